@@ -85,3 +85,25 @@ def test_sample_token_keeps_ids_on_the_device_and_validates(cabi):
         cabi.sample_tokens(torch.randn(2, 8))
     with pytest.raises(RuntimeError, match="top_k"):
         cabi.sample_tokens(x, top_k=-1, do_sample=True)
+
+
+@pytest.mark.parametrize("vocab,top_k,kind", [
+    (33, 50, "normal"), (1023, 7, "normal"), (1025, 1024, "normal"),       # fewer entries than threads; the cut at the thread count
+    (5000, 1025, "normal"),                                                # above it: radix select
+    (50257, 1000, "normal"), (32000, 50, "rounded"),                       # long runs of equal logits: more candidates than are kept
+    (4096, 40, "zeros"), (4096, 40, "masked"),                             # -0 and +0 at the cut; -inf entries
+])
+def test_draws_of_every_selection_path(cabi, vocab, top_k, kind):
+    g = torch.Generator().manual_seed(vocab + top_k)
+    x = 3.0 * torch.randn(48, vocab, generator=g)
+    if kind == "rounded":
+        x = x.round()
+    elif kind == "zeros":
+        x = torch.where(x > 0.5, 0.0, -0.0)
+    elif kind == "masked":
+        x[:, ::3] = float("-inf")
+    k = min(top_k, vocab)
+    got = cabi.sample_tokens(x.cuda(), 0.9, k, True, seed=77, step=vocab).cpu()
+    want = ko.sample_tokens(x, 0.9, k, True, seed=77, step=vocab)
+    # as above: exp differs in the last bit, a draw on a boundary may move to the neighbour
+    assert int((got != want).sum()) <= 1, (got, want)
