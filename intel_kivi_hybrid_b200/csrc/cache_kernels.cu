@@ -300,6 +300,9 @@ flush_values_fast_kernel(TokenSource src, uint8_t* __restrict__ v_codes, float* 
 // that token rows follow each other without a gap (tok_stride == 128), which
 // turns the 32 row offsets into immediates.
 // grid = (ceil(2*n_groups / 4), units), 4 warps per CTA.
+// Bound by issue slots before HBM with scalar arithmetic; with the two channels of
+// a lane in one fp32x2 operation, keys + values + window of 256 units x 8192 bf16
+// tokens went from 243 to 207 us (6.5 TB/s), fp32 from 401 to 385 us (6.3 TB/s).
 template <typename TF, bool HALF_EVEN, bool DENSE>
 __global__ void __launch_bounds__(128)
 flush_keys_direct_kernel(const TF* __restrict__ fresh, int64_t unit_stride, int64_t tok_stride_arg,
@@ -336,16 +339,15 @@ flush_keys_direct_kernel(const TF* __restrict__ fresh, int64_t unit_stride, int6
     if (r0 != 0.0f && r1 != 0.0f) {
 #pragma unroll
         for (int j = 0; j < Q; ++j) {
-            float m0[4], m1[4];
+            float2 m[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 float a, b;
                 P::widen(w[4 * j + e], a, b);
-                m0[e] = code_magic_rcp<HALF_EVEN>(a, mn0, s0, r0);
-                m1[e] = code_magic_rcp<HALF_EVEN>(b, mn1, s1, r1);
+                m[e] = code_magic_rcp2<HALF_EVEN>(make_float2(a, b), make_float2(-mn0, -mn1), make_float2(-s0, -s1), make_float2(r0, r1));
             }
             *reinterpret_cast<uint16_t*>(dst + j * 64) =
-                (uint16_t)(pack4_magic(m0[0], m0[1], m0[2], m0[3]) | (pack4_magic(m1[0], m1[1], m1[2], m1[3]) << 8));
+                (uint16_t)(pack4_magic(m[0].x, m[1].x, m[2].x, m[3].x) | (pack4_magic(m[0].y, m[1].y, m[2].y, m[3].y) << 8));
         }
     } else {
         // a scale too large for a reciprocal (rare): plain divisions, the values
@@ -423,8 +425,9 @@ flush_values_direct_kernel(const TF* __restrict__ fresh, int64_t unit_stride, in
         for (int r = 0; r < G / 4; ++r) {
             float x[4];
             row.quad(r, x);
-            sc[r * 16] = (uint8_t)pack4_magic(code_magic_rcp<HALF_EVEN>(x[0], mn, scale, rcp), code_magic_rcp<HALF_EVEN>(x[1], mn, scale, rcp),
-                                              code_magic_rcp<HALF_EVEN>(x[2], mn, scale, rcp), code_magic_rcp<HALF_EVEN>(x[3], mn, scale, rcp));
+            const float2 m01 = code_magic_rcp2<HALF_EVEN>(make_float2(x[0], x[1]), both(-mn), both(-scale), both(rcp));
+            const float2 m23 = code_magic_rcp2<HALF_EVEN>(make_float2(x[2], x[3]), both(-mn), both(-scale), both(rcp));
+            sc[r * 16] = (uint8_t)pack4_magic(m01.x, m01.y, m23.x, m23.y);
         }
     } else {
         // a scale too large for a reciprocal (rare): plain divisions on re-read values
@@ -451,26 +454,53 @@ flush_values_direct_kernel(const TF* __restrict__ fresh, int64_t unit_stride, in
         reinterpret_cast<float4*>(v_zeros + t_first * (D / G))[threadIdx.x - 96] = reinterpret_cast<const float4*>(s_zero)[threadIdx.x - 96];
 }
 
-// Copies virtual tokens [tau_from, tau_to) of the new tensor into their ring
-// slots (slot = (res_start + tau) % R); tokens already in the ring stay put.
+// Copies virtual tokens [tau_from, tau_from + n_tok) of the new tensor into their
+// ring slots (the first one `slot0`; n_tok is at most R); tokens already in the
+// ring stay put.  VEC consecutive elements per thread, one flat index over
+// (tensor, unit, token, piece): a single decode token of a large batch and the
+// window a prefill leaves behind both fill the machine.  VEC = 8: every pointer
+// and stride is a multiple of 16 bytes and D of 8; 12.6 MB of bf16 (256 units x
+// 96 tokens) took 25 us with one element per thread and 64-bit divisions.
+// Launched with programmatic stream serialization behind the flush kernels, which
+// read the ring: nothing is written before they have completed.
+template <typename TR, typename TF, int VEC>
 __global__ void __launch_bounds__(256)
-ring_append_kernel(TokenSource src, void* __restrict__ k_ring, void* __restrict__ v_ring,
-                   const void* __restrict__ fresh_v, int64_t unit_stride_v, int64_t tok_stride_v,
-                   int64_t tau_from, int64_t tau_to) {
-    const int D = src.D;
-    const int u = blockIdx.y;
-    const int64_t n = (tau_to - tau_from) * D;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t tau = tau_from + i / D;
-        const int d = (int)(i % D);
-        const int slot = (int)((src.res_start + tau) % src.R);
-        const int64_t o = ((int64_t)u * src.R + slot) * D + d;
-        const int64_t tn = tau - src.res_len;
-        float kv = load_as_float(src.fresh, src.fresh_dtype, (int64_t)u * src.unit_stride + tn * src.tok_stride + d);
-        float vv = load_as_float(fresh_v, src.fresh_dtype, (int64_t)u * unit_stride_v + tn * tok_stride_v + d);
-        store_from_float(k_ring, src.ring_dtype, o, kv);
-        store_from_float(v_ring, src.ring_dtype, o, vv);
+ring_append_kernel(const TF* __restrict__ new_k, const TF* __restrict__ new_v, TR* __restrict__ k_ring, TR* __restrict__ v_ring,
+                   int64_t unit_stride_k, int64_t tok_stride_k, int64_t unit_stride_v, int64_t tok_stride_v,
+                   int64_t first_tok, int n_tok, int slot0, int R, int D, uint32_t n_items) {   // n_items < 2^31
+    cudaGridDependencySynchronize();
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= n_items) return;
+    const uint32_t pieces = (uint32_t)(D / VEC);
+    const uint32_t row = i / pieces, d = (i - row * pieces) * VEC;          // row = (tensor, unit, token)
+    const uint32_t uu = row / (uint32_t)n_tok, t = row - uu * (uint32_t)n_tok;
+    const uint32_t units = n_items / (2u * pieces * (uint32_t)n_tok);
+    const bool is_v = uu >= units;
+    const int64_t u = is_v ? uu - units : uu;
+    int slot = slot0 + (int)t;
+    if (slot >= R) slot -= R;
+    const TF* src = (is_v ? new_v + u * unit_stride_v + (first_tok + t) * tok_stride_v : new_k + u * unit_stride_k + (first_tok + t) * tok_stride_k) + d;
+    TR* dst = (is_v ? v_ring : k_ring) + (u * R + slot) * (int64_t)D + d;
+    if constexpr (VEC == 8 && sizeof(TR) == sizeof(TF)) {
+#pragma unroll
+        for (int j = 0; j < (int)sizeof(TF) / 2; ++j) reinterpret_cast<uint4*>(dst)[j] = __ldg(reinterpret_cast<const uint4*>(src) + j);
+    } else if constexpr (VEC == 8) {
+        float v[8];
+        Load8<TF>::run(src, v);
+        if constexpr (sizeof(TR) == 4) {
+            reinterpret_cast<float4*>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
+            reinterpret_cast<float4*>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
+        } else {
+            uint32_t w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const __nv_bfloat162 p = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+                w[j] = *reinterpret_cast<const uint32_t*>(&p);
+            }
+            *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    } else {
+        store_from_float(dst, sizeof(TR) == 2 ? KIVI_BF16 : KIVI_F32, 0, load_as_float(src, sizeof(TF) == 2 ? KIVI_BF16 : KIVI_F32, 0));
     }
 }
 
@@ -636,6 +666,24 @@ import_keys_kernel(kivi_layer L, const uint8_t* __restrict__ packed, const float
     }
 }
 
+// Launch on `st`; with `overlap` as a programmatic dependent of the kernel before
+// it, whose last blocks it may then run beside.  Only for kernels that either do
+// not depend on that one or wait for it themselves (cudaGridDependencySynchronize).
+template <typename... P, typename... A>
+cudaError_t launch(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, bool overlap, A... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 }  // namespace
 
 int validate_layer(const kivi_layer* L) {
@@ -707,17 +755,20 @@ extern "C" int kivi_cache_update(const kivi_layer* L, int64_t quant_len, int res
                  (long long)ql_out, (long long)L->max_tokens);
     cudaStream_t st = (cudaStream_t)stream;
     int launches = 0;
+    auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+    const int esz = elem_size(new_dtype);
     TokenSource sk{L->k_res, new_k, L->res_dtype, new_dtype, R, D, res_start, res_len, unit_stride_k, tok_stride_k};
     TokenSource sv{L->v_res, new_v, L->res_dtype, new_dtype, R, D, res_start, res_len, unit_stride_v, tok_stride_v};
     const int64_t max_groups = L->max_tokens / G;
+    // The flush kernels of one call write disjoint arrays and read what was there
+    // before the call, so each may start while the one before it drains; the ring
+    // append, which overwrites slots they read, waits for them.
     if (f > 0) {
         const int64_t group0 = quant_len / G;
         KIVI_REQUIRE(f <= 0x7fffffff && L->num_units <= 65535, "grid too large");
         const int threads = D >= 256 ? 256 : (D >= 128 ? 128 : (D >= 64 ? 64 : 32));
         const size_t smem = (size_t)D * G / 4;
         const bool he = rounding == KIVI_ROUND_HALF_EVEN;
-        auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
-        const int esz = elem_size(new_dtype);
         const bool fast_k = D == 128 && G == 32 && al16(new_k) && al16(L->k_res) && al16(L->k_codes) &&
                             al16(L->k_scales) && al16(L->k_zeros) &&
                             (unit_stride_k * esz) % 16 == 0 && (tok_stride_k * esz) % 16 == 0;
@@ -730,8 +781,8 @@ extern "C" int kivi_cache_update(const kivi_layer* L, int64_t quant_len, int res
             if (fast_k) {
 #define KIVI_FK(TR, TF)                                                                                              \
                 do {                                                                                                 \
-                    if (he) flush_keys_fast_kernel<TR, TF, true><<<grid, 128, 0, st>>>(sk, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0); \
-                    else flush_keys_fast_kernel<TR, TF, false><<<grid, 128, 0, st>>>(sk, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0);   \
+                    if (he) KIVI_CUDA_OK(launch(flush_keys_fast_kernel<TR, TF, true>, grid, 128, 0, st, launches > 0, sk, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0)); \
+                    else KIVI_CUDA_OK(launch(flush_keys_fast_kernel<TR, TF, false>, grid, 128, 0, st, launches > 0, sk, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0));   \
                 } while (0)
                 if (L->res_dtype == KIVI_F32 && new_dtype == KIVI_F32) KIVI_FK(float, float);
                 else if (L->res_dtype == KIVI_F32) KIVI_FK(float, __nv_bfloat16);
@@ -739,13 +790,12 @@ extern "C" int kivi_cache_update(const kivi_layer* L, int64_t quant_len, int res
                 else KIVI_FK(__nv_bfloat16, __nv_bfloat16);
 #undef KIVI_FK
             } else if (G == 32) {
-                if (he) flush_keys_kernel<32, true><<<grid, threads, smem, st>>>(sk, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0, G);
-                else flush_keys_kernel<32, false><<<grid, threads, smem, st>>>(sk, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0, G);
+                if (he) KIVI_CUDA_OK(launch(flush_keys_kernel<32, true>, grid, threads, smem, st, launches > 0, sk, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0, G));
+                else KIVI_CUDA_OK(launch(flush_keys_kernel<32, false>, grid, threads, smem, st, launches > 0, sk, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0, G));
             } else {
-                if (he) flush_keys_kernel<0, true><<<grid, threads, smem, st>>>(sk, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0, G);
-                else flush_keys_kernel<0, false><<<grid, threads, smem, st>>>(sk, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0, G);
+                if (he) KIVI_CUDA_OK(launch(flush_keys_kernel<0, true>, grid, threads, smem, st, launches > 0, sk, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0, G));
+                else KIVI_CUDA_OK(launch(flush_keys_kernel<0, false>, grid, threads, smem, st, launches > 0, sk, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0, G));
             }
-            KIVI_LAUNCH_OK();
             launches += 1;
         }
         if (g_ring < f) {
@@ -756,16 +806,15 @@ extern "C" int kivi_cache_update(const kivi_layer* L, int64_t quant_len, int res
             do {                                                                                                     \
                 const TF* p = reinterpret_cast<const TF*>(new_k) + first * tok_stride_k;                             \
                 if (tok_stride_k == D) {                                                                             \
-                    if (he) flush_keys_direct_kernel<TF, true, true><<<grid, 128, 0, st>>>(p, unit_stride_k, tok_stride_k, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0 + g_ring, n_direct); \
-                    else flush_keys_direct_kernel<TF, false, true><<<grid, 128, 0, st>>>(p, unit_stride_k, tok_stride_k, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0 + g_ring, n_direct);   \
+                    if (he) KIVI_CUDA_OK(launch(flush_keys_direct_kernel<TF, true, true>, grid, 128, 0, st, launches > 0, p, unit_stride_k, tok_stride_k, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0 + g_ring, n_direct)); \
+                    else KIVI_CUDA_OK(launch(flush_keys_direct_kernel<TF, false, true>, grid, 128, 0, st, launches > 0, p, unit_stride_k, tok_stride_k, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0 + g_ring, n_direct));   \
                 } else {                                                                                             \
-                    if (he) flush_keys_direct_kernel<TF, true, false><<<grid, 128, 0, st>>>(p, unit_stride_k, tok_stride_k, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0 + g_ring, n_direct); \
-                    else flush_keys_direct_kernel<TF, false, false><<<grid, 128, 0, st>>>(p, unit_stride_k, tok_stride_k, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0 + g_ring, n_direct);   \
+                    if (he) KIVI_CUDA_OK(launch(flush_keys_direct_kernel<TF, true, false>, grid, 128, 0, st, launches > 0, p, unit_stride_k, tok_stride_k, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0 + g_ring, n_direct)); \
+                    else KIVI_CUDA_OK(launch(flush_keys_direct_kernel<TF, false, false>, grid, 128, 0, st, launches > 0, p, unit_stride_k, tok_stride_k, L->k_codes, L->k_scales, L->k_zeros, max_groups, group0 + g_ring, n_direct));   \
                 }                                                                                                    \
             } while (0)
             if (new_dtype == KIVI_F32) KIVI_DK(float); else KIVI_DK(__nv_bfloat16);
 #undef KIVI_DK
-            KIVI_LAUNCH_OK();
             launches += 1;
         }
         const int64_t n_tok = (int64_t)f * G;
@@ -779,8 +828,8 @@ extern "C" int kivi_cache_update(const kivi_layer* L, int64_t quant_len, int res
                 dim3 gridv((unsigned)((t_ring + 63) / 64), (unsigned)L->num_units);
 #define KIVI_FV(TR, TF)                                                                                              \
                 do {                                                                                                 \
-                    if (he) flush_values_fast_kernel<TR, TF, true><<<gridv, 256, 0, st>>>(sv, L->v_codes, L->v_scales, L->v_zeros, L->max_tokens, quant_len, t_ring); \
-                    else flush_values_fast_kernel<TR, TF, false><<<gridv, 256, 0, st>>>(sv, L->v_codes, L->v_scales, L->v_zeros, L->max_tokens, quant_len, t_ring);   \
+                    if (he) KIVI_CUDA_OK(launch(flush_values_fast_kernel<TR, TF, true>, gridv, 256, 0, st, launches > 0, sv, L->v_codes, L->v_scales, L->v_zeros, L->max_tokens, quant_len, t_ring)); \
+                    else KIVI_CUDA_OK(launch(flush_values_fast_kernel<TR, TF, false>, gridv, 256, 0, st, launches > 0, sv, L->v_codes, L->v_scales, L->v_zeros, L->max_tokens, quant_len, t_ring));   \
                 } while (0)
                 if (L->res_dtype == KIVI_F32 && new_dtype == KIVI_F32) KIVI_FV(float, float);
                 else if (L->res_dtype == KIVI_F32) KIVI_FV(float, __nv_bfloat16);
@@ -790,10 +839,9 @@ extern "C" int kivi_cache_update(const kivi_layer* L, int64_t quant_len, int res
             } else {
                 const int64_t items = n_tok * (D / G);
                 dim3 gridv((unsigned)((items + 255) / 256), (unsigned)L->num_units);
-                if (he) flush_values_kernel<true><<<gridv, 256, 0, st>>>(sv, L->v_codes, L->v_scales, L->v_zeros, L->max_tokens, quant_len, n_tok, G);
-                else flush_values_kernel<false><<<gridv, 256, 0, st>>>(sv, L->v_codes, L->v_scales, L->v_zeros, L->max_tokens, quant_len, n_tok, G);
+                if (he) KIVI_CUDA_OK(launch(flush_values_kernel<true>, gridv, 256, 0, st, launches > 0, sv, L->v_codes, L->v_scales, L->v_zeros, L->max_tokens, quant_len, n_tok, G));
+                else KIVI_CUDA_OK(launch(flush_values_kernel<false>, gridv, 256, 0, st, launches > 0, sv, L->v_codes, L->v_scales, L->v_zeros, L->max_tokens, quant_len, n_tok, G));
             }
-            KIVI_LAUNCH_OK();
             launches += 1;
         }
         if (t_ring < n_tok) {
@@ -804,13 +852,12 @@ extern "C" int kivi_cache_update(const kivi_layer* L, int64_t quant_len, int res
 #define KIVI_DV(TF)                                                                                                  \
             do {                                                                                                     \
                 const TF* p = reinterpret_cast<const TF*>(new_v) + (t_ring - res_len) * tok_stride_v;                \
-                if (he) flush_values_direct_kernel<TF, true, KIVI_STAGE(TF)><<<gridv, 128, 0, st>>>(p, unit_stride_v, tok_stride_v, L->v_codes, L->v_scales, L->v_zeros, L->max_tokens, quant_len + t_ring); \
-                else flush_values_direct_kernel<TF, false, KIVI_STAGE(TF)><<<gridv, 128, 0, st>>>(p, unit_stride_v, tok_stride_v, L->v_codes, L->v_scales, L->v_zeros, L->max_tokens, quant_len + t_ring);   \
+                if (he) KIVI_CUDA_OK(launch(flush_values_direct_kernel<TF, true, KIVI_STAGE(TF)>, gridv, 128, 0, st, launches > 0, p, unit_stride_v, tok_stride_v, L->v_codes, L->v_scales, L->v_zeros, L->max_tokens, quant_len + t_ring)); \
+                else KIVI_CUDA_OK(launch(flush_values_direct_kernel<TF, false, KIVI_STAGE(TF)>, gridv, 128, 0, st, launches > 0, p, unit_stride_v, tok_stride_v, L->v_codes, L->v_scales, L->v_zeros, L->max_tokens, quant_len + t_ring));   \
             } while (0)
             if (new_dtype == KIVI_F32) KIVI_DV(float); else KIVI_DV(__nv_bfloat16);
 #undef KIVI_DV
 #undef KIVI_STAGE
-            KIVI_LAUNCH_OK();
             launches += 1;
         }
     }
@@ -819,13 +866,34 @@ extern "C" int kivi_cache_update(const kivi_layer* L, int64_t quant_len, int res
     const int64_t total = (int64_t)res_len + n_new;
     const int64_t tau_from = (int64_t)f * G > res_len ? (int64_t)f * G : res_len;
     if (tau_from < total) {
-        const int64_t n = (total - tau_from) * D;
-        unsigned bx = (unsigned)((n + 255) / 256);
-        if (bx > 64) bx = 64;
-        dim3 grid(bx, (unsigned)L->num_units);
-        ring_append_kernel<<<grid, 256, 0, st>>>(sk, L->k_res, L->v_res, new_v, unit_stride_v, tok_stride_v, tau_from, total);
-        KIVI_LAUNCH_OK();
-        launches += 1;
+        const int n_tok = (int)(total - tau_from);            // at most R
+        const int64_t first = tau_from - res_len;             // index in the new tensor
+        const bool vec = D % 8 == 0 && al16(new_k) && al16(new_v) && al16(L->k_res) && al16(L->v_res) &&
+                         (unit_stride_k * esz) % 16 == 0 && (tok_stride_k * esz) % 16 == 0 &&
+                         (unit_stride_v * esz) % 16 == 0 && (tok_stride_v * esz) % 16 == 0;
+        const int pieces = D / (vec ? 8 : 1);
+        // the kernel's index has 31 bits: a window too large for one launch goes in runs of units and tokens
+        const int64_t most = (1ll << 31) - 1;
+        const int tok_step = (int)(most / (2 * pieces) < n_tok ? most / (2 * pieces) : n_tok);
+        const int64_t unit_room = most / (2ll * pieces * tok_step);
+        const int unit_step = (int)(unit_room < L->num_units ? unit_room : L->num_units);
+        auto go = [&](auto tr, auto tf, int u0, int nu, int t0, int nt) -> cudaError_t {
+            using TR = decltype(tr);
+            using TF = decltype(tf);
+            const int64_t items = 2ll * nu * nt * pieces, ring0 = (int64_t)u0 * R * D;
+            return launch(vec ? ring_append_kernel<TR, TF, 8> : ring_append_kernel<TR, TF, 1>, dim3((unsigned)((items + 255) / 256)), 256, 0, st, true,
+                          reinterpret_cast<const TF*>(new_k) + u0 * unit_stride_k, reinterpret_cast<const TF*>(new_v) + u0 * unit_stride_v,
+                          reinterpret_cast<TR*>(L->k_res) + ring0, reinterpret_cast<TR*>(L->v_res) + ring0, unit_stride_k, tok_stride_k,
+                          unit_stride_v, tok_stride_v, first + t0, nt, (int)((res_start + tau_from + t0) % R), R, D, (uint32_t)items);
+        };
+        const bool rf = L->res_dtype == KIVI_F32, nf = new_dtype == KIVI_F32;
+        for (int u0 = 0; u0 < L->num_units; u0 += unit_step)
+            for (int t0 = 0; t0 < n_tok; t0 += tok_step) {
+                const int nu = L->num_units - u0 < unit_step ? L->num_units - u0 : unit_step, nt = n_tok - t0 < tok_step ? n_tok - t0 : tok_step;
+                KIVI_CUDA_OK(rf ? (nf ? go(float{}, float{}, u0, nu, t0, nt) : go(float{}, __nv_bfloat16{}, u0, nu, t0, nt))
+                                : (nf ? go(__nv_bfloat16{}, float{}, u0, nu, t0, nt) : go(__nv_bfloat16{}, __nv_bfloat16{}, u0, nu, t0, nt)));
+                launches += 1;
+            }
     }
     if (quant_len_out) *quant_len_out = ql_out;
     if (res_start_out) *res_start_out = (int)((res_start + (int64_t)f * G) % R);

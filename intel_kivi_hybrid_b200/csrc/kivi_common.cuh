@@ -90,15 +90,41 @@ __device__ __forceinline__ float code_magic(float x, float mn, float scale, floa
     return __fadd_rd(__fadd_rd(t, 0.5f), 8388608.0f);
 }
 
-// code_magic for a group whose reciprocal exists (rcp != 0): no branch per element
+// ---- two fp32 operations per instruction ----------------------------------------
+// Each half is rounded exactly like the scalar operation.  The packed form has no
+// higher rate on the FMA pipe, but takes one issue slot instead of two, and issue
+// slots are what the quantize kernels run out of.  Never feed mul2 straight into
+// add2 where the two roundings must both happen: the compiler fuses that pair.
+#define KIVI_F32X2_BINARY(name, op)                                                                               \
+    __device__ __forceinline__ float2 name(float2 a, float2 b) {                                                  \
+        float2 d;                                                                                                 \
+        asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t" op " z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}" \
+            : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                                     \
+        return d;                                                                                                 \
+    }
+KIVI_F32X2_BINARY(add2, "add.rn.f32x2")
+KIVI_F32X2_BINARY(add2_rd, "add.rm.f32x2")
+KIVI_F32X2_BINARY(mul2, "mul.rn.f32x2")
+#undef KIVI_F32X2_BINARY
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+
+// code_magic of two elements of groups whose reciprocal exists (rcp != 0): no branch
+// per element.  The groups' numbers come negated where they are subtracted (min,
+// scale): x + (-min) and fma(-scale, q0, a) are the same operations.
 template <bool HALF_EVEN>
-__device__ __forceinline__ float code_magic_rcp(float x, float mn, float scale, float rcp) {
-    const float a = __fsub_rn(x, mn);
-    const float q0 = __fmul_rn(a, rcp);
-    const float e = __fmaf_rn(-scale, q0, a);
-    const float t = __fmaf_rn(e, rcp, q0);
-    if (HALF_EVEN) return __fadd_rn(t, 8388608.0f);
-    return __fadd_rd(__fadd_rd(t, 0.5f), 8388608.0f);
+__device__ __forceinline__ float2 code_magic_rcp2(float2 x, float2 neg_min, float2 neg_scale, float2 rcp) {
+    const float2 a = add2(x, neg_min);
+    const float2 q0 = mul2(a, rcp);
+    const float2 e = fma2(neg_scale, q0, a);
+    const float2 t = fma2(e, rcp, q0);
+    if (HALF_EVEN) return add2(t, both(8388608.0f));
+    return add2_rd(add2_rd(t, both(0.5f)), both(8388608.0f));
 }
 
 // the code as a float in {0, 1, 2, 3}

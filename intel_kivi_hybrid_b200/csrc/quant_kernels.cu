@@ -110,16 +110,16 @@ group_quant_kernel(const T* __restrict__ in, uint8_t* __restrict__ packed,
         // reciprocal (>= 1e30) take the plain-division twin of the same code
         auto emit = [&](auto has_rcp) {
             constexpr bool RCP = decltype(has_rcp)::value;
-            auto magic = [&](float x) {
-                if constexpr (RCP) return code_magic_rcp<HALF_EVEN>(x, mn, scale, rcp);
-                else return code_magic<HALF_EVEN>(x, mn, scale, rcp);
+            auto magic2 = [&](float x, float y) {
+                if constexpr (RCP) return code_magic_rcp2<HALF_EVEN>(make_float2(x, y), both(-mn), both(-scale), both(rcp));
+                else return make_float2(code_magic<HALF_EVEN>(x, mn, scale, rcp), code_magic<HALF_EVEN>(y, mn, scale, rcp));
             };
             if (MODE == 0) {
                 uint32_t bytes[(BPL + 3) / 4] = {};
 #pragma unroll
                 for (int b = 0; b < BPL; ++b) {
-                    const uint32_t byte = pack4_magic(magic(v[it][4 * b + 0]), magic(v[it][4 * b + 1]),
-                                                      magic(v[it][4 * b + 2]), magic(v[it][4 * b + 3]));
+                    const float2 m01 = magic2(v[it][4 * b + 0], v[it][4 * b + 1]), m23 = magic2(v[it][4 * b + 2], v[it][4 * b + 3]);
+                    const uint32_t byte = pack4_magic(m01.x, m01.y, m23.x, m23.y);
                     bytes[b / 4] |= byte << (8 * (b % 4));
                 }
                 uint8_t* dst = s_codes + lg[it] * (G / 4) + sub * BPL;
@@ -134,12 +134,9 @@ group_quant_kernel(const T* __restrict__ in, uint8_t* __restrict__ packed,
                 float* o = rt_out + g * G + sub * EPL;
 #pragma unroll
                 for (int k = 0; k < EPL / 4; ++k) {
-                    float4 r;
-                    r.x = dequant(__fsub_rn(magic(v[it][4 * k + 0]), 8388608.0f), scale, mn);
-                    r.y = dequant(__fsub_rn(magic(v[it][4 * k + 1]), 8388608.0f), scale, mn);
-                    r.z = dequant(__fsub_rn(magic(v[it][4 * k + 2]), 8388608.0f), scale, mn);
-                    r.w = dequant(__fsub_rn(magic(v[it][4 * k + 3]), 8388608.0f), scale, mn);
-                    reinterpret_cast<float4*>(o)[k] = r;
+                    const float2 m01 = magic2(v[it][4 * k + 0], v[it][4 * k + 1]), m23 = magic2(v[it][4 * k + 2], v[it][4 * k + 3]);
+                    const float2 a = add2(m01, both(-8388608.0f)), b = add2(m23, both(-8388608.0f));
+                    reinterpret_cast<float4*>(o)[k] = make_float4(dequant(a.x, scale, mn), dequant(a.y, scale, mn), dequant(b.x, scale, mn), dequant(b.y, scale, mn));
                 }
             }
         };
@@ -243,9 +240,9 @@ group_quant_bf16_rows_kernel(const __nv_bfloat16* __restrict__ in, uint8_t* __re
             for (int r = 0; r < 8; ++r) {
                 float x[4];
                 row[k].quad(r, x);
-                w[2 * k + (r >> 2)] |= pack4_magic(code_magic_rcp<HALF_EVEN>(x[0], mn, scale, rcp), code_magic_rcp<HALF_EVEN>(x[1], mn, scale, rcp),
-                                                   code_magic_rcp<HALF_EVEN>(x[2], mn, scale, rcp), code_magic_rcp<HALF_EVEN>(x[3], mn, scale, rcp))
-                                       << (8 * (r & 3));
+                const float2 m01 = code_magic_rcp2<HALF_EVEN>(make_float2(x[0], x[1]), both(-mn), both(-scale), both(rcp));
+                const float2 m23 = code_magic_rcp2<HALF_EVEN>(make_float2(x[2], x[3]), both(-mn), both(-scale), both(rcp));
+                w[2 * k + (r >> 2)] |= pack4_magic(m01.x, m01.y, m23.x, m23.y) << (8 * (r & 3));
             }
         if (NR == 1) {
             *reinterpret_cast<uint2*>(packed + g * 8) = make_uint2(w[0], w[1]);

@@ -553,3 +553,27 @@ def test_tensor_core_keeps_enough_bits_for_subnormal_codes(cabi):
     bits = cabi.mma_alignment_bits()
     print(f"[tensor core] 1 + 2^-k - 1 is exact up to k = {bits}")
     assert bits >= 24
+
+
+@pytest.mark.parametrize("D,G,R,ring,new,shift,strided", [
+    (128, 32, 128, torch.bfloat16, torch.bfloat16, 0, False), (64, 16, 96, torch.float32, torch.float32, 0, True),
+    (128, 32, 64, torch.float32, torch.bfloat16, 0, True), (64, 32, 128, torch.bfloat16, torch.float32, 0, False),
+    (12, 4, 8, torch.float32, torch.float32, 0, False),                     # head_dim not a multiple of eight
+    (128, 32, 128, torch.bfloat16, torch.bfloat16, 1, False),               # new tensor off the 16-byte grid
+])
+def test_ring_append_keeps_the_window(cabi, D, G, R, ring, new, shift, strided):
+    """The window after chunks of every length (single tokens, wrap-around, bulk) is
+    the last res_len tokens, bit for bit (fp32 to a bf16 ring: rounded to nearest)."""
+    U, g = 3, torch.Generator(device="cuda").manual_seed(D + R)
+    T = 6 * R
+    st = cabi.LayerStore(U, D, G, R, T, ring, "cuda")
+    wide = D + 8 if strided else D
+    flat = [torch.randn(U * T * wide + shift, generator=g, device="cuda").to(new)[shift:].view(U, T, wide)[..., :D] for _ in range(2)]
+    t = 0
+    for n in (1, 2, R // 2 + 1, 1, R - 1, 3, 1, R + G + 1, 1):
+        st.update(flat[0][:, t:t + n], flat[1][:, t:t + n])
+        t += n
+        assert st.quant_len + st.res_len == t
+        idx = (torch.arange(st.res_len, device="cuda") + st.res_start) % R
+        for x, buf in ((flat[0], st.k_res), (flat[1], st.v_res)):
+            assert torch.equal(buf[:, idx], x[:, t - st.res_len:t].to(ring)), (n, t)
