@@ -18,7 +18,10 @@
 // Per 32-token chunk a warp does: lane = token for the q.k scores (each lane
 // walks the D channels of its token), a warp max, exp2, then lane = 4 channels
 // for p.V (each lane walks the chunk's tokens).
+#include "async_copy.cuh"
 #include "kivi_common.cuh"
+
+#include <atomic>
 
 namespace kivi {
 
@@ -233,6 +236,409 @@ attn_fp32_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
             if (mw != -INFINITY) ls += ml_s[(w * NREP + h) * 2 + 1] * exp2f(mw - M[h]);
         }
         part_ml[(pbase + h) * 2] = M[h];
+        part_ml[(pbase + h) * 2 + 1] = ls;
+    }
+}
+
+// ---- fp32 kernel for head_dim 64 and 128 -----------------------------------------
+// Same arithmetic (k = code*scale + zero in one fp32 rounding, fp32 FMAs for both
+// contractions), organised so that the FMA pipe is what bounds it:
+//   * every warp streams its own token groups into a private two-stage ring in shared
+//     memory with bulk copies (the six arrays of a group are contiguous runs);
+//   * q.k: a lane takes four tokens x D/4 channels, exactly what its 32-bit code
+//     words hold (4 tokens x 4 channels), so a code is read once, a dequantized
+//     key serves all heads, and a query or scale read serves four tokens; the lanes
+//     of a token quad then exchange partial sums and lane l ends with token l;
+//   * p.v: a lane takes four channels, a word is again 4 tokens x 4 channels;
+//   * a code becomes a float with one byte permute (2^23 + c) and half a packed
+//     subtract; dequantization and both contractions are packed two to an instruction
+//     (same rate on the FMA pipe, half the issue slots);
+//   * a running maximum is only worked out when a score exceeds it.
+// What bounds it: the FMA pipe.  A lane's 256 codes of a group cost one FMA per code and
+// head (512 cycles of the SM quarter per head, two per packed instruction) and about
+// 1500 cycles of conversion; measured 2150 / 4100 / 6700 cycles per group with 1 / 4 / 8
+// heads, against 13000 with four heads in the generic kernel (dependent 32-bit loads,
+// an integer conversion per code).  32 units x 8k tokens, 4 heads: 99 -> 36 us;
+// 32 x 32k, 1 head: 259 -> 65 us; 12 units x 712 tokens, head_dim 64: 18.4 -> 6.4 us.
+// Error against 64 bits is about half of the generic kernel's (shorter chains of adds).
+template <int D> struct Fp32Tile {
+    static constexpr int kBytes = D / 4;               // packed value bytes of a token
+    static constexpr int kTokPar = 32 / kBytes;        // token quads a warp takes side by side in p.v (2 for D = 64)
+};
+
+// score of one token per lane and head -> weight; running maximum, sum and outputs of the warp
+template <int NREP, int NO>
+__device__ __forceinline__ void absorb(float (&s)[NREP], bool valid, float* __restrict__ p_slot, float (&m)[NREP], float (&l)[NREP], float2 (&o)[NREP][NO]) {
+    bool above = false;
+#pragma unroll
+    for (int h = 0; h < NREP; ++h) {
+        s[h] = valid ? s[h] : -INFINITY;
+        above |= s[h] > m[h];
+    }
+    if (__any_sync(0xffffffffu, above)) {
+#pragma unroll
+        for (int h = 0; h < NREP; ++h) {
+            float mx = s[h];
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+            const float m_new = fmaxf(m[h], mx);
+            const float alpha = m_new == -INFINITY ? 1.0f : exp2f(m[h] - m_new);       // 0 on the first chunk
+            m[h] = m_new;
+            l[h] *= alpha;
+#pragma unroll
+            for (int i = 0; i < NO; ++i) o[h][i] = mul2(o[h][i], both(alpha));
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < NREP; ++h) {
+        const float p = valid ? exp2f(s[h] - m[h]) : 0.0f;
+        l[h] += p;
+        p_slot[h] = p;
+    }
+}
+
+template <int NREP> __device__ __forceinline__ void load_weights(const float* __restrict__ p, float (&w)[NREP]) {
+    if constexpr (NREP % 4 == 0) {
+#pragma unroll
+        for (int h = 0; h < NREP; h += 4) {
+            const float4 t = *reinterpret_cast<const float4*>(p + h);
+            w[h] = t.x; w[h + 1] = t.y; w[h + 2] = t.z; w[h + 3] = t.w;
+        }
+    } else if constexpr (NREP % 2 == 0) {
+#pragma unroll
+        for (int h = 0; h < NREP; h += 2) {
+            const float2 t = *reinterpret_cast<const float2*>(p + h);
+            w[h] = t.x; w[h + 1] = t.y;
+        }
+    } else {
+#pragma unroll
+        for (int h = 0; h < NREP; ++h) w[h] = p[h];
+    }
+}
+
+// the four 2-bit fields at bits 0-1 of the bytes of t, as floats
+__device__ __forceinline__ void codes_to_float(uint32_t t, float2& a, float2& b) {
+    const float2 x = make_float2(__uint_as_float(__byte_perm(t, 0x4B000000u, 0x7440)), __uint_as_float(__byte_perm(t, 0x4B000000u, 0x7441)));
+    const float2 y = make_float2(__uint_as_float(__byte_perm(t, 0x4B000000u, 0x7442)), __uint_as_float(__byte_perm(t, 0x4B000000u, 0x7443)));
+    a = add2(x, both(-8388608.0f));
+    b = add2(y, both(-8388608.0f));
+}
+
+template <typename T> __device__ __forceinline__ void load4(const T* p, float (&v)[4]);
+template <> __device__ __forceinline__ void load4<float>(const float* p, float (&v)[4]) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p));
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+template <> __device__ __forceinline__ void load4<__nv_bfloat16>(const __nv_bfloat16* p, float (&v)[4]) {
+    const uint2 t = __ldg(reinterpret_cast<const uint2*>(p));
+    v[0] = __uint_as_float(t.x << 16); v[1] = __uint_as_float(t.x & 0xffff0000u);
+    v[2] = __uint_as_float(t.y << 16); v[3] = __uint_as_float(t.y & 0xffff0000u);
+}
+
+// window tokens of one warp (every kWarps-th run of 32): lane (tl, cq) scores tokens
+// tl + 8j, j = 0..3, over channels cq*D/4 .. ; lane = token tl + 8*cq afterwards
+template <int NREP, int D, typename T>
+__device__ __forceinline__ void ring_tokens(const T* __restrict__ k_res, const T* __restrict__ v_res, int R, int res_start, int res_len,
+                                            const float* __restrict__ q_s, float scale_log2, float* __restrict__ p_s, int lane, int warp,
+                                            float (&m)[NREP], float (&l)[NREP], float2 (&o)[NREP][2]) {
+    constexpr int kTokPar = Fp32Tile<D>::kTokPar, kBytes = Fp32Tile<D>::kBytes;
+    const int tl = lane >> 2, cq = lane & 3;
+    for (int t0 = 32 * warp; t0 < res_len; t0 += 32 * kWarps) {
+        const int ntok = res_len - t0 < 32 ? res_len - t0 : 32;
+        float2 acc[4][NREP];
+        const T* row[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            int slot = res_start + t0 + (tl + 8 * j < ntok ? tl + 8 * j : 0);
+            if (slot >= R) slot -= R;
+            row[j] = k_res + (int64_t)slot * D + cq * (D / 4);
+#pragma unroll
+            for (int h = 0; h < NREP; ++h) acc[j][h] = make_float2(0.0f, 0.0f);
+        }
+#pragma unroll 2
+        for (int c = 0; c < D / 4; c += 4) {
+            float kv[4][4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) load4<T>(row[j] + c, kv[j]);
+#pragma unroll
+            for (int h = 0; h < NREP; ++h) {
+                const float4 q4 = *reinterpret_cast<const float4*>(q_s + h * D + cq * (D / 4) + c);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    acc[j][h] = fma2(make_float2(q4.x, q4.y), make_float2(kv[j][0], kv[j][1]), acc[j][h]);
+                    acc[j][h] = fma2(make_float2(q4.z, q4.w), make_float2(kv[j][2], kv[j][3]), acc[j][h]);
+                }
+            }
+        }
+        float s[NREP];
+#pragma unroll
+        for (int h = 0; h < NREP; ++h) {
+            float a[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                a[j] = acc[j][h].x + acc[j][h].y;
+                a[j] += __shfl_xor_sync(0xffffffffu, a[j], 1);
+                a[j] += __shfl_xor_sync(0xffffffffu, a[j], 2);
+            }
+            s[h] = (cq == 0 ? a[0] : cq == 1 ? a[1] : cq == 2 ? a[2] : a[3]) * scale_log2;
+        }
+        __syncwarp();
+        absorb<NREP, 2>(s, tl + 8 * cq < ntok, p_s + (tl + 8 * cq) * NREP, m, l, o);
+        __syncwarp();
+        const int b = lane % kBytes, tp = lane / kBytes;
+        for (int k0 = 0; k0 < ntok; k0 += 8 * kTokPar) {
+            float vv[8][4];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int tk = k0 + k * kTokPar + tp;
+                int slot = res_start + t0 + (tk < ntok ? tk : 0);
+                if (slot >= R) slot -= R;
+                load4<T>(v_res + (int64_t)slot * D + 4 * b, vv[k]);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int tk = k0 + k * kTokPar + tp;
+                float w[NREP];
+                load_weights<NREP>(p_s + (tk < ntok ? tk : 0) * NREP, w);
+#pragma unroll
+                for (int h = 0; h < NREP; ++h) {
+                    const float2 pp = both(tk < ntok ? w[h] : 0.0f);
+                    o[h][0] = fma2(pp, make_float2(vv[k][0], vv[k][1]), o[h][0]);
+                    o[h][1] = fma2(pp, make_float2(vv[k][2], vv[k][3]), o[h][1]);
+                }
+            }
+        }
+    }
+}
+
+__device__ int g_fp32_copy_fault = 0;
+
+// Shared memory: warps' stage rings [kWarps][2][stage_bytes] (a warp's ring doubles as
+// its [NREP][D] output buffer) | queries [NREP][D] | weights [kWarps][32][NREP] |
+// mbarriers [kWarps][2] | (max, sum) [kWarps][NREP][2]
+template <int NREP, int D>
+__global__ void __launch_bounds__(kWarps * 32, NREP <= 2 ? 4 : NREP <= 6 ? 3 : 2)
+attn_fp32_tile_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
+                      const void* __restrict__ q, int q_dtype, float scale_log2,
+                      int nq_splits, int groups_per_split, int n_splits, int stage_bytes,
+                      float* __restrict__ part_o, float* __restrict__ part_ml) {
+    constexpr int kBytes = Fp32Tile<D>::kBytes, kTokPar = Fp32Tile<D>::kTokPar;
+    const int G = L.group_size, ng = D / G;
+    const int u = blockIdx.y, split = blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    uint8_t* ring = smem_raw + warp * 2 * stage_bytes;
+    float* q_s = reinterpret_cast<float*>(smem_raw + kWarps * 2 * stage_bytes);
+    float* p_s = q_s + NREP * D + warp * 32 * NREP;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(q_s + NREP * D + kWarps * 32 * NREP);
+    float* ml_s = reinterpret_cast<float*>(bars + kWarps * 2);
+    cudaTriggerProgrammaticLaunchCompletion();            // the fold may become resident now, it waits for this grid's end
+
+    const bool is_ring = split >= nq_splits;
+    const int64_t g_begin = is_ring ? 0 : (int64_t)split * groups_per_split;
+    int64_t g_end = is_ring ? 0 : g_begin + groups_per_split;
+    if (g_end > quant_len / G) g_end = quant_len / G;
+    const int n_my = (int)(g_end - g_begin) > warp ? ((int)(g_end - g_begin) - warp + kWarps - 1) / kWarps : 0;
+    // the six pieces of a group: key codes, scales, zeros, value codes, scales, zeros
+    const uint32_t code_bytes = (uint32_t)(D * G / 4), meta_bytes = D * 4;
+    const uint32_t bar0 = smem_u32(bars + warp * 2), ring0 = smem_u32(ring);
+    const uint64_t policy = l2_stream_policy();
+    const uint8_t* my_src = nullptr;
+    uint32_t my_bytes = 0, my_dst = 0;
+    auto issue = [&](int i) {                             // the warp's i-th group
+        const uint32_t bar = bar0 + 8 * (i & 1);
+        if (lane == 0) mbar_expect_tx(bar, 2 * code_bytes + 4 * meta_bytes);
+        __syncwarp();
+        if (lane < 6) bulk_g2s(ring0 + (i & 1) * stage_bytes + my_dst, my_src + (int64_t)i * kWarps * my_bytes, my_bytes, bar, policy);
+    };
+    if (n_my > 0) {
+        const uint8_t* base = lane == 0 ? L.k_codes
+                            : lane == 1 ? reinterpret_cast<const uint8_t*>(L.k_scales)
+                            : lane == 2 ? reinterpret_cast<const uint8_t*>(L.k_zeros)
+                            : lane == 3 ? L.v_codes
+                            : lane == 4 ? reinterpret_cast<const uint8_t*>(L.v_scales)
+                                        : reinterpret_cast<const uint8_t*>(L.v_zeros);
+        my_bytes = (lane == 0 || lane == 3) ? code_bytes : meta_bytes;
+        my_dst = lane <= 3 ? (lane == 0 ? 0u : code_bytes + (lane - 1) * meta_bytes) : 2 * code_bytes + (lane - 2) * meta_bytes;
+        my_src = base + ((int64_t)u * (L.max_tokens / G) + g_begin + warp) * my_bytes;
+        if (lane == 0) { mbar_init(bar0, 1); mbar_init(bar0 + 8, 1); mbar_init_fence(); }
+        __syncwarp();
+        issue(0);
+        if (n_my > 1) issue(1);
+    }
+    for (int i = threadIdx.x; i < NREP * D; i += blockDim.x)
+        q_s[i] = load_as_float(q, q_dtype, (int64_t)u * NREP * D + i);
+    __syncthreads();
+
+    float m[NREP], l[NREP];
+    float2 o[NREP][2];
+#pragma unroll
+    for (int h = 0; h < NREP; ++h) { m[h] = -INFINITY; l[h] = 0.0f; o[h][0] = make_float2(0.0f, 0.0f); o[h][1] = o[h][0]; }
+
+    if (is_ring) {
+        const int64_t r0 = (int64_t)u * L.residual_cap * D;
+        if (L.res_dtype == KIVI_BF16)
+            ring_tokens<NREP, D, __nv_bfloat16>(reinterpret_cast<const __nv_bfloat16*>(L.k_res) + r0, reinterpret_cast<const __nv_bfloat16*>(L.v_res) + r0,
+                                                L.residual_cap, res_start, res_len, q_s, scale_log2, p_s, lane, warp, m, l, o);
+        else
+            ring_tokens<NREP, D, float>(reinterpret_cast<const float*>(L.k_res) + r0, reinterpret_cast<const float*>(L.v_res) + r0,
+                                        L.residual_cap, res_start, res_len, q_s, scale_log2, p_s, lane, warp, m, l, o);
+    } else {
+        const int j = lane >> 2, cq = lane & 3;           // q.k: token quad, channels 16*i + 4*cq
+        const int b = lane % kBytes, tp = lane / kBytes;  // p.v: packed byte (four channels), token quads tp, tp + kTokPar, ...
+        const int gd = 4 * b / G;
+        const bool blocks = value_blocks(D, G);
+        int i = 0;
+        for (; i < n_my; ++i) {
+            if (!mbar_wait(bar0 + 8 * (i & 1), (uint32_t)(i >> 1) & 1u)) break;
+            __syncwarp();
+            const uint8_t* kc = ring + (i & 1) * stage_bytes;
+            const float* ks = reinterpret_cast<const float*>(kc + code_bytes);
+            const float* kz = ks + D;
+            const uint8_t* vc = kc + code_bytes + 2 * meta_bytes;
+            const float* vs = reinterpret_cast<const float*>(vc + code_bytes);
+            const float* vz = vs + D;
+            for (int c0 = 0; c0 < G; c0 += 32) {          // 32 tokens at a time (fewer when G has no 32)
+                const int nt = G - c0 < 32 ? G - c0 : 32;
+                float2 acc[4][NREP];
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+#pragma unroll
+                    for (int h = 0; h < NREP; ++h) acc[e][h] = make_float2(0.0f, 0.0f);
+                const uint8_t* krow = kc + (c0 / 4 + (4 * j < nt ? j : 0)) * 64 + cq * 16;
+#pragma unroll
+                for (int hh = 0; hh < D / 64; ++hh) {
+                    const uint4 wv = *reinterpret_cast<const uint4*>(krow + hh * 16 * G);
+                    const uint32_t w4[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+                    for (int mm = 0; mm < 4; ++mm) {
+                        const int ch = 64 * hh + 16 * mm + 4 * cq;
+                        const float4 s4 = *reinterpret_cast<const float4*>(ks + ch), z4 = *reinterpret_cast<const float4*>(kz + ch);
+                        float2 k01[4], k23[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            codes_to_float((w4[mm] >> (2 * e)) & 0x03030303u, k01[e], k23[e]);
+                            k01[e] = fma2(k01[e], make_float2(s4.x, s4.y), make_float2(z4.x, z4.y));
+                            k23[e] = fma2(k23[e], make_float2(s4.z, s4.w), make_float2(z4.z, z4.w));
+                        }
+#pragma unroll
+                        for (int h = 0; h < NREP; ++h) {
+                            const float4 q4 = *reinterpret_cast<const float4*>(q_s + h * D + ch);
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                acc[e][h] = fma2(make_float2(q4.x, q4.y), k01[e], acc[e][h]);
+                                acc[e][h] = fma2(make_float2(q4.z, q4.w), k23[e], acc[e][h]);
+                            }
+                        }
+                    }
+                }
+                // sums over the four lanes of a quad; lane 4j + cq keeps token 4j + cq
+                float s[NREP];
+#pragma unroll
+                for (int h = 0; h < NREP; ++h) {
+                    float a[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) a[e] = acc[e][h].x + acc[e][h].y;
+                    const bool hi = (cq & 2) != 0, odd = (cq & 1) != 0;
+                    const float x0 = (hi ? a[2] : a[0]) + __shfl_xor_sync(0xffffffffu, hi ? a[0] : a[2], 2);
+                    const float x1 = (hi ? a[3] : a[1]) + __shfl_xor_sync(0xffffffffu, hi ? a[1] : a[3], 2);
+                    s[h] = ((odd ? x1 : x0) + __shfl_xor_sync(0xffffffffu, odd ? x0 : x1, 1)) * scale_log2;
+                }
+                __syncwarp();                             // the weights of the chunk before have been read
+                absorb<NREP, 2>(s, lane < nt, p_s + lane * NREP, m, l, o);
+                __syncwarp();
+                for (int qd = tp; 4 * qd < nt; qd += kTokPar) {
+                    const int t = c0 + 4 * qd;            // tokens t .. t+3 of the group
+                    uint32_t w;
+                    int row, row_step;                    // scale / zero index of token t + n: row + n * row_step
+                    if (blocks) {                         // word (gd, kappa, r, c): four tokens of one byte (kivi_common.cuh)
+                        w = *reinterpret_cast<const uint32_t*>(vc + ((b >> 3) * 64 + (qd >> 2) * 32 + (b & 7) * 4 + (qd & 3)) * 4);
+                        row = (16 * (qd >> 2) + (qd & 3)) * 4 + gd; row_step = 16;
+                    } else {                              // one row per token
+                        const uint8_t* r0 = vc + t * kBytes + b;
+                        w = (uint32_t)r0[0] | ((uint32_t)r0[kBytes] << 8) | ((uint32_t)r0[2 * kBytes] << 16) | ((uint32_t)r0[3 * kBytes] << 24);
+                        row = t * ng + gd; row_step = ng;
+                    }
+                    // v[i]: channel 4b + i of tokens (0, 1) and (2, 3)
+                    float2 c01[4], c23[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) codes_to_float((w >> (2 * e)) & 0x03030303u, c01[e], c23[e]);
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) {
+                        const float sc = vs[row + n * row_step], zc = vz[row + n * row_step];
+                        const float2 a = n < 2 ? (n == 0 ? make_float2(c01[0].x, c01[1].x) : make_float2(c01[0].y, c01[1].y))
+                                               : (n == 2 ? make_float2(c23[0].x, c23[1].x) : make_float2(c23[0].y, c23[1].y));
+                        const float2 c = n < 2 ? (n == 0 ? make_float2(c01[2].x, c01[3].x) : make_float2(c01[2].y, c01[3].y))
+                                               : (n == 2 ? make_float2(c23[2].x, c23[3].x) : make_float2(c23[2].y, c23[3].y));
+                        const float2 v01 = fma2(a, both(sc), both(zc)), v23 = fma2(c, both(sc), both(zc));
+                        float wt[NREP];
+                        load_weights<NREP>(p_s + (4 * qd + n) * NREP, wt);
+#pragma unroll
+                        for (int h = 0; h < NREP; ++h) {
+                            o[h][0] = fma2(both(wt[h]), v01, o[h][0]);
+                            o[h][1] = fma2(both(wt[h]), v23, o[h][1]);
+                        }
+                    }
+                }
+            }
+            __syncwarp();
+            if (i + 2 < n_my) issue(i + 2);
+        }
+        if (i < n_my) {
+            // A copy did not land within the bound: the ones still under way get a second
+            // bounded wait before the ring is reused, then the warp reports nothing.
+            if (lane == 0) atomicExch(&g_fp32_copy_fault, 1);
+            for (int k = i; k < i + 2 && k < n_my; ++k) mbar_wait(bar0 + 8 * (k & 1), (uint32_t)(k >> 1) & 1u);
+#pragma unroll
+            for (int h = 0; h < NREP; ++h) { m[h] = -INFINITY; l[h] = 0.0f; o[h][0] = make_float2(0.0f, 0.0f); o[h][1] = o[h][0]; }
+        }
+    }
+
+    // ---- fold the warps ---------------------------------------------------------------
+#pragma unroll
+    for (int h = 0; h < NREP; ++h) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) l[h] += __shfl_xor_sync(0xffffffffu, l[h], off);
+        if (lane == 0) { ml_s[(warp * NREP + h) * 2] = m[h]; ml_s[(warp * NREP + h) * 2 + 1] = l[h]; }
+        if constexpr (kTokPar == 2) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                o[h][i].x += __shfl_xor_sync(0xffffffffu, o[h][i].x, 16);
+                o[h][i].y += __shfl_xor_sync(0xffffffffu, o[h][i].y, 16);
+            }
+        }
+    }
+    __syncthreads();
+    float* mine = reinterpret_cast<float*>(ring);
+#pragma unroll
+    for (int h = 0; h < NREP; ++h) {
+        float M = -INFINITY;
+#pragma unroll
+        for (int w2 = 0; w2 < kWarps; ++w2) M = fmaxf(M, ml_s[(w2 * NREP + h) * 2]);
+        const float f = m[h] == -INFINITY ? 0.0f : exp2f(m[h] - M);
+        if (lane < kBytes)
+            *reinterpret_cast<float4*>(mine + h * D + 4 * lane) = make_float4(f * o[h][0].x, f * o[h][0].y, f * o[h][1].x, f * o[h][1].y);
+    }
+    __syncthreads();
+    const int64_t pbase = ((int64_t)u * n_splits + split) * NREP;
+    for (int i = threadIdx.x * 4; i < NREP * D; i += blockDim.x * 4) {
+        float4 a = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(smem_raw) + i);
+#pragma unroll
+        for (int w2 = 1; w2 < kWarps; ++w2) {
+            const float4 c = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(smem_raw + w2 * 2 * stage_bytes) + i);
+            a.x += c.x; a.y += c.y; a.z += c.z; a.w += c.w;
+        }
+        *reinterpret_cast<float4*>(part_o + pbase * D + i) = a;
+    }
+    if (threadIdx.x < NREP) {
+        const int h = threadIdx.x;
+        float M = -INFINITY, ls = 0.0f;
+        for (int w2 = 0; w2 < kWarps; ++w2) M = fmaxf(M, ml_s[(w2 * NREP + h) * 2]);
+        for (int w2 = 0; w2 < kWarps; ++w2) {
+            const float mw = ml_s[(w2 * NREP + h) * 2];
+            if (mw != -INFINITY) ls += ml_s[(w2 * NREP + h) * 2 + 1] * exp2f(mw - M);
+        }
+        part_ml[(pbase + h) * 2] = M;
         part_ml[(pbase + h) * 2 + 1] = ls;
     }
 }
@@ -522,6 +928,17 @@ merge_gather_kernel(const float* __restrict__ part_o, const float* __restrict__ 
 
 }  // namespace
 
+int fp32_fault_word(int* out) {
+    KIVI_CUDA_OK(cudaMemcpyFromSymbol(out, g_fp32_copy_fault, sizeof(int)));
+    return KIVI_OK;
+}
+
+int fp32_fault_clear() {
+    const int zero = 0;
+    KIVI_CUDA_OK(cudaMemcpyToSymbol(g_fp32_copy_fault, &zero, sizeof(int)));
+    return KIVI_OK;
+}
+
 int gather_fault_word(int* out) {
     KIVI_CUDA_OK(cudaMemcpyFromSymbol(out, g_gather_fault, sizeof(int)));
     return KIVI_OK;
@@ -594,23 +1011,52 @@ int run_merge_token_shards(const float* parts, int n_shards, int64_t rows, int D
     return KIVI_OK;
 }
 
+// The tile kernel takes head_dim 64 and 128 with 16-byte aligned arrays and groups of
+// whole 16-byte pieces (any group size: D*G/4 bytes of codes are a multiple of 16);
+// everything else -- other head_dims, odd alignments -- takes the generic kernel.
+static bool tile_kernel_ok(const kivi_layer* L) {
+    auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+    return (L->head_dim == 64 || L->head_dim == 128) && al(L->k_res) && al(L->v_res) && al(L->k_codes) && al(L->k_scales) &&
+           al(L->k_zeros) && al(L->v_codes) && al(L->v_scales) && al(L->v_zeros);
+}
+
+template <int NREP, int D>
+static int launch_tile(const kivi_layer* L, int64_t quant_len, int res_start, int res_len, const void* q, int q_dtype, float scale_log2,
+                       int nq_splits, int gps, int n_splits, float* part_o, float* part_ml, cudaStream_t st) {
+    static std::atomic<int> smem_set[64];
+    // two stages of one group per warp, and never less than the warp's [NREP][D] output buffer
+    int stage = 2 * (D * L->group_size / 4) + 4 * D * 4;
+    if (stage < NREP * D * 2) stage = NREP * D * 2;
+    const int smem = kWarps * 2 * stage + 4 * (NREP * D + kWarps * 32 * NREP) + 8 * kWarps * 2 + 4 * kWarps * NREP * 2;
+    int dev = 0;
+    KIVI_CUDA_OK(cudaGetDevice(&dev));
+    KIVI_REQUIRE(dev >= 0 && dev < 64, "device ordinal %d out of range", dev);
+    if (smem > 48 * 1024 && smem_set[dev].load(std::memory_order_acquire) < smem) {
+        KIVI_CUDA_OK(cudaFuncSetAttribute(attn_fp32_tile_kernel<NREP, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        smem_set[dev].store(smem, std::memory_order_release);
+    }
+    dim3 grid((unsigned)n_splits, (unsigned)L->num_units);
+    attn_fp32_tile_kernel<NREP, D><<<grid, kWarps * 32, smem, st>>>(*L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits,
+                                                                    stage, part_o, part_ml);
+    KIVI_LAUNCH_OK();
+    return KIVI_OK;
+}
+
 template <int NREP>
 static int launch_fp32(const kivi_layer* L, int64_t quant_len, int res_start, int res_len,
                        const void* q, int q_dtype, float scale_log2, int nq_splits, int gps,
-                       int n_splits, float* part_o, float* part_ml, cudaStream_t st,
-                       int split_base = 0, int grid_x = -1) {
+                       int n_splits, float* part_o, float* part_ml, cudaStream_t st) {
     const int D = L->head_dim;
+    if (tile_kernel_ok(L))
+        return D == 64 ? launch_tile<NREP, 64>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, st)
+                       : launch_tile<NREP, 128>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, st);
     const int DB = D > 128 ? 2 : 1;
     const size_t smem = sizeof(float) * ((size_t)NREP * D + kWarps * 2 * D + kWarps * 32 * NREP +
                                          kWarps * NREP * 2 + (size_t)NREP * DB * 128);
-    dim3 grid((unsigned)(grid_x < 0 ? n_splits : grid_x), (unsigned)L->num_units);
-    if (DB == 1) {
-        if (smem > 48 * 1024) KIVI_CUDA_OK(cudaFuncSetAttribute(attn_fp32_kernel<NREP, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attn_fp32_kernel<NREP, 1><<<grid, kWarps * 32, smem, st>>>(*L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, split_base, n_splits, part_o, part_ml);
-    } else {
-        if (smem > 48 * 1024) KIVI_CUDA_OK(cudaFuncSetAttribute(attn_fp32_kernel<NREP, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attn_fp32_kernel<NREP, 2><<<grid, kWarps * 32, smem, st>>>(*L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, split_base, n_splits, part_o, part_ml);
-    }
+    dim3 grid((unsigned)n_splits, (unsigned)L->num_units);
+    auto kernel = DB == 1 ? attn_fp32_kernel<NREP, 1> : attn_fp32_kernel<NREP, 2>;
+    if (smem > 48 * 1024) KIVI_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<grid, kWarps * 32, smem, st>>>(*L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, 0, n_splits, part_o, part_ml);
     KIVI_LAUNCH_OK();
     return KIVI_OK;
 }

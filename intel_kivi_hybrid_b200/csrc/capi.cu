@@ -58,6 +58,8 @@ int run_merge_token_shards(const float* parts, int n_shards, int64_t rows, int D
                            float* lse_out, cudaStream_t st);
 int run_mma_alignment_probe(int* bits_out);
 int attn_mma_fault_word(int* out);
+int fp32_fault_word(int* out);
+int fp32_fault_clear();
 int gather_fault_word(int* out);
 int attn_mma_fault_clear();
 int gather_fault_clear();
@@ -73,15 +75,17 @@ extern "C" int kivi_version(void) { return 100; }
 extern "C" int kivi_last_launch_count(void) { return g_launches; }
 extern "C" int kivi_device_fault(int* word_out) {
     KIVI_REQUIRE(word_out != nullptr, "word_out is null");
-    int copy_wait = 0, peer_wait = 0;
+    int copy_wait = 0, copy_wait_fp32 = 0, peer_wait = 0;
     if (int rc = attn_mma_fault_word(&copy_wait)) return rc;
+    if (int rc = fp32_fault_word(&copy_wait_fp32)) return rc;
     if (int rc = gather_fault_word(&peer_wait)) return rc;
-    *word_out = (copy_wait ? 1 : 0) | (peer_wait ? 2 : 0);
+    *word_out = (copy_wait || copy_wait_fp32 ? 1 : 0) | (peer_wait ? 2 : 0);
     return KIVI_OK;
 }
 
 extern "C" int kivi_device_fault_clear(void) {
     if (int rc = attn_mma_fault_clear()) return rc;
+    if (int rc = fp32_fault_clear()) return rc;
     return gather_fault_clear();
 }
 
@@ -154,16 +158,37 @@ static int clamp_splits(int64_t s, int64_t n_groups) {
     return (int)s;
 }
 
-// CUDA-core kernel: aim at ~8 CTAs of 128 threads per SM, never below 4 token
-// groups per CTA.
-static int plan_splits_fp32(int num_units, int64_t n_groups, int requested) {
+// CUDA-core kernels.  The generic one (head_dim other than 64 and 128): ~8 CTAs of
+// 128 threads per SM, never below 4 token groups per CTA.  The tile kernel is bound by
+// the FMA pipe, so what counts is how evenly whole rounds (one group per warp, four
+// per CTA) spread over the SMs: a round costs c_round of SM time (fitted on B200:
+// 1.0 / 1.9 / 3.3 us with 1 / 4 / 8 heads at head_dim 128, groups of 32), and a CTA
+// alone on its SM takes about 1.2 us longer per round than its share.  32 units x 8k
+// tokens, four heads: 8 pieces 35.9 us, 37 (the generic rule) 39.3; 192 units x 1k,
+// head_dim 64: 2 pieces 14.3, 7 pieces 16.1.
+static int plan_splits_fp32(int num_units, int64_t n_groups, int requested, int head_dim, int group_size, int n_rep, int n_res, int sms) {
     if (n_groups <= 0) return 0;
     if (requested > 0) return clamp_splits(requested, n_groups);
-    const int64_t target = (int64_t)num_sms() * 8;
-    int64_t s = (target + num_units - 1) / num_units;
-    const int64_t cap = (n_groups + 3) / 4;
-    if (s > cap) s = cap;
-    return clamp_splits(s, n_groups);
+    const int n_sms = sms > 0 ? sms : 148;
+    if (head_dim != 64 && head_dim != 128) {
+        const int64_t target = (int64_t)n_sms * 8;
+        int64_t s = (target + num_units - 1) / num_units;
+        const int64_t cap = (n_groups + 3) / 4;
+        if (s > cap) s = cap;
+        return clamp_splits(s, n_groups);
+    }
+    const double c_round = (0.7 + 0.32 * n_rep) * head_dim / 128.0 * group_size / 32.0, c_alone = 1.2, c_cta = 0.3;
+    int best = 1;
+    double best_t = 0.0;
+    for (int s = 1; s <= kMaxSplitsC && s <= n_groups; ++s) {
+        const int64_t per_cta = (n_groups + s - 1) / s;
+        const double rounds = (double)((per_cta + 3) / 4);
+        const double per_sm = (double)(((int64_t)num_units * s + n_sms - 1) / n_sms);
+        const double shared = per_sm * (rounds * c_round + c_cta) + (double)num_units * n_res * c_round / n_sms, alone = rounds * (c_round + c_alone);
+        const double t = (shared > alone ? shared : alone) + (s <= 16 ? 0.1 * s : 1.0 + 0.02 * s);
+        if (s == 1 || t < best_t - 1e-9) { best = s; best_t = t; }
+    }
+    return best;
 }
 
 // Tensor-core kernel: how many pieces to cut every unit's quantized history into.
@@ -236,7 +261,7 @@ extern "C" int kivi_decode_attention_plan(int num_units, int64_t quant_len, int 
     if (ctas_per_sm <= 0) ctas_per_sm = attn_mma_ctas_per_sm();
     *tensor_cores_out = use_mma ? 1 : 0;
     *quant_splits_out = use_mma ? plan_splits_mma(num_units * ((n_rep + 3) / 4), n_groups, num_splits, n_res, sms, ctas_per_sm)
-                                : plan_splits_fp32(num_units, n_groups, num_splits);
+                                : plan_splits_fp32(num_units, n_groups, num_splits, head_dim, group_size, n_rep, n_res, sms);
     *residual_parts_out = n_res;
     return KIVI_OK;
 }
@@ -273,7 +298,7 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
     int n_res_splits = res_len > 0 ? 1 : 0, res_chunk = res_len;
     if (use_mma) attn_mma_residual_plan(res_len, &n_res_splits, &res_chunk);
     const int nq_splits = use_mma ? plan_splits_mma(L->num_units * ((n_rep + 3) / 4), n_groups, num_splits, n_res_splits, num_sms(), attn_mma_ctas_per_sm())
-                                  : plan_splits_fp32(L->num_units, n_groups, num_splits);
+                                  : plan_splits_fp32(L->num_units, n_groups, num_splits, D, G, n_rep, n_res_splits, num_sms());
     const int gps = nq_splits > 0 ? (int)((n_groups + nq_splits - 1) / nq_splits) : 0;
     const int n_splits = nq_splits + n_res_splits;
     const size_t need = (size_t)L->num_units * n_splits * n_rep * (D + 2) * sizeof(float);

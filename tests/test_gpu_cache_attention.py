@@ -577,3 +577,33 @@ def test_ring_append_keeps_the_window(cabi, D, G, R, ring, new, shift, strided):
         idx = (torch.arange(st.res_len, device="cuda") + st.res_start) % R
         for x, buf in ((flat[0], st.k_res), (flat[1], st.v_res)):
             assert torch.equal(buf[:, idx], x[:, t - st.res_len:t].to(ring)), (n, t)
+
+
+@pytest.mark.parametrize("D,G,n_rep,n_quant,n_res,res_start,dtype", [
+    (64, 4, 1, 36, 0, 0, torch.float32),             # groups of four tokens: one of eight token quads in use
+    (128, 8, 3, 8 * 9, 5, 60, torch.float32), (64, 16, 2, 16 * 33, 31, 40, torch.bfloat16),
+    (64, 64, 8, 64 * 5, 33, 0, torch.float32),       # two runs of 32 tokens per group
+    (128, 128, 7, 128 * 3, 64, 1, torch.bfloat16), (128, 32, 5, 32 * 17, 1, 63, torch.float32),
+    (128, 32, 1, 0, 64, 10, torch.float32),          # nothing quantized
+    (64, 32, 6, 32, 0, 0, torch.bfloat16),           # one group, empty ring
+    (32, 8, 4, 64, 20, 50, torch.float32), (256, 64, 2, 128, 20, 50, torch.float32),      # other head_dims: generic kernel
+])
+def test_attention_fp32_kernels_at_their_edges(cabi, D, G, n_rep, n_quant, n_res, res_start, dtype):
+    """fp32-arithmetic kernels against 64 bits on the cache's own dequantized keys and
+    values.  Bound 1e-5 of the row's largest element (fp32 activations): sums of at
+    most n_quant + n_res + D products in fp32, 2^-24 * sqrt(600) = 1.5e-6 per rounding chain."""
+    U, g = 3, torch.Generator(device="cuda").manual_seed(D * G + n_rep)
+    T = n_quant + n_res
+    st = cabi.LayerStore(U, D, G, 128, max(n_quant, G), dtype, "cuda")
+    k, v = (torch.randn(U, T, D, generator=g, device="cuda").to(dtype) for _ in range(2))
+    cabi.load_state(st, k, v, n_quant)
+    st.k_res, st.v_res = (torch.roll(x, res_start, dims=1).contiguous() for x in (st.k_res, st.v_res))
+    st.c.k_res, st.c.v_res, st.res_start = st.k_res.data_ptr(), st.v_res.data_ptr(), res_start
+    q = torch.randn(U, n_rep, D, generator=g, device="cuda").to(dtype)
+    kd, vd = st.materialize()
+    w = torch.softmax(q.double() @ kd.double().transpose(1, 2) * D ** -0.5, dim=-1)
+    ref = w @ vd.double()
+    for splits in (0, 1, 3):
+        out = st.attention(q, n_rep=n_rep, path=cabi.ATTN_FP32, out_dtype=torch.float32, num_splits=splits)
+        err = ((out.double() - ref).abs().amax(-1) / ref.abs().amax(-1)).max().item()
+        assert err < 1e-5, (splits, err)
