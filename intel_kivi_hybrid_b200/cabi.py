@@ -16,6 +16,7 @@ from . import _build
 F32, BF16 = 0, 1
 ROUND_HALF_AWAY, ROUND_HALF_EVEN = 0, 1
 ATTN_AUTO, ATTN_FP32, ATTN_MMA = 0, 1, 2
+_OUT_DTYPES = {None: -1, torch.float32: F32, torch.bfloat16: BF16}      # None: the queries' own
 
 _c = ctypes
 _i64, _int, _vp, _f = _c.c_int64, _c.c_int, _c.c_void_p, _c.c_float
@@ -100,6 +101,25 @@ def _load():
 
 
 lib = _load()
+
+
+_ops = None
+
+
+def _native_ops():
+    """The compiled extension over the same library, whose calls cost a fraction of a
+    ctypes call; None where it is not built, or where the library is not the in-tree
+    one it links against."""
+    global _ops
+    if _ops is None:
+        _ops = False
+        if not os.environ.get("KIVI_CUDA_LIB"):
+            try:
+                from .extension.loader import kivi_native
+                _ops = kivi_native if hasattr(kivi_native, "cache_attention") else False
+            except ImportError:
+                pass
+    return _ops or None
 
 
 def _check(rc):
@@ -228,7 +248,7 @@ class LayerStore:
                        self.k_codes.data_ptr(), self.k_scales.data_ptr(), self.k_zeros.data_ptr(),
                        self.v_codes.data_ptr(), self.v_scales.data_ptr(), self.v_zeros.data_ptr(),
                        self.k_res.data_ptr(), self.v_res.data_ptr())
-        self._ws = None
+        self._ws, self._ws_for = None, None
 
     def reset(self):
         self.quant_len, self.res_start, self.res_len = 0, 0, 0
@@ -264,15 +284,22 @@ class LayerStore:
                                           seq_len, _stream()))
 
     def workspace(self, n_rep, num_splits=0):
+        if self._ws is not None and self._ws_for == (n_rep, num_splits):
+            return self._ws
         need = lib.kivi_decode_attention_workspace(self.num_units, n_rep, self.D, num_splits)
+        self._ws_for = (n_rep, num_splits)
         if self._ws is None or self._ws.numel() < need:
             self._ws = torch.empty(need, dtype=torch.uint8, device=self.device)
         return self._ws
 
     def attention(self, q, out=None, n_rep=None, sm_scale=0.0, num_splits=0, path=ATTN_AUTO, out_dtype=None):
         """q: [num_units, n_rep, D] (or anything contiguous with that many elements)."""
-        _dev(q)
         n_rep = n_rep or q.numel() // (self.num_units * self.D)
+        ops = _native_ops()
+        if ops is not None and out_dtype in _OUT_DTYPES:
+            return ops.cache_attention(_c.addressof(self.c), self.quant_len, self.res_start, self.res_len, q, out,
+                                       self.workspace(n_rep, num_splits), n_rep, sm_scale, num_splits, path, _OUT_DTYPES[out_dtype])
+        _dev(q)
         if out is None:
             out = torch.empty(q.shape, dtype=out_dtype or q.dtype, device=q.device)
         ws = self.workspace(n_rep, num_splits)

@@ -325,6 +325,9 @@ class KiviCache:
         assert st is not None, "decode_attention() before any add_tokens()"
         B, Hq, D = q.shape
         n_rep = Hq // self.num_kv_heads
+        if self.shard is None and B == self.batch_size and Hq == n_rep * self.num_kv_heads:
+            # [B, Hq, D] is [units, n_rep, D] in memory
+            return st.attention(q.contiguous(), n_rep=n_rep, out_dtype=out_dtype, num_splits=num_splits, sm_scale=sm_scale)
         u0, u1 = self._units
         q_units = q.reshape(B * self.num_kv_heads, n_rep, D)[u0:u1].contiguous()
         if self._tokens is not None:

@@ -241,6 +241,21 @@ static int plan_splits_mma(int num_units, int64_t n_groups, int requested, int n
     return best;
 }
 
+// The piece count of either kernel.  The models above walk up to 128 candidates (1-2 us);
+// a decode loop asks for the same shape again and again, so each thread remembers
+// its last question -- the answer depends on nothing else.
+static int plan_splits(bool mma, int num_units, int64_t n_groups, int requested, int head_dim, int group_size, int n_rep, int n_res,
+                       int sms, int ctas_per_sm) {
+    const int64_t key[10] = {mma, num_units, n_groups, requested, head_dim, group_size, n_rep, n_res, sms, ctas_per_sm};
+    static thread_local int64_t last_key[10];
+    static thread_local int last = -1;
+    if (last >= 0 && memcmp(key, last_key, sizeof(key)) == 0) return last;
+    last = mma ? plan_splits_mma(num_units * ((n_rep + 3) / 4), n_groups, requested, n_res, sms, ctas_per_sm)
+               : plan_splits_fp32(num_units, n_groups, requested, head_dim, group_size, n_rep, n_res, sms);
+    memcpy(last_key, key, sizeof(key));
+    return last;
+}
+
 extern "C" int kivi_decode_attention_plan(int num_units, int64_t quant_len, int res_len, int head_dim, int group_size,
                                           int n_rep, int q_dtype, int num_splits, int path, int sms, int ctas_per_sm,
                                           int* tensor_cores_out, int* quant_splits_out, int* residual_parts_out) {
@@ -260,8 +275,7 @@ extern "C" int kivi_decode_attention_plan(int num_units, int64_t quant_len, int 
     if (sms <= 0) sms = num_sms();
     if (ctas_per_sm <= 0) ctas_per_sm = attn_mma_ctas_per_sm();
     *tensor_cores_out = use_mma ? 1 : 0;
-    *quant_splits_out = use_mma ? plan_splits_mma(num_units * ((n_rep + 3) / 4), n_groups, num_splits, n_res, sms, ctas_per_sm)
-                                : plan_splits_fp32(num_units, n_groups, num_splits, head_dim, group_size, n_rep, n_res, sms);
+    *quant_splits_out = plan_splits(use_mma, num_units, n_groups, num_splits, head_dim, group_size, n_rep, n_res, sms, ctas_per_sm);
     *residual_parts_out = n_res;
     return KIVI_OK;
 }
@@ -297,8 +311,7 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
     }
     int n_res_splits = res_len > 0 ? 1 : 0, res_chunk = res_len;
     if (use_mma) attn_mma_residual_plan(res_len, &n_res_splits, &res_chunk);
-    const int nq_splits = use_mma ? plan_splits_mma(L->num_units * ((n_rep + 3) / 4), n_groups, num_splits, n_res_splits, num_sms(), attn_mma_ctas_per_sm())
-                                  : plan_splits_fp32(L->num_units, n_groups, num_splits, D, G, n_rep, n_res_splits, num_sms());
+    const int nq_splits = plan_splits(use_mma, L->num_units, n_groups, num_splits, D, G, n_rep, n_res_splits, num_sms(), use_mma ? attn_mma_ctas_per_sm() : 0);
     const int gps = nq_splits > 0 ? (int)((n_groups + nq_splits - 1) / nq_splits) : 0;
     const int n_splits = nq_splits + n_res_splits;
     const size_t need = (size_t)L->num_units * n_splits * n_rep * (D + 2) * sizeof(float);

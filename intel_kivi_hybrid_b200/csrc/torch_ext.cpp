@@ -280,6 +280,35 @@ int dtype_code(const torch::Tensor& t, const char* name) {
     return t.scalar_type() == torch::kFloat32 ? KIVI_F32 : KIVI_BF16;
 }
 
+// Attention of a layer store of the Python package: `layer` is the address of its
+// struct kivi_layer.  Everything between the Python call and the launches happens
+// here (checks, output allocation, stream lookup): a decode step over a short context
+// is bound by the host, and the same calls made one by one from Python cost 18 us of
+// its 26.  out_dtype: KIVI_F32, KIVI_BF16 or -1 for q's.
+torch::Tensor cache_attention(int64_t layer, int64_t quant_len, int res_start, int res_len, const torch::Tensor& q,
+                              const c10::optional<torch::Tensor>& out, const torch::Tensor& workspace, int n_rep, double sm_scale,
+                              int num_splits, int path, int out_dtype) {
+    auto fail = [](const std::string& what) { throw std::runtime_error(what); };
+    if (!q.is_cuda()) fail("tensor must be on a CUDA device");
+    if (!q.is_contiguous()) fail("tensor must be contiguous");
+    auto code = [&](const torch::Tensor& t) {
+        if (t.scalar_type() == torch::kFloat32) return KIVI_F32;
+        if (t.scalar_type() != torch::kBFloat16)
+            fail(std::string("unsupported dtype torch.") + (t.scalar_type() == torch::kHalf ? "float16" : t.scalar_type() == torch::kDouble ? "float64" : torch::toString(t.scalar_type())) +
+                 ": expected float32 or bfloat16");
+        return KIVI_BF16;
+    };
+    const int q_dtype = code(q);
+    c10::cuda::CUDAGuard guard(q.device());
+    const torch::Tensor o = out.has_value() ? *out
+                                            : at::empty(q.sizes(), q.options().dtype(out_dtype < 0 ? q.scalar_type() : out_dtype == KIVI_F32 ? torch::kFloat32 : torch::kBFloat16));
+    const int rc = kivi_decode_attention(reinterpret_cast<const kivi_layer*>(layer), quant_len, res_start, res_len, q.data_ptr(), q_dtype, o.data_ptr(),
+                                         code(o), n_rep, (float)sm_scale, workspace.data_ptr(), (size_t)workspace.numel(), num_splits, path,
+                                         at::cuda::getCurrentCUDAStream().stream());
+    if (rc != KIVI_OK) fail("kivi_cuda error " + std::to_string(rc) + ": " + kivi_last_error());
+    return o;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -400,6 +429,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("v_zeros"), py::arg("k_res"), py::arg("v_res"), py::arg("quant_len"), py::arg("res_start"), py::arg("res_len"),
           py::arg("out"), py::arg("group_size"), py::arg("workspace") = py::none(), py::arg("sm_scale") = 0.0,
           py::arg("num_splits") = 0, py::arg("path") = 0);
+    m.def("cache_attention", &cache_attention, py::call_guard<py::gil_scoped_release>(),
+          "decode_attention over the layer struct at an address (used by cabi.LayerStore); returns the output tensor.",
+          py::arg("layer"), py::arg("quant_len"), py::arg("res_start"), py::arg("res_len"), py::arg("q"), py::arg("out"), py::arg("workspace"),
+          py::arg("n_rep"), py::arg("sm_scale"), py::arg("num_splits"), py::arg("path"), py::arg("out_dtype"));
     m.def("decode_attention_workspace", [](int num_units, int n_rep, int head_dim, int num_splits) {
               return (int64_t)kivi_decode_attention_workspace(num_units, n_rep, head_dim, num_splits); },
           "Bytes of scratch decode_attention needs.", py::arg("num_units"), py::arg("n_rep"), py::arg("head_dim"), py::arg("num_splits") = 0);

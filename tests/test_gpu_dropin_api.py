@@ -355,3 +355,37 @@ def test_reference_flush_sequence_over_the_extension_reproduces_its_served_cache
     assert flushes == int(sm["long__total_flushes"])
     assert torch.equal(served_k.cpu(), torch.from_numpy(sm["long__served_k"]))
     assert torch.equal(served_v.cpu(), torch.from_numpy(sm["long__served_v"]))
+
+
+@pytest.mark.parametrize("dtype,D,n_rep", [(torch.bfloat16, 128, 4), (torch.float32, 64, 1), (torch.float32, 128, 3)])
+def test_native_attention_call_equals_the_ctypes_call(monkeypatch, dtype, D, n_rep):
+    """LayerStore.attention goes through the compiled extension; the ctypes binding of
+    the same library call is what it is compared with: results bit for bit, the same
+    refusals."""
+    from intel_kivi_hybrid_b200 import cabi
+    g = torch.Generator(device="cuda").manual_seed(5)
+    st = cabi.LayerStore(6, D, 32, 128, 512, dtype, "cuda")
+    k, v = (torch.randn(6, 333, D, generator=g, device="cuda").to(dtype) for _ in range(2))
+    st.update(k, v)
+    q = torch.randn(6, n_rep, D, generator=g, device="cuda").to(dtype)
+    assert cabi._native_ops() is not None
+
+    def calls():
+        out = torch.full_like(q, 7.0)
+        got = [st.attention(q), st.attention(q, n_rep=n_rep, num_splits=3, sm_scale=0.2), st.attention(q, out_dtype=torch.float32),
+               st.attention(q, out_dtype=torch.bfloat16), st.attention(q, out=out), st.attention(q.view(2, 3 * n_rep, D), n_rep=n_rep, path=cabi.ATTN_FP32)]
+        assert got[4].data_ptr() == out.data_ptr()
+        refused = []
+        for bad in (lambda: st.attention(q.cpu(), n_rep=n_rep), lambda: st.attention(q[..., ::2], n_rep=n_rep), lambda: st.attention(q.half(), n_rep=n_rep),
+                    lambda: st.attention(q, out_dtype=torch.float16), lambda: st.attention(q, num_splits=1000), lambda: st.attention(q, n_rep=9)):
+            with pytest.raises(RuntimeError) as e:
+                bad()
+            refused.append(str(e.value))
+        return got, refused
+
+    native = calls()
+    monkeypatch.setattr(cabi, "_ops", False)
+    general = calls()
+    for a, b in zip(native[0], general[0]):
+        assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(a, b)
+    assert native[1] == general[1]
