@@ -33,11 +33,14 @@ constexpr int kWarps = 4;
 template <int NREP, int DB>
 __global__ void __launch_bounds__(kWarps * 32)
 attn_fp32_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
-                 const void* __restrict__ q, int q_dtype, float scale_log2,
-                 int nq_splits, int groups_per_split, int split_base, int n_splits,
+                 const void* q, int q_dtype, float scale_log2,
+                 int nq_splits, int groups_per_split, int n_splits,
                  float* __restrict__ part_o, float* __restrict__ part_ml) {
+    stream_order();
+    q = settled(q);
+    settle_layer(L);
     const int D = L.head_dim, G = L.group_size, Q = G / 4, W = D < 64 ? D : 64, ng = D / G;
-    const int u = blockIdx.y, split = blockIdx.x + split_base;
+    const int u = blockIdx.y, split = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t max_groups = L.max_tokens / G;
 
@@ -419,7 +422,7 @@ __device__ int g_fp32_copy_fault = 0;
 template <int NREP, int D>
 __global__ void __launch_bounds__(kWarps * 32, NREP <= 2 ? 4 : NREP <= 6 ? 3 : 2)
 attn_fp32_tile_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
-                      const void* __restrict__ q, int q_dtype, float scale_log2,
+                      const void* q, int q_dtype, float scale_log2,
                       int nq_splits, int groups_per_split, int n_splits, int stage_bytes,
                       float* __restrict__ part_o, float* __restrict__ part_ml) {
     constexpr int kBytes = Fp32Tile<D>::kBytes, kTokPar = Fp32Tile<D>::kTokPar;
@@ -432,7 +435,10 @@ attn_fp32_tile_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_le
     float* p_s = q_s + NREP * D + warp * 32 * NREP;
     uint64_t* bars = reinterpret_cast<uint64_t*>(q_s + NREP * D + kWarps * 32 * NREP);
     float* ml_s = reinterpret_cast<float*>(bars + kWarps * 2);
-    cudaTriggerProgrammaticLaunchCompletion();            // the fold may become resident now, it waits for this grid's end
+    cudaTriggerProgrammaticLaunchCompletion();            // the kernel that folds the partials may become resident, it waits for this grid's end
+    stream_order();
+    q = settled(q);
+    settle_layer(L);
 
     const bool is_ring = split >= nq_splits;
     const int64_t g_begin = is_ring ? 0 : (int64_t)split * groups_per_split;
@@ -817,14 +823,14 @@ struct LocalSink {
 };
 
 __global__ void __launch_bounds__(kMergeWarps * 32)
-merge_splits_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+merge_splits_kernel(const float* part_o, const float* part_ml,
                     void* __restrict__ out, int out_dtype, int n_splits, int nrep, int64_t rows, int D,
                     float* __restrict__ lse) {
-    // launched with programmatic stream serialization: the launch may overlap the
-    // tail of the attention kernel, the partials may not be read before that
-    // kernel has completed
+    // the launch may overlap the tail of the attention kernel, the partials may not
+    // be read before that kernel has completed
     __shared__ __align__(16) float fold_s[kMergeWarps][128];
-    cudaGridDependencySynchronize();
+    stream_order();
+    part_o = settled(part_o); part_ml = settled(part_ml);
     if (n_splits >= kMergeWideFrom) {                     // grid = rows: the whole CTA on one row
         merge_row_wide(part_o, part_ml, n_splits, nrep, (int64_t)blockIdx.x, D, LocalSink{out, out_dtype}, lse, fold_s);
         return;
@@ -866,9 +872,10 @@ struct PeerSink {
 constexpr uint32_t kPeerSpinLimit = 5u << 20;      // default bound: x 200 ns sleeps, about a second
 
 __global__ void __launch_bounds__(kMergeWarps * 32)
-merge_gather_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+merge_gather_kernel(const float* part_o, const float* part_ml,
                     kivi_peer_gather g, int out_dtype, int n_splits, int nrep, int64_t rows, int D) {
     cudaGridDependencySynchronize();
+    part_o = settled(part_o); part_ml = settled(part_ml);
     // Epoch kept on the device (a call replayed from a CUDA graph): every CTA
     // reads the counter here; the last CTA stores it back after all CTAs have
     // counted themselves in, that is after all of them have read it.
@@ -956,22 +963,11 @@ int gather_fault_clear() {
 int run_merge(const float* part_o, const float* part_ml, void* out, const kivi_peer_gather* gather, float* lse,
               int out_dtype, int num_units, int n_rep, int n_splits, int D, cudaStream_t st) {
     const int64_t rows = (int64_t)num_units * n_rep;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(n_splits >= kMergeWideFrom ? rows : (rows + kMergeWarps - 1) / kMergeWarps));
-    cfg.blockDim = dim3(kMergeWarps * 32);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (gather) {
-        kivi_peer_gather g = *gather;
-        KIVI_CUDA_OK(cudaLaunchKernelEx(&cfg, merge_gather_kernel, part_o, part_ml, g, out_dtype, n_splits, n_rep, rows, D));
-    } else {
-        KIVI_CUDA_OK(cudaLaunchKernelEx(&cfg, merge_splits_kernel, part_o, part_ml, out, out_dtype, n_splits, n_rep, rows, D, lse));
-    }
+    const dim3 grid((unsigned)(n_splits >= kMergeWideFrom ? rows : (rows + kMergeWarps - 1) / kMergeWarps));
+    if (gather)
+        KIVI_CUDA_OK(launch(merge_gather_kernel, grid, kMergeWarps * 32, 0, st, true, part_o, part_ml, *gather, out_dtype, n_splits, n_rep, rows, D));
+    else
+        KIVI_CUDA_OK(launch(merge_splits_kernel, grid, kMergeWarps * 32, 0, st, true, part_o, part_ml, out, out_dtype, n_splits, n_rep, rows, D, lse));
     return KIVI_OK;
 }
 
@@ -1036,9 +1032,8 @@ static int launch_tile(const kivi_layer* L, int64_t quant_len, int res_start, in
         smem_set[dev].store(smem, std::memory_order_release);
     }
     dim3 grid((unsigned)n_splits, (unsigned)L->num_units);
-    attn_fp32_tile_kernel<NREP, D><<<grid, kWarps * 32, smem, st>>>(*L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits,
-                                                                    stage, part_o, part_ml);
-    KIVI_LAUNCH_OK();
+    KIVI_CUDA_OK(launch(attn_fp32_tile_kernel<NREP, D>, grid, kWarps * 32, (size_t)smem, st, true, *L, quant_len, res_start, res_len, q, q_dtype, scale_log2,
+                        nq_splits, gps, n_splits, stage, part_o, part_ml));
     return KIVI_OK;
 }
 
@@ -1056,8 +1051,7 @@ static int launch_fp32(const kivi_layer* L, int64_t quant_len, int res_start, in
     dim3 grid((unsigned)n_splits, (unsigned)L->num_units);
     auto kernel = DB == 1 ? attn_fp32_kernel<NREP, 1> : attn_fp32_kernel<NREP, 2>;
     if (smem > 48 * 1024) KIVI_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<grid, kWarps * 32, smem, st>>>(*L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, 0, n_splits, part_o, part_ml);
-    KIVI_LAUNCH_OK();
+    KIVI_CUDA_OK(launch(kernel, grid, kWarps * 32, smem, st, true, *L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml));
     return KIVI_OK;
 }
 

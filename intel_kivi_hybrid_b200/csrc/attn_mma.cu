@@ -481,7 +481,7 @@ __device__ __forceinline__ void residual_part(
 // buffers in warp order (deterministic) and writes one partial.
 __global__ void __launch_bounds__(kWarps * 32, KIVI_MMA_MIN_CTAS)
 attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
-                const void* __restrict__ q, int q_dtype,
+                const void* q, int q_dtype,
                 float scale_log2, int n_rep, int gps, int nq_splits, int n_res_splits, int res_chunk,
                 float* __restrict__ part_o, float* __restrict__ part_ml) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -490,9 +490,12 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
     uint64_t* bars = reinterpret_cast<uint64_t*>(q_s + 4 * kD);                  // [kWarps][kStages]
     float* ml_s = reinterpret_cast<float*>(bars + kWarps * kStages);             // [kWarps][4][2]
 
-    // the kernel that folds the partials is queued with programmatic stream
-    // serialization: let it become resident now, it waits for this grid's end
+    // the kernel that folds the partials is the only one queued as a dependent: its few
+    // small blocks may become resident from here on, it waits for this grid's end
     cudaTriggerProgrammaticLaunchCompletion();
+    stream_order();
+    q = settled(q);
+    settle_layer(L);
 
     // grid order: all quantized pieces (unit-major), then all residual-ring CTAs --
     // the long CTAs start first, the short ones fill the end
@@ -770,9 +773,8 @@ int run_attn_mma(const kivi_layer* L, int64_t quant_len, int res_start, int res_
                  int n_res_splits, int res_chunk, float* part_o, float* part_ml, cudaStream_t st) {
     if (int rc = ensure_smem_attr(nullptr)) return rc;
     dim3 grid((unsigned)(nq_splits + n_res_splits) * (unsigned)L->num_units * (unsigned)((n_rep + 3) / 4));
-    attn_mma_kernel<<<grid, kWarps * 32, kSmemBytes, st>>>(*L, quant_len, res_start, res_len, q, q_dtype, scale_log2,
-                                                         n_rep, gps, nq_splits, n_res_splits, res_chunk, part_o, part_ml);
-    KIVI_LAUNCH_OK();
+    KIVI_CUDA_OK(launch(attn_mma_kernel, grid, kWarps * 32, kSmemBytes, st, true, *L, quant_len, res_start, res_len, q, q_dtype, scale_log2,
+                        n_rep, gps, nq_splits, n_res_splits, res_chunk, part_o, part_ml));
     return KIVI_OK;
 }
 

@@ -465,10 +465,11 @@ flush_values_direct_kernel(const TF* __restrict__ fresh, int64_t unit_stride, in
 // read the ring: nothing is written before they have completed.
 template <typename TR, typename TF, int VEC>
 __global__ void __launch_bounds__(256)
-ring_append_kernel(const TF* __restrict__ new_k, const TF* __restrict__ new_v, TR* __restrict__ k_ring, TR* __restrict__ v_ring,
+ring_append_kernel(const TF* new_k, const TF* new_v, TR* __restrict__ k_ring, TR* __restrict__ v_ring,
                    int64_t unit_stride_k, int64_t tok_stride_k, int64_t unit_stride_v, int64_t tok_stride_v,
                    int64_t first_tok, int n_tok, int slot0, int R, int D, uint32_t n_items) {   // n_items < 2^31
-    cudaGridDependencySynchronize();
+    stream_order();
+    new_k = settled(new_k); new_v = settled(new_v);
     const uint32_t i = blockIdx.x * 256u + threadIdx.x;
     if (i >= n_items) return;
     const uint32_t pieces = (uint32_t)(D / VEC);
@@ -513,6 +514,9 @@ ring_append_kernel(const TF* __restrict__ new_k, const TF* __restrict__ new_v, T
 __global__ void __launch_bounds__(256)
 materialize_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len, int64_t t_begin,
                    float* __restrict__ k_out, float* __restrict__ v_out) {
+    let_in_early();
+    stream_order();
+    settle_layer(L);
     const int D = L.head_dim, G = L.group_size, Q = G / 4, W = D < 64 ? D : 64, ng = D / G, D4 = D / 4;
     const int u = blockIdx.y;
     const int64_t T = quant_len + res_len;
@@ -585,6 +589,9 @@ __global__ void __launch_bounds__(256)
 materialize_groups_kernel(kivi_layer L, int64_t n_groups, int64_t T,
                           float* __restrict__ k_out, float* __restrict__ v_out) {
     constexpr int D = 128, G = 32;
+    let_in_early();
+    stream_order();
+    settle_layer(L);
     const int u = blockIdx.y, lane = threadIdx.x & 31;
     const int64_t g = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (g >= n_groups) return;
@@ -664,24 +671,6 @@ import_keys_kernel(kivi_layer L, const uint8_t* __restrict__ packed, const float
             L.k_codes[gb * (D * Q) + kblock_offset(d, j, Q, W)] = (uint8_t)byte;
         }
     }
-}
-
-// Launch on `st`; with `overlap` as a programmatic dependent of the kernel before
-// it, whose last blocks it may then run beside.  Only for kernels that either do
-// not depend on that one or wait for it themselves (cudaGridDependencySynchronize).
-template <typename... P, typename... A>
-cudaError_t launch(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, bool overlap, A... args) {
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = overlap ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
 }  // namespace
@@ -920,8 +909,7 @@ extern "C" int kivi_cache_materialize(const kivi_layer* L, int64_t quant_len, in
         al16(L->k_scales) && al16(L->k_zeros) && al16(L->v_codes)) {
         const int64_t n_groups = quant_len / 32;
         dim3 grid((unsigned)((n_groups + 7) / 8), (unsigned)L->num_units);
-        materialize_groups_kernel<<<grid, 256, 0, st>>>(*L, n_groups, quant_len + res_len, k_out, v_out);
-        KIVI_LAUNCH_OK();
+        KIVI_CUDA_OK(launch(materialize_groups_kernel, grid, 256, 0, st, true, *L, n_groups, quant_len + res_len, k_out, v_out));
         ++launches;
         t_begin = quant_len;
     }
@@ -930,8 +918,7 @@ extern "C" int kivi_cache_materialize(const kivi_layer* L, int64_t quant_len, in
         unsigned bx = (unsigned)((rest + 255) / 256);
         if (bx > 4096) bx = 4096;
         dim3 grid(bx, (unsigned)L->num_units);
-        materialize_kernel<<<grid, 256, 0, st>>>(*L, quant_len, res_start, res_len, t_begin, k_out, v_out);
-        KIVI_LAUNCH_OK();
+        KIVI_CUDA_OK(launch(materialize_kernel, grid, 256, 0, st, true, *L, quant_len, res_start, res_len, t_begin, k_out, v_out));
         ++launches;
     }
     note_launches(launches);

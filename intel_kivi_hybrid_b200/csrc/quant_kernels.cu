@@ -48,7 +48,7 @@ template <> struct Vec<__nv_bfloat16> {
 // MODE 0: write packed + scales + zeros.  MODE 1: write the round trip (fp32).
 template <typename T, int LPG, int K, bool HALF_EVEN, int MODE>
 __global__ void __launch_bounds__(kThreads)
-group_quant_kernel(const T* __restrict__ in, uint8_t* __restrict__ packed,
+group_quant_kernel(const T* in, uint8_t* __restrict__ packed,
                    float* __restrict__ scales, float* __restrict__ zeros,
                    float* __restrict__ rt_out, int64_t num_groups) {
     constexpr int VEC = Vec<T>::N;
@@ -64,6 +64,9 @@ group_quant_kernel(const T* __restrict__ in, uint8_t* __restrict__ packed,
     __shared__ __align__(16) float s_scale[MODE == 0 ? TILE_GROUPS : 4];
     __shared__ __align__(16) float s_zero[MODE == 0 ? TILE_GROUPS : 4];
 
+    let_in_early();
+    stream_order();
+    in = settled(in);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = lane % LPG;
     const int64_t tile_g0 = (int64_t)blockIdx.x * TILE_GROUPS;
@@ -171,9 +174,12 @@ group_quant_kernel(const T* __restrict__ in, uint8_t* __restrict__ packed,
 // One thread per group, any G % 4 == 0, any alignment.
 template <bool HALF_EVEN, int MODE>
 __global__ void __launch_bounds__(kThreads)
-group_quant_generic_kernel(const void* __restrict__ in, int in_dtype, uint8_t* __restrict__ packed,
+group_quant_generic_kernel(const void* in, int in_dtype, uint8_t* __restrict__ packed,
                            float* __restrict__ scales, float* __restrict__ zeros,
                            float* __restrict__ rt_out, int64_t num_groups, int G) {
+    let_in_early();
+    stream_order();
+    in = settled(in);
     const int64_t g = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     if (g >= num_groups) return;
     const int64_t base = g * G;
@@ -212,9 +218,12 @@ group_quant_generic_kernel(const void* __restrict__ in, int in_dtype, uint8_t* _
 // scales and zeros: no shuffles, no staging, no barrier.
 template <bool HALF_EVEN, int NR>
 __global__ void __launch_bounds__(kThreads)
-group_quant_bf16_rows_kernel(const __nv_bfloat16* __restrict__ in, uint8_t* __restrict__ packed,
+group_quant_bf16_rows_kernel(const __nv_bfloat16* in, uint8_t* __restrict__ packed,
                              float* __restrict__ scales, float* __restrict__ zeros, int64_t num_groups) {
     constexpr int G = 32 * NR;
+    let_in_early();
+    stream_order();
+    in = settled(in);
     const int64_t g = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     if (g >= num_groups) return;
     const __nv_bfloat16* src = in + g * G;
@@ -271,10 +280,9 @@ int launch_bf16_rows(const void* in, uint8_t* packed, float* scales, float* zero
     KIVI_REQUIRE(blocks <= 0x7fffffffLL, "too many groups for one launch: %lld", (long long)num_groups);
     const __nv_bfloat16* p = reinterpret_cast<const __nv_bfloat16*>(in);
     if (rounding == KIVI_ROUND_HALF_EVEN)
-        group_quant_bf16_rows_kernel<true, NR><<<(unsigned)blocks, kThreads, 0, st>>>(p, packed, scales, zeros, num_groups);
+        KIVI_CUDA_OK(launch(group_quant_bf16_rows_kernel<true, NR>, dim3((unsigned)blocks), kThreads, 0, st, true, p, packed, scales, zeros, num_groups));
     else
-        group_quant_bf16_rows_kernel<false, NR><<<(unsigned)blocks, kThreads, 0, st>>>(p, packed, scales, zeros, num_groups);
-    KIVI_LAUNCH_OK();
+        KIVI_CUDA_OK(launch(group_quant_bf16_rows_kernel<false, NR>, dim3((unsigned)blocks), kThreads, 0, st, true, p, packed, scales, zeros, num_groups));
     note_launches(1);
     return KIVI_OK;
 }
@@ -298,9 +306,11 @@ __device__ __forceinline__ float4 dequant_byte(uint32_t p, float s, float z) {
 }
 
 __global__ void __launch_bounds__(kThreads)
-group_dequant_kernel(const uint8_t* __restrict__ packed, const float* __restrict__ scales,
-                     const float* __restrict__ zeros, float* __restrict__ out,
+group_dequant_kernel(const uint8_t* packed, const float* scales, const float* zeros, float* __restrict__ out,
                      int64_t total_bytes, int bytes_per_group, int group_shift, bool vec_ok) {
+    let_in_early();
+    stream_order();
+    packed = settled(packed); scales = settled(scales); zeros = settled(zeros);
     const int64_t tile = (int64_t)kDqUnroll * kThreads;
     for (int64_t b0 = (int64_t)blockIdx.x * tile; b0 < total_bytes; b0 += (int64_t)gridDim.x * tile) {
         uint32_t p[kDqUnroll];
@@ -339,19 +349,18 @@ int launch_fast(const void* in, uint8_t* packed, float* scales, float* zeros, fl
     const int64_t blocks = (num_groups + TILE_GROUPS - 1) / TILE_GROUPS;
     KIVI_REQUIRE(blocks <= 0x7fffffffLL, "too many groups for one launch: %lld", (long long)num_groups);
     const T* p = reinterpret_cast<const T*>(in);
-    dim3 grid((unsigned)blocks), block(kThreads);
+    dim3 grid((unsigned)blocks);
     if (mode == 0) {
         if (rounding == KIVI_ROUND_HALF_EVEN)
-            group_quant_kernel<T, LPG, K, true, 0><<<grid, block, 0, st>>>(p, packed, scales, zeros, rt, num_groups);
+            KIVI_CUDA_OK(launch(group_quant_kernel<T, LPG, K, true, 0>, dim3(grid), kThreads, 0, st, true, p, packed, scales, zeros, rt, num_groups));
         else
-            group_quant_kernel<T, LPG, K, false, 0><<<grid, block, 0, st>>>(p, packed, scales, zeros, rt, num_groups);
+            KIVI_CUDA_OK(launch(group_quant_kernel<T, LPG, K, false, 0>, dim3(grid), kThreads, 0, st, true, p, packed, scales, zeros, rt, num_groups));
     } else {
         if (rounding == KIVI_ROUND_HALF_EVEN)
-            group_quant_kernel<T, LPG, K, true, 1><<<grid, block, 0, st>>>(p, packed, scales, zeros, rt, num_groups);
+            KIVI_CUDA_OK(launch(group_quant_kernel<T, LPG, K, true, 1>, dim3(grid), kThreads, 0, st, true, p, packed, scales, zeros, rt, num_groups));
         else
-            group_quant_kernel<T, LPG, K, false, 1><<<grid, block, 0, st>>>(p, packed, scales, zeros, rt, num_groups);
+            KIVI_CUDA_OK(launch(group_quant_kernel<T, LPG, K, false, 1>, dim3(grid), kThreads, 0, st, true, p, packed, scales, zeros, rt, num_groups));
     }
-    KIVI_LAUNCH_OK();
     note_launches(1);
     return KIVI_OK;
 }
@@ -399,19 +408,18 @@ int run_group_quant(const void* in, int in_dtype, uint8_t* packed, float* scales
     }
     const int64_t blocks = (num_groups + kThreads - 1) / kThreads;
     KIVI_REQUIRE(blocks <= 0x7fffffffLL, "too many groups for one launch: %lld", (long long)num_groups);
-    dim3 grid((unsigned)blocks), block(kThreads);
+    dim3 grid((unsigned)blocks);
     if (mode == 0) {
         if (rounding == KIVI_ROUND_HALF_EVEN)
-            group_quant_generic_kernel<true, 0><<<grid, block, 0, st>>>(in, in_dtype, packed, scales, zeros, rt, num_groups, G);
+            KIVI_CUDA_OK(launch(group_quant_generic_kernel<true, 0>, dim3(grid), kThreads, 0, st, true, in, in_dtype, packed, scales, zeros, rt, num_groups, G));
         else
-            group_quant_generic_kernel<false, 0><<<grid, block, 0, st>>>(in, in_dtype, packed, scales, zeros, rt, num_groups, G);
+            KIVI_CUDA_OK(launch(group_quant_generic_kernel<false, 0>, dim3(grid), kThreads, 0, st, true, in, in_dtype, packed, scales, zeros, rt, num_groups, G));
     } else {
         if (rounding == KIVI_ROUND_HALF_EVEN)
-            group_quant_generic_kernel<true, 1><<<grid, block, 0, st>>>(in, in_dtype, packed, scales, zeros, rt, num_groups, G);
+            KIVI_CUDA_OK(launch(group_quant_generic_kernel<true, 1>, dim3(grid), kThreads, 0, st, true, in, in_dtype, packed, scales, zeros, rt, num_groups, G));
         else
-            group_quant_generic_kernel<false, 1><<<grid, block, 0, st>>>(in, in_dtype, packed, scales, zeros, rt, num_groups, G);
+            KIVI_CUDA_OK(launch(group_quant_generic_kernel<false, 1>, dim3(grid), kThreads, 0, st, true, in, in_dtype, packed, scales, zeros, rt, num_groups, G));
     }
-    KIVI_LAUNCH_OK();
     note_launches(1);
     return KIVI_OK;
 }
@@ -427,8 +435,7 @@ int run_group_dequant(const uint8_t* packed, const float* scales, const float* z
     if (blocks > cap) blocks = cap;
     int shift = -1;
     for (int k = 0; k < 31; ++k) if ((G / 4) == (1 << k)) shift = k;
-    group_dequant_kernel<<<(unsigned)blocks, kThreads, 0, st>>>(packed, scales, zeros, out, total_bytes, G / 4, shift, aligned16(out));
-    KIVI_LAUNCH_OK();
+    KIVI_CUDA_OK(launch(group_dequant_kernel, dim3((unsigned)blocks), kThreads, 0, st, true, packed, scales, zeros, out, total_bytes, G / 4, shift, aligned16(out)));
     note_launches(1);
     return KIVI_OK;
 }

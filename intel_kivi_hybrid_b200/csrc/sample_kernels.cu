@@ -86,7 +86,7 @@ __device__ __forceinline__ uint32_t kth_key(uint32_t key, int k) {
 // rows with NaN take a radix select over the row instead.  128 rows x 50257 fp32,
 // top 50: 238 us with 256 threads per row, seven passes and two serial scans.
 __global__ void __launch_bounds__(kThreads)
-sample_kernel(const void* __restrict__ logits, int dtype, int vocab, int64_t row_stride,
+sample_kernel(const void* logits, int dtype, int vocab, int64_t row_stride,
               float temperature, int top_k, int do_sample, uint64_t seed, uint64_t step, int64_t* __restrict__ ids) {
     __shared__ float red_f[kWarps];
     __shared__ int red_i[kWarps];
@@ -97,6 +97,8 @@ sample_kernel(const void* __restrict__ logits, int dtype, int vocab, int64_t row
     __shared__ double cand_w[kCand];
     __shared__ uint32_t sel_prefix;
     __shared__ int sel_remaining, pick_s, n_cand_s;
+    stream_order();
+    logits = settled(logits);
     // the reference divides: logits / max(temperature, 1e-8)
     auto scaled = [&](int i) { return __fdiv_rn(logit_at(logits, dtype, (int64_t)blockIdx.x * row_stride + i), temperature); };
     const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -283,8 +285,7 @@ sample_kernel(const void* __restrict__ logits, int dtype, int vocab, int64_t row
 int run_sample(const void* logits, int dtype, int batch, int vocab, int64_t row_stride, float temperature, int top_k,
                int do_sample, uint64_t seed, uint64_t step, int64_t* ids, cudaStream_t st) {
     const float t = temperature > 1e-8f ? temperature : 1e-8f;
-    sample_kernel<<<batch, kThreads, 0, st>>>(logits, dtype, vocab, row_stride, t, top_k, do_sample, seed, step, ids);
-    KIVI_LAUNCH_OK();
+    KIVI_CUDA_OK(launch(sample_kernel, dim3((unsigned)batch), kThreads, 0, st, true, logits, dtype, vocab, row_stride, t, top_k, do_sample, seed, step, ids));
     return KIVI_OK;
 }
 
