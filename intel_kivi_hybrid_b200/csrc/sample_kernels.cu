@@ -15,7 +15,7 @@ namespace {
 
 constexpr int kThreads = 1024;
 constexpr int kWarps = kThreads / 32;
-constexpr int kCand = 2048;               // candidates of a top-k cut that are kept in shared memory
+constexpr int kCand = 512;                 // candidates of a top-k cut that are kept in shared memory
 
 __device__ __forceinline__ float logit_at(const void* p, int dtype, int64_t i) { return load_as_float(p, dtype, i); }
 
@@ -52,21 +52,12 @@ __device__ __forceinline__ MaxIdx better(MaxIdx a, MaxIdx b) {      // larger va
     return a;
 }
 
-// The k-th largest of the keys of all threads' entries (two each, `n` of them in
-// all, absent ones 0): 32 rounds of bisection on the bits, each one barrier that
-// also counts.  Every thread gets the answer.
-__device__ __forceinline__ uint32_t kth_key(uint32_t key0, uint32_t key1, int k) {
+// The k-th largest of the threads' keys by bisection on the bits from 31 down to
+// `last_bit` (the lower bits 0): one barrier per bit, which also counts.  Every thread
+// gets the answer; at least k keys are >= it.
+__device__ __forceinline__ uint32_t kth_key(uint32_t key, int k, int last_bit) {
     uint32_t t = 0u;
-    for (int bit = 31; bit >= 0; --bit) {
-        const uint32_t probe = t | (1u << bit);
-        const int above = __syncthreads_count(key0 >= probe) + __syncthreads_count(key1 >= probe);
-        if (above >= k) t = probe;
-    }
-    return t;
-}
-__device__ __forceinline__ uint32_t kth_key(uint32_t key, int k) {
-    uint32_t t = 0u;
-    for (int bit = 31; bit >= 0; --bit) {
+    for (int bit = 31; bit >= last_bit; --bit) {
         const uint32_t probe = t | (1u << bit);
         if (__syncthreads_count(key >= probe) >= k) t = probe;
     }
@@ -78,13 +69,15 @@ __device__ __forceinline__ uint32_t kth_key(uint32_t key, int k) {
 // many loads are in flight: one pass for the maximum (strided over the threads,
 // coalesced, eight loads in flight), one more to draw.
 //
-// Top-k cut: at least k entries are >= the k-th largest of the threads' own maxima,
-// so one pass that collects the entries above that bound into shared memory (about
-// k of them for unrelated logits) leaves a set small enough to find the exact k-th
-// value, sort by index and draw from without reading the row again.  k above the
-// number of threads, more than kCand candidates (long runs of equal logits) and
-// rows with NaN take a radix select over the row instead.  128 rows x 50257 fp32,
-// top 50: 238 us with 256 threads per row, seven passes and two serial scans.
+// Top-k cut: at least k entries are >= the k-th largest of the threads' own maxima
+// (its upper 16 bits are bound enough), so one pass that collects the entries above
+// that bound into shared memory (a few more than k for unrelated logits) leaves a set
+// small enough to rank every entry by counting and to draw from without reading the
+// row again: an entry is kept when fewer than k are greater, which is what comparing
+// it with the k-th value says.  k above the number of threads, more than kCand
+// candidates (k above about 400, long runs of equal logits) and rows with NaN take a
+// radix select over the row instead.  128 rows x 50257 fp32, top 50: 238 us with 256
+// threads per row, seven passes and two serial scans, 16 us now.
 __global__ void __launch_bounds__(kThreads)
 sample_kernel(const void* logits, int dtype, int vocab, int64_t row_stride,
               float temperature, int top_k, int do_sample, uint64_t seed, uint64_t step, int64_t* __restrict__ ids) {
@@ -135,9 +128,14 @@ sample_kernel(const void* logits, int dtype, int vocab, int64_t row_stride,
 
     float kth = -INFINITY;
     if (top_k > 0 && top_k < vocab) {
-        const uint32_t bound = (top_k <= kThreads && !row_nan) ? kth_key(my_key, top_k) : 0u;
+        const uint32_t bound = (top_k <= kThreads && !row_nan) ? kth_key(my_key, top_k, 16) : 0u;
         if (bound != 0u) {                                  // CTA-uniform
-            const float least = key_to_float(bound);        // compared as a number: -0 counts as +0, as in the cut itself
+            // compared as a number: -0 counts as +0, as in the cut itself (the keys between 0 and
+            // that of -inf are NaN patterns: cutting the lower bits may end there)
+            const float least = bound < 0x007fffffu ? -INFINITY : key_to_float(bound);
+            // what is clearly below is dropped without a division (a quotient that lost bits in
+            // the subnormals does not say what is clear)
+            const float clear = fabsf(least) > 1e-30f && fabsf(least) < 1e30f ? (least - fabsf(least) * 1e-5f) * temperature : -INFINITY;
             // ---- collect what is not below the bound -------------------------------
             for (int i0 = tid; i0 < vocab; i0 += 8 * kThreads) {
                 float x[8];
@@ -145,8 +143,9 @@ sample_kernel(const void* logits, int dtype, int vocab, int64_t row_stride,
                 for (int j = 0; j < 8; ++j) x[j] = i0 + j * kThreads < vocab ? logit_at(logits, dtype, base + i0 + j * kThreads) : -INFINITY;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
+                    if (!(x[j] >= clear) || i0 + j * kThreads >= vocab) continue;
                     const float y = __fdiv_rn(x[j], temperature);
-                    if (i0 + j * kThreads < vocab && y >= least) {
+                    if (y >= least) {
                         const int at = atomicAdd(&n_cand_s, 1);
                         if (at < kCand) { cand_x[at] = y; cand_i[at] = i0 + j * kThreads; }
                     }
@@ -155,29 +154,20 @@ sample_kernel(const void* logits, int dtype, int vocab, int64_t row_stride,
             __syncthreads();
             const int n = n_cand_s;
             if (n <= kCand) {
-                const int i0 = tid, i1 = tid + kThreads;
-                const uint32_t key0 = i0 < n ? ordered_key(cand_x[i0]) : 0u, key1 = i1 < n ? ordered_key(cand_x[i1]) : 0u;
-                const float cut = key_to_float(kth_key(key0, key1, top_k));
-                // masses in index order: every candidate's place is the number of smaller indices
-                float x[2]; int idx[2], place[2];
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const int c = tid + j * kThreads;
-                    x[j] = c < n ? cand_x[c] : 0.0f; idx[j] = c < n ? cand_i[c] : 0x7fffffff; place[j] = 0;
-                }
+                // an entry's place in index order and how many are greater, by counting
+                const float x = tid < n ? cand_x[tid] : 0.0f;
+                const int idx = tid < n ? cand_i[tid] : 0;
+                int place = 0, greater = 0;
                 if (tid < n)
                     for (int c = 0; c < n; ++c) {
-                        const int other = cand_i[c];
-                        place[0] += other < idx[0]; place[1] += other < idx[1];
+                        place += cand_i[c] < idx;
+                        greater += cand_x[c] > x;
                     }
-                __syncthreads();                            // all have read the unsorted indices
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-                    if (tid + j * kThreads < n) {
-                        cand_i[place[j]] = idx[j];
-                        cand_w[place[j]] = x[j] >= cut ? (double)expf(x[j] - m) : 0.0;
-                        cand_x[place[j]] = x[j];
-                    }
+                __syncthreads();                            // all have read the unsorted entries
+                if (tid < n) {
+                    cand_i[place] = idx;
+                    cand_w[place] = greater < top_k ? (double)expf(x - m) : 0.0;
+                }
                 __syncthreads();
                 if (warp == 0) {
                     // running masses in index order, the first one past the target is the draw

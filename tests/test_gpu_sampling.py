@@ -92,6 +92,7 @@ def test_sample_token_keeps_ids_on_the_device_and_validates(cabi):
     (5000, 1025, "normal"),                                                # above it: radix select
     (50257, 1000, "normal"), (32000, 50, "rounded"),                       # long runs of equal logits: more candidates than are kept
     (4096, 40, "zeros"), (4096, 40, "masked"),                             # -0 and +0 at the cut; -inf entries
+    (1023, 1000, "masked"), (700, 500, "masked"),                          # -inf at the cut: more asked for than is finite
 ])
 def test_draws_of_every_selection_path(cabi, vocab, top_k, kind):
     g = torch.Generator().manual_seed(vocab + top_k)
