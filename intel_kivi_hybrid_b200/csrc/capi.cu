@@ -208,13 +208,18 @@ static int plan_splits_fp32(int num_units, int64_t n_groups, int requested, int 
 //   * the quantized CTAs all resident at once: the time of one of them (the ring
 //     CTAs fill the free slots, or follow the first ring CTAs that finish);
 //   * several waves: total CTA time over the slots, plus a ragged end of about
-//     a third of a CTA.
+//     a third of a CTA; a CTA's fixed time is 7.5 us there.
+// The ring CTAs count where they decide how many CTAs share an SM: the one-CTA rate
+// needs all CTAs, ring included, on SMs of their own (32 units x 2k tokens: 3 pieces
+// 9.7 us, 4 pieces 10.7), and at the two-CTA count the ring CTAs must fit beside the
+// quantized ones (256 units x 4k with 256 + 256 CTAs: 49.6 us in one piece, 45.3 in
+// two, 44.0 in three; 192 units x 2k: one piece 24.3 us, three 26.3).
 static int plan_splits_mma(int num_units, int64_t n_groups, int requested, int n_res_splits, int sms, int ctas_per_sm) {
     if (n_groups <= 0) return 0;
     if (requested > 0) return clamp_splits(requested, n_groups);
     const int n_sms = sms > 0 ? sms : 148, per_sm = ctas_per_sm > 0 ? ctas_per_sm : 3;
     const double slots = (double)per_sm * n_sms;
-    const double c0 = 6.0, c1_one = 0.16, c1_two = 0.24, c1_three = 0.33, c1_full = 0.36;
+    const double c0 = 6.0, c0_waves = 7.5, c1_one = 0.16, c1_two = 0.24, c1_crowded = 0.31, c1_three = 0.33, c1_full = 0.36;
     const double t_ring = 7.0, c_start = 0.015, ragged = 0.3;
     const int64_t s_max = n_groups < kMaxSplitsC ? n_groups : kMaxSplitsC;
     int best = 1;
@@ -227,10 +232,12 @@ static int plan_splits_mma(int num_units, int64_t n_groups, int requested, int n
             // the fullest SM sets the pace.  The two-CTA rate only holds up to about
             // 1.75 CTAs per SM on average: with 288 or 296 CTAs on 148 SMs a CTA was
             // measured at 0.27-0.32 us per group, as if some SMs already held three.
-            const double c1 = quant <= n_sms ? c1_one : quant <= 1.75 * n_sms ? c1_two : quant <= 3.0 * n_sms ? c1_three : c1_full;
+            const double c1 = quant + ring <= n_sms ? c1_one
+                            : quant <= 1.75 * n_sms ? (quant + ring <= slots ? c1_two : c1_crowded)
+                            : quant <= 3.0 * n_sms ? c1_three : c1_full;
             t = c0 + c1 * per_cta + c_start * (quant + ring);
         } else {
-            t = (quant * (c0 + c1_full * per_cta) + ring * t_ring) / slots + ragged * (c0 + c1_full * per_cta);
+            t = (quant * (c0_waves + c1_full * per_cta) + ring * t_ring) / slots + ragged * (c0_waves + c1_full * per_cta);
             // just over one wave: never cheaper than a full single wave of such CTAs
             const double one_wave = c0 + c1_three * per_cta + c_start * slots;
             if (t < one_wave) t = one_wave;
