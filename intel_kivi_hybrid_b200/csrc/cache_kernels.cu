@@ -23,6 +23,11 @@
 namespace kivi {
 namespace {
 
+// Last statement of the flush kernels that start while the one before them drains:
+// nothing they do depends on it, but what comes after this kernel waits for this
+// kernel only, so this one must not be over before the one before it is.
+__device__ __forceinline__ void after_predecessor() { cudaGridDependencySynchronize(); }
+
 struct TokenSource {
     const void* ring;     // [units][R][D] of ring_dtype
     const void* fresh;    // new tokens
@@ -209,6 +214,7 @@ flush_values_kernel(TokenSource src, uint8_t* __restrict__ v_codes, float* __res
         }
         dst[vcode_offset(t, gd * (G / 4) + i / 4, D, G)] = (uint8_t)byte;
     }
+    after_predecessor();
 }
 
 // Values, fast path for D = 128, G = 32: four consecutive lanes share one
@@ -286,6 +292,7 @@ flush_values_fast_kernel(TokenSource src, uint8_t* __restrict__ v_codes, float* 
         gs[i] = reinterpret_cast<const float4*>(s_scale)[i];
         gz[i] = reinterpret_cast<const float4*>(s_zero)[i];
     }
+    after_predecessor();
 }
 
 // ---- bulk prefill: groups cut straight out of the new tensor ----------------
@@ -366,6 +373,7 @@ flush_keys_direct_kernel(const TF* __restrict__ fresh, int64_t unit_stride, int6
                 (uint16_t)(pack4_magic(m0[0], m0[1], m0[2], m0[3]) | (pack4_magic(m1[0], m1[1], m1[2], m1[3]) << 8));
         }
     }
+    after_predecessor();
 }
 
 // Values for D = 128, G = 32, every token in the new tensor: a thread owns one
@@ -452,6 +460,7 @@ flush_values_direct_kernel(const TF* __restrict__ fresh, int64_t unit_stride, in
         reinterpret_cast<float4*>(v_scales + t_first * (D / G))[threadIdx.x - 64] = reinterpret_cast<const float4*>(s_scale)[threadIdx.x - 64];
     else
         reinterpret_cast<float4*>(v_zeros + t_first * (D / G))[threadIdx.x - 96] = reinterpret_cast<const float4*>(s_zero)[threadIdx.x - 96];
+    after_predecessor();
 }
 
 // Copies virtual tokens [tau_from, tau_from + n_tok) of the new tensor into their
@@ -750,8 +759,8 @@ extern "C" int kivi_cache_update(const kivi_layer* L, int64_t quant_len, int res
     TokenSource sv{L->v_res, new_v, L->res_dtype, new_dtype, R, D, res_start, res_len, unit_stride_v, tok_stride_v};
     const int64_t max_groups = L->max_tokens / G;
     // The flush kernels of one call write disjoint arrays and read what was there
-    // before the call, so each may start while the one before it drains; the ring
-    // append, which overwrites slots they read, waits for them.
+    // before the call, so each may start while the one before it drains (and ends
+    // after it); the ring append, which overwrites slots they read, waits for them.
     if (f > 0) {
         const int64_t group0 = quant_len / G;
         KIVI_REQUIRE(f <= 0x7fffffff && L->num_units <= 65535, "grid too large");
