@@ -19,6 +19,7 @@
 // walks the D channels of its token), a warp max, exp2, then lane = 4 channels
 // for p.V (each lane walks the chunk's tokens).
 #include "async_copy.cuh"
+#include "cluster_fold.cuh"
 #include "kivi_common.cuh"
 
 #include <atomic>
@@ -424,7 +425,7 @@ __global__ void __launch_bounds__(kWarps * 32, NREP <= 2 ? 4 : NREP <= 6 ? 3 : 2
 attn_fp32_tile_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
                       const void* q, int q_dtype, float scale_log2,
                       int nq_splits, int groups_per_split, int n_splits, int stage_bytes,
-                      float* __restrict__ part_o, float* __restrict__ part_ml) {
+                      float* __restrict__ part_o, float* __restrict__ part_ml, ClusterOut direct) {
     constexpr int kBytes = Fp32Tile<D>::kBytes, kTokPar = Fp32Tile<D>::kTokPar;
     const int G = L.group_size, ng = D / G;
     const int u = blockIdx.y, split = blockIdx.x;
@@ -634,8 +635,10 @@ attn_fp32_tile_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_le
             const float4 c = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(smem_raw + w2 * 2 * stage_bytes) + i);
             a.x += c.x; a.y += c.y; a.z += c.z; a.w += c.w;
         }
-        *reinterpret_cast<float4*>(part_o + pbase * D + i) = a;
+        // (the queries and the weights have been read for the last time)
+        *reinterpret_cast<float4*>(direct.out ? q_s + i : part_o + pbase * D + i) = a;
     }
+    float* const ml_out = direct.out ? q_s + NREP * D : part_ml + pbase * 2;
     if (threadIdx.x < NREP) {
         const int h = threadIdx.x;
         float M = -INFINITY, ls = 0.0f;
@@ -644,16 +647,15 @@ attn_fp32_tile_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_le
             const float mw = ml_s[(w2 * NREP + h) * 2];
             if (mw != -INFINITY) ls += ml_s[(w2 * NREP + h) * 2 + 1] * exp2f(mw - M);
         }
-        part_ml[(pbase + h) * 2] = M;
-        part_ml[(pbase + h) * 2 + 1] = ls;
+        ml_out[h * 2] = M;
+        ml_out[h * 2 + 1] = ls;
     }
+    if (direct.out) cluster_fold(q_s, ml_out, NREP, D, (int64_t)u * NREP, direct);
 }
 
 }  // namespace
 
 namespace {
-
-__device__ __forceinline__ void store_quad(void* p, int dtype, int64_t i, float4 v);
 
 // out[u][h][:] = sum_s o_s * 2^(m_s - M) / sum_s l_s * 2^(m_s - M)
 // One warp per output row (row = u*n_rep + h), kMergeWarps rows per CTA; partials
@@ -792,27 +794,6 @@ __device__ __forceinline__ void merge_row_wide(const float* __restrict__ part_o,
             if (active) sink(row * D + d, make_float4(t.x * inv, t.y * inv, t.z * inv, t.w * inv));
         }
         __syncthreads();                                  // fold_s is rewritten by the next 128 channels
-    }
-}
-
-// four consecutive output elements starting at element i (i % 4 == 0): one 8- or
-// 16-byte store when the buffer allows it
-__device__ __forceinline__ void store_quad(void* p, int dtype, int64_t i, float4 v) {
-    if (dtype == KIVI_BF16) {
-        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p) + i;
-        if ((reinterpret_cast<uintptr_t>(o) & 7u) == 0) {
-            const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-            uint2 w;
-            w.x = *reinterpret_cast<const uint32_t*>(&lo); w.y = *reinterpret_cast<const uint32_t*>(&hi);
-            *reinterpret_cast<uint2*>(o) = w;
-        } else {
-            o[0] = __float2bfloat16_rn(v.x); o[1] = __float2bfloat16_rn(v.y);
-            o[2] = __float2bfloat16_rn(v.z); o[3] = __float2bfloat16_rn(v.w);
-        }
-    } else {
-        float* o = reinterpret_cast<float*>(p) + i;
-        if ((reinterpret_cast<uintptr_t>(o) & 15u) == 0) *reinterpret_cast<float4*>(o) = v;
-        else { o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
     }
 }
 
@@ -1010,7 +991,7 @@ int run_merge_token_shards(const float* parts, int n_shards, int64_t rows, int D
 // The tile kernel takes head_dim 64 and 128 with 16-byte aligned arrays and groups of
 // whole 16-byte pieces (any group size: D*G/4 bytes of codes are a multiple of 16);
 // everything else -- other head_dims, odd alignments -- takes the generic kernel.
-static bool tile_kernel_ok(const kivi_layer* L) {
+bool attn_fp32_tile_ok(const kivi_layer* L) {
     auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     return (L->head_dim == 64 || L->head_dim == 128) && al(L->k_res) && al(L->v_res) && al(L->k_codes) && al(L->k_scales) &&
            al(L->k_zeros) && al(L->v_codes) && al(L->v_scales) && al(L->v_zeros);
@@ -1018,7 +999,7 @@ static bool tile_kernel_ok(const kivi_layer* L) {
 
 template <int NREP, int D>
 static int launch_tile(const kivi_layer* L, int64_t quant_len, int res_start, int res_len, const void* q, int q_dtype, float scale_log2,
-                       int nq_splits, int gps, int n_splits, float* part_o, float* part_ml, cudaStream_t st) {
+                       int nq_splits, int gps, int n_splits, float* part_o, float* part_ml, const ClusterOut& direct, cudaStream_t st) {
     static std::atomic<int> smem_set[64];
     // two stages of one group per warp, and never less than the warp's [NREP][D] output buffer
     int stage = 2 * (D * L->group_size / 4) + 4 * D * 4;
@@ -1032,19 +1013,19 @@ static int launch_tile(const kivi_layer* L, int64_t quant_len, int res_start, in
         smem_set[dev].store(smem, std::memory_order_release);
     }
     dim3 grid((unsigned)n_splits, (unsigned)L->num_units);
-    KIVI_CUDA_OK(launch(attn_fp32_tile_kernel<NREP, D>, grid, kWarps * 32, (size_t)smem, st, true, *L, quant_len, res_start, res_len, q, q_dtype, scale_log2,
-                        nq_splits, gps, n_splits, stage, part_o, part_ml));
+    KIVI_CUDA_OK(launch_cluster(attn_fp32_tile_kernel<NREP, D>, direct.out ? n_splits : 0, grid, kWarps * 32, (size_t)smem, st, true, *L, quant_len, res_start, res_len, q, q_dtype, scale_log2,
+                        nq_splits, gps, n_splits, stage, part_o, part_ml, direct));
     return KIVI_OK;
 }
 
 template <int NREP>
 static int launch_fp32(const kivi_layer* L, int64_t quant_len, int res_start, int res_len,
                        const void* q, int q_dtype, float scale_log2, int nq_splits, int gps,
-                       int n_splits, float* part_o, float* part_ml, cudaStream_t st) {
+                       int n_splits, float* part_o, float* part_ml, const ClusterOut& direct, cudaStream_t st) {
     const int D = L->head_dim;
-    if (tile_kernel_ok(L))
-        return D == 64 ? launch_tile<NREP, 64>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, st)
-                       : launch_tile<NREP, 128>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, st);
+    if (attn_fp32_tile_ok(L))
+        return D == 64 ? launch_tile<NREP, 64>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, direct, st)
+                       : launch_tile<NREP, 128>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, direct, st);
     const int DB = D > 128 ? 2 : 1;
     const size_t smem = sizeof(float) * ((size_t)NREP * D + kWarps * 2 * D + kWarps * 32 * NREP +
                                          kWarps * NREP * 2 + (size_t)NREP * DB * 128);
@@ -1057,16 +1038,16 @@ static int launch_fp32(const kivi_layer* L, int64_t quant_len, int res_start, in
 
 int run_attn_fp32(const kivi_layer* L, int64_t quant_len, int res_start, int res_len,
                   const void* q, int q_dtype, int n_rep, float scale_log2, int nq_splits, int gps,
-                  int n_splits, float* part_o, float* part_ml, cudaStream_t st) {
+                  int n_splits, float* part_o, float* part_ml, const ClusterOut& direct, cudaStream_t st) {
     switch (n_rep) {
-        case 1: return launch_fp32<1>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, st);
-        case 2: return launch_fp32<2>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, st);
-        case 3: return launch_fp32<3>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, st);
-        case 4: return launch_fp32<4>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, st);
-        case 5: return launch_fp32<5>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, st);
-        case 6: return launch_fp32<6>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, st);
-        case 7: return launch_fp32<7>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, st);
-        case 8: return launch_fp32<8>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, st);
+        case 1: return launch_fp32<1>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, direct, st);
+        case 2: return launch_fp32<2>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, direct, st);
+        case 3: return launch_fp32<3>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, direct, st);
+        case 4: return launch_fp32<4>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, direct, st);
+        case 5: return launch_fp32<5>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, direct, st);
+        case 6: return launch_fp32<6>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, direct, st);
+        case 7: return launch_fp32<7>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, direct, st);
+        case 8: return launch_fp32<8>(L, quant_len, res_start, res_len, q, q_dtype, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, direct, st);
         default: break;
     }
     set_error("n_rep (%d) outside 1..8", n_rep);

@@ -31,6 +31,7 @@
 // Every wait on an mbarrier is bounded; on expiry the warp raises the device
 // fault word, stops consuming and its partial is written as "empty".
 #include "async_copy.cuh"
+#include "cluster_fold.cuh"
 #include "kivi_common.cuh"
 
 #include <cuda_fp16.h>
@@ -479,11 +480,15 @@ __device__ __forceinline__ void residual_part(
 // (max, sum) of the warps.  When a warp is done, its ring doubles as the
 // [4][128] buffer its scaled output goes to; the CTA then adds the warps'
 // buffers in warp order (deterministic) and writes one partial.
+//
+// FOLD: the CTAs of a unit and head block are a cluster and fold their partials
+// themselves (a template, so that the wide grids keep their registers).
+template <bool FOLD>
 __global__ void __launch_bounds__(kWarps * 32, KIVI_MMA_MIN_CTAS)
 attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
                 const void* q, int q_dtype,
                 float scale_log2, int n_rep, int gps, int nq_splits, int n_res_splits, int res_chunk,
-                float* __restrict__ part_o, float* __restrict__ part_ml) {
+                float* __restrict__ part_o, float* __restrict__ part_ml, ClusterOut direct) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     uint8_t* stage_mem = smem_raw;                                               // [kWarps][kStages][kStageBytes]
     float* q_s = reinterpret_cast<float*>(smem_raw + kWarps * kStages * kStageBytes);   // [4][128]
@@ -504,10 +509,15 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
     // read of the piece mostly comes from L2).
     const int head_blocks = (n_rep + 3) >> 2;
     const int n_quant_ctas = (int)L.num_units * head_blocks * nq_splits;
-    const bool is_res = (int)blockIdx.x >= n_quant_ctas;
+    // When the partials are folded inside clusters (FOLD), the CTAs of a unit and
+    // head block lie side by side instead: pieces, then ring parts.
+    const int n_all = nq_splits + n_res_splits;
+    const int in_row = (int)blockIdx.x % n_all;
+    const bool is_res = FOLD ? in_row >= nq_splits : (int)blockIdx.x >= n_quant_ctas;
     const int rel = is_res ? (int)blockIdx.x - n_quant_ctas : (int)blockIdx.x;
     const int per_unit = is_res ? n_res_splits : nq_splits;
-    const int uv = rel / per_unit, sub = rel - uv * per_unit;
+    const int uv = FOLD ? (int)blockIdx.x / n_all : rel / per_unit;
+    const int sub = FOLD ? (is_res ? in_row - nq_splits : in_row) : rel - uv * per_unit;
     const int u = uv / head_blocks, head0 = 4 * (uv - u * head_blocks);
     const int n_heads = n_rep - head0 < 4 ? n_rep - head0 : 4;       // heads of this CTA: head0 .. head0 + n_heads - 1
     const int n_splits_total = nq_splits + n_res_splits;
@@ -690,7 +700,9 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
     __syncthreads();
 
     // ---- the CTA's partial: warps added in warp order ------------------------------
+    // (for the fold inside a cluster it stays in shared memory, behind the first warp's buffer)
     const int64_t pbase = ((int64_t)u * n_splits_total + slot) * n_rep + head0;
+    float* const cta_o = reinterpret_cast<float*>(stage_mem) + 4 * kD;
     for (int i = threadIdx.x; i < kD; i += blockDim.x) {
         const int h = i >> 5, cc = (i & 31) * 4;
         if (h < n_heads) {
@@ -700,9 +712,10 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
                 const float4 b = *reinterpret_cast<const float4*>(stage_mem + w2 * kStages * kStageBytes + h * kD * 4 + cc * 4);
                 a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
             }
-            *reinterpret_cast<float4*>(part_o + (pbase + h) * kD + cc) = a;
+            *reinterpret_cast<float4*>(FOLD ? cta_o + h * kD + cc : part_o + (pbase + h) * kD + cc) = a;
         }
     }
+    float* const ml_out = FOLD ? cta_o + 4 * kD : part_ml + pbase * 2;
     if (threadIdx.x < n_heads) {
         const int h = threadIdx.x;
         float Mh = -INFINITY, ls = 0.0f;
@@ -711,14 +724,15 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
             const float mw = ml_s[(w2 * 4 + h) * 2];
             if (mw != -INFINITY) ls += ml_s[(w2 * 4 + h) * 2 + 1] * ex2(mw - Mh);
         }
-        part_ml[(pbase + h) * 2] = Mh;
-        part_ml[(pbase + h) * 2 + 1] = ls;
+        ml_out[h * 2] = Mh;
+        ml_out[h * 2 + 1] = ls;
     }
+    if constexpr (FOLD) cluster_fold(cta_o, ml_out, n_heads, kD, (int64_t)u * n_rep + head0, direct);
 }
 
 constexpr size_t kSmemBytes = (size_t)kWarps * kStages * kStageBytes + 4 * kD * 4 + kWarps * kStages * 8 +
                               kWarps * 4 * 2 * 4;
-static_assert(kStages * kStageBytes >= 4 * kD * 4, "a warp's ring doubles as its [4][128] fold buffer");
+static_assert(kStages * kStageBytes >= 2 * 4 * kD * 4 + 32, "a warp's ring doubles as its [4][128] fold buffer, the first also holds the CTA's partial");
 static_assert(kWarps * 32 >= 32, "at least one warp");
 
 }  // namespace
@@ -746,7 +760,8 @@ static int ensure_smem_attr(int* dev_out) {
     KIVI_CUDA_OK(cudaGetDevice(&dev));
     KIVI_REQUIRE(dev >= 0 && dev < 64, "device ordinal %d out of range", dev);
     if (!attr_set[dev].load(std::memory_order_acquire)) {
-        KIVI_CUDA_OK(cudaFuncSetAttribute(attn_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+        KIVI_CUDA_OK(cudaFuncSetAttribute(attn_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+        KIVI_CUDA_OK(cudaFuncSetAttribute(attn_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
         attr_set[dev].store(true, std::memory_order_release);
     }
     if (dev_out) *dev_out = dev;
@@ -761,7 +776,7 @@ int attn_mma_ctas_per_sm() {
     if (ensure_smem_attr(&dev) != KIVI_OK) return 0;
     int n = cached[dev].load(std::memory_order_acquire);
     if (n == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_mma_kernel, kWarps * 32, kSmemBytes) != cudaSuccess || n <= 0)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_mma_kernel<false>, kWarps * 32, kSmemBytes) != cudaSuccess || n <= 0)
             return 0;
         cached[dev].store(n, std::memory_order_release);
     }
@@ -770,11 +785,11 @@ int attn_mma_ctas_per_sm() {
 
 int run_attn_mma(const kivi_layer* L, int64_t quant_len, int res_start, int res_len,
                  const void* q, int q_dtype, int n_rep, float scale_log2, int nq_splits, int gps,
-                 int n_res_splits, int res_chunk, float* part_o, float* part_ml, cudaStream_t st) {
+                 int n_res_splits, int res_chunk, float* part_o, float* part_ml, const ClusterOut& direct, cudaStream_t st) {
     if (int rc = ensure_smem_attr(nullptr)) return rc;
     dim3 grid((unsigned)(nq_splits + n_res_splits) * (unsigned)L->num_units * (unsigned)((n_rep + 3) / 4));
-    KIVI_CUDA_OK(launch(attn_mma_kernel, grid, kWarps * 32, kSmemBytes, st, true, *L, quant_len, res_start, res_len, q, q_dtype, scale_log2,
-                        n_rep, gps, nq_splits, n_res_splits, res_chunk, part_o, part_ml));
+    KIVI_CUDA_OK(launch_cluster(direct.out ? attn_mma_kernel<true> : attn_mma_kernel<false>, direct.out ? nq_splits + n_res_splits : 0, grid, kWarps * 32, kSmemBytes, st, true, *L, quant_len, res_start, res_len, q, q_dtype, scale_log2,
+                        n_rep, gps, nq_splits, n_res_splits, res_chunk, part_o, part_ml, direct));
     return KIVI_OK;
 }
 

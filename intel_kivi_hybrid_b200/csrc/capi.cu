@@ -6,6 +6,7 @@
 
 #include <mutex>
 
+#include "cluster_fold.cuh"
 #include "kivi_common.cuh"
 
 namespace kivi {
@@ -45,13 +46,14 @@ int validate_layer(const kivi_layer* L);
 int validate_state(const kivi_layer* L, int64_t quant_len, int res_start, int res_len);
 int run_attn_fp32(const kivi_layer* L, int64_t quant_len, int res_start, int res_len,
                   const void* q, int q_dtype, int n_rep, float scale_log2, int nq_splits, int gps,
-                  int n_splits, float* part_o, float* part_ml, cudaStream_t st);
+                  int n_splits, float* part_o, float* part_ml, const ClusterOut& direct, cudaStream_t st);
+bool attn_fp32_tile_ok(const kivi_layer* L);
 bool attn_mma_supported(const kivi_layer* L, int n_rep, const void* q);
 void attn_mma_residual_plan(int res_len, int* n_res_splits, int* res_chunk);
 int attn_mma_ctas_per_sm();
 int run_attn_mma(const kivi_layer* L, int64_t quant_len, int res_start, int res_len,
                  const void* q, int q_dtype, int n_rep, float scale_log2, int nq_splits, int gps,
-                 int n_res_splits, int res_chunk, float* part_o, float* part_ml, cudaStream_t st);
+                 int n_res_splits, int res_chunk, float* part_o, float* part_ml, const ClusterOut& direct, cudaStream_t st);
 int run_sample(const void* logits, int dtype, int batch, int vocab, int64_t row_stride, float temperature, int top_k,
                int do_sample, uint64_t seed, uint64_t step, int64_t* ids, cudaStream_t st);
 int run_merge_token_shards(const float* parts, int n_shards, int64_t rows, int D, void* out, int out_dtype,
@@ -150,6 +152,13 @@ extern "C" size_t kivi_decode_attention_workspace(int num_units, int n_rep, int 
     if (num_splits <= 0 || num_splits > kMaxSplitsC) num_splits = kMaxSplitsC;
     return (size_t)num_units * (num_splits + 8) * n_rep * (head_dim + 2) * sizeof(float);
 }
+
+// Up to this many CTAs, and eight pieces a row, the fold runs inside clusters of the
+// attention kernel.
+#ifndef KIVI_FUSED_MAX
+#define KIVI_FUSED_MAX 148
+#endif
+constexpr int64_t kFusedMaxCtas = KIVI_FUSED_MAX;
 
 static int clamp_splits(int64_t s, int64_t n_groups) {
     if (s > kMaxSplitsC) s = kMaxSplitsC;
@@ -331,10 +340,15 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
     const float scale_log2 = sm_scale * 1.4426950408889634f;
     cudaStream_t st = (cudaStream_t)stream;
 
+    const int64_t ctas = (int64_t)L->num_units * (use_mma ? (n_rep + 3) / 4 : 1) * n_splits;
+    ClusterOut direct{nullptr, out_dtype, lse};
+    if (!gather && n_splits <= kClusterFoldMax && ctas <= kFusedMaxCtas && (use_mma || attn_fp32_tile_ok(L))) direct.out = out;
+
     int rc = use_mma
-        ? run_attn_mma(L, quant_len, res_start, res_len, q, q_dtype, n_rep, scale_log2, nq_splits, gps, n_res_splits, res_chunk, part_o, part_ml, st)
-        : run_attn_fp32(L, quant_len, res_start, res_len, q, q_dtype, n_rep, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, st);
+        ? run_attn_mma(L, quant_len, res_start, res_len, q, q_dtype, n_rep, scale_log2, nq_splits, gps, n_res_splits, res_chunk, part_o, part_ml, direct, st)
+        : run_attn_fp32(L, quant_len, res_start, res_len, q, q_dtype, n_rep, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, direct, st);
     if (rc) return rc;
+    if (direct.out) { note_launches(1); return KIVI_OK; }
     if (int rc2 = run_merge(part_o, part_ml, out, gather, lse, out_dtype, L->num_units, n_rep, n_splits, D, st)) return rc2;
     note_launches(2);
     return KIVI_OK;

@@ -66,19 +66,33 @@ __device__ __forceinline__ void settle_layer(kivi_layer& L) {
 
 // Launch on `st`; with `overlap` as a programmatic dependent of the kernel before it.
 // Only for kernels that either do not depend on that one or wait for it themselves.
+// cluster > 0: clusters of that many blocks along x.
 template <typename... P, typename... A>
-cudaError_t launch(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, bool overlap, A... args) {
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+cudaError_t launch_cluster(void (*kernel)(P...), int cluster, dim3 grid, unsigned block, size_t smem, cudaStream_t st, bool overlap, A... args) {
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (overlap) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 0) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = (unsigned)cluster;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = attr;
-    cfg.numAttrs = overlap ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+template <typename... P, typename... A>
+cudaError_t launch(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, bool overlap, A... args) {
+    return launch_cluster(kernel, 0, grid, block, smem, st, overlap, args...);
 }
 #endif
 
@@ -206,6 +220,27 @@ __device__ __forceinline__ float load_as_float(const void* p, int dtype, int64_t
 __device__ __forceinline__ void store_from_float(void* p, int dtype, int64_t i, float v) {
     if (dtype == KIVI_BF16) reinterpret_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16_rn(v);
     else reinterpret_cast<float*>(p)[i] = v;
+}
+
+// four consecutive output elements starting at element i (i % 4 == 0): one 8- or
+// 16-byte store when the buffer allows it
+__device__ __forceinline__ void store_quad(void* p, int dtype, int64_t i, float4 v) {
+    if (dtype == KIVI_BF16) {
+        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p) + i;
+        if ((reinterpret_cast<uintptr_t>(o) & 7u) == 0) {
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+            uint2 w;
+            w.x = *reinterpret_cast<const uint32_t*>(&lo); w.y = *reinterpret_cast<const uint32_t*>(&hi);
+            *reinterpret_cast<uint2*>(o) = w;
+        } else {
+            o[0] = __float2bfloat16_rn(v.x); o[1] = __float2bfloat16_rn(v.y);
+            o[2] = __float2bfloat16_rn(v.z); o[3] = __float2bfloat16_rn(v.w);
+        }
+    } else {
+        float* o = reinterpret_cast<float*>(p) + i;
+        if ((reinterpret_cast<uintptr_t>(o) & 15u) == 0) *reinterpret_cast<float4*>(o) = v;
+        else { o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
+    }
 }
 
 // ---- groups kept in registers as loaded -----------------------------------------
