@@ -289,17 +289,37 @@ class LayerStore:
         need = lib.kivi_decode_attention_workspace(self.num_units, n_rep, self.D, num_splits)
         self._ws_for = (n_rep, num_splits)
         if self._ws is None or self._ws.numel() < need:
-            self._ws = torch.empty(need, dtype=torch.uint8, device=self.device)
+            self._ws = torch.empty(need, dtype=torch.uint8, device=self.k_codes.device)
         return self._ws
 
+    def _operands(self, q, n_rep, out=None, like_q=True):
+        """Refuse, before anything is launched, operands the kernels would read or
+        write out of range: they take raw pointers.  q holds one row per (unit, head);
+        like_q: the call allocates an output of q's shape, so q holds nothing else.
+        (Head counts the library does not take are left to the library's own message.)"""
+        _dev(self.k_codes, q)
+        if not 1 <= n_rep <= 8:
+            return
+        need = self.num_units * n_rep * self.D
+        if q.numel() < need or (like_q and q.numel() != need):
+            raise RuntimeError(f"q holds {q.numel()} elements, the cache needs {need}")
+        if out is not None:
+            if out.device != q.device and (out.is_cuda or not out.is_pinned()):
+                raise RuntimeError("out must be on the device of q or in pinned host memory")
+            if not out.is_contiguous():
+                raise RuntimeError("tensor must be contiguous")
+            if out.numel() < need:
+                raise RuntimeError(f"out holds {out.numel()} elements, the cache needs {need}")
+
     def attention(self, q, out=None, n_rep=None, sm_scale=0.0, num_splits=0, path=ATTN_AUTO, out_dtype=None):
-        """q: [num_units, n_rep, D] (or anything contiguous with that many elements)."""
+        """q: [num_units, n_rep, D] (or anything contiguous with that many elements); out,
+        if given, holds at least as many, on q's device or in pinned host memory."""
         n_rep = n_rep or q.numel() // (self.num_units * self.D)
         ops = _native_ops()
         if ops is not None and out_dtype in _OUT_DTYPES:
             return ops.cache_attention(_c.addressof(self.c), self.quant_len, self.res_start, self.res_len, q, out,
                                        self.workspace(n_rep, num_splits), n_rep, sm_scale, num_splits, path, _OUT_DTYPES[out_dtype])
-        _dev(q)
+        self._operands(q, n_rep, out, like_q=out is None)
         if out is None:
             out = torch.empty(q.shape, dtype=out_dtype or q.dtype, device=q.device)
         ws = self.workspace(n_rep, num_splits)
@@ -313,8 +333,8 @@ class LayerStore:
         returns (out [like q], lse [num_units, n_rep] fp32).  use_ring=False
         attends to the quantized store only (a rank of a sequence-sharded cache
         that leaves the replicated ring to another rank)."""
-        _dev(q)
         n_rep = n_rep or q.numel() // (self.num_units * self.D)
+        self._operands(q, n_rep)
         out = torch.empty(q.shape, dtype=out_dtype or q.dtype, device=q.device)
         lse = torch.empty(self.num_units, n_rep, dtype=torch.float32, device=q.device)
         ws = self.workspace(n_rep, num_splits)
@@ -326,7 +346,7 @@ class LayerStore:
     def attention_gather(self, q, desc: "PeerGatherDesc", out_dtype, n_rep, sm_scale=0.0, num_splits=0, path=ATTN_AUTO):
         """kivi_decode_attention_gather: the output rows of this store's units go
         straight into every rank's gathered buffer (see parallel.PeerGather)."""
-        _dev(q)
+        self._operands(q, n_rep, like_q=False)
         ws = self.workspace(n_rep, num_splits)
         odt = F32 if out_dtype == torch.float32 else BF16
         _check(lib.kivi_decode_attention_gather(_c.byref(self.c), self.quant_len, self.res_start, self.res_len,
@@ -368,6 +388,7 @@ class LayerStore:
         workspace tensor.  `out` must be preallocated by the caller: nothing is
         allocated on this path."""
         _dev(q, out)
+        self._operands(q, n_rep, out, like_q=False)
         _check(lib.kivi_decode_attention_noalloc(_c.byref(self.c), self.quant_len, self.res_start, self.res_len,
                                                  q.data_ptr(), _dt(q), out.data_ptr(), _dt(out), n_rep,
                                                  float(sm_scale), num_splits, path, _stream()))

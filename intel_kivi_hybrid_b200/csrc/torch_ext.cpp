@@ -291,6 +291,21 @@ torch::Tensor cache_attention(int64_t layer, int64_t quant_len, int res_start, i
     auto fail = [](const std::string& what) { throw std::runtime_error(what); };
     if (!q.is_cuda()) fail("tensor must be on a CUDA device");
     if (!q.is_contiguous()) fail("tensor must be contiguous");
+    if (workspace.device() != q.device())
+        fail("all tensors of one call must be on the same device, got " + workspace.device().str() + " and " + q.device().str());
+    const kivi_layer* L = reinterpret_cast<const kivi_layer*>(layer);
+    // the kernels take raw pointers: what is too short is refused here (a head count the
+    // library does not take is left to its own message)
+    if (n_rep >= 1 && n_rep <= 8) {
+        const int64_t need = (int64_t)L->num_units * n_rep * L->head_dim;
+        if (out.has_value() ? q.numel() < need : q.numel() != need)
+            fail("q holds " + std::to_string(q.numel()) + " elements, the cache needs " + std::to_string(need));
+        if (out.has_value()) {
+            if (out->device() != q.device() && (out->is_cuda() || !out->is_pinned())) fail("out must be on the device of q or in pinned host memory");
+            if (!out->is_contiguous()) fail("tensor must be contiguous");
+            if (out->numel() < need) fail("out holds " + std::to_string(out->numel()) + " elements, the cache needs " + std::to_string(need));
+        }
+    }
     auto code = [&](const torch::Tensor& t) {
         if (t.scalar_type() == torch::kFloat32) return KIVI_F32;
         if (t.scalar_type() != torch::kBFloat16)
@@ -302,7 +317,7 @@ torch::Tensor cache_attention(int64_t layer, int64_t quant_len, int res_start, i
     c10::cuda::CUDAGuard guard(q.device());
     const torch::Tensor o = out.has_value() ? *out
                                             : at::empty(q.sizes(), q.options().dtype(out_dtype < 0 ? q.scalar_type() : out_dtype == KIVI_F32 ? torch::kFloat32 : torch::kBFloat16));
-    const int rc = kivi_decode_attention(reinterpret_cast<const kivi_layer*>(layer), quant_len, res_start, res_len, q.data_ptr(), q_dtype, o.data_ptr(),
+    const int rc = kivi_decode_attention(L, quant_len, res_start, res_len, q.data_ptr(), q_dtype, o.data_ptr(),
                                          code(o), n_rep, (float)sm_scale, workspace.data_ptr(), (size_t)workspace.numel(), num_splits, path,
                                          at::cuda::getCurrentCUDAStream().stream());
     if (rc != KIVI_OK) fail("kivi_cuda error " + std::to_string(rc) + ": " + kivi_last_error());

@@ -389,3 +389,45 @@ def test_native_attention_call_equals_the_ctypes_call(monkeypatch, dtype, D, n_r
     for a, b in zip(native[0], general[0]):
         assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(a, b)
     assert native[1] == general[1]
+
+
+def test_attention_refuses_operands_the_kernels_would_overrun(monkeypatch):
+    """The kernels take raw pointers: a q or an out too short for the cache, an out in
+    pageable host memory or with gaps are refused before the launch, by the extension
+    and by the ctypes binding alike; what fits (a longer buffer, pinned host memory) works."""
+    from intel_kivi_hybrid_b200 import cabi
+    from kivi_sycl import KiviCache
+    U, n_rep, D = 6, 4, 128
+    st = cabi.LayerStore(U, D, 32, 128, 512, torch.bfloat16, "cuda")
+    k, v = (torch.randn(U, 333, D, device="cuda").bfloat16() for _ in range(2))
+    st.update(k, v)
+    q = torch.randn(U, n_rep, D, device="cuda").bfloat16()
+    out = torch.empty(U, n_rep, D, device="cuda")
+    cache = KiviCache(num_layers=1, head_dim=D, device=DEV)
+    cache.add_tokens(((k.view(2, 3, 333, D), v.view(2, 3, 333, D)),))
+    assert cabi._native_ops() is not None
+    messages = []
+    for native in (True, False):
+        if not native:
+            monkeypatch.setattr(cabi, "_ops", False)
+        want = st.attention(q, out_dtype=torch.float32)
+        longer = torch.empty(U * n_rep * D + 64, device="cuda")
+        pinned = torch.empty(U, n_rep, D).pin_memory()
+        st.attention(q, out=longer, n_rep=n_rep)
+        st.attention(torch.cat([q, q[:1]]), out=out, n_rep=n_rep)
+        st.attention(q, out=pinned)
+        torch.cuda.synchronize()
+        assert torch.equal(longer[:want.numel()].view_as(want), want) and torch.equal(out, want) and torch.equal(pinned, want.cpu())
+        for bad in (lambda: st.attention(q[:5], n_rep=n_rep), lambda: st.attention(torch.cat([q, q[:1]]), n_rep=n_rep),
+                    lambda: st.attention(q[:5], out=out, n_rep=n_rep), lambda: st.attention(q, out=out[:5]),
+                    lambda: st.attention(q, out=torch.empty(U, n_rep, 2 * D, device="cuda")[..., ::2]), lambda: st.attention(q, out=out.cpu()),
+                    lambda: cache.decode_attention(0, torch.zeros(2, 12, 64, device="cuda").bfloat16()),
+                    lambda: cache.decode_attention(0, torch.zeros(2, 12, 256, device="cuda").bfloat16()),
+                    lambda: st.attention_lse(q[:5], n_rep=n_rep), lambda: st.attention_noalloc(q, out[:5], n_rep),
+                    lambda: st.attention_gather(q[:5], None, torch.float32, n_rep)):
+            with pytest.raises(RuntimeError) as e:
+                bad()
+            messages.append(str(e.value))
+    half = len(messages) // 2
+    assert messages[:half] == messages[half:]
+    assert all("elements" in m or "contiguous" in m or "pinned" in m for m in messages)
