@@ -997,20 +997,28 @@ bool attn_fp32_tile_ok(const kivi_layer* L) {
            al(L->k_zeros) && al(L->v_codes) && al(L->v_scales) && al(L->v_zeros);
 }
 
+// Bytes of one stage (one group of a warp): two stages of a warp also hold its [NREP][D] outputs.
+template <int NREP, int D> constexpr int tile_stage_bytes(int group_size) {
+    const int stage = 2 * (D * group_size / 4) + 4 * D * 4;
+    return stage < NREP * D * 2 ? NREP * D * 2 : stage;
+}
+template <int NREP, int D> constexpr int tile_smem_bytes(int group_size) {
+    return kWarps * 2 * tile_stage_bytes<NREP, D>(group_size) + 4 * (NREP * D + kWarps * 32 * NREP) + 8 * kWarps * 2 + 4 * kWarps * NREP * 2;
+}
+
 template <int NREP, int D>
 static int launch_tile(const kivi_layer* L, int64_t quant_len, int res_start, int res_len, const void* q, int q_dtype, float scale_log2,
                        int nq_splits, int gps, int n_splits, float* part_o, float* part_ml, const ClusterOut& direct, cudaStream_t st) {
-    static std::atomic<int> smem_set[64];
-    // two stages of one group per warp, and never less than the warp's [NREP][D] output buffer
-    int stage = 2 * (D * L->group_size / 4) + 4 * D * 4;
-    if (stage < NREP * D * 2) stage = NREP * D * 2;
-    const int smem = kWarps * 2 * stage + 4 * (NREP * D + kWarps * 32 * NREP) + 8 * kWarps * 2 + 4 * kWarps * NREP * 2;
+    // The limit is set once per device to what the largest group (G = D) takes: threads
+    // that come here together with different group sizes all write the same value.
+    static std::atomic<bool> limit_set[64];
+    const int stage = tile_stage_bytes<NREP, D>(L->group_size), smem = tile_smem_bytes<NREP, D>(L->group_size);
     int dev = 0;
     KIVI_CUDA_OK(cudaGetDevice(&dev));
     KIVI_REQUIRE(dev >= 0 && dev < 64, "device ordinal %d out of range", dev);
-    if (smem > 48 * 1024 && smem_set[dev].load(std::memory_order_acquire) < smem) {
-        KIVI_CUDA_OK(cudaFuncSetAttribute(attn_fp32_tile_kernel<NREP, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        smem_set[dev].store(smem, std::memory_order_release);
+    if (smem > 48 * 1024 && !limit_set[dev].load(std::memory_order_acquire)) {
+        KIVI_CUDA_OK(cudaFuncSetAttribute(attn_fp32_tile_kernel<NREP, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_bytes<NREP, D>(D)));
+        limit_set[dev].store(true, std::memory_order_release);
     }
     dim3 grid((unsigned)n_splits, (unsigned)L->num_units);
     KIVI_CUDA_OK(launch_cluster(attn_fp32_tile_kernel<NREP, D>, direct.out ? n_splits : 0, grid, kWarps * 32, (size_t)smem, st, true, *L, quant_len, res_start, res_len, q, q_dtype, scale_log2,

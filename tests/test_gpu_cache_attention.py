@@ -7,6 +7,8 @@ max|out-ref| / max|ref| (`rel_err`).  The tests also print the element-wise
 figure max |out-ref| / max(|ref|, 1e-3 * max|ref| of the row) (`elem_err`),
 which weighs the same absolute error against each element's own magnitude."""
 import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -607,3 +609,63 @@ def test_attention_fp32_kernels_at_their_edges(cabi, D, G, n_rep, n_quant, n_res
         out = st.attention(q, n_rep=n_rep, path=cabi.ATTN_FP32, out_dtype=torch.float32, num_splits=splits)
         err = ((out.double() - ref).abs().amax(-1) / ref.abs().amax(-1)).max().item()
         assert err < 1e-5, (splits, err)
+
+
+_TWO_THREADS_CPP = r"""
+#include <atomic>
+#include <thread>
+#include "kivi_cuda.h"
+extern "C" void together(const kivi_layer* const* layers, const void* q, void* const* outs, void* const* ws, size_t ws_bytes, int64_t tokens,
+                         int n_rep, int* rc) {
+    std::atomic<int> ready{0};
+    auto work = [&](int i) {
+        ready.fetch_add(1);
+        while (ready.load() < 2) {}
+        rc[i] = kivi_decode_attention(layers[i], tokens, 0, 0, q, KIVI_F32, outs[i], KIVI_F32, n_rep, 0.0f, ws[i], ws_bytes, 0, KIVI_ATTN_FP32, nullptr);
+    };
+    std::thread a(work, 0), b(work, 1);
+    a.join(); b.join();
+}
+"""
+_TWO_THREADS = r"""
+import ctypes, sys, torch
+sys.path.insert(0, sys.argv[1])
+from intel_kivi_hybrid_b200 import cabi
+together = ctypes.CDLL(sys.argv[2]).together
+D, T, U, failed = 128, 256, 2, []
+stores = [cabi.LayerStore(U, D, G, 128, T, torch.float32, "cuda") for G in (128, 64)]
+for st in stores:
+    cabi.load_state(st, torch.randn(U, T, D, device="cuda"), torch.randn(U, T, D, device="cuda"), T)
+torch.cuda.synchronize()
+vp = ctypes.c_void_p
+for n_rep in range(1, 9):                       # each head count is a kernel of its own, met here for the first time
+    q = torch.randn(U, n_rep, D, device="cuda")
+    outs, ws, rc = [torch.empty_like(q) for _ in stores], [st.workspace(n_rep) for st in stores], (ctypes.c_int * 2)()
+    torch.cuda.synchronize()
+    two = lambda p: (vp * 2)(*p)
+    together(two([ctypes.addressof(st.c) for st in stores]), vp(q.data_ptr()), two([o.data_ptr() for o in outs]), two([w.data_ptr() for w in ws]),
+             ctypes.c_size_t(ws[0].numel()), ctypes.c_int64(T), n_rep, rc)
+    failed += [(n_rep, st.G, "together") for st, c in zip(stores, rc) if c]
+    for st in stores:
+        try:
+            st.attention(q, n_rep=n_rep)
+        except RuntimeError as e:
+            failed.append((n_rep, st.G, str(e)))
+torch.cuda.synchronize()
+print("failed:", failed)
+sys.exit(1 if failed else 0)
+"""
+
+
+def test_first_fp32_attention_calls_from_two_threads(tmp_path):
+    """Groups of 64 and of 128 tokens need different amounts of shared memory of the same
+    kernel: two host threads that launch it for the first time together must not leave it
+    with the smaller limit.  A process of its own: a kernel is met for the first time once."""
+    from intel_kivi_hybrid_b200 import _build
+    (tmp_path / "two.cpp").write_text(_TWO_THREADS_CPP)
+    (tmp_path / "two.py").write_text(_TWO_THREADS)
+    lib = str(tmp_path / "two.so")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-pthread", "-I" + os.path.join(_build.ROOT, "include"), str(tmp_path / "two.cpp"),
+                    "-o", lib, "-L" + _build.PKG, "-l:libkivi_cuda.so", "-Wl,-rpath," + _build.PKG], check=True)
+    p = subprocess.run([sys.executable, str(tmp_path / "two.py"), _build.ROOT, lib], capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stdout + p.stderr
