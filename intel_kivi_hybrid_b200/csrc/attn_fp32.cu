@@ -991,9 +991,10 @@ int run_merge_token_shards(const float* parts, int n_shards, int64_t rows, int D
 // The tile kernel takes head_dim 64 and 128 with 16-byte aligned arrays and groups of
 // whole 16-byte pieces (any group size: D*G/4 bytes of codes are a multiple of 16);
 // everything else -- other head_dims, odd alignments -- takes the generic kernel.
+bool attn_fp32_tile_head_dim(int head_dim) { return head_dim == 64 || head_dim == 128; }
 bool attn_fp32_tile_ok(const kivi_layer* L) {
     auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
-    return (L->head_dim == 64 || L->head_dim == 128) && al(L->k_res) && al(L->v_res) && al(L->k_codes) && al(L->k_scales) &&
+    return attn_fp32_tile_head_dim(L->head_dim) && al(L->k_res) && al(L->v_res) && al(L->k_codes) && al(L->k_scales) &&
            al(L->k_zeros) && al(L->v_codes) && al(L->v_scales) && al(L->v_zeros);
 }
 

@@ -48,6 +48,7 @@ int run_attn_fp32(const kivi_layer* L, int64_t quant_len, int res_start, int res
                   const void* q, int q_dtype, int n_rep, float scale_log2, int nq_splits, int gps,
                   int n_splits, float* part_o, float* part_ml, const ClusterOut& direct, cudaStream_t st);
 bool attn_fp32_tile_ok(const kivi_layer* L);
+bool attn_fp32_tile_head_dim(int head_dim);
 bool attn_mma_supported(const kivi_layer* L, int n_rep, const void* q);
 void attn_mma_residual_plan(int res_len, int* n_res_splits, int* res_chunk);
 int attn_mma_ctas_per_sm();
@@ -167,33 +168,31 @@ static int clamp_splits(int64_t s, int64_t n_groups) {
     return (int)s;
 }
 
-// CUDA-core kernels.  The generic one (head_dim other than 64 and 128): ~8 CTAs of
-// 128 threads per SM, never below 4 token groups per CTA.  The tile kernel is bound by
-// the FMA pipe, so what counts is how evenly whole rounds (one group per warp, four
-// per CTA) spread over the SMs: a round costs c_round of SM time (fitted on B200:
-// 1.0 / 1.9 / 3.3 us with 1 / 4 / 8 heads at head_dim 128, groups of 32), and a CTA
-// alone on its SM takes about 1.2 us longer per round than its share.  32 units x 8k
-// tokens, four heads: 8 pieces 35.9 us, 37 (the generic rule) 39.3; 192 units x 1k,
-// head_dim 64: 2 pieces 14.3, 7 pieces 16.1.
-static int plan_splits_fp32(int num_units, int64_t n_groups, int requested, int head_dim, int group_size, int n_rep, int n_res, int sms) {
-    if (n_groups <= 0) return 0;
-    if (requested > 0) return clamp_splits(requested, n_groups);
-    const int n_sms = sms > 0 ? sms : 148;
-    if (head_dim != 64 && head_dim != 128) {
-        const int64_t target = (int64_t)n_sms * 8;
-        int64_t s = (target + num_units - 1) / num_units;
-        const int64_t cap = (n_groups + 3) / 4;
-        if (s > cap) s = cap;
-        return clamp_splits(s, n_groups);
-    }
+// Generic CUDA-core kernel (head_dim other than 64 and 128, arrays off the 16-byte
+// grid): ~8 CTAs of 128 threads per SM, never below 4 token groups per CTA.
+static int plan_splits_generic(int num_units, int64_t n_groups, int sms) {
+    const int64_t target = (int64_t)sms * 8;
+    int64_t s = (target + num_units - 1) / num_units;
+    const int64_t cap = (n_groups + 3) / 4;
+    if (s > cap) s = cap;
+    return clamp_splits(s, n_groups);
+}
+
+// The tile kernel is bound by the FMA pipe, so what counts is how evenly whole rounds
+// (one group per warp, four per CTA) spread over the SMs: a round costs c_round of SM
+// time (fitted on B200: 1.0 / 1.9 / 3.3 us with 1 / 4 / 8 heads at head_dim 128,
+// groups of 32), and a CTA alone on its SM takes about 1.2 us longer per round than its
+// share.  32 units x 8k tokens, four heads: 8 pieces 35.9 us, 37 (the generic rule)
+// 39.3; 192 units x 1k, head_dim 64: 2 pieces 14.3, 7 pieces 16.1.
+static int plan_splits_tile(int num_units, int64_t n_groups, int head_dim, int group_size, int n_rep, int n_res, int sms) {
     const double c_round = (0.7 + 0.32 * n_rep) * head_dim / 128.0 * group_size / 32.0, c_alone = 1.2, c_cta = 0.3;
     int best = 1;
     double best_t = 0.0;
     for (int s = 1; s <= kMaxSplitsC && s <= n_groups; ++s) {
         const int64_t per_cta = (n_groups + s - 1) / s;
         const double rounds = (double)((per_cta + 3) / 4);
-        const double per_sm = (double)(((int64_t)num_units * s + n_sms - 1) / n_sms);
-        const double shared = per_sm * (rounds * c_round + c_cta) + (double)num_units * n_res * c_round / n_sms, alone = rounds * (c_round + c_alone);
+        const double per_sm = (double)(((int64_t)num_units * s + sms - 1) / sms);
+        const double shared = per_sm * (rounds * c_round + c_cta) + (double)num_units * n_res * c_round / sms, alone = rounds * (c_round + c_alone);
         const double t = (shared > alone ? shared : alone) + (s <= 16 ? 0.1 * s : 1.0 + 0.02 * s);
         if (s == 1 || t < best_t - 1e-9) { best = s; best_t = t; }
     }
@@ -223,10 +222,8 @@ static int plan_splits_fp32(int num_units, int64_t n_groups, int requested, int 
 // 9.7 us, 4 pieces 10.7), and at the two-CTA count the ring CTAs must fit beside the
 // quantized ones (256 units x 4k with 256 + 256 CTAs: 49.6 us in one piece, 45.3 in
 // two, 44.0 in three; 192 units x 2k: one piece 24.3 us, three 26.3).
-static int plan_splits_mma(int num_units, int64_t n_groups, int requested, int n_res_splits, int sms, int ctas_per_sm) {
-    if (n_groups <= 0) return 0;
-    if (requested > 0) return clamp_splits(requested, n_groups);
-    const int n_sms = sms > 0 ? sms : 148, per_sm = ctas_per_sm > 0 ? ctas_per_sm : 3;
+static int plan_splits_mma(int num_units, int64_t n_groups, int n_res_splits, int n_sms, int ctas_per_sm) {
+    const int per_sm = ctas_per_sm > 0 ? ctas_per_sm : 3;
     const double slots = (double)per_sm * n_sms;
     const double c0 = 6.0, c0_waves = 7.5, c1_one = 0.16, c1_two = 0.24, c1_crowded = 0.31, c1_three = 0.33, c1_full = 0.36;
     const double t_ring = 7.0, c_start = 0.015, ragged = 0.3;
@@ -257,17 +254,24 @@ static int plan_splits_mma(int num_units, int64_t n_groups, int requested, int n
     return best;
 }
 
-// The piece count of either kernel.  The models above walk up to 128 candidates (1-2 us);
+// The piece count of a kernel.  The models above walk up to 128 candidates (1-2 us);
 // a decode loop asks for the same shape again and again, so each thread remembers
 // its last question -- the answer depends on nothing else.
-static int plan_splits(bool mma, int num_units, int64_t n_groups, int requested, int head_dim, int group_size, int n_rep, int n_res,
+enum class AttnKernel { kGeneric, kTile, kMma };
+static int plan_splits(AttnKernel kernel, int num_units, int64_t n_groups, int requested, int head_dim, int group_size, int n_rep, int n_res,
                        int sms, int ctas_per_sm) {
-    const int64_t key[10] = {mma, num_units, n_groups, requested, head_dim, group_size, n_rep, n_res, sms, ctas_per_sm};
-    static thread_local int64_t last_key[10];
+    if (n_groups <= 0) return 0;
+    if (requested > 0) return clamp_splits(requested, n_groups);
+    if (sms <= 0) sms = 148;
+    const int64_t key[9] = {(int64_t)kernel, num_units, n_groups, head_dim, group_size, n_rep, n_res, sms, ctas_per_sm};
+    static thread_local int64_t last_key[9];
     static thread_local int last = -1;
     if (last >= 0 && memcmp(key, last_key, sizeof(key)) == 0) return last;
-    last = mma ? plan_splits_mma(num_units * ((n_rep + 3) / 4), n_groups, requested, n_res, sms, ctas_per_sm)
-               : plan_splits_fp32(num_units, n_groups, requested, head_dim, group_size, n_rep, n_res, sms);
+    switch (kernel) {
+        case AttnKernel::kMma: last = plan_splits_mma(num_units * ((n_rep + 3) / 4), n_groups, n_res, sms, ctas_per_sm); break;
+        case AttnKernel::kTile: last = plan_splits_tile(num_units, n_groups, head_dim, group_size, n_rep, n_res, sms); break;
+        case AttnKernel::kGeneric: last = plan_splits_generic(num_units, n_groups, sms); break;
+    }
     memcpy(last_key, key, sizeof(key));
     return last;
 }
@@ -291,7 +295,9 @@ extern "C" int kivi_decode_attention_plan(int num_units, int64_t quant_len, int 
     if (sms <= 0) sms = num_sms();
     if (ctas_per_sm <= 0) ctas_per_sm = attn_mma_ctas_per_sm();
     *tensor_cores_out = use_mma ? 1 : 0;
-    *quant_splits_out = plan_splits(use_mma, num_units, n_groups, num_splits, head_dim, group_size, n_rep, n_res, sms, ctas_per_sm);
+    // (arrays on the 16-byte grid, as every allocator places them)
+    const AttnKernel kernel = use_mma ? AttnKernel::kMma : attn_fp32_tile_head_dim(head_dim) ? AttnKernel::kTile : AttnKernel::kGeneric;
+    *quant_splits_out = plan_splits(kernel, num_units, n_groups, num_splits, head_dim, group_size, n_rep, n_res, sms, ctas_per_sm);
     *residual_parts_out = n_res;
     return KIVI_OK;
 }
@@ -327,7 +333,8 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
     }
     int n_res_splits = res_len > 0 ? 1 : 0, res_chunk = res_len;
     if (use_mma) attn_mma_residual_plan(res_len, &n_res_splits, &res_chunk);
-    const int nq_splits = plan_splits(use_mma, L->num_units, n_groups, num_splits, D, G, n_rep, n_res_splits, num_sms(), use_mma ? attn_mma_ctas_per_sm() : 0);
+    const AttnKernel kernel = use_mma ? AttnKernel::kMma : attn_fp32_tile_ok(L) ? AttnKernel::kTile : AttnKernel::kGeneric;
+    const int nq_splits = plan_splits(kernel, L->num_units, n_groups, num_splits, D, G, n_rep, n_res_splits, num_sms(), use_mma ? attn_mma_ctas_per_sm() : 0);
     const int gps = nq_splits > 0 ? (int)((n_groups + nq_splits - 1) / nq_splits) : 0;
     const int n_splits = nq_splits + n_res_splits;
     const size_t need = (size_t)L->num_units * n_splits * n_rep * (D + 2) * sizeof(float);
@@ -342,7 +349,7 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
 
     const int64_t ctas = (int64_t)L->num_units * (use_mma ? (n_rep + 3) / 4 : 1) * n_splits;
     ClusterOut direct{nullptr, out_dtype, lse};
-    if (!gather && n_splits <= kClusterFoldMax && ctas <= kFusedMaxCtas && (use_mma || attn_fp32_tile_ok(L))) direct.out = out;
+    if (!gather && n_splits <= kClusterFoldMax && ctas <= kFusedMaxCtas && kernel != AttnKernel::kGeneric) direct.out = out;
 
     int rc = use_mma
         ? run_attn_mma(L, quant_len, res_start, res_len, q, q_dtype, n_rep, scale_log2, nq_splits, gps, n_res_splits, res_chunk, part_o, part_ml, direct, st)

@@ -307,3 +307,33 @@ def test_token_shard_plan_gives_every_group_to_one_rank():
         for g in range(40):                                           # single groups: exactly one owner
             assert sum(p.owns(g) for p in plans) == 1
         assert sum(p.serves_ring for p in plans) == 1
+
+
+def _partials_needed(D, G, n_rep, U, T, shift, workspace_bytes=16, num_splits=0):
+    """Bytes of partials kivi_decode_attention asks for, read from its refusal: the
+    workspace handed over is too small, or misaligned (None then), so that nothing is
+    launched on the addresses made up here.  shift: offset of one array from the 16-byte grid."""
+    from intel_kivi_hybrid_b200 import cabi
+    p = 0x10000
+    layer = cabi.Layer(U, D, G, 128, T, cabi.F32, 0, p, p + shift, p, p, p, p, p, p)
+    rc = cabi.lib.kivi_decode_attention(ctypes.byref(layer), T, 0, 96, p, cabi.F32, p, cabi.F32, n_rep, 0.0, 0x10008, workspace_bytes,
+                                        num_splits, cabi.ATTN_FP32, None)
+    said = cabi.lib.kivi_last_error().decode()
+    assert rc == 1, said
+    if "aligned" in said:
+        return None
+    return int(re.search(r"(\d+) needed", said).group(1))
+
+
+@pytest.mark.parametrize("D,n_rep,U,T", [(64, 1, 192, 1024), (128, 4, 32, 8192), (128, 1, 12, 512)])
+def test_unaligned_arrays_get_the_plan_of_the_kernel_that_serves_them(D, n_rep, U, T):
+    """Arrays off the 16-byte grid go to the generic kernel, whose rule is about eight
+    CTAs per SM and at least four groups per CTA, not the tile kernel's."""
+    from intel_kivi_hybrid_b200 import cabi
+    if torch.cuda.is_available() and torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("counts below are for 148 SMs")
+    row = U * n_rep * (D + 2) * 4
+    generic = min(-(-8 * 148 // U), -(-(T // 32) // 4), 128)
+    assert _partials_needed(D, 32, n_rep, U, T, shift=4) == (generic + 1) * row
+    tile = cabi.attention_plan(U, T, 96, head_dim=D, n_rep=n_rep, q_dtype=cabi.F32, sms=148)[1]
+    assert _partials_needed(D, 32, n_rep, U, T, shift=0) == (tile + 1) * row
