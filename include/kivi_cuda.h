@@ -250,7 +250,9 @@ int kivi_merge_token_shards(const float* parts, int n_shards, int64_t rows, int 
  * Limit: num_units * (splits + residual parts) * n_rep * (head_dim + 2) * 4
  * bytes must fit in the array; a larger problem is refused with
  * KIVI_ERR_INVALID_ARGUMENT and a message naming the limit (pass a smaller
- * num_splits, or use kivi_decode_attention with your own workspace).
+ * num_splits, or use kivi_decode_attention with your own workspace).  With
+ * num_splits = 0 a cut too fine for the array gives way to a coarser one (about
+ * eight CTAs per SM) before the call is refused.
  * The first call on each device looks up the array's device address (no
  * allocation, but make that first call before starting a stream capture).
  * All calls on a device share the one array and nothing in it needs to start

@@ -334,10 +334,18 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
     int n_res_splits = res_len > 0 ? 1 : 0, res_chunk = res_len;
     if (use_mma) attn_mma_residual_plan(res_len, &n_res_splits, &res_chunk);
     const AttnKernel kernel = use_mma ? AttnKernel::kMma : attn_fp32_tile_ok(L) ? AttnKernel::kTile : AttnKernel::kGeneric;
-    const int nq_splits = plan_splits(kernel, L->num_units, n_groups, num_splits, D, G, n_rep, n_res_splits, num_sms(), use_mma ? attn_mma_ctas_per_sm() : 0);
+    int nq_splits = plan_splits(kernel, L->num_units, n_groups, num_splits, D, G, n_rep, n_res_splits, num_sms(), use_mma ? attn_mma_ctas_per_sm() : 0);
+    const auto partial_bytes = [&](int pieces) { return (size_t)L->num_units * (pieces + n_res_splits) * n_rep * (D + 2) * sizeof(float); };
+    // The tile kernel's plan cuts large problems finer than the generic rule (300 units x
+    // 8k tokens: 16 pieces against 4): where its partials do not fit the scratch but the
+    // coarser cut's do, that one is taken.
+    if (num_splits == 0 && kernel == AttnKernel::kTile && partial_bytes(nq_splits) > workspace_bytes) {
+        const int coarse = plan_splits(AttnKernel::kGeneric, L->num_units, n_groups, 0, D, G, n_rep, n_res_splits, num_sms(), 0);
+        if (partial_bytes(coarse) <= workspace_bytes) nq_splits = coarse;
+    }
     const int gps = nq_splits > 0 ? (int)((n_groups + nq_splits - 1) / nq_splits) : 0;
     const int n_splits = nq_splits + n_res_splits;
-    const size_t need = (size_t)L->num_units * n_splits * n_rep * (D + 2) * sizeof(float);
+    const size_t need = partial_bytes(nq_splits);
     KIVI_REQUIRE(workspace != nullptr && workspace_bytes >= need,
                  "workspace too small: %zu bytes given, %zu needed", workspace_bytes, need);
     KIVI_REQUIRE((reinterpret_cast<uintptr_t>(workspace) & 15u) == 0, "workspace must be 16-byte aligned");

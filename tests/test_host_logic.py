@@ -337,3 +337,21 @@ def test_unaligned_arrays_get_the_plan_of_the_kernel_that_serves_them(D, n_rep, 
     assert _partials_needed(D, 32, n_rep, U, T, shift=4) == (generic + 1) * row
     tile = cabi.attention_plan(U, T, 96, head_dim=D, n_rep=n_rep, q_dtype=cabi.F32, sms=148)[1]
     assert _partials_needed(D, 32, n_rep, U, T, shift=0) == (tile + 1) * row
+
+
+@pytest.mark.parametrize("D,n_rep,U,T", [(128, 4, 300, 8192), (128, 4, 256, 65536), (128, 1, 2048, 32768), (128, 2, 300, 32768)])
+def test_a_plan_too_fine_for_the_scratch_gives_way_to_a_coarser_one(D, n_rep, U, T):
+    """8 MiB is what kivi_decode_attention_noalloc has.  The automatic piece count of these
+    fp32 shapes needs more, about eight CTAs per SM need less: not refused.  A count the
+    caller asks for is still taken as it is, and what no rule fits is still refused."""
+    from intel_kivi_hybrid_b200 import cabi
+    if torch.cuda.is_available() and torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("counts below are for 148 SMs")
+    scratch = 8 << 20
+    row = U * n_rep * (D + 2) * 4
+    planned = cabi.attention_plan(U, T, 96, head_dim=D, n_rep=n_rep, q_dtype=cabi.F32, sms=148)[1]
+    coarse = min(-(-8 * 148 // U), -(-(T // 32) // 4), 128)
+    assert (planned + 1) * row > scratch >= (coarse + 1) * row
+    assert _partials_needed(D, 32, n_rep, U, T, 0, workspace_bytes=scratch) is None                         # accepted (no further than the alignment check)
+    assert _partials_needed(D, 32, n_rep, U, T, 0, workspace_bytes=scratch, num_splits=planned) == (planned + 1) * row
+    assert _partials_needed(D, 32, n_rep, U, T, 0, workspace_bytes=(coarse + 1) * row - 1) == (planned + 1) * row

@@ -57,3 +57,18 @@ def test_noalloc_entry_point_refuses_what_does_not_fit():
         st.attention_noalloc(q, out, n_rep, num_splits=64)       # 1024*64*4*130*4 B = 136 MB > 8 MiB
     st.attention_noalloc(q, out, n_rep, num_splits=2)            # 4.3 MB: accepted
     torch.cuda.synchronize()
+
+
+def test_noalloc_takes_a_coarser_cut_where_the_planned_one_does_not_fit():
+    """300 units x 8192 fp32 tokens: the plan's 16 pieces need 10.6 MB, the coarser rule's four fit."""
+    from intel_kivi_hybrid_b200 import cabi
+    D, n_rep, U, T = 128, 4, 300, 8192
+    st = cabi.LayerStore(U, D, 32, 128, T, torch.float32, "cuda")
+    k = torch.randn(U, T, D, device="cuda")
+    cabi.load_state(st, k, k, T)
+    q = torch.randn(U, n_rep, D, device="cuda")
+    out = torch.empty_like(q)
+    assert (cabi.attention_plan(U, T, 0, n_rep=n_rep, q_dtype=cabi.F32)[1]) * U * n_rep * (D + 2) * 4 > 8 << 20
+    st.attention_noalloc(q, out, n_rep)
+    assert torch.equal(out, st.attention(q, n_rep=n_rep, num_splits=4))
+    assert cabi.device_fault() == 0
