@@ -93,20 +93,22 @@ sample_kernel(const void* logits, int dtype, int vocab, int64_t row_stride,
     stream_order();
     logits = settled(logits);
     // the reference divides: logits / max(temperature, 1e-8)
-    auto scaled = [&](int i) { return __fdiv_rn(logit_at(logits, dtype, (int64_t)blockIdx.x * row_stride + i), temperature); };
+    auto scaled = [&](uint32_t i) { return __fdiv_rn(logit_at(logits, dtype, (int64_t)blockIdx.x * row_stride + i), temperature); };
     const int row = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t base = (int64_t)row * row_stride;
 
     // ---- row maximum and its first index (also the argmax answer) ----------------
     MaxIdx best{-INFINITY, 0x7fffffff};
     bool nan = false;
-    for (int i0 = tid; i0 < vocab; i0 += 8 * kThreads) {
+    // (indices are unsigned: a row may have up to 2^31 - 1 entries, and the walks step past its end)
+    const uint32_t n_row = (uint32_t)vocab;
+    for (uint32_t i0 = tid; i0 < n_row; i0 += 8 * kThreads) {
         float x[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = i0 + j * kThreads < vocab ? logit_at(logits, dtype, base + i0 + j * kThreads) : -INFINITY;
+        for (int j = 0; j < 8; ++j) x[j] = i0 + j * kThreads < n_row ? logit_at(logits, dtype, base + (i0 + j * kThreads)) : -INFINITY;
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-            if (i0 + j * kThreads < vocab) { best = better(best, MaxIdx{x[j], i0 + j * kThreads}); nan |= x[j] != x[j]; }
+            if (i0 + j * kThreads < n_row) { best = better(best, MaxIdx{x[j], (int)(i0 + j * kThreads)}); nan |= x[j] != x[j]; }
     }
     // largest scaled logit of this thread as a key; 0 (below every number's key) without one
     const uint32_t my_key = best.i == 0x7fffffff ? 0u : ordered_key(__fdiv_rn(best.v, temperature));
@@ -137,17 +139,17 @@ sample_kernel(const void* logits, int dtype, int vocab, int64_t row_stride,
             // the subnormals does not say what is clear)
             const float clear = fabsf(least) > 1e-30f && fabsf(least) < 1e30f ? (least - fabsf(least) * 1e-5f) * temperature : -INFINITY;
             // ---- collect what is not below the bound -------------------------------
-            for (int i0 = tid; i0 < vocab; i0 += 8 * kThreads) {
+            for (uint32_t i0 = tid; i0 < n_row; i0 += 8 * kThreads) {
                 float x[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) x[j] = i0 + j * kThreads < vocab ? logit_at(logits, dtype, base + i0 + j * kThreads) : -INFINITY;
+                for (int j = 0; j < 8; ++j) x[j] = i0 + j * kThreads < n_row ? logit_at(logits, dtype, base + (i0 + j * kThreads)) : -INFINITY;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    if (!(x[j] >= clear) || i0 + j * kThreads >= vocab) continue;
+                    if (!(x[j] >= clear) || i0 + j * kThreads >= n_row) continue;
                     const float y = __fdiv_rn(x[j], temperature);
                     if (y >= least) {
                         const int at = atomicAdd(&n_cand_s, 1);
-                        if (at < kCand) { cand_x[at] = y; cand_i[at] = i0 + j * kThreads; }
+                        if (at < kCand) { cand_x[at] = y; cand_i[at] = (int)(i0 + j * kThreads); }
                     }
                 }
             }
@@ -204,7 +206,7 @@ sample_kernel(const void* logits, int dtype, int vocab, int64_t row_stride,
             __syncthreads();
             const uint32_t prefix = sel_prefix;
             const uint32_t mask = pass == 0 ? 0u : (0xffffffffu << (shift + 8));
-            for (int i = tid; i < vocab; i += kThreads) {
+            for (uint32_t i = tid; i < n_row; i += kThreads) {
                 const uint32_t key = ordered_key(scaled(i));
                 if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
             }
@@ -224,13 +226,13 @@ sample_kernel(const void* logits, int dtype, int vocab, int64_t row_stride,
     }
 
     // ---- softmax weights over the kept entries: a contiguous segment per warp ---------
-    const int seg = (vocab + kWarps - 1) / kWarps;
-    const int s0 = min(vocab, warp * seg), s1 = min(vocab, s0 + seg);
+    const uint32_t seg = (n_row + kWarps - 1) / kWarps;
+    const uint32_t s0 = min(n_row, warp * seg), s1 = min(n_row, s0 + seg);
     double mine = 0.0;
-    for (int i0 = s0 + lane; i0 < s1; i0 += 8 * 32) {
+    for (uint32_t i0 = s0 + lane; i0 < s1; i0 += 8 * 32) {
         float x[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = i0 + 32 * j < s1 ? logit_at(logits, dtype, base + i0 + 32 * j) : 0.0f;
+        for (int j = 0; j < 8; ++j) x[j] = i0 + 32 * j < s1 ? logit_at(logits, dtype, base + (i0 + 32 * j)) : 0.0f;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const float y = __fdiv_rn(x[j], temperature);
@@ -249,16 +251,16 @@ sample_kernel(const void* logits, int dtype, int vocab, int64_t row_stride,
     if (mine > 0.0 && before <= target && target < before + mine) {
         double run = before;
         int pick = -1, last_kept = -1;
-        for (int i0 = s0; i0 < s1 && pick < 0; i0 += 32) {
-            const int i = i0 + lane;
+        for (uint32_t i0 = s0; i0 < s1 && pick < 0; i0 += 32) {
+            const uint32_t i = i0 + lane;
             const float y = i < s1 ? scaled(i) : 0.0f;
             const bool kept = i < s1 && y >= kth;
             double incl = kept ? (double)expf(y - m) : 0.0;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) { const double v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
             const unsigned keep = __ballot_sync(0xffffffffu, kept), past = __ballot_sync(0xffffffffu, kept && run + incl > target);
-            if (past) pick = i0 + __ffs(past) - 1;
-            if (keep) last_kept = i0 + 31 - __clz(keep);
+            if (past) pick = (int)i0 + __ffs(past) - 1;
+            if (keep) last_kept = (int)i0 + 31 - __clz(keep);
             run += __shfl_sync(0xffffffffu, incl, 31);
         }
         // the walk adds the same numbers in another order than the sum above: should the

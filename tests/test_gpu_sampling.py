@@ -108,3 +108,17 @@ def test_draws_of_every_selection_path(cabi, vocab, top_k, kind):
     want = ko.sample_tokens(x, 0.9, k, True, seed=77, step=vocab)
     # as above: exp differs in the last bit, a draw on a boundary may move to the neighbour
     assert int((got != want).sum()) <= 1, (got, want)
+
+
+def test_longest_row_the_interface_takes(cabi):
+    """2^31 - 1 entries: the walks over a row step past its end, where a signed index
+    would wrap round to before its beginning."""
+    V = 2 ** 31 - 1
+    x = torch.full((1, V), -100.0, device="cuda", dtype=torch.bfloat16)
+    x[0, V - 1] = 1.0
+    assert cabi.sample_tokens(x, do_sample=False).item() == V - 1
+    assert cabi.sample_tokens(x, 1.0, 1, True, seed=3, step=1).item() == V - 1
+    assert cabi.sample_tokens(x, 1.0, 0, True, seed=3, step=1).item() == V - 1     # the other entries weigh 2^31 e^-101
+    x[0, 0] = x[0, 2 ** 30 + 5] = 1.0
+    drawn = {cabi.sample_tokens(x, 1.0, 3, True, seed=3, step=s).item() for s in range(8)}
+    assert drawn <= {0, 2 ** 30 + 5, V - 1} and len(drawn) > 1
