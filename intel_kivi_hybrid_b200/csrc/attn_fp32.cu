@@ -436,7 +436,7 @@ attn_fp32_tile_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_le
     float* p_s = q_s + NREP * D + warp * 32 * NREP;
     uint64_t* bars = reinterpret_cast<uint64_t*>(q_s + NREP * D + kWarps * 32 * NREP);
     float* ml_s = reinterpret_cast<float*>(bars + kWarps * 2);
-    cudaTriggerProgrammaticLaunchCompletion();            // the kernel that folds the partials may become resident, it waits for this grid's end
+    if (direct.out == nullptr) cudaTriggerProgrammaticLaunchCompletion();      // the kernel that folds the partials may become resident (attn_mma.cu)
     stream_order();
     q = settled(q);
     settle_layer(L);

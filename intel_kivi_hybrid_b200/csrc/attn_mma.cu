@@ -495,9 +495,11 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
     uint64_t* bars = reinterpret_cast<uint64_t*>(q_s + 4 * kD);                  // [kWarps][kStages]
     float* ml_s = reinterpret_cast<float*>(bars + kWarps * kStages);             // [kWarps][4][2]
 
-    // the kernel that folds the partials is the only one queued as a dependent: its few
-    // small blocks may become resident from here on, it waits for this grid's end
-    cudaTriggerProgrammaticLaunchCompletion();
+    // With a fold kernel behind this one, its few small blocks may become resident from
+    // here on (it waits for this grid's end).  Without (FOLD), what comes next can be
+    // another attention call, whose blocks would take places beside this one's while
+    // other SMs stay empty: let in before the fold in the cluster (cluster_fold.cuh).
+    if constexpr (!FOLD) cudaTriggerProgrammaticLaunchCompletion();
     stream_order();
     q = settled(q);
     settle_layer(L);

@@ -30,6 +30,11 @@ struct ClusterOut {                              // where the outputs go; out ==
 // of the cluster calls it.
 __device__ __forceinline__ void cluster_fold(float* part_s, float* ml_s, int n_heads, int D, int64_t row0, const ClusterOut& to) {
     namespace cg = cooperative_groups;
+    // What follows in the stream may become resident while the clusters fold: that hides
+    // its launch, and by now few SMs are left to be unevenly taken.  32 units x 2k tokens,
+    // attention calls back to back 9.6 us (let in at the kernel's start 12.2, at its end
+    // 9.4), append and attention in turn 10.1 (10.1, 10.4); 64 x 512 8.2 (10.1, 8.7).
+    cudaTriggerProgrammaticLaunchCompletion();
     cg::cluster_group cluster = cg::this_cluster();
     const int n = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
     cluster.sync();
