@@ -154,12 +154,14 @@ extern "C" size_t kivi_decode_attention_workspace(int num_units, int n_rep, int 
     return (size_t)num_units * (num_splits + 8) * n_rep * (head_dim + 2) * sizeof(float);
 }
 
-// Up to this many CTAs, and eight pieces a row, the fold runs inside clusters of the
-// attention kernel.
-#ifndef KIVI_FUSED_MAX
-#define KIVI_FUSED_MAX 148
-#endif
-constexpr int64_t kFusedMaxCtas = KIVI_FUSED_MAX;
+// The fold runs inside clusters of the attention kernel up to one CTA per SM and eight
+// pieces a row; more CTAs leave their partials to the fold kernel.  A cluster's CTAs are
+// placed together and hold their places until the slowest is done: with CTAs to spare
+// that costs less than the second launch and the partials' way through memory, with
+// SMs shared it costs more.  us, fold in the cluster / by its own kernel:
+//   tensor cores, 4 heads: 80 CTAs 8.2 / 8.9, 96 8.8 / 9.0, 200 11.5 / 11.0, 256 12.0 / 11.4, 384 12.7 / 13.6 and 27.7 / 24.5, 512 57 / 39
+//   fp32: 20 CTAs 5.1 / 6.1, 60 9.3 / 10.8, 128 7.2 / 8.5 and 11.1 / 11.2, 320 15.0 / 13.3 and 8.3 / 9.6, 800 49 / 43
+static bool folds_in_cluster(int64_t ctas, int pieces, int sms) { return pieces <= kClusterFoldMax && ctas <= sms; }
 
 static int clamp_splits(int64_t s, int64_t n_groups) {
     if (s > kMaxSplitsC) s = kMaxSplitsC;
@@ -203,52 +205,50 @@ static int plan_splits_tile(int num_units, int64_t n_groups, int head_dim, int g
 // Evaluates a small cost model for every candidate count and keeps the cheapest
 // (ties: fewer pieces).  `slots` CTAs are resident at a time (SMs x CTAs per SM).
 // Constants in microseconds, fitted to CUDA-event times on B200 at about 1.9 GHz
-// (units x tokens from 1 x 128k and 16 x 1k to 512 x 32k): a CTA costs c0 of
-// fixed time (first copy, query staging, the fold of its warps) plus c1 per token
-// group, a residual-ring CTA t_ring, starting a CTA c_start, folding the pieces
-// of a unit c_fold.  c1 depends on how many CTAs share an SM (an SM with three
-// CTAs delivers 8.3-9 groups per us, with two 7.4-8, with one 5.7-6): 0.16 /
-// 0.24 / 0.33 us per group for a single wave with at most 1 / 2 / 3 quantized
-// CTAs per SM, 0.36 in the steady state of several waves.  The fold of more
-// than 16 pieces is done by a whole CTA per output row and costs less per
-// piece.  The grid lists the
-// quantized pieces first and the short ring CTAs last, so:
-//   * the quantized CTAs all resident at once: the time of one of them (the ring
-//     CTAs fill the free slots, or follow the first ring CTAs that finish);
+// (1 x 128k and 4 x 96 to 512 x 32k units x tokens, 1 to 32 pieces each): a CTA costs
+// c0 of fixed time (first copy, query staging, the fold of its warps) plus c1 per token
+// group, starting a CTA c_start, a piece of a unit c_piece, pieces that no cluster folds
+// c_merge.  c1 depends on how many CTAs share an SM: one at most, one beside ring CTAs,
+// up to 1.75 quantized ones on average (288 or 296 on 148 SMs run as if some held three),
+// up to 2.25, up to three; c1_full is the steady state of several waves.  The fold of more
+// than 16 pieces is done by a whole CTA per output row and costs less per piece.  The
+// grid lists the quantized pieces first and the short ring CTAs last, so:
+//   * the quantized CTAs all resident at once: the time of one of them; ring CTAs beyond
+//     the slots follow the first CTAs that finish, c_over per CTA and SM
+//     (140 units x 2k: 140 + 140 CTAs 18.7 us, 420 + 140 23.3);
 //   * several waves: total CTA time over the slots, plus a ragged end of about
-//     a third of a CTA; a CTA's fixed time is 7.5 us there.
-// The ring CTAs count where they decide how many CTAs share an SM: the one-CTA rate
-// needs all CTAs, ring included, on SMs of their own (32 units x 2k tokens: 3 pieces
-// 9.7 us, 4 pieces 10.7), and at the two-CTA count the ring CTAs must fit beside the
-// quantized ones (256 units x 4k with 256 + 256 CTAs: 49.6 us in one piece, 45.3 in
-// two, 44.0 in three; 192 units x 2k: one piece 24.3 us, three 26.3).
+//     a third of a CTA; a CTA's fixed time is c0_waves there.
+// At the two-CTA count the ring CTAs must fit beside the quantized ones, or c1 is that of
+// a crowded SM (256 units x 4k: one piece 51 us, two 44, three 45).
+// Against the best count measured at 308 shapes this is 2 % off on average; where two
+// counts lie close it may take the second (160 units x 8k: two pieces 7 % behind four).
 static int plan_splits_mma(int num_units, int64_t n_groups, int n_res_splits, int n_sms, int ctas_per_sm) {
     const int per_sm = ctas_per_sm > 0 ? ctas_per_sm : 3;
     const double slots = (double)per_sm * n_sms;
-    const double c0 = 6.0, c0_waves = 7.5, c1_one = 0.16, c1_two = 0.24, c1_crowded = 0.31, c1_three = 0.33, c1_full = 0.36;
-    const double t_ring = 7.0, c_start = 0.015, ragged = 0.3;
+    const double c0 = 6.0, c0_waves = 7.5, c1_one = 0.17, c1_beside = 0.20, c1_two = 0.24, c1_crowded = 0.31, c1_some_three = 0.315, c1_three = 0.33, c1_full = 0.36;
+    const double t_ring = 7.0, c_start = 0.015, c_piece = 0.1, c_merge = 0.2, c_over = 1.8, ragged = 0.3;
     const int64_t s_max = n_groups < kMaxSplitsC ? n_groups : kMaxSplitsC;
     int best = 1;
     double best_t = 0.0;
     for (int64_t s = 1; s <= s_max; ++s) {
-        const double quant = (double)num_units * (double)s, ring = (double)num_units * n_res_splits;
+        const double quant = (double)num_units * (double)s, ring = (double)num_units * n_res_splits, ctas = quant + ring;
         const double per_cta = (double)((n_groups + s - 1) / s);
         double t;
         if (quant <= slots) {
-            // the fullest SM sets the pace.  The two-CTA rate only holds up to about
-            // 1.75 CTAs per SM on average: with 288 or 296 CTAs on 148 SMs a CTA was
-            // measured at 0.27-0.32 us per group, as if some SMs already held three.
-            const double c1 = quant + ring <= n_sms ? c1_one
-                            : quant <= 1.75 * n_sms ? (quant + ring <= slots ? c1_two : c1_crowded)
+            const double c1 = ctas <= n_sms ? c1_one
+                            : quant <= n_sms ? c1_beside
+                            : quant <= 1.75 * n_sms ? (ctas <= slots ? c1_two : c1_crowded)
+                            : quant <= 2.25 * n_sms ? c1_some_three
                             : quant <= 3.0 * n_sms ? c1_three : c1_full;
-            t = c0 + c1 * per_cta + c_start * (quant + ring);
+            t = c0 + c1 * per_cta + c_start * ctas + (ctas > slots ? c_over * (ctas - slots) / n_sms : 0.0);
         } else {
             t = (quant * (c0_waves + c1_full * per_cta) + ring * t_ring) / slots + ragged * (c0_waves + c1_full * per_cta);
             // just over one wave: never cheaper than a full single wave of such CTAs
             const double one_wave = c0 + c1_three * per_cta + c_start * slots;
             if (t < one_wave) t = one_wave;
         }
-        t += s <= 16 ? 0.1 * (double)s : 1.0 + 0.02 * (double)s;
+        if (!folds_in_cluster((int64_t)ctas, (int)s + n_res_splits, n_sms)) t += c_merge;
+        t += s <= 16 ? c_piece * (double)s : 10 * c_piece + 0.02 * (double)s;
         if (s == 1 || t < best_t - 1e-9) { best = (int)s; best_t = t; }
     }
     return best;
@@ -357,7 +357,7 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
 
     const int64_t ctas = (int64_t)L->num_units * (use_mma ? (n_rep + 3) / 4 : 1) * n_splits;
     ClusterOut direct{nullptr, out_dtype, lse};
-    if (!gather && n_splits <= kClusterFoldMax && ctas <= kFusedMaxCtas && kernel != AttnKernel::kGeneric) direct.out = out;
+    if (!gather && folds_in_cluster(ctas, n_splits, num_sms()) && kernel != AttnKernel::kGeneric) direct.out = out;
 
     int rc = use_mma
         ? run_attn_mma(L, quant_len, res_start, res_len, q, q_dtype, n_rep, scale_log2, nq_splits, gps, n_res_splits, res_chunk, part_o, part_ml, direct, st)

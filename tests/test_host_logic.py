@@ -355,3 +355,15 @@ def test_a_plan_too_fine_for_the_scratch_gives_way_to_a_coarser_one(D, n_rep, U,
     assert _partials_needed(D, 32, n_rep, U, T, 0, workspace_bytes=scratch) is None                         # accepted (no further than the alignment check)
     assert _partials_needed(D, 32, n_rep, U, T, 0, workspace_bytes=scratch, num_splits=planned) == (planned + 1) * row
     assert _partials_needed(D, 32, n_rep, U, T, 0, workspace_bytes=(coarse + 1) * row - 1) == (planned + 1) * row
+
+
+@pytest.mark.parametrize("units,tokens,n_rep,pieces", [
+    (48, 2048, 4, 3),       # 11.5 us; in two pieces 13.2
+    (148, 1024, 8, 2),      # two head blocks a unit: 21.9 us, in one piece 24.2
+    (140, 2048, 4, 2),      # 19.2 us; in three pieces, whose ring CTAs find no place beside them, 23.3
+    (37, 3968, 4, 4),       # 13.0 us; in three pieces 16.4
+    (32, 2048, 4, 3),       # 10.0 us, folded in a cluster; in four pieces 11.0
+])
+def test_attention_split_plan_takes_the_measured_counts(units, tokens, n_rep, pieces):
+    from intel_kivi_hybrid_b200 import cabi
+    assert cabi.attention_plan(units, tokens, 96, n_rep=n_rep, sms=148, ctas_per_sm=3)[1] == pieces
