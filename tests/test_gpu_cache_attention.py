@@ -611,6 +611,91 @@ def test_attention_fp32_kernels_at_their_edges(cabi, D, G, n_rep, n_quant, n_res
         assert err < 1e-5, (splits, err)
 
 
+@pytest.mark.parametrize("D,G,n_rep,n_res,res_start,ring", [
+    (64, 32, 3, 20, 120, torch.float32), (64, 16, 8, 128, 127, torch.bfloat16),
+    (128, 32, 1, 33, 96, torch.bfloat16), (128, 128, 4, 100, 101, torch.float32), (128, 8, 8, 128, 65, torch.float32)])
+def test_attention_fp32_tile_kernel_across_the_end_of_the_ring(cabi, D, G, n_rep, n_res, res_start, ring):
+    """The window lies across the end of a ring of 128 slots, in each kind of the tile
+    kernel's ring code: both head_dims, both ring types, one and several heads.
+    Bound as in the test of the kernels' edges above."""
+    U, R, n_quant = 3, 128, 2 * G
+    assert res_start + n_res > R
+    g = torch.Generator(device="cuda").manual_seed(D + G + n_rep)
+    st = cabi.LayerStore(U, D, G, R, n_quant, ring, "cuda")
+    k, v = (torch.randn(U, n_quant + n_res, D, generator=g, device="cuda").to(ring) for _ in range(2))
+    cabi.load_state(st, k, v, n_quant)
+    for buf in (st.k_res, st.v_res):
+        buf.copy_(torch.roll(buf, res_start, dims=1))
+    st.res_start = res_start
+    q = torch.randn(U, n_rep, D, generator=g, device="cuda")
+    kd, vd = st.materialize()
+    assert torch.equal(kd[:, n_quant:], k[:, n_quant:].float())
+    ref = torch.softmax(q.double() @ kd.double().transpose(1, 2) * D ** -0.5, dim=-1) @ vd.double()
+    assert rel_err(st.attention(q, n_rep=n_rep), ref) < TOL_F32
+
+
+@pytest.mark.parametrize("D,G,n_rep,path,dtype", [
+    (64, 32, 1, "fp32", torch.float32), (64, 64, 8, "fp32", torch.bfloat16), (128, 32, 4, "fp32", torch.float32), (128, 128, 7, "fp32", torch.float32),
+    (128, 32, 1, "mma", torch.bfloat16), (128, 32, 3, "mma", torch.bfloat16), (128, 32, 8, "mma", torch.bfloat16)])
+def test_fold_in_a_cluster_gives_the_bits_of_the_fold_kernel(cabi, D, G, n_rep, path, dtype):
+    """Few units fold inside clusters of the attention kernel, many leave it to the fold
+    kernel; a unit's output and log-sum-exp do not depend on which, bit for bit, for
+    every piece count a cluster takes."""
+    few, many, n_quant, n_res = 3, 160, 8 * G, 40             # 160 units: more CTAs than SMs whatever the cut
+    g = torch.Generator(device="cuda").manual_seed(D + n_rep)
+    k, v = (torch.randn(few, n_quant + n_res, D, generator=g, device="cuda").to(dtype) for _ in range(2))
+    q = torch.randn(few, n_rep, D, generator=g, device="cuda").to(dtype)
+    kernel = cabi.ATTN_FP32 if path == "fp32" else cabi.ATTN_MMA
+    for res in (n_res, 0):
+        outs = []
+        for U in (few, many):
+            st = cabi.LayerStore(U, D, G, 128, n_quant, dtype, "cuda")
+            pad = lambda x: torch.cat([x, x[:1].expand(U - few, *x.shape[1:])])
+            cabi.load_state(st, pad(k)[:, :n_quant + res], pad(v)[:, :n_quant + res], n_quant)
+            per = []
+            for pieces in range(1, 8):
+                out, lse = st.attention_lse(pad(q).contiguous(), n_rep=n_rep, num_splits=pieces, path=kernel, out_dtype=torch.float32)
+                launches = cabi.lib.kivi_last_launch_count()
+                assert launches == (1 if U == few else 2), (U, pieces, launches)
+                per.append((out[:few], lse[:few]))
+            outs.append(per)
+        for (o1, l1), (o2, l2) in zip(*outs):
+            assert torch.equal(o1, o2) and torch.equal(l1, l2)
+
+
+@pytest.mark.parametrize("D,dtype,U,n_rep", [(128, torch.bfloat16, 8, 4), (64, torch.float32, 12, 1), (128, torch.bfloat16, 200, 1), (32, torch.float32, 2, 2)])
+def test_queued_steps_equal_synchronised_steps(cabi, D, dtype, U, n_rep):
+    """Launches overlap the kernels before them in their stream: append, flush,
+    attention and sampling of 70 steps queued without a pause (flushes among them) leave the
+    same bits as the same steps with the GPU idle before each call."""
+    G = 8 if D == 32 else 32                                   # (head_dim 32: the generic kernels)
+    steps, T0 = 70, 200
+    g = torch.Generator(device="cuda").manual_seed(U)
+    k, v = (torch.randn(U, T0 + steps, D, generator=g, device="cuda").to(dtype) for _ in range(2))
+    q = torch.randn(steps, U, n_rep, D, generator=g, device="cuda").to(dtype)
+    results = []
+    for queued in (True, False):
+        st = cabi.LayerStore(U, D, G, 128, 512, dtype, "cuda")
+        wait = (lambda: None) if queued else torch.cuda.synchronize
+        outs, ids = [], []
+        torch.cuda.synchronize()
+        st.update(k[:, :T0], v[:, :T0])
+        for i in range(steps):
+            wait()
+            st.update(k[:, T0 + i:T0 + i + 1], v[:, T0 + i:T0 + i + 1])
+            wait()
+            outs.append(st.attention(q[i], n_rep=n_rep))
+            wait()
+            outs.append(st.attention(q[i], n_rep=n_rep, num_splits=1))
+            wait()
+            ids.append(cabi.sample_tokens(outs[-1].view(U, -1), 1.0, 5, True, seed=i))
+        torch.cuda.synchronize()
+        results.append((torch.stack(outs), torch.stack(ids), *st.materialize(), st.k_res.clone(), st.v_res.clone()))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+    assert cabi.device_fault() == 0
+
+
 _TWO_THREADS_CPP = r"""
 #include <atomic>
 #include <thread>
