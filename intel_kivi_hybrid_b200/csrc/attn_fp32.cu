@@ -246,7 +246,7 @@ attn_fp32_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
 
 // ---- fp32 kernel for head_dim 64 and 128 -----------------------------------------
 // Same arithmetic (k = code*scale + zero in one fp32 rounding, fp32 FMAs for both
-// contractions), organised so that the FMA pipe is what bounds it:
+// contractions), organised so that little is left beside the FMAs:
 //   * every warp streams its own token groups into a private two-stage ring in shared
 //     memory with bulk copies (the six arrays of a group are contiguous runs);
 //   * q.k: a lane takes four tokens x D/4 channels, exactly what its 32-bit code
@@ -258,12 +258,17 @@ attn_fp32_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
 //     subtract; dequantization and both contractions are packed two to an instruction
 //     (same rate on the FMA pipe, half the issue slots);
 //   * a running maximum is only worked out when a score exceeds it.
-// What bounds it: the FMA pipe.  A lane's 256 codes of a group cost one FMA per code and
-// head (512 cycles of the SM quarter per head, two per packed instruction) and about
-// 1500 cycles of conversion; measured 2150 / 4100 / 6700 cycles per group with 1 / 4 / 8
-// heads, against 13000 with four heads in the generic kernel (dependent 32-bit loads,
-// an integer conversion per code).  32 units x 8k tokens, 4 heads: 99 -> 36 us;
-// 32 x 32k, 1 head: 259 -> 65 us; 12 units x 712 tokens, head_dim 64: 18.4 -> 6.4 us.
+// What bounds it: no single pipe.  A lane's 256 codes of a group cost one FMA per code and
+// head (256 cycles of the SM quarter per head: two per packed instruction, which does two)
+// and about 1000 cycles of conversion (a byte permute, half a packed add and half a packed
+// FMA per code), so four heads need 2000 of the 3800-4100 cycles a group takes.  Counters
+// on 160 units x 8k, four heads: 2060 instructions per group and warp, issue slots 60 %
+// busy, FMA pipe 53 %, ALU 43 %, shared-memory pipe (query, weight and scale reads) 46 %,
+// with 11 warps on an SM (162 registers) to cover the latencies in between.
+// Measured 2150 / 4100 / 6700 cycles per group with 1 / 4 / 8 heads, against 13000 with
+// four heads in the generic kernel (dependent 32-bit loads, an integer conversion per
+// code).  32 units x 8k tokens, 4 heads: 99 -> 37 us; 32 x 32k, 1 head: 259 -> 67 us;
+// 12 units x 712 tokens, head_dim 64: 18.4 -> 5.1 us (with the fold in a cluster).
 // Error against 64 bits is about half of the generic kernel's (shorter chains of adds).
 template <int D> struct Fp32Tile {
     static constexpr int kBytes = D / 4;               // packed value bytes of a token

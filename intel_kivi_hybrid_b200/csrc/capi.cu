@@ -180,12 +180,15 @@ static int plan_splits_generic(int num_units, int64_t n_groups, int sms) {
     return clamp_splits(s, n_groups);
 }
 
-// The tile kernel is bound by the FMA pipe, so what counts is how evenly whole rounds
-// (one group per warp, four per CTA) spread over the SMs: a round costs c_round of SM
-// time (fitted on B200: 1.0 / 1.9 / 3.3 us with 1 / 4 / 8 heads at head_dim 128,
-// groups of 32), and a CTA alone on its SM takes about 1.2 us longer per round than its
-// share.  32 units x 8k tokens, four heads: 8 pieces 35.9 us, 37 (the generic rule)
-// 39.3; 192 units x 1k, head_dim 64: 2 pieces 14.3, 7 pieces 16.1.
+// Tile kernel: what counts is how evenly whole rounds (one group per warp, four per CTA)
+// spread over the SMs: a round costs c_round of SM time (fitted on B200: 1.0 / 1.9 / 3.3
+// us with 1 / 4 / 8 heads at head_dim 128, groups of 32), and a CTA alone on its SM takes
+// about 1.2 us longer per round than its share.  The model tells good counts from bad
+// ones, not the best from the next: us at the count it takes, the best one, the generic
+// rule's -- 192 units x 1k, head_dim 64: 2 pieces 14.6, the same, 7 pieces 18.6; 32 x 2k,
+// four heads: 8 pieces 14.9, the same, 37 pieces 25.1; 32 x 8k, four heads: 32 pieces
+// 37.4, 8 pieces 35.7, 37 pieces 40.6; 32 x 8k, eight heads: 32 pieces 60.5, 8 pieces
+// 52.9, 37 pieces 66.8; 8 x 32k, four heads: 37 pieces 42.3, 32 pieces 35.5, 128 pieces 36.6.
 static int plan_splits_tile(int num_units, int64_t n_groups, int head_dim, int group_size, int n_rep, int n_res, int sms) {
     const double c_round = (0.7 + 0.32 * n_rep) * head_dim / 128.0 * group_size / 32.0, c_alone = 1.2, c_cta = 0.3;
     int best = 1;

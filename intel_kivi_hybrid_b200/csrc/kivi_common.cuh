@@ -35,23 +35,32 @@ int num_sms();
 #define KIVI_LAUNCH_OK()  KIVI_CUDA_OK(cudaGetLastError())
 
 // ---- overlapping launches ------------------------------------------------------
-// Kernels of this library are launched as programmatic dependents of whatever runs
+// Most kernels of this library are launched as programmatic dependents of whatever runs
 // before them in their stream: their blocks may become resident once every block of
 // that kernel has finished (or has let them in), which hides launch latency and
-// prologue.  A kernel calls stream_order() before it touches memory: it waits until
-// everything before it has completed.  Pointers it reads from go through settled()
-// afterwards: a load the compiler takes for invariant (ld.global.nc) could otherwise
-// be moved ahead of the wait.
+// prologue.  Three disciplines keep the order of memory:
+//   * wait first (all but those below): the kernel calls stream_order() before it touches
+//     memory, which waits until everything before it has completed.  Pointers it reads
+//     from go through settled() afterwards: a load the compiler takes for invariant
+//     (ld.global.nc) could otherwise be moved ahead of the wait;
+//   * wait last: the flush kernels of one kivi_cache_update.  The first is launched
+//     plainly, the others may start beside it: they write disjoint arrays and read what
+//     was there before the call.  Each waits at its end, so that what follows a kernel
+//     and waits for it waits for the ones before it too (cache_kernels.cu);
+//   * plain launch, ordered by the stream: the first flush kernel, import_keys_kernel,
+//     merge_token_shards_kernel, the alignment probe.
 //
 // Letting dependents in early (let_in_early) pays for a streaming kernel of more
 // blocks than the GPU holds at a time: its dependents then fill the ragged last wave
 // (quantize + dequantize of 4 x 8 x 4096 tokens: 65.6 -> 57.9 us).  With fewer blocks
 // the dependents are dealt out over SMs that are unevenly taken and stay uneven when
 // it is their turn (sampling 128 rows: 28.7 -> 44.9 us), so it is left to the end there.
+// The attention kernels have rules of their own (attn_mma.cu, cluster_fold.cuh).
+constexpr unsigned kResidentBlocks = 148u * 8u;      // B200: 148 SMs x 2048 threads; every kernel that asks has blocks of 256
 #ifdef __CUDACC__
 __device__ __forceinline__ void stream_order() { cudaGridDependencySynchronize(); }
 __device__ __forceinline__ void let_in_early() {
-    if (gridDim.x * gridDim.y > 148u * 8u) cudaTriggerProgrammaticLaunchCompletion();      // 8 blocks of 256 threads fill an SM
+    if (gridDim.x * gridDim.y > kResidentBlocks) cudaTriggerProgrammaticLaunchCompletion();
 }
 template <typename T> __device__ __forceinline__ T* settled(T* p) {
     asm volatile("" : "+l"(p));
