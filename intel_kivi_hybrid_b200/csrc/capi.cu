@@ -337,13 +337,14 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
     int n_res_splits = res_len > 0 ? 1 : 0, res_chunk = res_len;
     if (use_mma) attn_mma_residual_plan(res_len, &n_res_splits, &res_chunk);
     const AttnKernel kernel = use_mma ? AttnKernel::kMma : attn_fp32_tile_ok(L) ? AttnKernel::kTile : AttnKernel::kGeneric;
-    int nq_splits = plan_splits(kernel, L->num_units, n_groups, num_splits, D, G, n_rep, n_res_splits, num_sms(), use_mma ? attn_mma_ctas_per_sm() : 0);
+    const int sms = num_sms();
+    int nq_splits = plan_splits(kernel, L->num_units, n_groups, num_splits, D, G, n_rep, n_res_splits, sms, use_mma ? attn_mma_ctas_per_sm() : 0);
     const auto partial_bytes = [&](int pieces) { return (size_t)L->num_units * (pieces + n_res_splits) * n_rep * (D + 2) * sizeof(float); };
     // The tile kernel's plan cuts large problems finer than the generic rule (300 units x
     // 8k tokens: 16 pieces against 4): where its partials do not fit the scratch but the
     // coarser cut's do, that one is taken.
     if (num_splits == 0 && kernel == AttnKernel::kTile && partial_bytes(nq_splits) > workspace_bytes) {
-        const int coarse = plan_splits(AttnKernel::kGeneric, L->num_units, n_groups, 0, D, G, n_rep, n_res_splits, num_sms(), 0);
+        const int coarse = plan_splits(AttnKernel::kGeneric, L->num_units, n_groups, 0, D, G, n_rep, n_res_splits, sms, 0);
         if (partial_bytes(coarse) <= workspace_bytes) nq_splits = coarse;
     }
     const int gps = nq_splits > 0 ? (int)((n_groups + nq_splits - 1) / nq_splits) : 0;
@@ -360,7 +361,7 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
 
     const int64_t ctas = (int64_t)L->num_units * (use_mma ? (n_rep + 3) / 4 : 1) * n_splits;
     ClusterOut direct{nullptr, out_dtype, lse};
-    if (!gather && folds_in_cluster(ctas, n_splits, num_sms()) && kernel != AttnKernel::kGeneric) direct.out = out;
+    if (!gather && folds_in_cluster(ctas, n_splits, sms) && kernel != AttnKernel::kGeneric) direct.out = out;
 
     int rc = use_mma
         ? run_attn_mma(L, quant_len, res_start, res_len, q, q_dtype, n_rep, scale_log2, nq_splits, gps, n_res_splits, res_chunk, part_o, part_ml, direct, st)
