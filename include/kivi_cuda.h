@@ -201,7 +201,8 @@ int kivi_decode_attention_max_splits(void);
  * arithmetic only, nothing is launched): whether the tensor-core kernel runs,
  * into how many pieces every unit's quantized history is cut (num_splits > 0 is
  * taken as given, 0 lets the library choose from the number of CTAs the GPU
- * holds at a time) and how many CTAs per unit take the residual ring.
+ * holds at a time) and how many CTAs per unit take the residual ring.  For arrays
+ * on the 16-byte grid; others take the generic kernel and its coarser cut.
  * sms / ctas_per_sm: the SM count and the tensor-core kernel's resident CTAs per
  * SM to plan for; <= 0 asks the current device (148 and 3 without one).
  * No counterpart in the reference. */
