@@ -388,9 +388,8 @@ int kivi_sample_tokens(const void* logits, int dtype, int batch, int vocab, int6
  * tensor core, adding the products 1 and 2^-k to the addend -1 in one m16n8k16
  * fp16 MMA, still returns exactly 2^-k -- i.e. how many bits below the largest
  * addend survive its alignment (25 on B200).  The tensor-core attention kernel
- * feeds 2-bit codes as fp16 subnormals and places them so that at least 20 of
- * those bits are left for every code; below 24 here its error bound does not
- * hold.  No counterpart in the reference. */
+ * contracts bytes, whose sums are exact integers, and does not depend on it.
+ * No counterpart in the reference. */
 int kivi_selftest_mma_alignment_bits(int* bits_out);
 
 /* number of kernels the last successful call on this thread launched */

@@ -5,28 +5,36 @@
 // Decode attention over 2-bit codes is instruction-bound before it is HBM-bound:
 // one quantized (token, kv_head) is 128 bytes of HBM but 256 codes that each
 // feed 4 query heads.  The GQA query-group tile therefore runs on the tensor
-// cores (mma.sync m16n8k16, fp32 accumulate) with the codes as the exact
-// operand, and everything that depends on scales and zeros is folded into the
-// small operand:
+// cores (mma.sync m16n8k32, bytes in, exact 32-bit integer sums) with the codes as
+// one operand, and everything that depends on scales and zeros is folded into the
+// small operand, a fixed-point number cut into bytes:
 //
 //   q.k   score[t,h] = sum_d (q[h,d]*s[g,d]) * c[d,t]  +  sum_d q[h,d]*z[g,d]
-//         A = codes of 16 tokens x 16 channels; a code is used where it lies in
-//         its 16-bit half, as the fp16 subnormal c*4^e*2^-24 (one AND per
-//         register pair); B = q*s split into fp16 hi + lo parts (the 8 columns
-//         are 4 heads x {hi, lo}), 22 significant bits; the zero term is an
-//         fp32 dot product per (group, head), computed once per column pair.
+//         A = codes of 16 tokens x 32 channels; a byte of four codes is an operand as
+//         it lies, and so is what three masks leave of it (below); B = q*s in 22 bits
+//         and a sign of the largest of the stage, three bytes and a constant (16
+//         columns = 4 heads x 4 bytes); the zero term is an fp32 dot product.
 //   p.v   out[h,d]   = sum_t (p[h,t]*s[t,gd]) * c[t,d]  +  sum_t p[h,t]*z[t,gd]
-//         A = codes of 16 channels x 16 tokens, same encoding; B = p*s in fp16
-//         (rounding errors of independent tokens average out), built once per
-//         column pair and exchanged by shuffle; the zero term accumulates in fp32.
-//   Requires |q*s*sm_scale*log2(e)| and p*s below 65504 (fp16 range).
+//         A = codes of 16 channels x 32 tokens, same encoding; B = p*s in 16 bits of
+//         the stage's largest (8 columns = 4 heads x 2 bytes); the zero term
+//         accumulates in fp32.
+//   Infinities, NaN and negative value scales take an fp32 form of their own.
+//
+// Bytes instead of fp16 (codes as subnormals, q*s in two parts): 16 codes cost three
+// ALU operations instead of nine, and every MMA contracts twice as many.  512 units x
+// 32k tokens 416 -> 353 us (6.15 TB/s, 0.94 of a plain copy), 32 x 128k 118 -> 99 us,
+// 128 x 4k 24.0 -> 21.9 us, and the error against the fp32 kernel falls to a seventh.
+// A group of 32 tokens takes about 470 instructions of a warp: 24 MMAs, 48 masks, 96
+// FMAs for the operands and the zero terms, 24 permutes, 44 shared-memory accesses.
 //
 // Data movement: every warp streams its own token groups from HBM into a
 // private shared-memory ring with bulk asynchronous copies (cp.async.bulk,
-// completion on an mbarrier; six lanes issue one copy each), two groups (8 KB)
-// per stage, and unpacks codes in registers.  The unit's queries sit in shared
-// memory, pre-scaled.  Nothing dequantized is ever written anywhere.  The
-// residual ring (full precision) is handled by extra CTAs with fp32 FMAs.
+// completion on an mbarrier), two groups (8 KB) per stage, and masks codes in
+// registers.  The small operands are made where their scales are read without
+// repetition (a lane takes four channels, or one token, for all four heads) and
+// travel through 2 KB of shared memory per warp to where the MMA wants them
+// (ldmatrix with byte transposition).  Nothing dequantized is ever written anywhere.
+// The residual ring (full precision) is handled by extra CTAs with fp32 FMAs.
 //
 // Every wait on an mbarrier is bounded; on expiry the warp raises the device
 // fault word, stops consuming and its partial is written as "empty".
@@ -42,191 +50,314 @@ namespace kivi {
 namespace {
 
 constexpr int kD = 128, kG = 32;
-#ifndef KIVI_MMA_WARPS
-#define KIVI_MMA_WARPS 4
-#endif
-#ifndef KIVI_MMA_GPS
-#define KIVI_MMA_GPS 2
-#endif
-#ifndef KIVI_MMA_STAGES
-#define KIVI_MMA_STAGES 2
-#endif
-#ifndef KIVI_MMA_JOINT
-#define KIVI_MMA_JOINT 1            /* 1: both groups of a stage share one softmax update */
-#endif
-#ifndef KIVI_MMA_CHAINS
-#define KIVI_MMA_CHAINS 2           /* independent accumulator chains per q.k tile */
-#endif
-#ifndef KIVI_MMA_MIN_CTAS
-#define KIVI_MMA_MIN_CTAS 3
-#endif
-constexpr int kWarps = KIVI_MMA_WARPS;     // warps per CTA, each with a private pipeline
-constexpr int kGPS = KIVI_MMA_GPS;         // token groups per pipeline stage
-constexpr int kStages = KIVI_MMA_STAGES;
+constexpr int kWarps = 4;              // warps per CTA, each with a private pipeline
+constexpr int kGPS = 2;                // token groups per pipeline stage
+constexpr int kStages = 2;
+constexpr int kScratchBytes = 2048;    // per warp, for operands on their way from lane to lane
 constexpr int kGroupBytes = 4096;      // kc 1024 | ks 512 | kz 512 | vc 1024 | vs 512 | vz 512
 constexpr int kStageBytes = kGPS * kGroupBytes;
 
 __device__ int g_fault_word = 0;
 
 // ---- PTX wrappers ------------------------------------------------------------
-__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+// accumulator c (+)= codes x digits, both unsigned bytes: exact 32-bit integers
+__device__ __forceinline__ void mma_u8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// same with a zero addend: starts an accumulator without initialising registers
-__device__ __forceinline__ void mma_f16_first(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
+// c = start + codes x digits: `start` stays in four registers of its own for the whole kernel
+__device__ __forceinline__ void mma_u8_from(const int (&start)[4], int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(start[0]), "r"(start[1]), "r"(start[2]), "r"(start[3]));
 }
-// {lo16, hi16} = {f16(lo), f16(hi)}
-__device__ __forceinline__ uint32_t pack_f16_rz(float lo, float hi) {
-    uint32_t r;
-    asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
+// Two 16 x 16 byte matrices, transposed: lane l gives the address of row l (0-15: first
+// matrix, 16-31: second); lane (gid, tig) gets, as bytes, rows 4*tig .. 4*tig+3 of column
+// gid and of column gid + 8 of the first (r[0], r[1]) and the second (r[2], r[3]).
+__device__ __forceinline__ void ldmatrix_t8(uint32_t (&r)[4], uint32_t row_addr) {
+    asm volatile("ldmatrix.sync.aligned.m16n16.x2.trans.shared.b8 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(row_addr) : "memory");
 }
-__device__ __forceinline__ uint32_t pack_f16_rn(float lo, float hi) {
-    uint32_t r;
-    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
+__device__ __forceinline__ void sts128(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ void sts64(uint32_t addr, uint32_t x, uint32_t y) {
+    asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(addr), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void sts32(uint32_t addr, float x) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(x) : "memory"); }
+__device__ __forceinline__ float4 lds128(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
 }
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// largest magnitude; NaN if any is
+__device__ __forceinline__ float max3_abs_nan(float a, float b, float c) {
+    float d;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(fabsf(a)), "f"(fabsf(b)), "f"(fabsf(c)));
+    return d;
+}
+__device__ __forceinline__ float warp_max_abs_nan(float a) {
+    float d;
+    asm volatile("redux.sync.max.abs.NaN.f32 %0, %1, 0xffffffff;" : "=f"(d) : "f"(a));
+    return d;
+}
+__device__ __forceinline__ uint32_t warp_max_u32(uint32_t a) {
+    uint32_t d;
+    asm volatile("redux.sync.max.u32 %0, %1, 0xffffffff;" : "=r"(d) : "r"(a));
+    return d;
+}
 
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 
-// ---- code -> MMA operand encoding ----------------------------------------------
-// A 2-bit code c sitting at bits 2e..2e+1 (e <= 4) of a 16-bit half is, read as
-// an fp16 bit pattern with a zero exponent field, the subnormal number
-// c * 4^e * 2^-24 -- exactly.  So one AND per register pair turns packed codes
-// into a tensor-core operand: no shift, no offset.  The factor 4^e * 2^-24
-// belongs to a whole accumulator row and is undone (exactly, a power of two)
-// when the accumulator is read.
+// ---- operands ------------------------------------------------------------------
+// A byte of packed codes c0 + 4 c1 + 16 c2 + 64 c3 is itself a tensor-core operand, and so
+// are the bytes left by masking away c0; c0 and c1; c0, c1 and c2: three ANDs turn a 32-bit
+// word (four bytes, four consecutive contraction indices) into four operands.  Neighbouring
+// accumulator rows then differ by the sum wanted of one code, times 4^e, which is taken out
+// (exactly) at the end.
+constexpr uint32_t kFrom1 = 0xfcfcfcfcu, kFrom2 = 0xf0f0f0f0u, kFrom3 = 0xc0c0c0c0u;
+constexpr float kRow1 = 0.25f, kRow2 = 0.0625f, kRow3 = 0.015625f;
+
+// The other operand is a fixed-point number cut into bytes, each byte a column of its own.
+// x = fma(w, F, M) leaves round(w * F) in the low bits of the float x.
 //
-// The tensor core aligns the products of one MMA on their exponent *fields* and
-// keeps about 26 bits below the largest (measured: truncation, not rounding).
-// A subnormal's field is fixed, so the zero bits above a low-lying code come out
-// of that budget: a code at e = 0 is left with 18 bits.  A 32-bit word holds
-// four bytes = four codes each; with the bytes of each half swapped (one PRMT,
-// in place of the shift that would otherwise bring the odd bytes down) the
-// first code of every byte can be taken from bits 8-9 (e = 4) and the other
-// three from where they lie (e = 1..3): no row is left with fewer than 20 bits.
-template <int E> __device__ __forceinline__ uint32_t code_pair(uint32_t w) {
-    static_assert(E >= 0 && E <= 4, "bits 10 and up are the exponent field");
-    return w & (0x00030003u << (2 * E));
-}
-__device__ __forceinline__ uint32_t swap_bytes_in_halves(uint32_t w) { return __byte_perm(w, 0u, 0x2301u); }
-constexpr float kRow0 = 65536.0f;             // first code of a byte, taken at e = 4:  2^24 * 4^-4
-constexpr float kRow1 = 4194304.0f;           // 2^24 * 4^-1
-constexpr float kRow2 = 1048576.0f;           // 2^24 * 4^-2
-constexpr float kRow3 = 262144.0f;            // 2^24 * 4^-3
-
-// The eight operand registers of one 32-bit word `w` of codes (bytes b0..b3; the
-// halves of a register are MMA k-slots): lo[e] = code e of bytes (b0, b2),
-// hi[e] = code e of bytes (b1, b3).
-struct CodeRegs { uint32_t lo[4], hi[4]; };
-__device__ __forceinline__ CodeRegs code_regs(uint32_t w) {
-    const uint32_t ws = swap_bytes_in_halves(w);
-    CodeRegs r;
-    r.lo[0] = code_pair<4>(ws); r.hi[0] = code_pair<4>(w);
-    r.lo[1] = code_pair<1>(w);  r.hi[1] = code_pair<1>(ws);
-    r.lo[2] = code_pair<2>(w);  r.hi[2] = code_pair<2>(ws);
-    r.lo[3] = code_pair<3>(w);  r.hi[3] = code_pair<3>(ws);
-    return r;
-}
+// q.k: M = 2^23 + 0x4b0000, |w * F| < 1.6 * 2^21: bytes 0 and 1 are digits, byte 2 is the top
+// digit plus 0x4b, byte 3 the constant 0x4b -- whose column is 0x4b * sum of the codes,
+// which is what the top digit's bias adds up to.  22 bits and a sign, against 22 bits of
+// each single element in an fp16 hi/lo pair whose sums the tensor core truncates at 20.
+// p.v: M = 2^23, 0 <= w * F <= 65535: two digits.
+// F follows the largest |w| of a stage and head: the bits of a positive float subtracted from
+// a constant give a float y with x * y between 2 and 2.25 times a power of two.
+//
+// Integer accumulators start at the bits of 2^23: read as floats they are 2^23 + sum, since
+// the sums stay below 2^23 (128 * 255 * 255), and differences of them are exact.
+constexpr float kTwo23 = 8388608.0f;
+constexpr int kTwo23Bits = 0x4b000000;
+constexpr float kMagicK = 8388608.0f + 4915200.0f;        // 2^23 + 0x4b0000
+constexpr float kSmallest = 7.888609052210118e-31f;       // 2^-100: weights below it count as zero beside it
+constexpr uint32_t kExponent = 0x7f800000u, kSmallestBits = 27u << 23;
+constexpr uint32_t kInverseK = 275u << 23;                // largest |w * F| is 2^21 .. 1.125 * 2^21
+constexpr uint32_t kInverseV = 269u << 23;                // 2^15 .. 1.125 * 2^15, and then times kFillV
+constexpr float kFillV = 1.7777f;                         // below 65535 / (1.125 * 2^15)
+constexpr float kGrowth = 8.0f;                           // weights up to 2^8 are let stand before the running maximum moves
 
 struct WarpState {
     float m, l;            // running max / sum of head `tig` (score layout)
-    float o[8][2];         // p.v sums of 8 channel tiles, rows gid / gid+8 (they still carry 4^I * 2^-24)
-    float oz[2];           // zero-point term of head gid>>1, channel groups 2*part and 2*part+1, partial over lanes
+    float o[8][2];         // p.v sums of head tig: channel 32*(t/2) + 4*gid + 2*(t%2) + r, times 4^(2*(t%2) + r)
+    float oz[4][4];        // zero-point term [head][channel group] of the tokens this lane weighs
 };
 
-// ---- one token group (32 tokens) in three phases ----------------------------------
-// q.k: scores of the lane's four tokens (4*gid + e) for head `tig`, log2 domain.
-// `qx` points at the lane's query slice in shared memory (head hB, pre-scaled,
-// channel 4*tig), `qzp`/`kz` at the slice the lane owns for the zero term: the
-// hi lane of a column pair takes the even 16-channel steps, the lo lane the odd
-// ones, so the dot product q.z is computed once, not twice.
-__device__ __forceinline__ void qk_phase(
-    const uint8_t* __restrict__ kc, const float* __restrict__ ks, const float* __restrict__ kz,
-    const float* __restrict__ qx, const float* __restrict__ qzp, uint32_t part_mask, int gid, int tig, float (&s)[4]) {
-    float c0[KIVI_MMA_CHAINS][4], c1[KIVI_MMA_CHAINS][4];
-    float qz = 0.0f;
+// what a lane holds for the whole kernel
+struct LaneView {
+    int gid, tig, lane;
+    float qk[4][4];        // [i][head]: pre-scaled queries of channel k_channel(lane, i)
+    float4 qz[4];          // head tig, channels 4 * zero_quad(i, gid) .. + 3
+    uint32_t scratch;      // the warp's 2 KB of shared memory for operands on their way from lane to lane
+    uint32_t k_rows, v_rows;   // row addresses of ldmatrix_t8 for the q.k and the p.v operand
+    uint32_t p_even, p_odd;    // where it leaves the weights of tokens 4*gid + 0, 2 and + 1, 3
+    uint32_t p_read, v_write;
+    int v_first;               // value words: contraction half read first
+    int start[4];              // 2^23 in each accumulator register
+};
+// The zero term q.z of a group: lane (gid, tig) takes head tig and the 16 channels 16*gid ..,
+// in an order that keeps the lanes of a half-warp off each other's banks.
+__device__ __forceinline__ int zero_quad(int i, int gid) { return 4 * gid + ((i + gid) & 3); }
+// The q.k operand of a group: one 16-byte row per pair of channels 16 apart (the two halves
+// of a 32-channel contraction step) and half of the columns; lane 8*j + y makes the rows of
+// step j and channels 2*y, 2*y + 1 of each half.  In odd steps the second half comes first,
+// so that the scales are read without bank conflicts.
+__device__ __forceinline__ int k_channel(int l, int i) {
+    const int j = l >> 3;
+    return 32 * j + 16 * ((i >> 1) ^ (j & 1)) + 2 * (l & 7) + (i & 1);
+}
+// Row of the weights of the token whose scales are row r of the group (kivi_common.cuh:
+// token 16*kappa + 4*c + n at row 16*kappa + 4*n + c), for the same reason.
+__device__ __forceinline__ int p_row(int r) { return r ^ ((r >> 4) << 2); }
+
+// ---- plain fp32 forms for values that no fixed-point number holds ------------------
+// (infinities and NaN in the queries, scales or weights, negative value scales):
+// dequantize as the fp32 kernels do, code * scale + zero.
+__device__ __noinline__ float4 scores_plain(const uint8_t* kc, const float* ks, const float* kz, const float4* q4, int gid) {
+    float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 1
+    for (int c4 = 0; c4 < 32; ++c4) {
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(kc + kblock_offset(4 * c4, gid, 8, 64));
+        const float4 s = *reinterpret_cast<const float4*>(ks + 4 * c4), z = *reinterpret_cast<const float4*>(kz + 4 * c4);
+        const float4 q = q4[c4];
+        const float sv[4] = {s.x, s.y, s.z, s.w}, zv[4] = {z.x, z.y, z.z, z.w}, qv[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-    for (int qh = 0; qh < 2; ++qh) {
-        const uint4 wv = *reinterpret_cast<const uint4*>(kc + qh * 512 + gid * 64 + tig * 16);
-        const uint32_t w[4] = {wv.x, wv.y, wv.z, wv.w};
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const int kt = 4 * qh + m;
-            const int ch = 64 * qh + 16 * m;                 // + 4*tig through the lane pointers
-            const float4 s4 = *reinterpret_cast<const float4*>(ks + ch);
-            const float4 q4 = *reinterpret_cast<const float4*>(qx + ch);
-            if ((m & 1) == 0) {                              // channel steps kt, kt+1 -> one of them per lane
-                const float4 z4 = *reinterpret_cast<const float4*>(kz + ch);
-                const float4 y4 = *reinterpret_cast<const float4*>(qzp + ch);
-                qz = fmaf(y4.x, z4.x, qz); qz = fmaf(y4.y, z4.y, qz);
-                qz = fmaf(y4.z, z4.z, qz); qz = fmaf(y4.w, z4.w, qz);
-            }
-            const float x0 = q4.x * s4.x, x1 = q4.y * s4.y, x2 = q4.z * s4.z, x3 = q4.w * s4.w;
-            // fp16 hi/lo split of q*s: hi lanes keep x truncated to 11 significant
-            // bits, lo lanes keep the remainder (part_mask = 0 on hi lanes)
-            const float r0 = x0 - __uint_as_float(__float_as_uint(x0) & part_mask);
-            const float r1 = x1 - __uint_as_float(__float_as_uint(x1) & part_mask);
-            const float r2 = x2 - __uint_as_float(__float_as_uint(x2) & part_mask);
-            const float r3 = x3 - __uint_as_float(__float_as_uint(x3) & part_mask);
-            const uint32_t b0 = pack_f16_rz(r0, r2);
-            const uint32_t b1 = pack_f16_rz(r1, r3);
-            const CodeRegs cr = code_regs(w[m]);
-            uint32_t a[4];
-            a[0] = cr.lo[0]; a[1] = cr.lo[1]; a[2] = cr.hi[0]; a[3] = cr.hi[1];          // tokens 4*gid, 4*gid + 1
-            if (kt < KIVI_MMA_CHAINS) mma_f16_first(c0[kt % KIVI_MMA_CHAINS], a, b0, b1);
-            else mma_f16(c0[kt % KIVI_MMA_CHAINS], a, b0, b1);
-            a[0] = cr.lo[2]; a[1] = cr.lo[3]; a[2] = cr.hi[2]; a[3] = cr.hi[3];          // tokens 4*gid + 2, + 3
-            if (kt < KIVI_MMA_CHAINS) mma_f16_first(c1[kt % KIVI_MMA_CHAINS], a, b0, b1);
-            else mma_f16(c1[kt % KIVI_MMA_CHAINS], a, b0, b1);
+            for (int n = 0; n < 4; ++n) a[n] = fmaf(qv[i], fmaf((float)((w >> (8 * i + 2 * n)) & 3u), sv[i], zv[i]), a[n]);
+    }
+    return make_float4(a[0], a[1], a[2], a[3]);
+}
+// channels 32*gd + 4*gid + 0..3 of one head
+__device__ __noinline__ float4 weighted_plain(const uint8_t* vc, const float* vs, const float* vz, const float* p, int gd, int gid, int tig) {
+    float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 1
+    for (int r = 0; r < 32; ++r) {
+        const int kap = r >> 4, n = (r >> 2) & 3, c = r & 3;
+        const uint32_t b = vc[(gd * 64 + kap * 32 + gid * 4 + c) * 4 + n];
+        const float s = vs[4 * r + gd], z = vz[4 * r + gd], ph = p[4 * p_row(r) + tig];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = fmaf(ph, fmaf((float)((b >> (2 * i)) & 3u), s, z), a[i]);
+    }
+    return make_float4(a[0], a[1], a[2], a[3]);
+}
+
+// ---- NG token groups (32 tokens each) in three phases -------------------------------
+// q.k: scores of the lane's four tokens (4*gid + n) of each group for head `tig`, log2 domain.
+template <int NG>
+__device__ __forceinline__ void qk_phase(const uint8_t* __restrict__ kc, const float* __restrict__ ks, const float* __restrict__ kz,
+                                         const LaneView& v, uint8_t* scratch, float (&s)[NG][4]) {
+    float w[NG][4][4], top[4] = {kSmallest, kSmallest, kSmallest, kSmallest}, qz[NG];
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+        const float2 sa = *reinterpret_cast<const float2*>(ks + 128 * g + k_channel(v.lane, 0)), sb = *reinterpret_cast<const float2*>(ks + 128 * g + k_channel(v.lane, 2));
+        const float sv[4] = {sa.x, sa.y, sb.x, sb.y};
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[g][i][h] = v.qk[i][h] * sv[i];
+            top[h] = max3_abs_nan(w[g][2][h], w[g][3][h], max3_abs_nan(w[g][0][h], w[g][1][h], top[h]));
         }
     }
 #pragma unroll
-    for (int step = KIVI_MMA_CHAINS / 2; step >= 1; step /= 2)
+    for (int h = 0; h < 4; ++h) top[h] = warp_max_abs_nan(top[h]);
 #pragma unroll
-        for (int ch_ = 0; ch_ < step; ++ch_)
+    for (int g = 0; g < NG; ++g) {
+        float z0 = 0.0f, z1 = 0.0f;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { c0[ch_][i] += c0[ch_ + step][i]; c1[ch_][i] += c1[ch_ + step][i]; }
-    // zero term of head gid>>1: the eight lanes of a column pair hold disjoint partials
-    qz += __shfl_xor_sync(0xffffffffu, qz, 1);
-    qz += __shfl_xor_sync(0xffffffffu, qz, 2);
-    qz += __shfl_xor_sync(0xffffffffu, qz, 4);
-    const float qz_t = __shfl_sync(0xffffffffu, qz, 8 * tig);
-    s[0] = fmaf(c0[0][0] + c0[0][1], kRow0, qz_t);   // token 4*gid
-    s[1] = fmaf(c0[0][2] + c0[0][3], kRow1, qz_t);   // token 4*gid + 1
-    s[2] = fmaf(c1[0][0] + c1[0][1], kRow2, qz_t);   // token 4*gid + 2
-    s[3] = fmaf(c1[0][2] + c1[0][3], kRow3, qz_t);   // token 4*gid + 3
+        for (int i = 0; i < 4; ++i) {
+            const float4 z = *reinterpret_cast<const float4*>(kz + 128 * g + 4 * zero_quad(i, v.gid));
+            z0 = fmaf(v.qz[i].x, z.x, z0); z1 = fmaf(v.qz[i].y, z.y, z1);
+            z0 = fmaf(v.qz[i].z, z.z, z0); z1 = fmaf(v.qz[i].w, z.w, z1);
+        }
+        qz[g] = z0 + z1;
+    }
+#pragma unroll
+    for (int off = 4; off <= 16; off *= 2)
+#pragma unroll
+        for (int g = 0; g < NG; ++g) qz[g] += __shfl_xor_sync(0xffffffffu, qz[g], off);
+    __syncwarp();                                           // the scratch is free
+    if (!((top[0] + top[1]) + (top[2] + top[3]) <= 3.0e38f)) {
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sts32(v.scratch + h * 512 + 4 * k_channel(v.lane, i), v.qk[i][h]);
+        __syncwarp();
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+            const float4 r = scores_plain(kc + 1024 * g, ks + 128 * g, kz + 128 * g, reinterpret_cast<const float4*>(scratch) + 32 * v.tig, v.gid);
+            s[g][0] = r.x; s[g][1] = r.y; s[g][2] = r.z; s[g][3] = r.w;
+        }
+        return;
+    }
+    float F[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) F[h] = __uint_as_float(kInverseK - __float_as_uint(top[h]));
+    const float unit = rcp_approx(v.tig == 0 ? F[0] : v.tig == 1 ? F[1] : v.tig == 2 ? F[2] : F[3]);
+    int c[NG][2][2][4];                                     // [rows of codes 0,1 / 2,3 and up][digits 0,1 / 2,const]
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+        if (g > 0) __syncwarp();                            // the operand of the group before has been read
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            uint32_t x[2][4];
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+#pragma unroll
+                for (int h = 0; h < 4; ++h) x[k][h] = __float_as_uint(fmaf(w[g][2 * k + e][h], F[h], kMagicK));
+            // columns: digits 0 and 1 of the four heads; digit 2 and the constant
+            sts128(v.scratch + 512 * e + 16 * v.lane, __byte_perm(x[0][0], x[0][1], 0x5410), __byte_perm(x[0][2], x[0][3], 0x5410),
+                   __byte_perm(x[1][0], x[1][1], 0x5410), __byte_perm(x[1][2], x[1][3], 0x5410));
+            sts128(v.scratch + 1024 + 512 * e + 16 * v.lane, __byte_perm(x[0][0], x[0][1], 0x7632), __byte_perm(x[0][2], x[0][3], 0x7632),
+                   __byte_perm(x[1][0], x[1][1], 0x7632), __byte_perm(x[1][2], x[1][3], 0x7632));
+        }
+        __syncwarp();
+        uint32_t b[4][4];                                   // step j: both halves of columns 0-7, of columns 8-15
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ldmatrix_t8(b[j], v.k_rows + 128 * j);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const uint4 wv = *reinterpret_cast<const uint4*>(kc + 1024 * g + half * 512 + v.gid * 64 + v.tig * 16);
+            const uint32_t cw[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+            for (int m = 0; m < 4; m += 2) {
+                const int j = 2 * half + m / 2;
+                const uint32_t wa = cw[m + (j & 1)], wb = cw[m + 1 - (j & 1)];
+#pragma unroll
+                for (int d = 0; d < 2; ++d) {
+                    if (j == 0) {
+                        mma_u8_from(v.start, c[g][0][d], wa, wa & kFrom1, wb, wb & kFrom1, b[j][2 * d], b[j][2 * d + 1]);
+                        mma_u8_from(v.start, c[g][1][d], wa & kFrom2, wa & kFrom3, wb & kFrom2, wb & kFrom3, b[j][2 * d], b[j][2 * d + 1]);
+                    } else {
+                        mma_u8(c[g][0][d], wa, wa & kFrom1, wb, wb & kFrom1, b[j][2 * d], b[j][2 * d + 1]);
+                        mma_u8(c[g][1][d], wa & kFrom2, wa & kFrom3, wb & kFrom2, wb & kFrom3, b[j][2 * d], b[j][2 * d + 1]);
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+        float y[5][3];                                      // digit 0, digit 1, unbiased digit 2 of the sums "code n and up"
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            const int t = n >> 1, r = 2 * (n & 1);
+            y[n][0] = __int_as_float(c[g][t][0][r]); y[n][1] = __int_as_float(c[g][t][0][r + 1]);
+            y[n][2] = __int_as_float(c[g][t][1][r]) - __int_as_float(c[g][t][1][r + 1]);
+        }
+        y[4][0] = kTwo23; y[4][1] = kTwo23; y[4][2] = 0.0f;
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            const float d0 = y[n][0] - y[n + 1][0], d1 = y[n][1] - y[n + 1][1], d2 = y[n][2] - y[n + 1][2];
+            const float row = n == 0 ? 1.0f : n == 1 ? kRow1 : n == 2 ? kRow2 : kRow3;
+            s[g][n] = fmaf(fmaf(d2, 65536.0f, fmaf(d1, 256.0f, d0)), unit * row, qz[g]);
+        }
+    }
 }
 
 // running max / sum update for NG groups at once; turns scores into weights
 template <int NG>
-__device__ __forceinline__ void softmax_phase(float (&s)[NG][4], int gid, int lane, WarpState& st) {
+__device__ __forceinline__ void softmax_phase(float (&s)[NG][4], WarpState& st) {
     float gmax = -INFINITY;
 #pragma unroll
     for (int g = 0; g < NG; ++g)
 #pragma unroll
         for (int e = 0; e < 4; ++e) gmax = fmaxf(gmax, s[g][e]);
-    gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 4));
-    gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 8));
-    gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 16));
-    if (__any_sync(0xffffffffu, gmax > st.m)) {
+    if (__any_sync(0xffffffffu, gmax > st.m + kGrowth)) {
+        gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 4));
+        gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 8));
+        gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 16));
         const float m_new = fmaxf(st.m, gmax);
         const float alpha = ex2(st.m - m_new);         // 0 when st.m == -inf
         st.m = m_new;
         st.l *= alpha;
 #pragma unroll
         for (int mt = 0; mt < 8; ++mt) { st.o[mt][0] *= alpha; st.o[mt][1] *= alpha; }
-        const float alpha_b = __shfl_sync(0xffffffffu, alpha, (lane & ~3) | (gid >> 1));
-        st.oz[0] *= alpha_b; st.oz[1] *= alpha_b;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const float alpha_h = __shfl_sync(0xffffffffu, alpha, h);
+#pragma unroll
+            for (int gd = 0; gd < 4; ++gd) st.oz[h][gd] *= alpha_h;
+        }
     }
 #pragma unroll
     for (int g = 0; g < NG; ++g)
@@ -234,99 +365,118 @@ __device__ __forceinline__ void softmax_phase(float (&s)[NG][4], int gid, int la
         for (int e = 0; e < 4; ++e) { s[g][e] = ex2(s[g][e] - st.m); st.l += s[g][e]; }
 }
 
-// p.v of one group; p[n] = weight of token 4*gid + n for head tig.
+// p.v of NG groups; p[g][n] = weight of token 4*gid + n of group g for head tig.
+// The weights first change hands: a lane comes to hold the four heads of the token whose
+// scales are row `lane` of the group, multiplies them with the four scales, and the digits
+// go out as rows of 16 bytes -- one per token and pair of channel groups, columns
+// [channel group][head][digit] -- that ldmatrix_t8 hands back as tensor-core operands.
 // Value block words (kivi_common.cuh): word (gd, kappa, r, c) holds natural byte
-// 8*gd + r (channels 32*gd + 4*r + i) of tokens 16*kappa + 4*c + n in bytes n.
-// A lane (gid, tig) reads word (gd, kappa, gid, tig): bytes 0/2 are its k-slots
-// 2tig / 2tig+1, bytes 1/3 its k-slots 2tig+8 / 2tig+9 (code_regs).
-// The hi and the lo lane of a column pair (gid, gid^1) hold the same head and the
-// same tokens, and only the hi lane's B column is ever read.  So the pair splits
-// the work by channel group: the hi lane builds p*s and the zero term for groups
-// 0,1, the lo lane for groups 2,3, and one exchange hands the hi lane the
-// operands it lacks (what the lo lane feeds into its own column is never read).
-template <bool FIRST>
-__device__ __forceinline__ void pv_phase(
-    const uint8_t* __restrict__ vc, const float* __restrict__ vs, const float* __restrict__ vz,
-    const float (&p)[4], int part, int gid, int tig, float (&acc)[8][4], WarpState& st) {
-    const uint32_t* vw = reinterpret_cast<const uint32_t*>(vc) + gid * 4 + tig;
+// 8*gd + r (channels 32*gd + 4*r + i) of tokens 16*kappa + 4*c + n in bytes n: four
+// consecutive contraction indices, as the tensor core wants them.
+template <int NG>
+__device__ __forceinline__ void pv_phase(const uint8_t* __restrict__ vc, const float* __restrict__ vs, const float* __restrict__ vz,
+                                         const float (&p)[NG][4], const LaneView& v, uint8_t* scratch, WarpState& st) {
+    __syncwarp();                                           // the scratch is free
 #pragma unroll
-    for (int kap = 0; kap < 2; ++kap) {
-        const int src = 4 * (4 * kap + tig) + (gid >> 1);   // lane holding tokens 16*kap + 4*tig + n, head gid>>1
-        float pe[4];
+    for (int g = 0; g < NG; ++g) {
+        sts32(v.p_even + 512 * g, p[g][0]); sts32(v.p_even + 512 * g + 128, p[g][2]);
+        sts32(v.p_odd + 512 * g, p[g][1]); sts32(v.p_odd + 512 * g + 128, p[g][3]);
+    }
+    __syncwarp();
+    float ph[NG][4], sv[NG][4];                             // weights [head], scales [channel group] of the lane's token
+    uint32_t top[4] = {kSmallestBits, kSmallestBits, kSmallestBits, kSmallestBits};
 #pragma unroll
-        for (int n = 0; n < 4; ++n) pe[n] = __shfl_sync(0xffffffffu, p[n], src);
-        // scales / zeros of token 16*kap + 4*tig + n sit at row 16*kap + 4*n + tig;
-        // the lane takes the two channel groups 2*part, 2*part + 1 of each row
-        float2 sv[4], zv[4];
+    for (int g = 0; g < NG; ++g) {
+        const float4 p4 = lds128(v.p_read + 512 * g);
+        const float4 s4 = *reinterpret_cast<const float4*>(vs + g * 128 + 4 * v.lane);
+        ph[g][0] = p4.x; ph[g][1] = p4.y; ph[g][2] = p4.z; ph[g][3] = p4.w;
+        sv[g][0] = s4.x; sv[g][1] = s4.y; sv[g][2] = s4.z; sv[g][3] = s4.w;
+        // as integers, the bits of negative numbers, infinities and NaN all lie above those of a finite one
+        const float smax = __uint_as_float(max(max(__float_as_uint(s4.x), __float_as_uint(s4.y)), max(__float_as_uint(s4.z), __float_as_uint(s4.w))));
 #pragma unroll
-        for (int n = 0; n < 4; ++n) {
-            sv[n] = *reinterpret_cast<const float2*>(vs + (16 * kap + 4 * n + tig) * 4 + 2 * part);
-            zv[n] = *reinterpret_cast<const float2*>(vz + (16 * kap + 4 * n + tig) * 4 + 2 * part);
-        }
+        for (int h = 0; h < 4; ++h) top[h] = max(top[h], __float_as_uint(ph[g][h] * smax));
+    }
 #pragma unroll
-        for (int n = 0; n < 4; ++n) {
-            st.oz[0] = fmaf(pe[n], zv[n].x, st.oz[0]);
-            st.oz[1] = fmaf(pe[n], zv[n].y, st.oz[1]);
-        }
-        uint32_t own[2][2], got[2][2];
-        own[0][0] = pack_f16_rn(pe[0] * sv[0].x, pe[2] * sv[2].x);     // k-slots 2tig, 2tig+1: tokens n = 0, 2
-        own[0][1] = pack_f16_rn(pe[1] * sv[1].x, pe[3] * sv[3].x);     // k-slots 2tig+8, +9:   tokens n = 1, 3
-        own[1][0] = pack_f16_rn(pe[0] * sv[0].y, pe[2] * sv[2].y);
-        own[1][1] = pack_f16_rn(pe[1] * sv[1].y, pe[3] * sv[3].y);
+    for (int h = 0; h < 4; ++h) top[h] = warp_max_u32(top[h]);
+    if (max(max(top[0], top[1]), max(top[2], top[3])) >= kExponent) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int g = 0; g < NG; ++g)
 #pragma unroll
-            for (int j = 0; j < 2; ++j) got[i][j] = __shfl_xor_sync(0xffffffffu, own[i][j], 4);
+            for (int gd = 0; gd < 4; ++gd) {
+                const float4 r = weighted_plain(vc + g * 1024, vs + g * 128, vz + g * 128, reinterpret_cast<const float*>(scratch + 512 * g), gd, v.gid, v.tig);
+                st.o[2 * gd][0] += r.x; st.o[2 * gd][1] += 4.0f * r.y;
+                st.o[2 * gd + 1][0] += 16.0f * r.z; st.o[2 * gd + 1][1] += 64.0f * r.w;
+            }
+        return;
+    }
 #pragma unroll
-        for (int gd = 0; gd < 4; ++gd) {
-            const uint32_t b0 = gd < 2 ? own[gd][0] : got[gd - 2][0];
-            const uint32_t b1 = gd < 2 ? own[gd][1] : got[gd - 2][1];
-            const CodeRegs cr = code_regs(vw[gd * 64 + kap * 32]);
-            uint32_t a[4];
-            a[0] = cr.lo[0]; a[1] = cr.lo[1]; a[2] = cr.hi[0]; a[3] = cr.hi[1];          // channels 4*gid, 4*gid + 1 of the group
-            if (FIRST && kap == 0) mma_f16_first(acc[2 * gd], a, b0, b1);
-            else mma_f16(acc[2 * gd], a, b0, b1);
-            a[0] = cr.lo[2]; a[1] = cr.lo[3]; a[2] = cr.hi[2]; a[3] = cr.hi[3];
-            if (FIRST && kap == 0) mma_f16_first(acc[2 * gd + 1], a, b0, b1);
-            else mma_f16(acc[2 * gd + 1], a, b0, b1);
+    for (int g = 0; g < NG; ++g) {
+        const float4 z4 = *reinterpret_cast<const float4*>(vz + g * 128 + 4 * v.lane);
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            st.oz[h][0] = fmaf(ph[g][h], z4.x, st.oz[h][0]); st.oz[h][1] = fmaf(ph[g][h], z4.y, st.oz[h][1]);
+            st.oz[h][2] = fmaf(ph[g][h], z4.z, st.oz[h][2]); st.oz[h][3] = fmaf(ph[g][h], z4.w, st.oz[h][3]);
         }
     }
-}
-
-// NG consecutive token groups of one pipeline stage, processed together: the
-// q.k and p.v phases of the groups are independent instruction streams, the
-// softmax update is done once for all NG*32 tokens.
-struct LaneView {
-    const float* qx;       // q_s + head*kD + 4*tig
-    const float* qzp;      // qx + 16*part
-    uint32_t part_mask;    // 0 on hi lanes, "keep 11 significant bits" on lo lanes
-    int part, gid, tig, lane;
-};
-
-template <int NG>
-__device__ __forceinline__ void process_groups(const uint8_t* __restrict__ sb, const LaneView& v, WarpState& st) {
-    float s[NG][4];
+    float F[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) F[h] = __uint_as_float(kInverseV - top[h]) * kFillV;
+    const float unit = rcp_approx(v.tig == 0 ? F[0] : v.tig == 1 ? F[1] : v.tig == 2 ? F[2] : F[3]);
+    __syncwarp();                                           // every lane has read its weights
+    // Rows of 16 bytes per channel group and contraction index k = 4*c + n: the columns
+    // [head][digit] of tokens 16*0 + k and 16*1 + k, in the other order for k >= 8 (the writes
+    // of a half-warp then touch every bank once; the codes are read in that order too).
 #pragma unroll
     for (int g = 0; g < NG; ++g)
-        qk_phase(sb + g * 1024, reinterpret_cast<const float*>(sb + kGPS * 1024 + g * 512) + 4 * v.tig,
-                 reinterpret_cast<const float*>(sb + kGPS * 1536 + g * 512) + 4 * v.tig + 16 * v.part,
-                 v.qx, v.qzp, v.part_mask, v.gid, v.tig, s[g]);
-    softmax_phase<NG>(s, v.gid, v.lane, st);
-    // The tensor core adds each product into its fp32 accumulator with
-    // truncation; against an accumulator that has grown over thousands of tokens
-    // that is a biased loss (all addends p*s*c are positive) which the later
-    // cancellation with the zero term amplifies.  So the MMAs of this stage go
-    // into fresh accumulators and join the running sums through ordinary adds
-    // (only the even columns are ever read).
-    float acc[8][4];
-    pv_phase<true>(sb + kGPS * 2048, reinterpret_cast<const float*>(sb + kGPS * 3072),
-                   reinterpret_cast<const float*>(sb + kGPS * 3584), s[0], v.part, v.gid, v.tig, acc, st);
 #pragma unroll
-    for (int g = 1; g < NG; ++g)
-        pv_phase<false>(sb + kGPS * 2048 + g * 1024, reinterpret_cast<const float*>(sb + kGPS * 3072 + g * 512),
-                        reinterpret_cast<const float*>(sb + kGPS * 3584 + g * 512), s[g], v.part, v.gid, v.tig, acc, st);
+        for (int gd = 0; gd < 4; ++gd) {
+            uint32_t x[4];
 #pragma unroll
-    for (int mt = 0; mt < 8; ++mt) { st.o[mt][0] += acc[mt][0]; st.o[mt][1] += acc[mt][2]; }
+            for (int h = 0; h < 4; ++h) x[h] = __float_as_uint(fmaf(ph[g][h] * sv[g][gd], F[h], kTwo23));
+            sts64(v.v_write + 1024 * g + 256 * gd, __byte_perm(x[0], x[1], 0x5410), __byte_perm(x[2], x[3], 0x5410));
+        }
+    __syncwarp();
+    int acc[8][4];
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+        const uint32_t* vw = reinterpret_cast<const uint32_t*>(vc + g * 1024) + v.lane;
+#pragma unroll
+        for (int gp = 0; gp < 2; ++gp) {
+            uint32_t b[4];
+            ldmatrix_t8(b, v.v_rows + 1024 * g + 512 * gp);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int gd = 2 * gp + e;
+                const uint32_t w0 = vw[gd * 64 + v.v_first], w1 = vw[gd * 64 + (v.v_first ^ 32)];
+                if (g == 0) {
+                    mma_u8_from(v.start, acc[2 * gd], w0, w0 & kFrom1, w1, w1 & kFrom1, b[2 * e], b[2 * e + 1]);
+                    mma_u8_from(v.start, acc[2 * gd + 1], w0 & kFrom2, w0 & kFrom3, w1 & kFrom2, w1 & kFrom3, b[2 * e], b[2 * e + 1]);
+                } else {
+                    mma_u8(acc[2 * gd], w0, w0 & kFrom1, w1, w1 & kFrom1, b[2 * e], b[2 * e + 1]);
+                    mma_u8(acc[2 * gd + 1], w0 & kFrom2, w0 & kFrom3, w1 & kFrom2, w1 & kFrom3, b[2 * e], b[2 * e + 1]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int gd = 0; gd < 4; ++gd)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int mt = 2 * gd + (i >> 1), r = 2 * (i & 1), mt1 = 2 * gd + ((i + 1) >> 1), r1 = 2 * ((i + 1) & 1);
+            const float n0 = i < 3 ? __int_as_float(acc[i < 3 ? mt1 : 0][r1]) : kTwo23, n1 = i < 3 ? __int_as_float(acc[i < 3 ? mt1 : 0][r1 + 1]) : kTwo23;
+            const float d0 = __int_as_float(acc[mt][r]) - n0, d1 = __int_as_float(acc[mt][r + 1]) - n1;
+            st.o[mt][i & 1] = fmaf(fmaf(d1, 256.0f, d0), unit, st.o[mt][i & 1]);
+        }
+}
+
+// NG consecutive token groups of one pipeline stage: the softmax update and the reading of
+// the p.v accumulators are done once for all NG*32 tokens.
+template <int NG>
+__device__ __forceinline__ void process_groups(const uint8_t* __restrict__ sb, const LaneView& v, uint8_t* scratch, WarpState& st) {
+    float s[NG][4];
+    qk_phase<NG>(sb, reinterpret_cast<const float*>(sb + kGPS * 1024), reinterpret_cast<const float*>(sb + kGPS * 1536), v, scratch, s);
+    softmax_phase<NG>(s, st);
+    pv_phase<NG>(sb + kGPS * 2048, reinterpret_cast<const float*>(sb + kGPS * 3072), reinterpret_cast<const float*>(sb + kGPS * 3584), s, v, scratch, st);
 }
 
 // ---- residual ring: full-precision tokens ---------------------------------------
@@ -359,6 +509,29 @@ template <> struct RowVec<__nv_bfloat16> {
         v[2] = __uint_as_float(t.y << 16); v[3] = __uint_as_float(t.y & 0xffff0000u);
     }
 };
+
+// The queries a lane holds, pre-scaled.  All loads are issued before the first is used
+// (absent heads read the last one's again and count as zero): one trip to memory, where a
+// branch around each load made twelve (3 us of a CTA's start).
+template <typename T>
+__device__ __forceinline__ void load_queries(const T* __restrict__ q, int n_heads, float scale_log2, LaneView& v) {
+    float a[4][4], b[4][4], z[4][4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const T* row = q + (h < n_heads ? h : n_heads - 1) * kD;
+        RowVec<T>::load4(row + (k_channel(v.lane, 0) & ~3), a[h]);
+        RowVec<T>::load4(row + (k_channel(v.lane, 2) & ~3), b[h]);
+        RowVec<T>::load4(q + (v.tig < n_heads ? v.tig : n_heads - 1) * kD + 4 * zero_quad(h, v.gid), z[h]);
+    }
+    const bool upper = v.lane & 1;                           // channels 2, 3 of a quad
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const float f = h < n_heads ? scale_log2 : 0.0f, fz = v.tig < n_heads ? scale_log2 : 0.0f;
+        v.qk[0][h] = h < n_heads ? f * (upper ? a[h][2] : a[h][0]) : 0.0f; v.qk[1][h] = h < n_heads ? f * (upper ? a[h][3] : a[h][1]) : 0.0f;
+        v.qk[2][h] = h < n_heads ? f * (upper ? b[h][2] : b[h][0]) : 0.0f; v.qk[3][h] = h < n_heads ? f * (upper ? b[h][3] : b[h][1]) : 0.0f;
+        v.qz[h] = v.tig < n_heads ? make_float4(fz * z[h][0], fz * z[h][1], fz * z[h][2], fz * z[h][3]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+}
 
 template <typename T>
 __device__ __forceinline__ void residual_part(
@@ -475,24 +648,25 @@ __device__ __forceinline__ void residual_part(
 // batch 16 x 4k).  Partial slots: quantized piece i -> i, residual part r ->
 // nq_splits + r.
 //
-// Shared memory: [kWarps][kStages][kStageBytes] stage rings | q_s [4][128] fp32
-// (the CTA's up to four query heads times sm_scale*log2(e), absent rows zero) | mbarriers |
-// (max, sum) of the warps.  When a warp is done, its ring doubles as the
-// [4][128] buffer its scaled output goes to; the CTA then adds the warps'
+// Shared memory: [kWarps][kStages][kStageBytes] stage rings | [kWarps][kScratchBytes]
+// (in ring CTAs the first holds the queries, [4][128] fp32 times sm_scale*log2(e), absent
+// rows zero) | mbarriers | (max, sum) of the warps.  When a warp is done, its ring doubles
+// as the [4][128] buffer its scaled output goes to; the CTA then adds the warps'
 // buffers in warp order (deterministic) and writes one partial.
 //
 // FOLD: the CTAs of a unit and head block are a cluster and fold their partials
 // themselves (a template, so that the wide grids keep their registers).
 template <bool FOLD>
-__global__ void __launch_bounds__(kWarps * 32, KIVI_MMA_MIN_CTAS)
+__global__ void __launch_bounds__(kWarps * 32, 3)
 attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
                 const void* q, int q_dtype,
                 float scale_log2, int n_rep, int gps, int nq_splits, int n_res_splits, int res_chunk,
                 float* __restrict__ part_o, float* __restrict__ part_ml, ClusterOut direct) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     uint8_t* stage_mem = smem_raw;                                               // [kWarps][kStages][kStageBytes]
-    float* q_s = reinterpret_cast<float*>(smem_raw + kWarps * kStages * kStageBytes);   // [4][128]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(q_s + 4 * kD);                  // [kWarps][kStages]
+    uint8_t* scratch_mem = smem_raw + kWarps * kStages * kStageBytes;            // [kWarps][kScratchBytes]
+    float* q_s = reinterpret_cast<float*>(scratch_mem);                          // [4][128], ring CTAs
+    uint64_t* bars = reinterpret_cast<uint64_t*>(scratch_mem + kWarps * kScratchBytes);   // [kWarps][kStages]
     float* ml_s = reinterpret_cast<float*>(bars + kWarps * kStages);             // [kWarps][4][2]
 
     // With a fold kernel behind this one, its few small blocks may become resident from
@@ -523,7 +697,7 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
     const int u = uv / head_blocks, head0 = 4 * (uv - u * head_blocks);
     const int n_heads = n_rep - head0 < 4 ? n_rep - head0 : 4;       // heads of this CTA: head0 .. head0 + n_heads - 1
     const int n_splits_total = nq_splits + n_res_splits;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);      // (known to be the same for all lanes)
     const int gid = lane >> 2, tig = lane & 3;
     uint8_t* wstage = stage_mem + warp * kStages * kStageBytes;
     float* fo = reinterpret_cast<float*>(wstage);                               // [4][128] once the ring is idle
@@ -539,25 +713,13 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
     const int my_n = n_chunks > warp ? (n_chunks - warp + kWarps - 1) / kWarps : 0;
     const uint32_t bar0 = smem_u32(bars + warp * kStages);
     const uint32_t stage0 = smem_u32(wstage);
-    // The six pieces of a chunk (key codes, scales, zeros, value codes, scales,
-    // zeros) are contiguous runs of 1024 or 512 bytes per token group; lane i < 6
-    // owns piece i and issues its copy, so a chunk costs one copy's instructions.
-    // Chunk c of this warp starts at group g_begin + (warp + kWarps*c)*kGPS.
-    const uint8_t* my_src = nullptr;
-    uint32_t my_bytes = 0, my_dst = 0;
+    // The six pieces of a chunk (key codes, scales, zeros, value codes, scales, zeros) are
+    // contiguous runs of 1024 or 512 bytes per token group.  One elected lane issues them
+    // from addresses that are the same for the whole warp (a bulk copy takes its operands
+    // from uniform registers: six lanes with an address each cost a loop of some 70
+    // instructions).  Chunk c of this warp starts at group g_begin + (warp + kWarps*c)*kGPS.
     if (!is_res) {
-        const uint8_t* base = lane == 0 ? L.k_codes
-                            : lane == 1 ? reinterpret_cast<const uint8_t*>(L.k_scales)
-                            : lane == 2 ? reinterpret_cast<const uint8_t*>(L.k_zeros)
-                            : lane == 3 ? L.v_codes
-                            : lane == 4 ? reinterpret_cast<const uint8_t*>(L.v_scales)
-                                        : reinterpret_cast<const uint8_t*>(L.v_zeros);
-        my_bytes = (lane == 0 || lane == 3) ? 1024u : 512u;
-        my_dst = lane == 0 ? 0u : lane == 1 ? kGPS * 1024u : lane == 2 ? kGPS * 1536u
-               : lane == 3 ? kGPS * 2048u : lane == 4 ? kGPS * 3072u : kGPS * 3584u;
-        const int64_t gw0 = (int64_t)u * (L.max_tokens / kG) + g_begin + (int64_t)warp * kGPS;
-        my_src = base + gw0 * my_bytes;
-        if (lane == 0) {
+        if (elect_one()) {
 #pragma unroll
             for (int s = 0; s < kStages; ++s) mbar_init(bar0 + 8 * s, 1);
             mbar_init_fence();
@@ -565,37 +727,38 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
         __syncwarp();
     }
     const uint64_t policy = l2_stream_policy();
+    const int64_t gw0 = (int64_t)u * (L.max_tokens / kG) + g_begin + (int64_t)warp * kGPS;
     auto issue = [&](int c) {                 // all lanes call it
         const int goff = (warp + kWarps * c) * kGPS;             // groups from g_begin
-        const int ng = (n_my_groups - goff) < kGPS ? (n_my_groups - goff) : kGPS;
+        const uint32_t ng = (n_my_groups - goff) < kGPS ? (n_my_groups - goff) : kGPS;
         const int s = c % kStages;
-        const uint32_t bar = bar0 + 8 * s;
-        if (lane == 0) mbar_expect_tx(bar, (uint32_t)ng * kGroupBytes);
+        const uint32_t bar = bar0 + 8 * s, dst = stage0 + s * kStageBytes;
+        const int64_t g = gw0 + (int64_t)c * (kWarps * kGPS);
+        if (elect_one()) {
+            mbar_expect_tx(bar, ng * kGroupBytes);
+            bulk_g2s(dst, L.k_codes + g * 1024, ng * 1024, bar, policy);
+            bulk_g2s(dst + kGPS * 1024, L.k_scales + g * 128, ng * 512, bar, policy);
+            bulk_g2s(dst + kGPS * 1536, L.k_zeros + g * 128, ng * 512, bar, policy);
+            bulk_g2s(dst + kGPS * 2048, L.v_codes + g * 1024, ng * 1024, bar, policy);
+            bulk_g2s(dst + kGPS * 3072, L.v_scales + g * 128, ng * 512, bar, policy);
+            bulk_g2s(dst + kGPS * 3584, L.v_zeros + g * 128, ng * 512, bar, policy);
+        }
         __syncwarp();
-        if (lane < 6)
-            bulk_g2s(stage0 + s * kStageBytes + my_dst, my_src + (int64_t)c * (kWarps * kGPS) * my_bytes,
-                     (uint32_t)ng * my_bytes, bar, policy);
     };
     for (int c = 0; c < kStages && c < my_n; ++c) issue(c);
 
-    // ---- queries -> shared memory, pre-scaled -----------------------------------
-    {
-        for (int i = threadIdx.x; i < kD; i += blockDim.x) {             // 128 float4 = [4][128]
-            const int hh = i >> 5, cc = (i & 31) * 4;
-            float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            if (hh < n_heads) {
-                const int64_t e = ((int64_t)u * n_rep + head0 + hh) * kD + cc;
-                if (q_dtype == KIVI_BF16) RowVec<__nv_bfloat16>::load4(reinterpret_cast<const __nv_bfloat16*>(q) + e, v);
-                else RowVec<float>::load4(reinterpret_cast<const float*>(q) + e, v);
-            }
-            *reinterpret_cast<float4*>(q_s + hh * kD + cc) =
-                make_float4(scale_log2 * v[0], scale_log2 * v[1], scale_log2 * v[2], scale_log2 * v[3]);
-        }
-    }
-    __syncthreads();
-
+    const int64_t q_row = (int64_t)u * n_rep + head0;
     if (is_res) {
         // ---------------- residual ring ----------------
+        for (int i = threadIdx.x; i < kD; i += blockDim.x) {             // [4][128], pre-scaled (absent heads: zeros)
+            float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if ((i >> 5) < n_heads) {
+                if (q_dtype == KIVI_BF16) RowVec<__nv_bfloat16>::load4(reinterpret_cast<const __nv_bfloat16*>(q) + q_row * kD + 4 * i, t);
+                else RowVec<float>::load4(reinterpret_cast<const float*>(q) + q_row * kD + 4 * i, t);
+            }
+            *reinterpret_cast<float4*>(q_s + 4 * i) = make_float4(scale_log2 * t[0], scale_log2 * t[1], scale_log2 * t[2], scale_log2 * t[3]);
+        }
+        __syncthreads();
         const int rs = sub;
         const int t_begin = rs * res_chunk;
         const int t_end = t_begin + res_chunk < res_len ? t_begin + res_chunk : res_len;
@@ -628,30 +791,43 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
     } else {
         // ---------------- quantized history ----------------
         LaneView v;
-        v.part = gid & 1; v.gid = gid; v.tig = tig; v.lane = lane;
-        v.qzp = q_s + (gid >> 1) * kD + 4 * tig + 16 * v.part;
-        v.qx = q_s + (gid >> 1) * kD + 4 * tig;
-        v.part_mask = v.part ? 0xffffe000u : 0u;   // keep 11 significant bits
+        v.gid = gid; v.tig = tig; v.lane = lane;
+        uint8_t* scratch = scratch_mem + warp * kScratchBytes;
+        v.scratch = smem_u32(scratch);
+        // row `lane & 15` of matrix `lane >> 4`
+        v.k_rows = v.scratch + 1024 * (lane >> 4) + 512 * (lane & 1) + 16 * ((lane >> 1) & 7);
+        v.v_rows = v.scratch + 256 * (lane >> 4) + 16 * (lane & 15);
+        {
+            const int kap = gid >> 2, k = 4 * tig + (gid & 3);            // as token quad; as row `lane` of the scales
+            v.p_even = v.scratch + 16 * (16 * kap + (gid & 3)) + 64 * kap + 4 * tig;
+            v.p_odd = v.scratch + 16 * (16 * kap + (gid & 3)) + 64 * (1 - kap) + 4 * tig;
+            v.p_read = v.scratch + 16 * p_row(lane);
+            v.v_write = v.scratch + 16 * k + 8 * ((lane >> 4) ^ (k >> 3));
+            v.v_first = 32 * (tig >> 1);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) asm volatile("mov.b32 %0, %1;" : "=r"(v.start[i]) : "n"(kTwo23Bits));
+        if (q_dtype == KIVI_BF16) load_queries(reinterpret_cast<const __nv_bfloat16*>(q) + q_row * kD, n_heads, scale_log2, v);
+        else load_queries(reinterpret_cast<const float*>(q) + q_row * kD, n_heads, scale_log2, v);
 
         WarpState st;
         st.m = -INFINITY; st.l = 0.0f;
 #pragma unroll
         for (int mt = 0; mt < 8; ++mt) { st.o[mt][0] = 0.0f; st.o[mt][1] = 0.0f; }
-        st.oz[0] = 0.0f; st.oz[1] = 0.0f;
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+#pragma unroll
+            for (int gd = 0; gd < 4; ++gd) st.oz[h][gd] = 0.0f;
 
         bool ok = true;
         int c = 0;
         for (; c < my_n; ++c) {
             const int s = c % kStages;
-            if (!mbar_wait(bar0 + 8 * s, (uint32_t)(c / kStages) & 1u)) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, mbar_wait(bar0 + 8 * s, (uint32_t)(c / kStages) & 1u))) { ok = false; break; }
             const int goff = (warp + kWarps * c) * kGPS;
             const uint8_t* sb = wstage + s * kStageBytes;
-#if KIVI_MMA_GPS == 2
-            if (n_my_groups - goff >= 2) process_groups<2>(sb, v, st);
-            else process_groups<1>(sb, v, st);
-#else
-            process_groups<1>(sb, v, st);
-#endif
+            if (n_my_groups - goff >= 2) process_groups<2>(sb, v, scratch, st);
+            else process_groups<1>(sb, v, scratch, st);
             __syncwarp();
             if (c + kStages < my_n) issue(c + kStages);
         }
@@ -666,23 +842,29 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
             st.m = -INFINITY; st.l = 0.0f;
 #pragma unroll
             for (int mt = 0; mt < 8; ++mt) { st.o[mt][0] = 0.0f; st.o[mt][1] = 0.0f; }
-            st.oz[0] = 0.0f; st.oz[1] = 0.0f;
+#pragma unroll
+            for (int h = 0; h < 4; ++h)
+#pragma unroll
+                for (int gd = 0; gd < 4; ++gd) st.oz[h][gd] = 0.0f;
         }
 
         // ---- fold the warp's lanes ----------------------------------------------
         st.l += __shfl_xor_sync(0xffffffffu, st.l, 4);
         st.l += __shfl_xor_sync(0xffffffffu, st.l, 8);
         st.l += __shfl_xor_sync(0xffffffffu, st.l, 16);
-        // zero term: lanes (gid, *) hold head gid>>1, channel groups 2*(gid&1) + {0, 1}
-        float ozt[4];
+        // zero term: every lane holds partial sums of all heads and channel groups
+        float* const oz_s = reinterpret_cast<float*>(scratch);                  // [lane][head][channel group]
+        __syncwarp();
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            float z = st.oz[i];
-            z += __shfl_xor_sync(0xffffffffu, z, 1);
-            z += __shfl_xor_sync(0xffffffffu, z, 2);
-            ozt[i] = __shfl_sync(0xffffffffu, z, 8 * tig);          // head tig, group i     <- hi lanes of gid 2*tig
-            ozt[2 + i] = __shfl_sync(0xffffffffu, z, 8 * tig + 4);  // head tig, group 2 + i <- lo lanes
-        }
+        for (int h = 0; h < 4; ++h) *reinterpret_cast<float4*>(oz_s + 16 * lane + 4 * h) = make_float4(st.oz[h][0], st.oz[h][1], st.oz[h][2], st.oz[h][3]);
+        __syncwarp();
+        float z = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) z += oz_s[16 * ((lane & 16) + i) + (lane & 15)];
+        z += __shfl_xor_sync(0xffffffffu, z, 16);
+        float ozt[4];                                                            // head tig
+#pragma unroll
+        for (int gd = 0; gd < 4; ++gd) ozt[gd] = __shfl_sync(0xffffffffu, z, 4 * tig + gd);
         if (gid == 0) { ml_s[(warp * 4 + tig) * 2] = st.m; ml_s[(warp * 4 + tig) * 2 + 1] = st.l; }
         __syncthreads();
         float M = -INFINITY;
@@ -693,8 +875,8 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
         for (int mt = 0; mt < 8; ++mt) {
             const int gd = mt >> 1;
             const int ch = 32 * gd + 4 * gid + 2 * (mt & 1);
-            // rows gid / gid+8 hold code index 2*(mt&1) / 2*(mt&1)+1 of their byte
-            const float r0 = (mt & 1) ? kRow2 : kRow0, r1 = (mt & 1) ? kRow3 : kRow1;
+            // code index 2*(mt&1) / 2*(mt&1)+1 of its byte
+            const float r0 = (mt & 1) ? kRow2 : 1.0f, r1 = (mt & 1) ? kRow3 : kRow1;
             *reinterpret_cast<float2*>(fo + tig * kD + ch) =
                 make_float2(f * fmaf(st.o[mt][0], r0, ozt[gd]), f * fmaf(st.o[mt][1], r1, ozt[gd]));
         }
@@ -732,8 +914,8 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
     if constexpr (FOLD) cluster_fold(cta_o, ml_out, n_heads, kD, (int64_t)u * n_rep + head0, direct);
 }
 
-constexpr size_t kSmemBytes = (size_t)kWarps * kStages * kStageBytes + 4 * kD * 4 + kWarps * kStages * 8 +
-                              kWarps * 4 * 2 * 4;
+constexpr size_t kSmemBytes = (size_t)kWarps * (kStages * kStageBytes + kScratchBytes) + kWarps * kStages * 8 + kWarps * 4 * 2 * 4;
+static_assert(kScratchBytes >= 4 * kD * 4, "ring CTAs keep the queries in the first warp's scratch");
 static_assert(kStages * kStageBytes >= 2 * 4 * kD * 4 + 32, "a warp's ring doubles as its [4][128] fold buffer, the first also holds the CTA's partial");
 static_assert(kWarps * 32 >= 32, "at least one warp");
 
@@ -799,8 +981,13 @@ int run_attn_mma(const kivi_layer* L, int64_t quant_len, int res_start, int res_
 // One m16n8k16 MMA per k: C = -1, products {1 * 1, 2^-a * 2^-b} with a + b = k.
 // If the unit kept every bit the result would be exactly 2^-k; it aligns the
 // addends on their exponent fields and truncates below a fixed distance from the
-// largest, so from some k on the small product is lost.  The kernel's accuracy
-// budget (code_regs above) assumes at least 24 bits.
+// largest, so from some k on the small product is lost.  (Why the kernel above
+// contracts bytes, whose sums are exact.)
+__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
 __global__ void mma_alignment_probe_kernel(int* kept_out) {
     const int lane = threadIdx.x, gid = lane >> 2, tig = lane & 3;
     int kept = 0;

@@ -663,6 +663,53 @@ def test_fold_in_a_cluster_gives_the_bits_of_the_fold_kernel(cabi, D, G, n_rep, 
             assert torch.equal(o1, o2) and torch.equal(l1, l2)
 
 
+@pytest.mark.parametrize("what", ["tiny", "huge", "mixed", "negative", "k_inf", "k_nan", "v_inf", "v_nan", "q_nan"])
+@pytest.mark.parametrize("tokens,n_rep", [(32, 1), (96, 4), (288, 3), (320, 8)])
+def test_attention_mma_at_the_edges_of_its_fixed_point_operands(cabi, what, tokens, n_rep):
+    """q*s and p*s go to the tensor cores as fixed-point numbers of the largest of a stage
+    (two groups; one at an odd end): scales of any size, of sizes far apart and negative
+    value scales give what the fp32 kernel gives; infinities and NaN come out where they do there.
+    A weight is off by 2^-16 of the stage's largest at most and its code is 3 at most; all 64
+    of a stage wrong the same way would be 64 * 3 * 2^-16 = 2.9e-3 of the largest value."""
+    U = 5
+    st = cabi.LayerStore(U, 128, 32, 128, tokens, torch.bfloat16, "cuda")
+    g = torch.Generator(device="cuda").manual_seed(tokens + n_rep)
+    for n in ("k_codes", "v_codes"):
+        getattr(st, n).random_(0, 256, generator=g)
+    for n, lo, hi in (("k_scales", 0.3, 1.2), ("v_scales", 0.3, 1.2), ("k_zeros", -2.0, -0.5), ("v_zeros", -2.0, -0.5)):
+        getattr(st, n).uniform_(lo, hi, generator=g)
+    st.quant_len = tokens
+    q = torch.randn(U, n_rep, 128, generator=g, device="cuda").bfloat16()
+    if what in ("tiny", "huge"):
+        f = 1e-30 if what == "tiny" else 1e30
+        for n in ("v_scales", "v_zeros"):
+            getattr(st, n).mul_(f)
+        for n in ("k_scales", "k_zeros"):
+            getattr(st, n).mul_(f)
+        q = (q.float() / f).bfloat16()
+    elif what == "mixed":                                       # one channel and one token a million times the others
+        st.k_scales[:, :, 7] *= 1e6
+        q[:, :, 7] *= 1e-6
+        st.v_scales.view(U, -1)[:, 5] *= 1e6
+    elif what == "negative":
+        st.v_scales.view(U, -1)[:, 11] *= -1
+        st.k_scales[:, 0, 3] *= -1
+    elif what in ("k_inf", "k_nan"):
+        st.k_scales[2, -1, 77] = float(what[2:])
+    elif what in ("v_inf", "v_nan"):
+        st.v_scales.view(U, -1)[2, 13] = float(what[2:])
+    elif what == "q_nan":
+        q[3, 0, 100] = float("nan")
+    got, want = (st.attention(q, n_rep=n_rep, path=p, out_dtype=torch.float32) for p in (cabi.ATTN_MMA, cabi.ATTN_FP32))
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert want.isfinite().any() and cabi.device_fault() == 0
+    if what in ("tiny", "huge", "mixed", "negative"):
+        assert want.isfinite().all()
+    ok = want.isfinite()
+    size = (st.v_scales.abs().nan_to_num(0, 0, 0).max() * 3 + st.v_zeros.abs().max()).item()
+    assert ((got - want)[ok].abs().max() / size).item() < 2.9e-3
+
+
 @pytest.mark.parametrize("D,dtype,U,n_rep", [(128, torch.bfloat16, 8, 4), (64, torch.float32, 12, 1), (128, torch.bfloat16, 200, 1), (32, torch.float32, 2, 2)])
 def test_queued_steps_equal_synchronised_steps(cabi, D, dtype, U, n_rep):
     """Launches overlap the kernels before them in their stream: append, flush,
