@@ -45,6 +45,7 @@
 #include <cuda_fp16.h>
 
 #include <atomic>
+#include <type_traits>
 
 namespace kivi {
 namespace {
@@ -86,6 +87,11 @@ __device__ __forceinline__ void sts64(uint32_t addr, uint32_t x, uint32_t y) {
     asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(addr), "r"(x), "r"(y) : "memory");
 }
 __device__ __forceinline__ void sts32(uint32_t addr, float x) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(x) : "memory"); }
+__device__ __forceinline__ float lds32(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
 __device__ __forceinline__ float4 lds128(uint32_t addr) {
     float4 v;
     asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
@@ -207,14 +213,15 @@ __device__ __noinline__ float4 scores_plain(const uint8_t* kc, const float* ks, 
     }
     return make_float4(a[0], a[1], a[2], a[3]);
 }
-// channels 32*gd + 4*gid + 0..3 of one head
+// channels 32*gd + 4*gid + 0..3 of one head (ONE: the only one, weights in the order of the scales)
+template <bool ONE>
 __device__ __noinline__ float4 weighted_plain(const uint8_t* vc, const float* vs, const float* vz, const float* p, int gd, int gid, int tig) {
     float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 1
     for (int r = 0; r < 32; ++r) {
         const int kap = r >> 4, n = (r >> 2) & 3, c = r & 3;
         const uint32_t b = vc[(gd * 64 + kap * 32 + gid * 4 + c) * 4 + n];
-        const float s = vs[4 * r + gd], z = vz[4 * r + gd], ph = p[4 * p_row(r) + tig];
+        const float s = vs[4 * r + gd], z = vz[4 * r + gd], ph = p[ONE ? r : 4 * p_row(r) + tig];
 #pragma unroll
         for (int i = 0; i < 4; ++i) a[i] = fmaf(ph, fmaf((float)((b >> (2 * i)) & 3u), s, z), a[i]);
     }
@@ -403,7 +410,7 @@ __device__ __forceinline__ void pv_phase(const uint8_t* __restrict__ vc, const f
         for (int g = 0; g < NG; ++g)
 #pragma unroll
             for (int gd = 0; gd < 4; ++gd) {
-                const float4 r = weighted_plain(vc + g * 1024, vs + g * 128, vz + g * 128, reinterpret_cast<const float*>(scratch + 512 * g), gd, v.gid, v.tig);
+                const float4 r = weighted_plain<false>(vc + g * 1024, vs + g * 128, vz + g * 128, reinterpret_cast<const float*>(scratch + 512 * g), gd, v.gid, v.tig);
                 st.o[2 * gd][0] += r.x; st.o[2 * gd][1] += 4.0f * r.y;
                 st.o[2 * gd + 1][0] += 16.0f * r.z; st.o[2 * gd + 1][1] += 64.0f * r.w;
             }
@@ -479,6 +486,225 @@ __device__ __forceinline__ void process_groups(const uint8_t* __restrict__ sb, c
     pv_phase<NG>(sb + kGPS * 2048, reinterpret_cast<const float*>(sb + kGPS * 3072), reinterpret_cast<const float*>(sb + kGPS * 3584), s, v, scratch, st);
 }
 
+// ---- one query head per KV head ------------------------------------------------------
+// With one head the columns that four would take hold other things instead: in q.k the two
+// groups of the stage (one operand for both, each lane reading the accumulators of its
+// group), in p.v the four channel groups (their contractions go to one accumulator, each
+// with the columns of the others at zero).  A quarter of the operand work, half of the
+// reading of accumulators.  256 units x 4k tokens 40.0 -> 31.3 us with the form for four
+// heads before, 512 x 8k 121 (fp16 form) -> 98, 32 x 8k 14.5 -> 11.5.
+struct OneView {
+    int gid, tig, lane;
+    float qk[4];           // pre-scaled query, channel k_channel(lane, i)
+    float4 qz[4];          // channels 4 * zero_quad_one(i, gid, tig) .. + 3
+    uint32_t scratch, k_rows, v_rows, p_write, v_write;
+    int v_first;
+    int start[4];
+};
+struct OneState {
+    float m, l;            // running max; sum over the lane's tokens
+    float o[4];            // channel 32*tig + 4*gid + i, times 4^i
+    float oz[4];           // zero-point term [channel group] of the tokens this lane weighs
+};
+// Zero term: lane (gid, tig) takes group tig; odd and even tig are two quads apart (bank conflicts).
+__device__ __forceinline__ int zero_quad_one(int i, int gid, int tig) { return 4 * gid + ((i + ((gid >> 1) & 1) + 2 * (tig & 1)) & 3); }
+
+// scores of the lane's tokens 4*gid + n of group tig (lanes with tig >= NG: -inf)
+template <int NG>
+__device__ __forceinline__ void qk_one(const uint8_t* __restrict__ kc, const float* __restrict__ ks, const float* __restrict__ kz,
+                                       const OneView& v, uint8_t* scratch, float (&s)[4]) {
+    float w[2][4], top = kSmallest;
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[g][i] = 0.0f;
+        if (g < NG) {
+            const float2 sa = *reinterpret_cast<const float2*>(ks + 128 * g + k_channel(v.lane, 0)), sb = *reinterpret_cast<const float2*>(ks + 128 * g + k_channel(v.lane, 2));
+            w[g][0] = v.qk[0] * sa.x; w[g][1] = v.qk[1] * sa.y; w[g][2] = v.qk[2] * sb.x; w[g][3] = v.qk[3] * sb.y;
+            top = max3_abs_nan(w[g][2], w[g][3], max3_abs_nan(w[g][0], w[g][1], top));
+        }
+    }
+    top = warp_max_abs_nan(top);
+    const int mine = v.tig < NG ? v.tig : 0;
+    float z0 = 0.0f, z1 = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 z = *reinterpret_cast<const float4*>(kz + 128 * mine + 4 * zero_quad_one(i, v.gid, v.tig));
+        z0 = fmaf(v.qz[i].x, z.x, z0); z1 = fmaf(v.qz[i].y, z.y, z1);
+        z0 = fmaf(v.qz[i].z, z.z, z0); z1 = fmaf(v.qz[i].w, z.w, z1);
+    }
+    float qz = z0 + z1;
+#pragma unroll
+    for (int off = 4; off <= 16; off *= 2) qz += __shfl_xor_sync(0xffffffffu, qz, off);
+    __syncwarp();                                           // the scratch is free
+    if (!(top <= 3.0e38f)) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sts32(v.scratch + 4 * k_channel(v.lane, i), v.qk[i]);
+        __syncwarp();
+        const float4 r = scores_plain(kc + 1024 * mine, ks + 128 * mine, kz + 128 * mine, reinterpret_cast<const float4*>(scratch), v.gid);
+        s[0] = r.x; s[1] = r.y; s[2] = r.z; s[3] = r.w;
+    } else {
+        const float F = __uint_as_float(kInverseK - __float_as_uint(top)), unit = rcp_approx(F);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            uint32_t x[2][2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+#pragma unroll
+                for (int g = 0; g < 2; ++g) x[k][g] = __float_as_uint(fmaf(w[g][2 * k + e], F, kMagicK));
+            // columns: digits 0 and 1 of the two groups; digit 2 and the constant
+            sts128(v.scratch + 512 * e + 16 * v.lane, __byte_perm(x[0][0], x[0][1], 0x5410), 0u, __byte_perm(x[1][0], x[1][1], 0x5410), 0u);
+            sts128(v.scratch + 1024 + 512 * e + 16 * v.lane, __byte_perm(x[0][0], x[0][1], 0x7632), 0u, __byte_perm(x[1][0], x[1][1], 0x7632), 0u);
+        }
+        __syncwarp();
+        uint32_t b[4][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ldmatrix_t8(b[j], v.k_rows + 128 * j);
+        int c[NG][2][2][4];
+#pragma unroll
+        for (int g = 0; g < NG; ++g)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint4 wv = *reinterpret_cast<const uint4*>(kc + 1024 * g + (j >> 1) * 512 + v.gid * 64 + v.tig * 16);
+                const uint32_t wa = j & 1 ? wv.w : wv.x, wb = j & 1 ? wv.z : wv.y;
+#pragma unroll
+                for (int d = 0; d < 2; ++d) {
+                    if (j == 0) {
+                        mma_u8_from(v.start, c[g][0][d], wa, wa & kFrom1, wb, wb & kFrom1, b[j][2 * d], b[j][2 * d + 1]);
+                        mma_u8_from(v.start, c[g][1][d], wa & kFrom2, wa & kFrom3, wb & kFrom2, wb & kFrom3, b[j][2 * d], b[j][2 * d + 1]);
+                    } else {
+                        mma_u8(c[g][0][d], wa, wa & kFrom1, wb, wb & kFrom1, b[j][2 * d], b[j][2 * d + 1]);
+                        mma_u8(c[g][1][d], wa & kFrom2, wa & kFrom3, wb & kFrom2, wb & kFrom3, b[j][2 * d], b[j][2 * d + 1]);
+                    }
+                }
+            }
+        float y[5][3];
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            const int t = n >> 1, r = 2 * (n & 1);
+            auto pick = [&](int d, int k) { return __int_as_float(NG == 2 && (v.tig & 1) ? c[NG - 1][t][d][r + k] : c[0][t][d][r + k]); };
+            y[n][0] = pick(0, 0); y[n][1] = pick(0, 1); y[n][2] = pick(1, 0) - pick(1, 1);
+        }
+        y[4][0] = kTwo23; y[4][1] = kTwo23; y[4][2] = 0.0f;
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            const float row = n == 0 ? 1.0f : n == 1 ? kRow1 : n == 2 ? kRow2 : kRow3;
+            s[n] = fmaf(fmaf(y[n][2] - y[n + 1][2], 65536.0f, fmaf(y[n][1] - y[n + 1][1], 256.0f, y[n][0] - y[n + 1][0])), unit * row, qz);
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < 4; ++n) s[n] = v.tig < NG ? s[n] : -INFINITY;
+}
+
+__device__ __forceinline__ void softmax_one(float (&s)[4], OneState& st) {
+    float gmax = fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3]));
+    if (__any_sync(0xffffffffu, gmax > st.m + kGrowth)) {
+#pragma unroll
+        for (int off = 1; off <= 16; off *= 2) gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, off));
+        const float m_new = fmaxf(st.m, gmax);
+        const float alpha = ex2(st.m - m_new);         // 0 when st.m == -inf
+        st.m = m_new;
+        st.l *= alpha;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { st.o[i] *= alpha; st.oz[i] *= alpha; }
+    }
+#pragma unroll
+    for (int n = 0; n < 4; ++n) { s[n] = ex2(s[n] - st.m); st.l += s[n]; }
+}
+
+template <int NG>
+__device__ __forceinline__ void pv_one(const uint8_t* __restrict__ vc, const float* __restrict__ vs, const float* __restrict__ vz,
+                                       const float (&p)[4], const OneView& v, uint8_t* scratch, OneState& st) {
+    __syncwarp();                                           // the scratch is free
+    if (v.tig < NG) {
+#pragma unroll
+        for (int n = 0; n < 4; ++n) sts32(v.p_write + 16 * n, p[n]);
+    }
+    __syncwarp();
+    float ph[NG], sv[NG][4];
+    uint32_t top = kSmallestBits;
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+        ph[g] = lds32(v.scratch + 128 * g + 4 * v.lane);
+        const float4 s4 = *reinterpret_cast<const float4*>(vs + g * 128 + 4 * v.lane);
+        sv[g][0] = s4.x; sv[g][1] = s4.y; sv[g][2] = s4.z; sv[g][3] = s4.w;
+        const float smax = __uint_as_float(max(max(__float_as_uint(s4.x), __float_as_uint(s4.y)), max(__float_as_uint(s4.z), __float_as_uint(s4.w))));
+        top = max(top, __float_as_uint(ph[g] * smax));
+    }
+    top = warp_max_u32(top);
+    if (top >= kExponent) {
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+            const float4 r = weighted_plain<true>(vc + g * 1024, vs + g * 128, vz + g * 128, reinterpret_cast<const float*>(scratch + 128 * g), v.tig, v.gid, 0);
+            st.o[0] += r.x; st.o[1] += 4.0f * r.y; st.o[2] += 16.0f * r.z; st.o[3] += 64.0f * r.w;
+        }
+        return;
+    }
+    const float F = __uint_as_float(kInverseV - top) * kFillV, unit = rcp_approx(F);
+    __syncwarp();                                           // every lane has read its weights
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+        const float4 z4 = *reinterpret_cast<const float4*>(vz + g * 128 + 4 * v.lane);
+        st.oz[0] = fmaf(ph[g], z4.x, st.oz[0]); st.oz[1] = fmaf(ph[g], z4.y, st.oz[1]);
+        st.oz[2] = fmaf(ph[g], z4.z, st.oz[2]); st.oz[3] = fmaf(ph[g], z4.w, st.oz[3]);
+        uint32_t x[4];
+#pragma unroll
+        for (int gd = 0; gd < 4; ++gd) x[gd] = __float_as_uint(fmaf(ph[g] * sv[g][gd], F, kTwo23));
+        sts64(v.v_write + 256 * g, __byte_perm(x[0], x[1], 0x5410), __byte_perm(x[2], x[3], 0x5410));       // columns [channel group][digit]
+    }
+    __syncwarp();
+    uint32_t b[4];
+    ldmatrix_t8(b, v.v_rows);                               // one matrix per group
+    int acc[2][4];
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+        const uint32_t* vw = reinterpret_cast<const uint32_t*>(vc + g * 1024) + v.lane;
+#pragma unroll
+        for (int gd = 0; gd < 4; ++gd) {
+            const uint32_t w0 = vw[gd * 64 + v.v_first], w1 = vw[gd * 64 + (v.v_first ^ 32)];
+            const bool own = (v.gid >> 1) == gd;             // the lane's column is of this channel group
+            const uint32_t b0 = own ? b[2 * g] : 0u, b1 = own ? b[2 * g + 1] : 0u;
+            if (g == 0 && gd == 0) {
+                mma_u8_from(v.start, acc[0], w0, w0 & kFrom1, w1, w1 & kFrom1, b0, b1);
+                mma_u8_from(v.start, acc[1], w0 & kFrom2, w0 & kFrom3, w1 & kFrom2, w1 & kFrom3, b0, b1);
+            } else {
+                mma_u8(acc[0], w0, w0 & kFrom1, w1, w1 & kFrom1, b0, b1);
+                mma_u8(acc[1], w0 & kFrom2, w0 & kFrom3, w1 & kFrom2, w1 & kFrom3, b0, b1);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = i >> 1, r = 2 * (i & 1), t1 = i < 3 ? (i + 1) >> 1 : 0, r1 = 2 * ((i + 1) & 1);
+        const float d0 = __int_as_float(acc[t][r]) - (i < 3 ? __int_as_float(acc[t1][r1]) : kTwo23);
+        const float d1 = __int_as_float(acc[t][r + 1]) - (i < 3 ? __int_as_float(acc[t1][r1 + 1]) : kTwo23);
+        st.o[i] = fmaf(fmaf(d1, 256.0f, d0), unit, st.o[i]);
+    }
+}
+
+template <int NG>
+__device__ __forceinline__ void process_groups(const uint8_t* __restrict__ sb, const OneView& v, uint8_t* scratch, OneState& st) {
+    float s[4];
+    qk_one<NG>(sb, reinterpret_cast<const float*>(sb + kGPS * 1024), reinterpret_cast<const float*>(sb + kGPS * 1536), v, scratch, s);
+    softmax_one(s, st);
+    pv_one<NG>(sb + kGPS * 2048, reinterpret_cast<const float*>(sb + kGPS * 3072), reinterpret_cast<const float*>(sb + kGPS * 3584), s, v, scratch, st);
+}
+
+__device__ __forceinline__ void clear(WarpState& st) {
+    st.m = -INFINITY; st.l = 0.0f;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) { st.o[t][0] = 0.0f; st.o[t][1] = 0.0f; }
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+#pragma unroll
+        for (int gd = 0; gd < 4; ++gd) st.oz[h][gd] = 0.0f;
+}
+__device__ __forceinline__ void clear(OneState& st) {
+    st.m = -INFINITY; st.l = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { st.o[i] = 0.0f; st.oz[i] = 0.0f; }
+}
+
 // ---- residual ring: full-precision tokens ---------------------------------------
 // CTA `rs` of the residual part handles window tokens [rs*chunk, (rs+1)*chunk).
 // A warp takes 32 tokens at a time: lane = (4 tokens, quarter of the channels)
@@ -531,6 +757,20 @@ __device__ __forceinline__ void load_queries(const T* __restrict__ q, int n_head
         v.qk[2][h] = h < n_heads ? f * (upper ? b[h][2] : b[h][0]) : 0.0f; v.qk[3][h] = h < n_heads ? f * (upper ? b[h][3] : b[h][1]) : 0.0f;
         v.qz[h] = v.tig < n_heads ? make_float4(fz * z[h][0], fz * z[h][1], fz * z[h][2], fz * z[h][3]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
+}
+
+template <typename T>
+__device__ __forceinline__ void load_queries(const T* __restrict__ q, int, float scale_log2, OneView& v) {
+    float a[4], b[4], z[4][4];
+    RowVec<T>::load4(q + (k_channel(v.lane, 0) & ~3), a);
+    RowVec<T>::load4(q + (k_channel(v.lane, 2) & ~3), b);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) RowVec<T>::load4(q + 4 * zero_quad_one(i, v.gid, v.tig), z[i]);
+    const bool upper = v.lane & 1;
+    v.qk[0] = scale_log2 * (upper ? a[2] : a[0]); v.qk[1] = scale_log2 * (upper ? a[3] : a[1]);
+    v.qk[2] = scale_log2 * (upper ? b[2] : b[0]); v.qk[3] = scale_log2 * (upper ? b[3] : b[1]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v.qz[i] = make_float4(scale_log2 * z[i][0], scale_log2 * z[i][1], scale_log2 * z[i][2], scale_log2 * z[i][3]);
 }
 
 template <typename T>
@@ -654,9 +894,10 @@ __device__ __forceinline__ void residual_part(
 // as the [4][128] buffer its scaled output goes to; the CTA then adds the warps'
 // buffers in warp order (deterministic) and writes one partial.
 //
+// ONE: one query head per KV head.
 // FOLD: the CTAs of a unit and head block are a cluster and fold their partials
 // themselves (a template, so that the wide grids keep their registers).
-template <bool FOLD>
+template <bool FOLD, bool ONE>
 __global__ void __launch_bounds__(kWarps * 32, 3)
 attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
                 const void* q, int q_dtype,
@@ -790,34 +1031,31 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
         }
     } else {
         // ---------------- quantized history ----------------
-        LaneView v;
+        std::conditional_t<ONE, OneView, LaneView> v;
         v.gid = gid; v.tig = tig; v.lane = lane;
         uint8_t* scratch = scratch_mem + warp * kScratchBytes;
         v.scratch = smem_u32(scratch);
         // row `lane & 15` of matrix `lane >> 4`
         v.k_rows = v.scratch + 1024 * (lane >> 4) + 512 * (lane & 1) + 16 * ((lane >> 1) & 7);
         v.v_rows = v.scratch + 256 * (lane >> 4) + 16 * (lane & 15);
-        {
-            const int kap = gid >> 2, k = 4 * tig + (gid & 3);            // as token quad; as row `lane` of the scales
+        // contraction index of the token whose scales are row `lane`
+        const int kap = gid >> 2, k = 4 * tig + (gid & 3);
+        v.v_write = v.scratch + 16 * k + 8 * (kap ^ (k >> 3));
+        v.v_first = 32 * (tig >> 1);
+        if constexpr (ONE) {
+            v.p_write = v.scratch + 128 * (tig & 1) + 4 * (16 * kap + (gid & 3));
+        } else {
             v.p_even = v.scratch + 16 * (16 * kap + (gid & 3)) + 64 * kap + 4 * tig;
             v.p_odd = v.scratch + 16 * (16 * kap + (gid & 3)) + 64 * (1 - kap) + 4 * tig;
             v.p_read = v.scratch + 16 * p_row(lane);
-            v.v_write = v.scratch + 16 * k + 8 * ((lane >> 4) ^ (k >> 3));
-            v.v_first = 32 * (tig >> 1);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) asm volatile("mov.b32 %0, %1;" : "=r"(v.start[i]) : "n"(kTwo23Bits));
         if (q_dtype == KIVI_BF16) load_queries(reinterpret_cast<const __nv_bfloat16*>(q) + q_row * kD, n_heads, scale_log2, v);
         else load_queries(reinterpret_cast<const float*>(q) + q_row * kD, n_heads, scale_log2, v);
 
-        WarpState st;
-        st.m = -INFINITY; st.l = 0.0f;
-#pragma unroll
-        for (int mt = 0; mt < 8; ++mt) { st.o[mt][0] = 0.0f; st.o[mt][1] = 0.0f; }
-#pragma unroll
-        for (int h = 0; h < 4; ++h)
-#pragma unroll
-            for (int gd = 0; gd < 4; ++gd) st.oz[h][gd] = 0.0f;
+        std::conditional_t<ONE, OneState, WarpState> st;
+        clear(st);
 
         bool ok = true;
         int c = 0;
@@ -837,48 +1075,60 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
             // those that were issued) a second bounded wait on its own phase
             // before the ring is reused, then report an empty partial.
             if (lane == 0) atomicExch(&g_fault_word, 1);
-            for (int k = c; k < c + kStages && k < my_n; ++k)
-                mbar_wait(bar0 + 8 * (k % kStages), (uint32_t)(k / kStages) & 1u);
-            st.m = -INFINITY; st.l = 0.0f;
-#pragma unroll
-            for (int mt = 0; mt < 8; ++mt) { st.o[mt][0] = 0.0f; st.o[mt][1] = 0.0f; }
-#pragma unroll
-            for (int h = 0; h < 4; ++h)
-#pragma unroll
-                for (int gd = 0; gd < 4; ++gd) st.oz[h][gd] = 0.0f;
+            for (int i = c; i < c + kStages && i < my_n; ++i)
+                mbar_wait(bar0 + 8 * (i % kStages), (uint32_t)(i / kStages) & 1u);
+            clear(st);
         }
 
         // ---- fold the warp's lanes ----------------------------------------------
-        st.l += __shfl_xor_sync(0xffffffffu, st.l, 4);
-        st.l += __shfl_xor_sync(0xffffffffu, st.l, 8);
-        st.l += __shfl_xor_sync(0xffffffffu, st.l, 16);
-        // zero term: every lane holds partial sums of all heads and channel groups
-        float* const oz_s = reinterpret_cast<float*>(scratch);                  // [lane][head][channel group]
-        __syncwarp();
+        if constexpr (ONE) {
 #pragma unroll
-        for (int h = 0; h < 4; ++h) *reinterpret_cast<float4*>(oz_s + 16 * lane + 4 * h) = make_float4(st.oz[h][0], st.oz[h][1], st.oz[h][2], st.oz[h][3]);
-        __syncwarp();
-        float z = 0.0f;
+            for (int off = 1; off <= 16; off *= 2) {
+                st.l += __shfl_xor_sync(0xffffffffu, st.l, off);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) z += oz_s[16 * ((lane & 16) + i) + (lane & 15)];
-        z += __shfl_xor_sync(0xffffffffu, z, 16);
-        float ozt[4];                                                            // head tig
+                for (int gd = 0; gd < 4; ++gd) st.oz[gd] += __shfl_xor_sync(0xffffffffu, st.oz[gd], off);
+            }
+            if (lane == 0) { ml_s[warp * 8] = st.m; ml_s[warp * 8 + 1] = st.l; }
+            __syncthreads();
+            float M = -INFINITY;
 #pragma unroll
-        for (int gd = 0; gd < 4; ++gd) ozt[gd] = __shfl_sync(0xffffffffu, z, 4 * tig + gd);
-        if (gid == 0) { ml_s[(warp * 4 + tig) * 2] = st.m; ml_s[(warp * 4 + tig) * 2 + 1] = st.l; }
-        __syncthreads();
-        float M = -INFINITY;
+            for (int w2 = 0; w2 < kWarps; ++w2) M = fmaxf(M, ml_s[w2 * 8]);
+            const float f = (st.m == -INFINITY) ? 0.0f : ex2(st.m - M);
+            const float z = tig == 0 ? st.oz[0] : tig == 1 ? st.oz[1] : tig == 2 ? st.oz[2] : st.oz[3];
+            *reinterpret_cast<float4*>(fo + 32 * tig + 4 * gid) =
+                make_float4(f * (st.o[0] + z), f * fmaf(st.o[1], kRow1, z), f * fmaf(st.o[2], kRow2, z), f * fmaf(st.o[3], kRow3, z));
+        } else {
+            st.l += __shfl_xor_sync(0xffffffffu, st.l, 4);
+            st.l += __shfl_xor_sync(0xffffffffu, st.l, 8);
+            st.l += __shfl_xor_sync(0xffffffffu, st.l, 16);
+            // zero term: every lane holds partial sums of all heads and channel groups
+            float* const oz_s = reinterpret_cast<float*>(scratch);                  // [lane][head][channel group]
+            __syncwarp();
 #pragma unroll
-        for (int w2 = 0; w2 < kWarps; ++w2) M = fmaxf(M, ml_s[(w2 * 4 + tig) * 2]);
-        const float f = (st.m == -INFINITY) ? 0.0f : ex2(st.m - M);
+            for (int h = 0; h < 4; ++h) *reinterpret_cast<float4*>(oz_s + 16 * lane + 4 * h) = make_float4(st.oz[h][0], st.oz[h][1], st.oz[h][2], st.oz[h][3]);
+            __syncwarp();
+            float z = 0.0f;
 #pragma unroll
-        for (int mt = 0; mt < 8; ++mt) {
-            const int gd = mt >> 1;
-            const int ch = 32 * gd + 4 * gid + 2 * (mt & 1);
-            // code index 2*(mt&1) / 2*(mt&1)+1 of its byte
-            const float r0 = (mt & 1) ? kRow2 : 1.0f, r1 = (mt & 1) ? kRow3 : kRow1;
-            *reinterpret_cast<float2*>(fo + tig * kD + ch) =
-                make_float2(f * fmaf(st.o[mt][0], r0, ozt[gd]), f * fmaf(st.o[mt][1], r1, ozt[gd]));
+            for (int i = 0; i < 16; ++i) z += oz_s[16 * ((lane & 16) + i) + (lane & 15)];
+            z += __shfl_xor_sync(0xffffffffu, z, 16);
+            float ozt[4];                                                            // head tig
+#pragma unroll
+            for (int gd = 0; gd < 4; ++gd) ozt[gd] = __shfl_sync(0xffffffffu, z, 4 * tig + gd);
+            if (gid == 0) { ml_s[(warp * 4 + tig) * 2] = st.m; ml_s[(warp * 4 + tig) * 2 + 1] = st.l; }
+            __syncthreads();
+            float M = -INFINITY;
+#pragma unroll
+            for (int w2 = 0; w2 < kWarps; ++w2) M = fmaxf(M, ml_s[(w2 * 4 + tig) * 2]);
+            const float f = (st.m == -INFINITY) ? 0.0f : ex2(st.m - M);
+#pragma unroll
+            for (int mt = 0; mt < 8; ++mt) {
+                const int gd = mt >> 1;
+                const int ch = 32 * gd + 4 * gid + 2 * (mt & 1);
+                // code index 2*(mt&1) / 2*(mt&1)+1 of its byte
+                const float r0 = (mt & 1) ? kRow2 : 1.0f, r1 = (mt & 1) ? kRow3 : kRow1;
+                *reinterpret_cast<float2*>(fo + tig * kD + ch) =
+                    make_float2(f * fmaf(st.o[mt][0], r0, ozt[gd]), f * fmaf(st.o[mt][1], r1, ozt[gd]));
+            }
         }
     }
     __syncthreads();
@@ -944,8 +1194,8 @@ static int ensure_smem_attr(int* dev_out) {
     KIVI_CUDA_OK(cudaGetDevice(&dev));
     KIVI_REQUIRE(dev >= 0 && dev < 64, "device ordinal %d out of range", dev);
     if (!attr_set[dev].load(std::memory_order_acquire)) {
-        KIVI_CUDA_OK(cudaFuncSetAttribute(attn_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
-        KIVI_CUDA_OK(cudaFuncSetAttribute(attn_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+        for (auto* kernel : {attn_mma_kernel<false, false>, attn_mma_kernel<true, false>, attn_mma_kernel<false, true>, attn_mma_kernel<true, true>})
+            KIVI_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
         attr_set[dev].store(true, std::memory_order_release);
     }
     if (dev_out) *dev_out = dev;
@@ -960,7 +1210,7 @@ int attn_mma_ctas_per_sm() {
     if (ensure_smem_attr(&dev) != KIVI_OK) return 0;
     int n = cached[dev].load(std::memory_order_acquire);
     if (n == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_mma_kernel<false>, kWarps * 32, kSmemBytes) != cudaSuccess || n <= 0)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_mma_kernel<false, false>, kWarps * 32, kSmemBytes) != cudaSuccess || n <= 0)
             return 0;
         cached[dev].store(n, std::memory_order_release);
     }
@@ -972,7 +1222,10 @@ int run_attn_mma(const kivi_layer* L, int64_t quant_len, int res_start, int res_
                  int n_res_splits, int res_chunk, float* part_o, float* part_ml, const ClusterOut& direct, cudaStream_t st) {
     if (int rc = ensure_smem_attr(nullptr)) return rc;
     dim3 grid((unsigned)(nq_splits + n_res_splits) * (unsigned)L->num_units * (unsigned)((n_rep + 3) / 4));
-    KIVI_CUDA_OK(launch_cluster(direct.out ? attn_mma_kernel<true> : attn_mma_kernel<false>, direct.out ? nq_splits + n_res_splits : 0, grid, kWarps * 32, kSmemBytes, st, true, *L, quant_len, res_start, res_len, q, q_dtype, scale_log2,
+    const bool fold = direct.out != nullptr;
+    auto* const kernel = n_rep == 1 ? (fold ? attn_mma_kernel<true, true> : attn_mma_kernel<false, true>)
+                                    : (fold ? attn_mma_kernel<true, false> : attn_mma_kernel<false, false>);
+    KIVI_CUDA_OK(launch_cluster(kernel, direct.out ? nq_splits + n_res_splits : 0, grid, kWarps * 32, kSmemBytes, st, true, *L, quant_len, res_start, res_len, q, q_dtype, scale_log2,
                         n_rep, gps, nq_splits, n_res_splits, res_chunk, part_o, part_ml, direct));
     return KIVI_OK;
 }
