@@ -124,12 +124,6 @@ __device__ __forceinline__ float rcp_approx(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p != 0;
-}
-
 // ---- operands ------------------------------------------------------------------
 // A byte of packed codes c0 + 4 c1 + 16 c2 + 64 c3 is itself a tensor-core operand, and so
 // are the bytes left by masking away c0; c0 and c1; c0, c1 and c2: three ANDs turn a 32-bit

@@ -62,6 +62,8 @@ int run_merge_token_shards(const float* parts, int n_shards, int64_t rows, int D
 int run_mma_alignment_probe(int* bits_out);
 int attn_mma_fault_word(int* out);
 int fp32_fault_word(int* out);
+int sample_fault_word(int* out);
+int sample_fault_clear();
 int fp32_fault_clear();
 int gather_fault_word(int* out);
 int attn_mma_fault_clear();
@@ -78,17 +80,19 @@ extern "C" int kivi_version(void) { return 100; }
 extern "C" int kivi_last_launch_count(void) { return g_launches; }
 extern "C" int kivi_device_fault(int* word_out) {
     KIVI_REQUIRE(word_out != nullptr, "word_out is null");
-    int copy_wait = 0, copy_wait_fp32 = 0, peer_wait = 0;
+    int copy_wait = 0, copy_wait_fp32 = 0, copy_wait_sample = 0, peer_wait = 0;
     if (int rc = attn_mma_fault_word(&copy_wait)) return rc;
     if (int rc = fp32_fault_word(&copy_wait_fp32)) return rc;
+    if (int rc = sample_fault_word(&copy_wait_sample)) return rc;
     if (int rc = gather_fault_word(&peer_wait)) return rc;
-    *word_out = (copy_wait || copy_wait_fp32 ? 1 : 0) | (peer_wait ? 2 : 0);
+    *word_out = (copy_wait || copy_wait_fp32 || copy_wait_sample ? 1 : 0) | (peer_wait ? 2 : 0);
     return KIVI_OK;
 }
 
 extern "C" int kivi_device_fault_clear(void) {
     if (int rc = attn_mma_fault_clear()) return rc;
     if (int rc = fp32_fault_clear()) return rc;
+    if (int rc = sample_fault_clear()) return rc;
     return gather_fault_clear();
 }
 

@@ -8,8 +8,10 @@
 // CDF in index order of a counter-based uniform number (Philox4x32-10 keyed by
 // (seed), counter (step, row)), so a CPU restatement reproduces it without
 // sharing any generator state, and the ids never have to leave the device.
+#include "async_copy.cuh"
 #include "kivi_common.cuh"
 
+#include <atomic>
 #include <type_traits>
 
 namespace kivi {
@@ -66,6 +68,75 @@ __device__ __forceinline__ uint32_t kth_key(uint32_t key, int k, int last_bit) {
     return t;
 }
 
+// A bound that at least k keys reach, for k up to an eighth of the threads, with two
+// barriers instead of sixteen: every warp finds its j-th largest key, and r warps (r j >= k)
+// reach the r-th largest of those.  About 1.7 k keys reach it, where the k-th largest is
+// reached by k; 1024 threads, k = 50: 2700 cycles by bisection, 600 this way (three bits
+// a step with counts by ballot and shared-memory atomics took 5000).
+template <int kWarps>
+__device__ __forceinline__ uint32_t bound_key(uint32_t key, int k, uint32_t* warp_s) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int j = (k + kWarps * 5 / 8 - 1) / (kWarps * 5 / 8), r = (k + j - 1) / j;
+    uint32_t largest = 0u;
+    for (int i = 0; i < j; ++i) {
+        largest = __reduce_max_sync(0xffffffffu, key);
+        const unsigned who = __ballot_sync(0xffffffffu, key == largest);
+        if (lane == __ffs(who) - 1) key = 0u;                // one of them is counted
+    }
+    if (lane == 0) warp_s[warp] = largest;
+    __syncthreads();
+    if (warp == 0) {                                        // (one warp: thirty-two would wait for each other's shuffles)
+        const uint32_t mine = lane < kWarps ? warp_s[lane] : 0u;
+        int before = 0;                                     // warps whose key comes before this lane's
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const uint32_t other = __shfl_sync(0xffffffffu, mine, w);
+            before += other > mine || (other == mine && w < lane);
+        }
+        if (lane < kWarps && before == r - 1) warp_s[kWarps] = mine;
+    }
+    __syncthreads();
+    return warp_s[kWarps];
+}
+
+__device__ __forceinline__ float max_nan(float a, float b) {              // NaN if either is
+    float d;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ float warp_max_nan(float a) {
+    float d;
+    asm volatile("redux.sync.max.NaN.f32 %0, %1, 0xffffffff;" : "=f"(d) : "f"(a));
+    return d;
+}
+// the entries of an aligned 16 bytes
+template <typename T> struct Granule;
+template <> struct Granule<float> {
+    static constexpr int kSize = 4;
+    __device__ static void load(const unsigned char* p, float (&x)[4]) {
+        const float4 v = *reinterpret_cast<const float4*>(p);
+        x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+    }
+};
+template <> struct Granule<__nv_bfloat16> {
+    static constexpr int kSize = 8;
+    __device__ static void load(const unsigned char* p, float (&x)[8]) {
+        const uint4 v = *reinterpret_cast<const uint4*>(p);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { x[2 * i] = __uint_as_float(w[i] << 16); x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
+    }
+};
+template <int N> __device__ __forceinline__ float largest(const float (&x)[N]) {
+    float m = max_nan(x[0], x[1]);
+#pragma unroll
+    for (int i = 2; i < N; i += 2) m = max_nan(m, max_nan(x[i], x[i + 1]));
+    return m;
+}
+
+__device__ int g_sample_fault = 0;
+constexpr int kChunks = 4;                 // pieces a staged row arrives in
+
 // Entries i0, i0 + step, ... of a row below `end`, kFlight loads in flight: whole blocks
 // of that many without a bounds test, the last one with.  (Indices are unsigned: a row
 // may have 2^31 - 1 entries, and the walk steps past its end.)
@@ -87,10 +158,11 @@ __device__ __forceinline__ void walk(const T* row, uint32_t i0, uint32_t end, ui
     }
 }
 
-// One CTA per row.  A row is a few hundred KB that one SM reads at its share of the
-// memory rate, so what counts is how often it is walked and how many loads are in
-// flight: one pass for the maximum (strided over the threads, coalesced, eight loads in
-// flight), one more to draw.
+// One CTA per row.  What a row costs is latency: how often it is walked, how many bytes are
+// in flight, and the barriers in between.  kStaged (rows that fit shared memory, one row per
+// SM): bulk copies bring the whole row into shared memory, everything in flight at once,
+// and both passes read it there, 16 bytes at a time: the maximum as the pieces arrive, then
+// the candidates or the draw.  Otherwise both passes read memory, strided over the threads.
 //
 // Top-k cut: at least k entries are >= the k-th largest of the threads' own maxima
 // (its upper 16 bits are bound enough), so one pass that collects the entries above
@@ -99,104 +171,231 @@ __device__ __forceinline__ void walk(const T* row, uint32_t i0, uint32_t end, ui
 // row again: an entry is kept when fewer than k are greater, which is what comparing
 // it with the k-th value says.  A larger k (cut_limit), more candidates than kCand (long
 // runs of equal logits) and rows with NaN take a radix select over the row instead.
-// 128 rows x 50257 fp32, top 50: 237 us with seven passes and two serial scans, 15 now.
+// 128 rows x 50257 fp32, top 50: 237 us with seven passes and two serial scans, 14.2 with two
+// passes over memory, bisection and one thread to a candidate, 10.6 now.
 //
 // What a call needs is a kernel of its own (Choice) and so is the number of threads a row
 // gets, so that the registers of one way do not cost another its occupancy.
 enum class Choice { kArgmax, kDraw, kTopK, kTopKRadix };
 
-template <typename T, int kThreads, Choice kChoice>
-__global__ void __launch_bounds__(kThreads, kThreads == 256 ? 8 : kThreads == 512 ? 3 : 1)
+template <typename T, int kThreads, Choice kChoice, bool kStaged>
+__global__ void __launch_bounds__(kThreads, kThreads == 256 ? 8 : kThreads == 512 && !kStaged ? 3 : 1)
 sample_kernel(const T* logits, int vocab, int64_t row_stride,
               float temperature, int top_k, uint64_t seed, uint64_t step, int64_t* __restrict__ ids) {
     constexpr int kWarps = kThreads / 32;
     constexpr int kFlight = kThreads == 256 && kChoice != Choice::kArgmax ? 4 : 8;     // (256: 32 registers, so that an SM holds eight rows)
     constexpr int kCand = cut_capacity(kThreads), kPer = (kCand + kThreads - 1) / kThreads;      // candidates; how many of them a thread ranks
+    constexpr bool kArg = kChoice == Choice::kArgmax;
     __shared__ float red_f[kWarps];
     __shared__ int red_i[kWarps];
     __shared__ double scan_s[kWarps];
     __shared__ int pick_s;
-    stream_order();
-    const T* row = settled(logits) + (int64_t)blockIdx.x * row_stride;
+    extern __shared__ __align__(128) unsigned char staged_s[];          // kStaged: the row at its own offset from a 16-byte boundary
     // the reference divides: logits / max(temperature, 1e-8)
     auto scaled = [&](float x) { return __fdiv_rn(x, temperature); };
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t n_row = (uint32_t)vocab;
-
-    // ---- row maximum and its first index (also the argmax answer) ----------------
-    MaxIdx best{-INFINITY, 0x7fffffff};
-    bool nan = false;
-    walk<kFlight>(row, tid, n_row, kThreads, [&](float x, uint32_t i) {
-        best = better(best, MaxIdx{x, (int)i});
-        if constexpr (kChoice == Choice::kTopK) nan |= x != x;
-    });
-    const MaxIdx mine_best = best;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        best = better(best, MaxIdx{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)});
-    if (lane == 0) { red_f[warp] = best.v; red_i[warp] = best.i; }
+    // (staged: worked out while the row is under way; else later, or it costs registers in the walk)
+    auto uniform = [&]() { return ((double)philox_first_word(seed, step, blockIdx.x) + 0.5) * (1.0 / 4294967296.0); };
+    double u = 0.0;
+    if constexpr (kStaged) u = uniform();
     if (tid == 0) pick_s = -1;
-    const bool row_nan = __syncthreads_or(nan);
-    best = MaxIdx{red_f[0], red_i[0]};
-    for (int w = 1; w < kWarps; ++w) best = better(best, MaxIdx{red_f[w], red_i[w]});
-    if (best.i == 0x7fffffff) best.i = 0;                  // a row of NaNs / -inf
-    if constexpr (kChoice == Choice::kArgmax) {
+    stream_order();
+    const T* const given = settled(logits) + (int64_t)blockIdx.x * row_stride;
+    const uint32_t skew = kStaged ? (uint32_t)(reinterpret_cast<uintptr_t>(given) & 15u) : 0u;
+    const T* const row = kStaged ? reinterpret_cast<const T*>(staged_s + skew) : given;
+
+    // largest entry and its first index; NaN does not count (a row of NaN: index 0)
+    auto find_best = [&](const T* from) {
+        MaxIdx best{-INFINITY, 0x7fffffff};
+        walk<kFlight>(from, tid, n_row, kThreads, [&](float x, uint32_t i) { best = better(best, MaxIdx{x, (int)i}); });
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            best = better(best, MaxIdx{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)});
+        if (lane == 0) { red_f[warp] = best.v; red_i[warp] = best.i; }
+        __syncthreads();
+        best = lane < kWarps ? MaxIdx{red_f[lane], red_i[lane]} : MaxIdx{-INFINITY, 0x7fffffff};
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            best = better(best, MaxIdx{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)});
+        if (best.i == 0x7fffffff) best.i = 0;
+        return best;
+    };
+    if constexpr (kArg) {
+        const MaxIdx best = find_best(row);
         if (tid == 0) ids[blockIdx.x] = best.i;
         return;
+    } else {
+    __shared__ uint32_t warp_key_s[kWarps + 1];
+    constexpr bool kCut = kChoice == Choice::kTopK;
+    __shared__ __align__(16) float cand_x[kCut ? kCand : 4];
+    __shared__ __align__(16) int cand_i[kCut ? kCand : 4];
+    __shared__ double cand_w[kCut ? kCand : 1];
+    __shared__ int n_cand_s;
+    if (kCut && tid == 0) n_cand_s = 0;                     // (barriers lie between this and its use)
+
+    // ---- largest entry of each thread and of the row (NaN if the row has one) ----------
+    float top = -INFINITY;
+    constexpr int kG = Granule<T>::kSize;
+    const uint32_t n_granules = (skew + n_row * (uint32_t)sizeof(T) + 15u) / 16u;       // kStaged
+    if constexpr (kStaged) {
+        __shared__ uint64_t bars[kChunks];
+        const uint32_t bar0 = smem_u32(bars);
+        const unsigned char* const base = reinterpret_cast<const unsigned char*>(given) - skew;
+        // granules that lie in the row as a whole are copied in kChunks pieces; the ragged
+        // ends are loaded entry by entry, places outside the row hold -inf
+        const uint32_t g0 = skew ? 1u : 0u, g1 = (skew + n_row * (uint32_t)sizeof(T)) / 16u;
+        const uint32_t per = g1 > g0 ? (g1 - g0 + kChunks - 1) / kChunks : 0u;
+        if (__shfl_sync(0xffffffffu, warp, 0) == 0 && elect_one()) {     // (operands of a bulk copy are the warp's, not a thread's)
+            const uint64_t policy = l2_stream_policy();
+#pragma unroll
+            for (int c = 0; c < kChunks; ++c) mbar_init(bar0 + 8 * c, 1);
+            mbar_init_fence();
+#pragma unroll
+            for (int c = 0; c < kChunks; ++c) {
+                const uint32_t from = g0 + c * per, to = min(from + per, g1);
+                if (from < to) {
+                    mbar_expect_tx(bar0 + 8 * c, (to - from) * 16u);
+                    bulk_g2s(smem_u32(staged_s) + from * 16u, base + (size_t)from * 16u, (to - from) * 16u, bar0 + 8 * c, policy);
+                }
+            }
+        }
+        for (int e = tid; e < 2 * kG; e += kThreads) {
+            const uint32_t g = e < kG ? 0u : n_granules - 1u;
+            if (e < kG ? g0 == 1u : (g1 < n_granules && (n_granules > 1u || g0 == 0u))) {
+                const int64_t i = (int64_t)(g * kG) + (e % kG) - (int64_t)(skew / sizeof(T));
+                const T x = i >= 0 && i < (int64_t)n_row ? given[i] : (T)(-INFINITY);
+                reinterpret_cast<T*>(staged_s)[g * kG + e % kG] = x;
+                top = max_nan(top, (float)x);
+            }
+        }
+        __syncthreads();                                    // the barriers are set up
+        bool arrived = true;
+        for (int c = 0; c < kChunks; ++c) {
+            const uint32_t from = g0 + c * per, to = min(from + per, g1);
+            if (from >= to) break;
+            if (!mbar_wait(bar0 + 8 * c, 0u)) { arrived = false; break; }
+            // (thread t takes granules t, t + kThreads, ... whatever the pieces)
+            for (uint32_t g = from + ((tid - from) & (kThreads - 1)); g < to; g += kThreads) {
+                float x[kG];
+                Granule<T>::load(staged_s + 16u * g, x);
+                top = max_nan(top, largest<kG>(x));
+            }
+        }
+        if (!__syncthreads_and(arrived)) {
+            // a copy did not land within the bound: raise the fault word, give all of them a
+            // second bounded wait, and read the row the plain way
+            if (tid == 0) atomicExch(&g_sample_fault, 1);
+            for (int c = 0; c < kChunks; ++c)
+                if (g0 + c * per < g1) mbar_wait(bar0 + 8 * c, 0u);
+            __syncthreads();
+            top = -INFINITY;
+            for (uint32_t i = tid; i < n_row; i += kThreads) {
+                const_cast<T*>(row)[i] = given[i];
+                top = max_nan(top, (float)given[i]);
+            }
+            __syncthreads();
+        }
+    } else {
+        walk<kFlight>(row, tid, n_row, kThreads, [&](float x, uint32_t) { top = max_nan(top, x); });
     }
-    const float m = scaled(best.v);
-    const double u = ((double)philox_first_word(seed, step, blockIdx.x) + 0.5) * (1.0 / 4294967296.0);
+    const float mine_top = top;
+    top = warp_max_nan(top);
+    if (lane == 0) red_f[warp] = top;
+    __syncthreads();
+    top = warp_max_nan(lane < kWarps ? red_f[lane] : -INFINITY);
+    const bool row_nan = top != top;                        // the same for all threads
+    if (row_nan) {
+        __syncthreads();
+        top = find_best(row).v;
+    }
+    const float m = scaled(top);
+    if constexpr (!kStaged) u = uniform();
+    // the fallback of a draw that finds no mass, called by one warp: first index of the maximum
+    auto argmax_index = [&]() {
+        int at = 0x7fffffff;
+        for (uint32_t i = lane; i < n_row && at == 0x7fffffff; i += 32)
+            if ((float)row[i] == top) at = (int)i;
+        at = __reduce_min_sync(0xffffffffu, at);
+        return at == 0x7fffffff ? 0 : at;
+    };
 
     float kth = -INFINITY;
-    if constexpr (kChoice == Choice::kTopK) {
-        __shared__ float cand_x[kCand];
-        __shared__ int cand_i[kCand];
-        __shared__ double cand_w[kCand];
-        __shared__ int n_cand_s;
-        if (tid == 0) n_cand_s = 0;                         // (the barriers of kth_key lie in between)
-        // largest scaled logit of this thread as a key; 0 (below every number's key) without one
-        const uint32_t my_key = mine_best.i == 0x7fffffff ? 0u : ordered_key(scaled(mine_best.v));
-        const uint32_t bound = row_nan ? 0u : kth_key(my_key, top_k, 16);
+    if constexpr (kCut) {
+        // A thread's largest logit as a key, of the logit itself: division by the temperature
+        // keeps the order.  (A thread without one: the key of -inf; fewer than k threads have
+        // one then, or the bound is no higher.)
+        const uint32_t my_key = ordered_key(mine_top);
+        const uint32_t bound = row_nan ? 0u : top_k <= kThreads / 8 ? bound_key<kWarps>(my_key, top_k, warp_key_s) : kth_key(my_key, top_k, 16);
         if (bound != 0u) {                                  // CTA-uniform
-            // compared as a number: -0 counts as +0, as in the cut itself (the keys between 0 and
-            // that of -inf are NaN patterns: cutting the lower bits may end there)
+            // Entries that the division rounds to the bound's quotient count too: the margin
+            // takes them in where quotients are normal numbers, else everything is taken (the
+            // keys between 0 and that of -inf are NaN patterns: cutting the lower bits may end there).
             const float least = bound < 0x007fffffu ? -INFINITY : key_to_float(bound);
-            // what is clearly below is dropped without a division (a quotient that lost bits in
-            // the subnormals does not say what is clear)
-            const float clear = fabsf(least) > 1e-30f && fabsf(least) < 1e30f ? (least - fabsf(least) * 1e-5f) * temperature : -INFINITY;
+            const float clear = fabsf(least) > 1e-20f && fabsf(least) < 1e20f && temperature < 1e8f ? least - fabsf(least) * 1e-5f : -INFINITY;
             // ---- collect what is not below the bound -------------------------------
-            walk<kFlight>(row, tid, n_row, kThreads, [&](float x, uint32_t i) {
+            auto collect = [&](float x, uint32_t i) {
                 if (!(x >= clear)) return;
-                const float y = scaled(x);
-                if (y >= least) {
-                    const int at = atomicAdd(&n_cand_s, 1);
-                    if (at < kCand) { cand_x[at] = y; cand_i[at] = (int)i; }
+                const int at = atomicAdd(&n_cand_s, 1);
+                if (at < kCand) { cand_x[at] = x; cand_i[at] = (int)i; }
+            };
+            if constexpr (kStaged) {
+                const uint32_t off = skew / (uint32_t)sizeof(T);
+#pragma unroll 4
+                for (uint32_t g = tid; g < n_granules; g += kThreads) {
+                    float x[kG];
+                    Granule<T>::load(staged_s + 16u * g, x);
+                    if (largest<kG>(x) >= clear) {
+#pragma unroll
+                        for (int e = 0; e < kG; ++e)
+                            if (g * kG + e - off < n_row) collect(x[e], g * kG + e - off);      // (unsigned: below the row counts as beyond)
+                    }
                 }
-            });
+            } else {
+                walk<kFlight>(row, tid, n_row, kThreads, collect);
+            }
             __syncthreads();
             const int n = n_cand_s;
             if (n <= kCand) {
-                // an entry's place in index order and how many are greater, by counting
-                float x[kPer];
-                int idx[kPer], place[kPer], greater[kPer];
+                // Scaled as the reference does; what only `clear` let through is below at least k
+                // others and falls out with them.
+                for (int c = tid; c < n; c += kThreads) cand_x[c] = scaled(cand_x[c]);
+                const int n4 = (n + 3) & ~3;                // (whole fours: beyond n is below everything)
+                if (tid < n4 - n) { cand_x[n + tid] = -INFINITY; cand_i[n + tid] = 0x7fffffff; }
+                __syncthreads();
+                // An entry's place in index order and how many are greater, by counting: as many
+                // threads to an entry as there are, each taking every `share`-th four others.
+                int share = 32;
+                while (share > 1 && (n * share > kThreads || 2 * share > n)) share >>= 1;
+                const int sub = tid & (share - 1), per_round = kThreads / share;
+                int idx[kPer], tally[kPer];                 // place | greater << 16
+                float w[kPer];
 #pragma unroll
                 for (int e = 0; e < kPer; ++e) {
-                    const int at = tid + e * kThreads;
-                    x[e] = at < n ? cand_x[at] : 0.0f;
-                    idx[e] = at < n ? cand_i[at] : 0;
-                    place[e] = greater[e] = 0;
-                    if (at < n)
-                        for (int c = 0; c < n; ++c) {
-                            place[e] += cand_i[c] < idx[e];
-                            greater[e] += cand_x[c] > x[e];
+                    const int at = tid / share + e * per_round;
+                    const bool valid = at < n;
+                    const float x = valid ? cand_x[at] : INFINITY;
+                    idx[e] = valid ? cand_i[at] : 0;
+                    int t = 0;
+                    if (valid) {
+#pragma unroll 2
+                        for (int c = 4 * sub; c < n; c += 4 * share) {
+                            const float4 xs = *reinterpret_cast<const float4*>(cand_x + c);
+                            const int4 is = *reinterpret_cast<const int4*>(cand_i + c);
+                            t += (is.x < idx[e]) + (is.y < idx[e]) + (is.z < idx[e]) + (is.w < idx[e]);
+                            t += (xs.x > x ? 65536 : 0) + (xs.y > x ? 65536 : 0) + (xs.z > x ? 65536 : 0) + (xs.w > x ? 65536 : 0);
                         }
+                    }
+                    for (int o = share >> 1; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+                    tally[e] = t;
+                    w[e] = x;
                 }
                 __syncthreads();                            // all have read the unsorted entries
 #pragma unroll
                 for (int e = 0; e < kPer; ++e)
-                    if (tid + e * kThreads < n) {
-                        cand_i[place[e]] = idx[e];
-                        cand_w[place[e]] = greater[e] < top_k ? (double)expf(x[e] - m) : 0.0;
+                    if (sub == 0 && tid / share + e * per_round < n) {
+                        cand_i[tally[e] & 0xffff] = idx[e];
+                        cand_w[tally[e] & 0xffff] = (tally[e] >> 16) < top_k ? (double)expf(w[e] - m) : 0.0;
                     }
                 __syncthreads();
                 if (warp == 0) {
@@ -221,7 +420,9 @@ sample_kernel(const T* logits, int vocab, int64_t row_stride,
                     }
                     // (rounding may leave the last running mass at the target: the last kept entry then;
                     // a total that is zero or not a number falls back to the argmax)
-                    if (lane == 0) ids[blockIdx.x] = !(total > 0.0) || total == INFINITY ? best.i : pick >= 0 ? cand_i[pick] : last_kept >= 0 ? cand_i[last_kept] : best.i;
+                    const int at = !(total > 0.0) || total == INFINITY ? -1 : pick >= 0 ? pick : last_kept;
+                    const int id = at >= 0 ? cand_i[at] : argmax_index();                       // (the same for the whole warp)
+                    if (lane == 0) ids[blockIdx.x] = id;
                 }
                 return;
             }
@@ -315,7 +516,11 @@ sample_kernel(const T* logits, int vocab, int64_t row_stride,
     }
     __syncthreads();
     // no segment claimed the target (total mass 0 or not finite): fall back to the argmax
-    if (tid == 0) ids[blockIdx.x] = pick_s >= 0 ? pick_s : best.i;
+    if (warp == 0) {
+        const int id = pick_s >= 0 ? pick_s : argmax_index();
+        if (lane == 0) ids[blockIdx.x] = id;
+    }
+    }
 }
 
 }  // namespace
@@ -338,14 +543,50 @@ static int sample_threads(int batch, int vocab, int cut) {
     return walk;
 }
 
+// Rows that fit the shared memory of an SM are staged there when every row has an SM of its own.
+constexpr size_t kStagedBytes = 208 * 1024;
+
+template <typename T, int kThreads, Choice kChoice>
+static cudaError_t allow_staged() {
+    static std::atomic<bool> done[64];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64 && done[dev].load(std::memory_order_acquire)) return cudaSuccess;
+    e = cudaFuncSetAttribute(sample_kernel<T, kThreads, kChoice, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStagedBytes);
+    if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev].store(true, std::memory_order_release);
+    return e;
+}
+
 template <typename T, int kThreads>
 static cudaError_t launch_sample(const T* logits, int batch, int vocab, int64_t row_stride, float temperature, int top_k, int do_sample,
                                  uint64_t seed, uint64_t step, int64_t* ids, cudaStream_t st) {
-    auto go = [&](auto kernel) { return launch(kernel, dim3((unsigned)batch), kThreads, 0, st, true, logits, vocab, row_stride, temperature, top_k, seed, step, ids); };
-    if (!do_sample) return go(sample_kernel<T, kThreads, Choice::kArgmax>);
-    if (top_k == 0) return go(sample_kernel<T, kThreads, Choice::kDraw>);
-    if (top_k <= cut_limit(kThreads)) return go(sample_kernel<T, kThreads, Choice::kTopK>);
-    return go(sample_kernel<T, kThreads, Choice::kTopKRadix>);
+    auto go = [&](auto kernel, size_t smem) { return launch(kernel, dim3((unsigned)batch), kThreads, smem, st, true, logits, vocab, row_stride, temperature, top_k, seed, step, ids); };
+    if (!do_sample) return go(sample_kernel<T, kThreads, Choice::kArgmax, false>, 0);
+    auto pick = [&](auto choice) {
+        constexpr Choice c = decltype(choice)::value;
+        if constexpr (kThreads > 256) {
+            const size_t bytes = ((size_t)vocab * sizeof(T) + 32) / 16 * 16;           // whole 16 bytes at any offset
+            if (batch <= num_sms() && bytes <= kStagedBytes) {
+                if (cudaError_t e = allow_staged<T, kThreads, c>(); e != cudaSuccess) return e;
+                return go(sample_kernel<T, kThreads, c, true>, bytes);
+            }
+        }
+        return go(sample_kernel<T, kThreads, c, false>, 0);
+    };
+    if (top_k == 0) return pick(std::integral_constant<Choice, Choice::kDraw>{});
+    if (top_k <= cut_limit(kThreads)) return pick(std::integral_constant<Choice, Choice::kTopK>{});
+    return pick(std::integral_constant<Choice, Choice::kTopKRadix>{});
+}
+
+int sample_fault_word(int* out) {
+    KIVI_CUDA_OK(cudaMemcpyFromSymbol(out, g_sample_fault, sizeof(int)));
+    return KIVI_OK;
+}
+int sample_fault_clear() {
+    const int zero = 0;
+    KIVI_CUDA_OK(cudaMemcpyToSymbol(g_sample_fault, &zero, sizeof(int)));
+    return KIVI_OK;
 }
 
 int run_sample(const void* logits, int dtype, int batch, int vocab, int64_t row_stride, float temperature, int top_k,

@@ -139,3 +139,31 @@ def test_every_thread_count_draws_the_same(cabi, batch, vocab, dtype):
             want = ko.sample_tokens(x.float(), 0.9, top_k or None, True, seed=5, step=top_k)
             # a draw on a boundary may move to the neighbour (exp differs in the last bit): about 1e-7 * vocab of the rows
             assert int((got != want).sum()) <= 1, (top_k, got, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("vocab,offset", [(2049, 0), (2050, 1), (2055, 3), (16385, 2), (16391, 7), (52999, 5), (53239, 1), (53241, 0), (106490, 3)])
+def test_rows_at_any_offset_from_sixteen_bytes(cabi, dtype, vocab, offset):
+    """Rows that fit shared memory arrive there by bulk copies of whole aligned 16 bytes,
+    their ragged ends by plain loads: every offset of a row against 16 bytes (the row stride
+    is odd, so the three rows differ), sizes around the largest row that fits (212992 bytes,
+    up to 30 of them padding) and just above it.  Neighbouring memory holds larger values than any row."""
+    g = torch.Generator().manual_seed(vocab)
+    x = (3.0 * torch.randn(3, vocab, generator=g)).to(dtype)
+    x[0, 0], x[1, vocab - 1], x[2, 1] = 30.0, 30.0, 30.0          # the draw of a peaked row is its peak: first, last, second entry
+    buf = torch.full((3, vocab + offset + 2 + (vocab + offset + 1) % 2), 100.0, dtype=dtype)
+    buf[:, offset:offset + vocab] = x
+    rows = buf.cuda()[:, offset:offset + vocab]
+    assert rows.stride(0) % 2 == 1
+    for top_k in (0, 50, 300, 1000):
+        got = cabi.sample_tokens(rows, 0.9, top_k, True, seed=3, step=top_k).cpu()
+        assert got.tolist() == [0, vocab - 1, 1], (top_k, got)
+    x[0, 0], x[1, vocab - 1], x[2, 1] = -30.0, -30.0, float("-inf")
+    buf[:, offset:offset + vocab] = x
+    rows = buf.cuda()[:, offset:offset + vocab]
+    wrong = 0
+    for top_k in (0, 50, 300, 1000):
+        got = cabi.sample_tokens(rows, 0.9, top_k, True, seed=5, step=top_k).cpu()
+        wrong += int((got != ko.sample_tokens(x.float(), 0.9, top_k or None, True, seed=5, step=top_k)).sum())
+    assert wrong <= 1                                             # (a draw on a boundary: see the oracle test above)
+    assert cabi.device_fault() == 0
