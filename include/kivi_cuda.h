@@ -188,7 +188,9 @@ int kivi_cache_import_keys(const kivi_layer* layer, const uint8_t* packed,
  * split); contents need not be preserved between calls.
  * num_splits: how many pieces the quantized history of a unit is cut into;
  * 0 = choose from the SM count.  path: KIVI_ATTN_AUTO picks the tensor-core
- * kernel when the shape allows it and the CUDA-core fp32 kernel otherwise.
+ * kernel when the shape allows it (fp32 queries: with longer operands, to fp32
+ * accuracy, and from the sizes on where it is faster) and the CUDA-core fp32
+ * kernel otherwise.
  * ---------------------------------------------------------------------- */
 #define KIVI_ATTN_AUTO 0
 #define KIVI_ATTN_FP32 1 /* CUDA-core fp32 kernel, any supported shape */
@@ -202,7 +204,9 @@ int kivi_decode_attention_max_splits(void);
  * into how many pieces every unit's quantized history is cut (num_splits > 0 is
  * taken as given, 0 lets the library choose from the number of CTAs the GPU
  * holds at a time) and how many CTAs per unit take the residual ring.  For arrays
- * on the 16-byte grid; others take the generic kernel and its coarser cut.
+ * on the 16-byte grid; others take the generic kernel and its coarser cut.  For fp32
+ * queries the piece count is the CUDA-core kernel's: where the tensor-core kernel
+ * serves them (KIVI_ATTN_AUTO) it is an upper bound.
  * sms / ctas_per_sm: the SM count and the tensor-core kernel's resident CTAs per
  * SM to plan for; <= 0 asks the current device (148 and 3 without one).
  * No counterpart in the reference. */

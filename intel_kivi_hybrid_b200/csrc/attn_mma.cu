@@ -149,10 +149,21 @@ constexpr float kRow1 = 0.25f, kRow2 = 0.0625f, kRow3 = 0.015625f;
 constexpr float kTwo23 = 8388608.0f;
 constexpr int kTwo23Bits = 0x4b000000;
 constexpr float kMagicK = 8388608.0f + 4915200.0f;        // 2^23 + 0x4b0000
+// Queries in fp32 (WIDE) take five digits for q.k and four for p.v: the rest r = w * F - x,
+// between -1/2 and 1/2, goes on as fma(r, 2^15, 2^23 + 0x4b00), whose low two bytes are two
+// more digits (the upper with the same bias); p.v has w * F < 2^23 and eight bits below that.
+// There the codes count from 1.5 (and the zero points from z + 1.5 s, the middle of a group's
+// range), or the two halves of a sum would cancel and leave their roundings: a contraction
+// with ones gives the sum of each digit, 1.5 times which is taken off the digit's sum.
+constexpr float kMiddle = 1.5f;
+constexpr uint32_t kOnes = 0x01010101u;
+constexpr float kMagicRest = 8388608.0f + 19200.0f;       // 2^23 + 0x4b00
+constexpr float kRestV = 255.49f;                         // 0 <= rest < 1 becomes 0 .. 255
 constexpr float kSmallest = 7.888609052210118e-31f;       // 2^-100: weights below it count as zero beside it
 constexpr uint32_t kExponent = 0x7f800000u, kSmallestBits = 27u << 23;
 constexpr uint32_t kInverseK = 275u << 23;                // largest |w * F| is 2^21 .. 1.125 * 2^21
 constexpr uint32_t kInverseV = 269u << 23;                // 2^15 .. 1.125 * 2^15, and then times kFillV
+constexpr uint32_t kInverseVWide = 276u << 23;            // 2^22 .. 1.125 * 2^22, and then times kFillV
 constexpr float kFillV = 1.7777f;                         // below 65535 / (1.125 * 2^15)
 constexpr float kGrowth = 8.0f;                           // weights up to 2^8 are let stand before the running maximum moves
 
@@ -173,6 +184,10 @@ struct LaneView {
     uint32_t p_read, v_write;
     int v_first;               // value words: contraction half read first
     int start[4];              // 2^23 in each accumulator register
+    // WIDE:
+    uint32_t rest_rows;        // as k_rows, for the third column block (from `spare`)
+    uint32_t ones[4];          // operand whose contraction sums the other one
+    const float4* q_zero;      // head tig's queries in shared memory, in place of qz
 };
 // The zero term q.z of a group: lane (gid, tig) takes head tig and the 16 channels 16*gid ..,
 // in an order that keeps the lanes of a half-warp off each other's banks.
@@ -224,18 +239,22 @@ __device__ __noinline__ float4 weighted_plain(const uint8_t* vc, const float* vs
 
 // ---- NG token groups (32 tokens each) in three phases -------------------------------
 // q.k: scores of the lane's four tokens (4*gid + n) of each group for head `tig`, log2 domain.
-template <int NG>
+// A score is s + fine; fine is 0 but for WIDE, where s is a multiple of the top digit's unit,
+// so that s less the running maximum, the number exponentiated, keeps all its bits.
+// `spare` (WIDE): the stage's key scales and zeros, kGPS * 1024 bytes, which take operands
+// once they have been read.
+template <int NG, bool WIDE>
 __device__ __forceinline__ void qk_phase(const uint8_t* __restrict__ kc, const float* __restrict__ ks, const float* __restrict__ kz,
-                                         const LaneView& v, uint8_t* scratch, float (&s)[NG][4]) {
-    float w[NG][4][4], top[4] = {kSmallest, kSmallest, kSmallest, kSmallest}, qz[NG];
+                                         const LaneView& v, uint8_t* scratch, uint32_t spare, float (&s)[NG][4], float (&fine)[NG][4]) {
+    float w[NG][4][4], sv[NG][4], top[4] = {kSmallest, kSmallest, kSmallest, kSmallest}, qz[NG];
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
         const float2 sa = *reinterpret_cast<const float2*>(ks + 128 * g + k_channel(v.lane, 0)), sb = *reinterpret_cast<const float2*>(ks + 128 * g + k_channel(v.lane, 2));
-        const float sv[4] = {sa.x, sa.y, sb.x, sb.y};
+        sv[g][0] = sa.x; sv[g][1] = sa.y; sv[g][2] = sb.x; sv[g][3] = sb.y;
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) w[g][i][h] = v.qk[i][h] * sv[i];
+            for (int i = 0; i < 4; ++i) w[g][i][h] = v.qk[i][h] * sv[g][i];
             top[h] = max3_abs_nan(w[g][2][h], w[g][3][h], max3_abs_nan(w[g][0][h], w[g][1][h], top[h]));
         }
     }
@@ -246,9 +265,14 @@ __device__ __forceinline__ void qk_phase(const uint8_t* __restrict__ kc, const f
         float z0 = 0.0f, z1 = 0.0f;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const float4 z = *reinterpret_cast<const float4*>(kz + 128 * g + 4 * zero_quad(i, v.gid));
-            z0 = fmaf(v.qz[i].x, z.x, z0); z1 = fmaf(v.qz[i].y, z.y, z1);
-            z0 = fmaf(v.qz[i].z, z.z, z0); z1 = fmaf(v.qz[i].w, z.w, z1);
+            float4 z = *reinterpret_cast<const float4*>(kz + 128 * g + 4 * zero_quad(i, v.gid));
+            if constexpr (WIDE) {
+                const float4 a = *reinterpret_cast<const float4*>(ks + 128 * g + 4 * zero_quad(i, v.gid));
+                z.x = fmaf(kMiddle, a.x, z.x); z.y = fmaf(kMiddle, a.y, z.y); z.z = fmaf(kMiddle, a.z, z.z); z.w = fmaf(kMiddle, a.w, z.w);
+            }
+            const float4 y = WIDE ? v.q_zero[zero_quad(i, v.gid)] : v.qz[i];
+            z0 = fmaf(y.x, z.x, z0); z1 = fmaf(y.y, z.y, z1);
+            z0 = fmaf(y.z, z.z, z0); z1 = fmaf(y.w, z.w, z1);
         }
         qz[g] = z0 + z1;
     }
@@ -267,82 +291,145 @@ __device__ __forceinline__ void qk_phase(const uint8_t* __restrict__ kc, const f
         for (int g = 0; g < NG; ++g) {
             const float4 r = scores_plain(kc + 1024 * g, ks + 128 * g, kz + 128 * g, reinterpret_cast<const float4*>(scratch) + 32 * v.tig, v.gid);
             s[g][0] = r.x; s[g][1] = r.y; s[g][2] = r.z; s[g][3] = r.w;
+#pragma unroll
+            for (int n = 0; n < 4; ++n) fine[g][n] = 0.0f;
         }
         return;
     }
-    float F[4];
+    float F[4], unit;
+    if constexpr (WIDE) {                                   // a power of two, so that unit = 1 / F exactly
 #pragma unroll
-    for (int h = 0; h < 4; ++h) F[h] = __uint_as_float(kInverseK - __float_as_uint(top[h]));
-    const float unit = rcp_approx(v.tig == 0 ? F[0] : v.tig == 1 ? F[1] : v.tig == 2 ? F[2] : F[3]);
-    int c[NG][2][2][4];                                     // [rows of codes 0,1 / 2,3 and up][digits 0,1 / 2,const]
+        for (int h = 0; h < 4; ++h) F[h] = __uint_as_float(kInverseK - (1u << 23) - (__float_as_uint(top[h]) & kExponent));
+        unit = __uint_as_float((254u << 23) - __float_as_uint(v.tig == 0 ? F[0] : v.tig == 1 ? F[1] : v.tig == 2 ? F[2] : F[3]));
+        // (the products are made again from here on: 32 of them would not stay in registers)
+#pragma unroll
+        for (int g = 0; g < NG; ++g)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) asm volatile("" : "+f"(sv[g][i]));
+    } else {
+#pragma unroll
+        for (int h = 0; h < 4; ++h) F[h] = __uint_as_float(kInverseK - __float_as_uint(top[h]));
+        unit = rcp_approx(v.tig == 0 ? F[0] : v.tig == 1 ? F[1] : v.tig == 2 ? F[2] : F[3]);
+    }
+    constexpr int kBlocks = WIDE ? 3 : 2;                   // column blocks: digits 0,1 / 2,const / rest 0,1
+    constexpr int kDigits = 2 * kBlocks - 1;
+    int c[WIDE ? 1 : NG][2][kBlocks][4];                    // [rows of codes 0,1 / 2,3 and up]
+    int sum[kBlocks][4];                                    // WIDE: every row the sum of the digits
+    auto read_scores = [&](int g) {
+        const int cg = WIDE ? 0 : g;
+        float below = 0.0f, y[5][kDigits], all[kDigits];    // digits (the biased ones less the constant) of the sums "code n and up"
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            const int t = n >> 1, r = 2 * (n & 1);
+            y[n][0] = __int_as_float(c[cg][t][0][r]); y[n][1] = __int_as_float(c[cg][t][0][r + 1]);
+            y[n][2] = __int_as_float(c[cg][t][1][r]) - __int_as_float(c[cg][t][1][r + 1]);
+            if constexpr (WIDE) {
+                y[n][3] = __int_as_float(c[cg][t][2][r]);
+                y[n][4] = __int_as_float(c[cg][t][2][r + 1]) - __int_as_float(c[cg][t][1][r + 1]);
+            }
+        }
+        y[4][0] = kTwo23; y[4][1] = kTwo23; y[4][2] = 0.0f;
+        if constexpr (WIDE) {
+            y[4][3] = kTwo23; y[4][4] = 0.0f;
+            all[0] = __int_as_float(sum[0][0]) - kTwo23; all[1] = __int_as_float(sum[0][1]) - kTwo23;
+            all[2] = __int_as_float(sum[1][0]) - __int_as_float(sum[1][1]);
+            all[3] = __int_as_float(sum[2][0]) - kTwo23; all[4] = __int_as_float(sum[2][1]) - __int_as_float(sum[1][1]);
+            below = fmaf(fmaf(all[4], 256.0f, all[3]), 0x1p-15f, all[0]);
+        }
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            const float row = n == 0 ? 1.0f : n == 1 ? kRow1 : n == 2 ? kRow2 : kRow3;
+            float d[kDigits];
+#pragma unroll
+            for (int i = 0; i < kDigits; ++i) d[i] = y[n][i] - y[n + 1][i];
+            if constexpr (WIDE) {
+                const float off = -kMiddle / row;
+                s[g][n] = fmaf(all[2], off, d[2]) * (65536.0f * row) * unit;
+                const float low = fmaf(below, off, fmaf(fmaf(d[4], 256.0f, d[3]), 0x1p-15f, d[0]));
+                fine[g][n] = fmaf(fmaf(fmaf(all[1], off, d[1]), 256.0f, low), unit * row, qz[g]);
+            } else {
+                s[g][n] = fmaf(fmaf(d[2], 65536.0f, fmaf(d[1], 256.0f, d[0])), unit * row, qz[g]);
+                fine[g][n] = 0.0f;
+            }
+        }
+    };
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
         if (g > 0) __syncwarp();                            // the operand of the group before has been read
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-            uint32_t x[2][4];
+            uint32_t x[2][4], rest[2][4];
 #pragma unroll
             for (int k = 0; k < 2; ++k)
 #pragma unroll
-                for (int h = 0; h < 4; ++h) x[k][h] = __float_as_uint(fmaf(w[g][2 * k + e][h], F[h], kMagicK));
+                for (int h = 0; h < 4; ++h) {
+                    const int i = 2 * k + e;
+                    if constexpr (WIDE) {
+                        const float y = v.qk[i][h] * sv[g][i], t = fmaf(y, F[h], kMagicK);
+                        x[k][h] = __float_as_uint(t);
+                        rest[k][h] = __float_as_uint(fmaf(fmaf(y, F[h], kMagicK - t), 32768.0f, kMagicRest));
+                    } else {
+                        x[k][h] = __float_as_uint(fmaf(w[g][i][h], F[h], kMagicK));
+                    }
+                }
             // columns: digits 0 and 1 of the four heads; digit 2 and the constant
             sts128(v.scratch + 512 * e + 16 * v.lane, __byte_perm(x[0][0], x[0][1], 0x5410), __byte_perm(x[0][2], x[0][3], 0x5410),
                    __byte_perm(x[1][0], x[1][1], 0x5410), __byte_perm(x[1][2], x[1][3], 0x5410));
             sts128(v.scratch + 1024 + 512 * e + 16 * v.lane, __byte_perm(x[0][0], x[0][1], 0x7632), __byte_perm(x[0][2], x[0][3], 0x7632),
                    __byte_perm(x[1][0], x[1][1], 0x7632), __byte_perm(x[1][2], x[1][3], 0x7632));
+            if constexpr (WIDE)
+                sts128(spare + 1024 * g + 512 * e + 16 * v.lane, __byte_perm(rest[0][0], rest[0][1], 0x5410), __byte_perm(rest[0][2], rest[0][3], 0x5410),
+                       __byte_perm(rest[1][0], rest[1][1], 0x5410), __byte_perm(rest[1][2], rest[1][3], 0x5410));
         }
         __syncwarp();
-        uint32_t b[4][4];                                   // step j: both halves of columns 0-7, of columns 8-15
+        uint32_t b[4][4], br[2][4];                         // step j: both halves of columns 0-7, of columns 8-15; steps 2j, 2j+1 of the rest
+        if constexpr (!WIDE) {                              // (WIDE has no registers to spare for all of them)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) ldmatrix_t8(b[j], v.k_rows + 128 * j);
+            for (int j = 0; j < 4; ++j) ldmatrix_t8(b[j], v.k_rows + 128 * j);
+        }
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const uint4 wv = *reinterpret_cast<const uint4*>(kc + 1024 * g + half * 512 + v.gid * 64 + v.tig * 16);
             const uint32_t cw[4] = {wv.x, wv.y, wv.z, wv.w};
 #pragma unroll
             for (int m = 0; m < 4; m += 2) {
-                const int j = 2 * half + m / 2;
+                const int j = 2 * half + m / 2, cg = WIDE ? 0 : g;
                 const uint32_t wa = cw[m + (j & 1)], wb = cw[m + 1 - (j & 1)];
+                if constexpr (WIDE) {
+                    ldmatrix_t8(b[j], v.k_rows + 128 * j);
+                    if (m == 0) ldmatrix_t8(br[half], spare + 1024 * g + v.rest_rows + 256 * half);
+                }
 #pragma unroll
-                for (int d = 0; d < 2; ++d) {
+                for (int d = 0; d < kBlocks; ++d) {
+                    const uint32_t b0 = d < 2 ? b[j][2 * d] : br[half][m], b1 = d < 2 ? b[j][2 * d + 1] : br[half][m + 1];
                     if (j == 0) {
-                        mma_u8_from(v.start, c[g][0][d], wa, wa & kFrom1, wb, wb & kFrom1, b[j][2 * d], b[j][2 * d + 1]);
-                        mma_u8_from(v.start, c[g][1][d], wa & kFrom2, wa & kFrom3, wb & kFrom2, wb & kFrom3, b[j][2 * d], b[j][2 * d + 1]);
+                        mma_u8_from(v.start, c[cg][0][d], wa, wa & kFrom1, wb, wb & kFrom1, b0, b1);
+                        mma_u8_from(v.start, c[cg][1][d], wa & kFrom2, wa & kFrom3, wb & kFrom2, wb & kFrom3, b0, b1);
+                        if constexpr (WIDE) mma_u8_from(v.start, sum[d], v.ones[0], v.ones[1], v.ones[2], v.ones[3], b0, b1);
                     } else {
-                        mma_u8(c[g][0][d], wa, wa & kFrom1, wb, wb & kFrom1, b[j][2 * d], b[j][2 * d + 1]);
-                        mma_u8(c[g][1][d], wa & kFrom2, wa & kFrom3, wb & kFrom2, wb & kFrom3, b[j][2 * d], b[j][2 * d + 1]);
+                        mma_u8(c[cg][0][d], wa, wa & kFrom1, wb, wb & kFrom1, b0, b1);
+                        mma_u8(c[cg][1][d], wa & kFrom2, wa & kFrom3, wb & kFrom2, wb & kFrom3, b0, b1);
+                        if constexpr (WIDE) mma_u8(sum[d], v.ones[0], v.ones[1], v.ones[2], v.ones[3], b0, b1);
                     }
                 }
             }
         }
+        if constexpr (WIDE) read_scores(g);                 // (registers: one group's accumulators at a time)
     }
+    if constexpr (!WIDE) {
 #pragma unroll
-    for (int g = 0; g < NG; ++g) {
-        float y[5][3];                                      // digit 0, digit 1, unbiased digit 2 of the sums "code n and up"
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-            const int t = n >> 1, r = 2 * (n & 1);
-            y[n][0] = __int_as_float(c[g][t][0][r]); y[n][1] = __int_as_float(c[g][t][0][r + 1]);
-            y[n][2] = __int_as_float(c[g][t][1][r]) - __int_as_float(c[g][t][1][r + 1]);
-        }
-        y[4][0] = kTwo23; y[4][1] = kTwo23; y[4][2] = 0.0f;
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-            const float d0 = y[n][0] - y[n + 1][0], d1 = y[n][1] - y[n + 1][1], d2 = y[n][2] - y[n + 1][2];
-            const float row = n == 0 ? 1.0f : n == 1 ? kRow1 : n == 2 ? kRow2 : kRow3;
-            s[g][n] = fmaf(fmaf(d2, 65536.0f, fmaf(d1, 256.0f, d0)), unit * row, qz[g]);
-        }
+        for (int g = 0; g < NG; ++g) read_scores(g);
     }
 }
 
 // running max / sum update for NG groups at once; turns scores into weights
 template <int NG>
-__device__ __forceinline__ void softmax_phase(float (&s)[NG][4], WarpState& st) {
+__device__ __forceinline__ void softmax_phase(float (&s)[NG][4], const float (&fine)[NG][4], WarpState& st) {
     float gmax = -INFINITY;
 #pragma unroll
     for (int g = 0; g < NG; ++g)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) gmax = fmaxf(gmax, s[g][e]);
+        for (int e = 0; e < 4; ++e) gmax = fmaxf(gmax, s[g][e] + fine[g][e]);
     if (__any_sync(0xffffffffu, gmax > st.m + kGrowth)) {
         gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 4));
         gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 8));
@@ -363,7 +450,7 @@ __device__ __forceinline__ void softmax_phase(float (&s)[NG][4], WarpState& st) 
 #pragma unroll
     for (int g = 0; g < NG; ++g)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) { s[g][e] = ex2(s[g][e] - st.m); st.l += s[g][e]; }
+        for (int e = 0; e < 4; ++e) { s[g][e] = ex2((s[g][e] - st.m) + fine[g][e]); st.l += s[g][e]; }
 }
 
 // p.v of NG groups; p[g][n] = weight of token 4*gid + n of group g for head tig.
@@ -374,9 +461,9 @@ __device__ __forceinline__ void softmax_phase(float (&s)[NG][4], WarpState& st) 
 // Value block words (kivi_common.cuh): word (gd, kappa, r, c) holds natural byte
 // 8*gd + r (channels 32*gd + 4*r + i) of tokens 16*kappa + 4*c + n in bytes n: four
 // consecutive contraction indices, as the tensor core wants them.
-template <int NG>
+template <int NG, bool WIDE>
 __device__ __forceinline__ void pv_phase(const uint8_t* __restrict__ vc, const float* __restrict__ vs, const float* __restrict__ vz,
-                                         const float (&p)[NG][4], const LaneView& v, uint8_t* scratch, WarpState& st) {
+                                         const float (&p)[NG][4], const LaneView& v, uint8_t* scratch, uint32_t spare, WarpState& st) {
     __syncwarp();                                           // the scratch is free
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
@@ -412,7 +499,11 @@ __device__ __forceinline__ void pv_phase(const uint8_t* __restrict__ vc, const f
     }
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
-        const float4 z4 = *reinterpret_cast<const float4*>(vz + g * 128 + 4 * v.lane);
+        float4 z4 = *reinterpret_cast<const float4*>(vz + g * 128 + 4 * v.lane);
+        if constexpr (WIDE) {
+            z4.x = fmaf(kMiddle, sv[g][0], z4.x); z4.y = fmaf(kMiddle, sv[g][1], z4.y);
+            z4.z = fmaf(kMiddle, sv[g][2], z4.z); z4.w = fmaf(kMiddle, sv[g][3], z4.w);
+        }
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
             st.oz[h][0] = fmaf(ph[g][h], z4.x, st.oz[h][0]); st.oz[h][1] = fmaf(ph[g][h], z4.y, st.oz[h][1]);
@@ -421,8 +512,10 @@ __device__ __forceinline__ void pv_phase(const uint8_t* __restrict__ vc, const f
     }
     float F[4];
 #pragma unroll
-    for (int h = 0; h < 4; ++h) F[h] = __uint_as_float(kInverseV - top[h]) * kFillV;
-    const float unit = rcp_approx(v.tig == 0 ? F[0] : v.tig == 1 ? F[1] : v.tig == 2 ? F[2] : F[3]);
+    for (int h = 0; h < 4; ++h) F[h] = __uint_as_float((WIDE ? kInverseVWide : kInverseV) - top[h]) * kFillV;
+    const float own = v.tig == 0 ? F[0] : v.tig == 1 ? F[1] : v.tig == 2 ? F[2] : F[3];
+    float unit = rcp_approx(own);
+    if constexpr (WIDE) unit = fmaf(unit, fmaf(-own, unit, 1.0f), unit);
     __syncwarp();                                           // every lane has read its weights
     // Rows of 16 bytes per channel group and contraction index k = 4*c + n: the columns
     // [head][digit] of tokens 16*0 + k and 16*1 + k, in the other order for k >= 8 (the writes
@@ -432,11 +525,64 @@ __device__ __forceinline__ void pv_phase(const uint8_t* __restrict__ vc, const f
 #pragma unroll
         for (int gd = 0; gd < 4; ++gd) {
             uint32_t x[4];
+            if constexpr (WIDE) {                           // below the 23 bits eight more: the rest of a number rounded down
 #pragma unroll
-            for (int h = 0; h < 4; ++h) x[h] = __float_as_uint(fmaf(ph[g][h] * sv[g][gd], F[h], kTwo23));
-            sts64(v.v_write + 1024 * g + 256 * gd, __byte_perm(x[0], x[1], 0x5410), __byte_perm(x[2], x[3], 0x5410));
+                for (int h = 0; h < 4; ++h) {
+                    const float y = ph[g][h] * sv[g][gd], t = __fmaf_rz(y, F[h], kTwo23), r = fmaf(fmaf(y, F[h], kTwo23 - t), kRestV, kTwo23);
+                    x[h] = __byte_perm(__float_as_uint(r), __float_as_uint(t), 0x6540);
+                }
+                const uint32_t row = (g == 0 ? v.v_write : v.v_write - v.scratch + spare) + 512 * gd;
+                sts64(row, __byte_perm(x[0], x[1], 0x5410), __byte_perm(x[2], x[3], 0x5410));
+                sts64(row + 256, __byte_perm(x[0], x[1], 0x7632), __byte_perm(x[2], x[3], 0x7632));
+            } else {
+#pragma unroll
+                for (int h = 0; h < 4; ++h) x[h] = __float_as_uint(fmaf(ph[g][h] * sv[g][gd], F[h], kTwo23));
+                sts64(v.v_write + 1024 * g + 256 * gd, __byte_perm(x[0], x[1], 0x5410), __byte_perm(x[2], x[3], 0x5410));
+            }
         }
     __syncwarp();
+    if constexpr (WIDE) {
+#pragma unroll
+        for (int gd = 0; gd < 4; ++gd) {
+            int acc[2][2][4], sum[2][4];                    // [rows of codes 0,1 / 2,3 and up][digits 0,1 / 2,3]; sums of the digits
+#pragma unroll
+            for (int g = 0; g < NG; ++g) {
+                const uint32_t* vw = reinterpret_cast<const uint32_t*>(vc + g * 1024) + v.lane;
+                uint32_t b[4];
+                ldmatrix_t8(b, (g == 0 ? v.v_rows : v.v_rows - v.scratch + spare) + 512 * gd);
+                const uint32_t w0 = vw[gd * 64 + v.v_first], w1 = vw[gd * 64 + (v.v_first ^ 32)];
+#pragma unroll
+                for (int d = 0; d < 2; ++d) {
+                    if (g == 0) {
+                        mma_u8_from(v.start, acc[0][d], w0, w0 & kFrom1, w1, w1 & kFrom1, b[2 * d], b[2 * d + 1]);
+                        mma_u8_from(v.start, acc[1][d], w0 & kFrom2, w0 & kFrom3, w1 & kFrom2, w1 & kFrom3, b[2 * d], b[2 * d + 1]);
+                        mma_u8_from(v.start, sum[d], v.ones[0], v.ones[1], v.ones[2], v.ones[3], b[2 * d], b[2 * d + 1]);
+                    } else {
+                        mma_u8(acc[0][d], w0, w0 & kFrom1, w1, w1 & kFrom1, b[2 * d], b[2 * d + 1]);
+                        mma_u8(acc[1][d], w0 & kFrom2, w0 & kFrom3, w1 & kFrom2, w1 & kFrom3, b[2 * d], b[2 * d + 1]);
+                        mma_u8(sum[d], v.ones[0], v.ones[1], v.ones[2], v.ones[3], b[2 * d], b[2 * d + 1]);
+                    }
+                }
+            }
+            float all[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) all[k] = __int_as_float(sum[k >> 1][k & 1]) - kTwo23;
+            const float below = fmaf(all[2], 256.0f, fmaf(all[0], 1.0f / kRestV, all[1]));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int mt = i >> 1, r = 2 * (i & 1), mt1 = i < 3 ? (i + 1) >> 1 : 0, r1 = 2 * ((i + 1) & 1);
+                const float off = i == 0 ? -kMiddle : i == 1 ? -4.0f * kMiddle : i == 2 ? -16.0f * kMiddle : -64.0f * kMiddle;
+                float d[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    d[k] = __int_as_float(acc[mt][k >> 1][r + (k & 1)]) - (i < 3 ? __int_as_float(acc[mt1][k >> 1][r1 + (k & 1)]) : kTwo23);
+                const float low = fmaf(below, off, fmaf(d[2], 256.0f, fmaf(d[0], 1.0f / kRestV, d[1])));
+                float& o = st.o[2 * gd + mt][i & 1];
+                o = fmaf(fmaf(fmaf(all[3], off, d[3]), 65536.0f, low), unit, o);
+            }
+        }
+        return;
+    }
     int acc[8][4];
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
@@ -472,12 +618,15 @@ __device__ __forceinline__ void pv_phase(const uint8_t* __restrict__ vc, const f
 
 // NG consecutive token groups of one pipeline stage: the softmax update and the reading of
 // the p.v accumulators are done once for all NG*32 tokens.
-template <int NG>
+template <int NG, bool WIDE>
 __device__ __forceinline__ void process_groups(const uint8_t* __restrict__ sb, const LaneView& v, uint8_t* scratch, WarpState& st) {
-    float s[NG][4];
-    qk_phase<NG>(sb, reinterpret_cast<const float*>(sb + kGPS * 1024), reinterpret_cast<const float*>(sb + kGPS * 1536), v, scratch, s);
-    softmax_phase<NG>(s, st);
-    pv_phase<NG>(sb + kGPS * 2048, reinterpret_cast<const float*>(sb + kGPS * 3072), reinterpret_cast<const float*>(sb + kGPS * 3584), s, v, scratch, st);
+    float s[NG][4], fine[NG][4];
+    const uint32_t spare = WIDE ? smem_u32(sb + kGPS * 1024) : 0u;
+    qk_phase<NG, WIDE>(sb, reinterpret_cast<const float*>(sb + kGPS * 1024), reinterpret_cast<const float*>(sb + kGPS * 1536), v, scratch, spare, s, fine);
+    softmax_phase<NG>(s, fine, st);
+    pv_phase<NG, WIDE>(sb + kGPS * 2048, reinterpret_cast<const float*>(sb + kGPS * 3072), reinterpret_cast<const float*>(sb + kGPS * 3584), s, v, scratch, spare, st);
+    // what was written over the stage comes before the copy that fills it again
+    if constexpr (WIDE) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
 // ---- one query head per KV head ------------------------------------------------------
@@ -676,7 +825,7 @@ __device__ __forceinline__ void pv_one(const uint8_t* __restrict__ vc, const flo
     }
 }
 
-template <int NG>
+template <int NG, bool>
 __device__ __forceinline__ void process_groups(const uint8_t* __restrict__ sb, const OneView& v, uint8_t* scratch, OneState& st) {
     float s[4];
     qk_one<NG>(sb, reinterpret_cast<const float*>(sb + kGPS * 1024), reinterpret_cast<const float*>(sb + kGPS * 1536), v, scratch, s);
@@ -888,10 +1037,10 @@ __device__ __forceinline__ void residual_part(
 // as the [4][128] buffer its scaled output goes to; the CTA then adds the warps'
 // buffers in warp order (deterministic) and writes one partial.
 //
-// ONE: one query head per KV head.
+// ONE: one query head per KV head.  WIDE: operands long enough for fp32 accuracy.
 // FOLD: the CTAs of a unit and head block are a cluster and fold their partials
 // themselves (a template, so that the wide grids keep their registers).
-template <bool FOLD, bool ONE>
+template <bool FOLD, bool WIDE, bool ONE>
 __global__ void __launch_bounds__(kWarps * 32, 3)
 attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
                 const void* q, int q_dtype,
@@ -903,6 +1052,7 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
     float* q_s = reinterpret_cast<float*>(scratch_mem);                          // [4][128], ring CTAs
     uint64_t* bars = reinterpret_cast<uint64_t*>(scratch_mem + kWarps * kScratchBytes);   // [kWarps][kStages]
     float* ml_s = reinterpret_cast<float*>(bars + kWarps * kStages);             // [kWarps][4][2]
+    float* const zero_s = ml_s + kWarps * 4 * 2;                                 // WIDE: [4][128] queries for the zero term
 
     // With a fold kernel behind this one, its few small blocks may become resident from
     // here on (it waits for this grid's end).  Without (FOLD), what comes next can be
@@ -983,16 +1133,19 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
     for (int c = 0; c < kStages && c < my_n; ++c) issue(c);
 
     const int64_t q_row = (int64_t)u * n_rep + head0;
-    if (is_res) {
-        // ---------------- residual ring ----------------
-        for (int i = threadIdx.x; i < kD; i += blockDim.x) {             // [4][128], pre-scaled (absent heads: zeros)
+    auto stage_queries = [&](float* dst) {                               // [4][128], pre-scaled (absent heads: zeros)
+        for (int i = threadIdx.x; i < kD; i += blockDim.x) {
             float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
             if ((i >> 5) < n_heads) {
                 if (q_dtype == KIVI_BF16) RowVec<__nv_bfloat16>::load4(reinterpret_cast<const __nv_bfloat16*>(q) + q_row * kD + 4 * i, t);
                 else RowVec<float>::load4(reinterpret_cast<const float*>(q) + q_row * kD + 4 * i, t);
             }
-            *reinterpret_cast<float4*>(q_s + 4 * i) = make_float4(scale_log2 * t[0], scale_log2 * t[1], scale_log2 * t[2], scale_log2 * t[3]);
+            *reinterpret_cast<float4*>(dst + 4 * i) = make_float4(scale_log2 * t[0], scale_log2 * t[1], scale_log2 * t[2], scale_log2 * t[3]);
         }
+    };
+    if (is_res) {
+        // ---------------- residual ring ----------------
+        stage_queries(q_s);
         __syncthreads();
         const int rs = sub;
         const int t_begin = rs * res_chunk;
@@ -1042,11 +1195,20 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
             v.p_even = v.scratch + 16 * (16 * kap + (gid & 3)) + 64 * kap + 4 * tig;
             v.p_odd = v.scratch + 16 * (16 * kap + (gid & 3)) + 64 * (1 - kap) + 4 * tig;
             v.p_read = v.scratch + 16 * p_row(lane);
+            v.rest_rows = 128 * (lane >> 4) + 512 * (lane & 1) + 16 * ((lane >> 1) & 7);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) asm volatile("mov.b32 %0, %1;" : "=r"(v.start[i]) : "n"(kTwo23Bits));
         if (q_dtype == KIVI_BF16) load_queries(reinterpret_cast<const __nv_bfloat16*>(q) + q_row * kD, n_heads, scale_log2, v);
         else load_queries(reinterpret_cast<const float*>(q) + q_row * kD, n_heads, scale_log2, v);
+
+        if constexpr (WIDE) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) asm volatile("mov.b32 %0, %1;" : "=r"(v.ones[i]) : "n"(kOnes));
+            v.q_zero = reinterpret_cast<const float4*>(zero_s) + 32 * tig;
+            stage_queries(zero_s);
+            __syncthreads();
+        }
 
         std::conditional_t<ONE, OneState, WarpState> st;
         clear(st);
@@ -1058,8 +1220,8 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
             if (!__all_sync(0xffffffffu, mbar_wait(bar0 + 8 * s, (uint32_t)(c / kStages) & 1u))) { ok = false; break; }
             const int goff = (warp + kWarps * c) * kGPS;
             const uint8_t* sb = wstage + s * kStageBytes;
-            if (n_my_groups - goff >= 2) process_groups<2>(sb, v, scratch, st);
-            else process_groups<1>(sb, v, scratch, st);
+            if (n_my_groups - goff >= 2) process_groups<2, WIDE>(sb, v, scratch, st);
+            else process_groups<1, WIDE>(sb, v, scratch, st);
             __syncwarp();
             if (c + kStages < my_n) issue(c + kStages);
         }
@@ -1159,6 +1321,7 @@ attn_mma_kernel(kivi_layer L, int64_t quant_len, int res_start, int res_len,
 }
 
 constexpr size_t kSmemBytes = (size_t)kWarps * (kStages * kStageBytes + kScratchBytes) + kWarps * kStages * 8 + kWarps * 4 * 2 * 4;
+constexpr size_t kSmemBytesWide = kSmemBytes + 4 * kD * 4;
 static_assert(kScratchBytes >= 4 * kD * 4, "ring CTAs keep the queries in the first warp's scratch");
 static_assert(kStages * kStageBytes >= 2 * 4 * kD * 4 + 32, "a warp's ring doubles as its [4][128] fold buffer, the first also holds the CTA's partial");
 static_assert(kWarps * 32 >= 32, "at least one warp");
@@ -1188,8 +1351,9 @@ static int ensure_smem_attr(int* dev_out) {
     KIVI_CUDA_OK(cudaGetDevice(&dev));
     KIVI_REQUIRE(dev >= 0 && dev < 64, "device ordinal %d out of range", dev);
     if (!attr_set[dev].load(std::memory_order_acquire)) {
-        for (auto* kernel : {attn_mma_kernel<false, false>, attn_mma_kernel<true, false>, attn_mma_kernel<false, true>, attn_mma_kernel<true, true>})
-            KIVI_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+        for (auto* kernel : {attn_mma_kernel<false, false, false>, attn_mma_kernel<true, false, false>, attn_mma_kernel<false, true, false>,
+                             attn_mma_kernel<true, true, false>, attn_mma_kernel<false, false, true>, attn_mma_kernel<true, false, true>})
+            KIVI_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytesWide));
         attr_set[dev].store(true, std::memory_order_release);
     }
     if (dev_out) *dev_out = dev;
@@ -1204,7 +1368,7 @@ int attn_mma_ctas_per_sm() {
     if (ensure_smem_attr(&dev) != KIVI_OK) return 0;
     int n = cached[dev].load(std::memory_order_acquire);
     if (n == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_mma_kernel<false, false>, kWarps * 32, kSmemBytes) != cudaSuccess || n <= 0)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_mma_kernel<false, false, false>, kWarps * 32, kSmemBytesWide) != cudaSuccess || n <= 0)
             return 0;
         cached[dev].store(n, std::memory_order_release);
     }
@@ -1212,14 +1376,15 @@ int attn_mma_ctas_per_sm() {
 }
 
 int run_attn_mma(const kivi_layer* L, int64_t quant_len, int res_start, int res_len,
-                 const void* q, int q_dtype, int n_rep, float scale_log2, int nq_splits, int gps,
+                 const void* q, int q_dtype, int n_rep, float scale_log2, bool wide, int nq_splits, int gps,
                  int n_res_splits, int res_chunk, float* part_o, float* part_ml, const ClusterOut& direct, cudaStream_t st) {
     if (int rc = ensure_smem_attr(nullptr)) return rc;
     dim3 grid((unsigned)(nq_splits + n_res_splits) * (unsigned)L->num_units * (unsigned)((n_rep + 3) / 4));
     const bool fold = direct.out != nullptr;
-    auto* const kernel = n_rep == 1 ? (fold ? attn_mma_kernel<true, true> : attn_mma_kernel<false, true>)
-                                    : (fold ? attn_mma_kernel<true, false> : attn_mma_kernel<false, false>);
-    KIVI_CUDA_OK(launch_cluster(kernel, direct.out ? nq_splits + n_res_splits : 0, grid, kWarps * 32, kSmemBytes, st, true, *L, quant_len, res_start, res_len, q, q_dtype, scale_log2,
+    auto* const kernel = wide ? (fold ? attn_mma_kernel<true, true, false> : attn_mma_kernel<false, true, false>)
+                       : n_rep == 1 ? (fold ? attn_mma_kernel<true, false, true> : attn_mma_kernel<false, false, true>)
+                                    : (fold ? attn_mma_kernel<true, false, false> : attn_mma_kernel<false, false, false>);
+    KIVI_CUDA_OK(launch_cluster(kernel, direct.out ? nq_splits + n_res_splits : 0, grid, kWarps * 32, wide ? kSmemBytesWide : kSmemBytes, st, true, *L, quant_len, res_start, res_len, q, q_dtype, scale_log2,
                         n_rep, gps, nq_splits, n_res_splits, res_chunk, part_o, part_ml, direct));
     return KIVI_OK;
 }

@@ -53,7 +53,7 @@ bool attn_mma_supported(const kivi_layer* L, int n_rep, const void* q);
 void attn_mma_residual_plan(int res_len, int* n_res_splits, int* res_chunk);
 int attn_mma_ctas_per_sm();
 int run_attn_mma(const kivi_layer* L, int64_t quant_len, int res_start, int res_len,
-                 const void* q, int q_dtype, int n_rep, float scale_log2, int nq_splits, int gps,
+                 const void* q, int q_dtype, int n_rep, float scale_log2, bool wide, int nq_splits, int gps,
                  int n_res_splits, int res_chunk, float* part_o, float* part_ml, const ClusterOut& direct, cudaStream_t st);
 int run_sample(const void* logits, int dtype, int batch, int vocab, int64_t row_stride, float temperature, int top_k,
                int do_sample, uint64_t seed, uint64_t step, int64_t* ids, cudaStream_t st);
@@ -261,10 +261,45 @@ static int plan_splits_mma(int num_units, int64_t n_groups, int n_res_splits, in
     return best;
 }
 
+// The tensor-core kernel with fp32 queries.  What counts are its stages (two groups a warp,
+// eight a CTA), each of which takes a warp c_one, c_two or c_three us by how many CTAs share
+// the SM, ring CTAs among them.  Fitted to 131 shapes (four heads, 1 to 512 units x 128 to
+// 131072 tokens, 1 to 128 pieces; the times to 11 %): its count is 3.5 % off the best on average.
+static int plan_splits_wide(int num_units, int64_t n_groups, int n_res_splits, int n_sms, int ctas_per_sm) {
+    const int per_sm = ctas_per_sm > 0 ? ctas_per_sm : 3;
+    const double slots = (double)per_sm * n_sms;
+    const double c0 = 6.84, c0_waves = 2.2, c_one = 1.97, c_two = 2.56, c_three = 4.32, c_merge = 1.8, c_over = 4.2, ragged = 0.48, c_start = 0.006, c_piece = 0.06;
+    int best = 1;
+    double best_t = 0.0;
+    for (int64_t s = 1; s <= kMaxSplitsC && s <= n_groups; ++s) {
+        const double quant = (double)num_units * (double)s, ring = (double)num_units * n_res_splits, ctas = quant + ring;
+        const double stages = (double)(((n_groups + s - 1) / s + 7) / 8);
+        double t;
+        if (quant <= slots) {
+            t = c0 + stages * (ctas <= n_sms ? c_one : ctas <= 2.0 * n_sms ? c_two : c_three) + (ctas > slots ? c_over * (ctas - slots) / n_sms : 0.0);
+        } else {
+            const double one = c0_waves + stages * c_three;
+            t = c0 - c0_waves + quant / slots * one + ragged * one + ring / slots * c_over;
+            if (t < c0 + stages * c_three) t = c0 + stages * c_three;
+        }
+        if (!folds_in_cluster((int64_t)ctas, (int)s + n_res_splits, n_sms)) t += c_merge + 0.02 * (double)s;
+        t += c_start * ctas + c_piece * (double)(s < 16 ? s : 16);
+        if (s == 1 || t < best_t - 1e-9) { best = (int)s; best_t = t; }
+    }
+    return best;
+}
+
+// fp32 queries: the tensor-core kernel costs the same for one to four heads, the CUDA-core
+// kernel about 1500 + 650 n_rep cycles of an SM quarter per group.  us, CUDA cores / tensor
+// cores, each at its best count.  Four heads: 32 units x 8k tokens 37.9 / 21.2, 192 x 4k 102 / 48,
+// 20 x 2k 16.4 / 10.4; 256 x 128 tokens (the ring counts most there) 19.4 / 27.6, 512 x 512
+// 51.5 / 50.1.  One head: 256 x 4k 74 / 65, 32 x 2k 12.3 / 13.7, 192 x 512 14.7 / 19.1.
+static bool wide_pays(int n_rep, int64_t n_groups) { return n_rep >= 3 && n_groups >= 32; }
+
 // The piece count of a kernel.  The models above walk up to 128 candidates (1-2 us);
 // a decode loop asks for the same shape again and again, so each thread remembers
 // its last question -- the answer depends on nothing else.
-enum class AttnKernel { kGeneric, kTile, kMma };
+enum class AttnKernel { kGeneric, kTile, kMma, kMmaWide };
 static int plan_splits(AttnKernel kernel, int num_units, int64_t n_groups, int requested, int head_dim, int group_size, int n_rep, int n_res,
                        int sms, int ctas_per_sm) {
     if (n_groups <= 0) return 0;
@@ -276,6 +311,12 @@ static int plan_splits(AttnKernel kernel, int num_units, int64_t n_groups, int r
     if (last >= 0 && memcmp(key, last_key, sizeof(key)) == 0) return last;
     switch (kernel) {
         case AttnKernel::kMma: last = plan_splits_mma(num_units * ((n_rep + 3) / 4), n_groups, n_res, sms, ctas_per_sm); break;
+        case AttnKernel::kMmaWide: {
+            const int finest = plan_splits_tile(num_units, n_groups, head_dim, group_size, n_rep, n_res > 0 ? 1 : 0, sms);
+            last = plan_splits_wide(num_units * ((n_rep + 3) / 4), n_groups, n_res, sms, ctas_per_sm);
+            if (last > finest) last = finest;
+            break;
+        }
         case AttnKernel::kTile: last = plan_splits_tile(num_units, n_groups, head_dim, group_size, n_rep, n_res, sms); break;
         case AttnKernel::kGeneric: last = plan_splits_generic(num_units, n_groups, sms); break;
     }
@@ -291,21 +332,24 @@ extern "C" int kivi_decode_attention_plan(int num_units, int64_t quant_len, int 
     KIVI_REQUIRE(num_splits >= 0 && num_splits <= kMaxSplitsC, "num_splits (%d) outside 0..%d", num_splits, kMaxSplitsC);
     KIVI_REQUIRE(tensor_cores_out && quant_splits_out && residual_parts_out, "output pointers must be given");
     const bool shape_ok = head_dim == 128 && group_size == 32 && n_rep >= 1 && n_rep <= 8;
+    const bool wide = path == KIVI_ATTN_AUTO && q_dtype == KIVI_F32 && shape_ok && wide_pays(n_rep, quant_len / group_size);
     const bool use_mma = path == KIVI_ATTN_MMA ? shape_ok : path == KIVI_ATTN_AUTO ? (shape_ok && q_dtype == KIVI_BF16) : false;
     if (path == KIVI_ATTN_MMA && !shape_ok) {
         set_error("tensor-core path needs head_dim 128, group_size 32, n_rep <= 8 (got %d, %d, %d)", head_dim, group_size, n_rep);
         return KIVI_ERR_UNSUPPORTED;
     }
-    int n_res = res_len > 0 ? 1 : 0, chunk = res_len;
-    if (use_mma) attn_mma_residual_plan(res_len, &n_res, &chunk);
+    int n_res = res_len > 0 ? 1 : 0, n_parts = n_res, chunk = res_len;
+    if (use_mma || wide) attn_mma_residual_plan(res_len, &n_parts, &chunk);
+    if (use_mma) n_res = n_parts;
     const int64_t n_groups = quant_len / group_size;
     if (sms <= 0) sms = num_sms();
     if (ctas_per_sm <= 0) ctas_per_sm = attn_mma_ctas_per_sm();
-    *tensor_cores_out = use_mma ? 1 : 0;
-    // (arrays on the 16-byte grid, as every allocator places them)
+    *tensor_cores_out = use_mma || wide ? 1 : 0;
+    // (arrays on the 16-byte grid, as every allocator places them; fp32 queries: the CUDA-core
+    // kernel's count, which the tensor-core kernel does not exceed)
     const AttnKernel kernel = use_mma ? AttnKernel::kMma : attn_fp32_tile_head_dim(head_dim) ? AttnKernel::kTile : AttnKernel::kGeneric;
     *quant_splits_out = plan_splits(kernel, num_units, n_groups, num_splits, head_dim, group_size, n_rep, n_res, sms, ctas_per_sm);
-    *residual_parts_out = n_res;
+    *residual_parts_out = n_parts;
     return KIVI_OK;
 }
 
@@ -326,7 +370,7 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
     KIVI_REQUIRE(L->num_units <= 65535, "num_units (%d) above 65535", L->num_units);
     const int D = L->head_dim, G = L->group_size;
     const int64_t n_groups = quant_len / G;
-    bool use_mma = false;
+    bool use_mma = false, wide = false;
     if (path == KIVI_ATTN_MMA) {
         if (!attn_mma_supported(L, n_rep, q)) {
             set_error("tensor-core path needs head_dim 128, group_size 32, n_rep <= 8 (got %d, %d, %d) and 16-byte aligned arrays", D, G, n_rep);
@@ -334,16 +378,34 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
         }
         use_mma = true;
     } else if (path == KIVI_ATTN_AUTO) {
-        // fp32 queries keep the all-fp32 kernel (1e-5 tolerance); bf16 queries take
-        // the tensor-core kernel when the shape allows it
-        use_mma = q_dtype == KIVI_BF16 && attn_mma_supported(L, n_rep, q);
+        // fp32 queries (1e-5 tolerance) take the tensor-core kernel with its longer operands
+        // where that is the faster one
+        wide = q_dtype == KIVI_F32;
+        use_mma = (!wide || wide_pays(n_rep, n_groups)) && attn_mma_supported(L, n_rep, q);
+        wide = wide && use_mma;
     }
-    int n_res_splits = res_len > 0 ? 1 : 0, res_chunk = res_len;
-    if (use_mma) attn_mma_residual_plan(res_len, &n_res_splits, &res_chunk);
-    const AttnKernel kernel = use_mma ? AttnKernel::kMma : attn_fp32_tile_ok(L) ? AttnKernel::kTile : AttnKernel::kGeneric;
     const int sms = num_sms();
-    int nq_splits = plan_splits(kernel, L->num_units, n_groups, num_splits, D, G, n_rep, n_res_splits, sms, use_mma ? attn_mma_ctas_per_sm() : 0);
+    AttnKernel kernel;
+    int n_res_splits, res_chunk, nq_splits;
     const auto partial_bytes = [&](int pieces) { return (size_t)L->num_units * (pieces + n_res_splits) * n_rep * (D + 2) * sizeof(float); };
+    const auto plan = [&]() {
+        n_res_splits = res_len > 0 ? 1 : 0; res_chunk = res_len;
+        if (use_mma) attn_mma_residual_plan(res_len, &n_res_splits, &res_chunk);
+        kernel = use_mma ? (wide ? AttnKernel::kMmaWide : AttnKernel::kMma) : attn_fp32_tile_ok(L) ? AttnKernel::kTile : AttnKernel::kGeneric;
+        nq_splits = plan_splits(kernel, L->num_units, n_groups, num_splits, D, G, n_rep, n_res_splits, sms, use_mma ? attn_mma_ctas_per_sm() : 0);
+    };
+    plan();
+    // fp32 queries on the tensor cores: where the partials do not fit the scratch, first fewer
+    // pieces (of an automatic count), then the CUDA-core kernel, which has one ring part at most
+    if (wide && partial_bytes(nq_splits) > workspace_bytes) {
+        const int64_t fit = (int64_t)(workspace_bytes / ((size_t)L->num_units * n_rep * (D + 2) * sizeof(float))) - n_res_splits;
+        if (num_splits == 0 && fit >= 1) {
+            nq_splits = (int)fit;
+        } else {
+            use_mma = wide = false;
+            plan();
+        }
+    }
     // The tile kernel's plan cuts large problems finer than the generic rule (300 units x
     // 8k tokens: 16 pieces against 4): where its partials do not fit the scratch but the
     // coarser cut's do, that one is taken.
@@ -368,7 +430,7 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
     if (!gather && folds_in_cluster(ctas, n_splits, sms) && kernel != AttnKernel::kGeneric) direct.out = out;
 
     int rc = use_mma
-        ? run_attn_mma(L, quant_len, res_start, res_len, q, q_dtype, n_rep, scale_log2, nq_splits, gps, n_res_splits, res_chunk, part_o, part_ml, direct, st)
+        ? run_attn_mma(L, quant_len, res_start, res_len, q, q_dtype, n_rep, scale_log2, wide, nq_splits, gps, n_res_splits, res_chunk, part_o, part_ml, direct, st)
         : run_attn_fp32(L, quant_len, res_start, res_len, q, q_dtype, n_rep, scale_log2, nq_splits, gps, n_splits, part_o, part_ml, direct, st);
     if (rc) return rc;
     if (direct.out) { note_launches(1); return KIVI_OK; }

@@ -6,6 +6,7 @@ Tolerances: fp32 activations 1e-5; bf16 activations 2e-3, on the error of a
 max|out-ref| / max|ref| (`rel_err`).  The tests also print the element-wise
 figure max |out-ref| / max(|ref|, 1e-3 * max|ref| of the row) (`elem_err`),
 which weighs the same absolute error against each element's own magnitude."""
+import ctypes
 import os
 import subprocess
 import sys
@@ -708,6 +709,76 @@ def test_attention_mma_at_the_edges_of_its_fixed_point_operands(cabi, what, toke
     ok = want.isfinite()
     size = (st.v_scales.abs().nan_to_num(0, 0, 0).max() * 3 + st.v_zeros.abs().max()).item()
     assert ((got - want)[ok].abs().max() / size).item() < 2.9e-3
+
+
+@pytest.mark.parametrize("n_quant,n_res,n_rep,splits", [(1024, 0, 3, 1), (1056, 77, 4, 0), (1312, 128, 5, 7), (4064, 200, 8, 0), (2080, 1, 4, 65)])
+def test_attention_fp32_queries_on_the_tensor_cores(cabi, n_quant, n_res, n_rep, splits):
+    """From three heads and 1024 tokens on fp32 queries are served there: whole and odd
+    stages, one to 65 pieces, one and two head blocks, several ring parts."""
+    assert cabi.attention_plan(2, n_quant, n_res, n_rep=n_rep, q_dtype=cabi.F32, num_splits=splits)[0]
+    err, oerr, _, _ = _attention_case(cabi, 1, 2, n_rep, 128, 32, 256, n_quant, n_res, torch.float32, 3, cabi.ATTN_AUTO, num_splits=splits)
+    print(f"[attn fp32 on tensor cores q={n_quant} r={n_res} heads={n_rep}] rel err {err:.2e} (fp32 oracle: {oerr:.2e})")
+    assert err < TOL_F32 and cabi.device_fault() == 0
+
+
+@pytest.mark.parametrize("what", ["tiny", "huge", "mixed", "negative", "k_inf", "v_nan", "q_nan"])
+def test_attention_fp32_queries_at_the_edges_of_fixed_point(cabi, what):
+    """As for bf16 queries above, with the longer operands: a weight is off by 2^-30 of the
+    stage's largest at most and a score by that of 128 channels, so the fp32 tolerance holds."""
+    U, tokens, n_rep = 3, 1056, 4
+    st = cabi.LayerStore(U, 128, 32, 128, tokens, torch.float32, "cuda")
+    g = torch.Generator(device="cuda").manual_seed(17)
+    for n in ("k_codes", "v_codes"):
+        getattr(st, n).random_(0, 256, generator=g)
+    for n, lo, hi in (("k_scales", 0.3, 1.2), ("v_scales", 0.3, 1.2), ("k_zeros", -2.0, -0.5), ("v_zeros", -2.0, -0.5)):
+        getattr(st, n).uniform_(lo, hi, generator=g)
+    st.quant_len = tokens
+    q = torch.randn(U, n_rep, 128, generator=g, device="cuda")
+    if what in ("tiny", "huge"):
+        f = 1e-30 if what == "tiny" else 1e30
+        for n in ("v_scales", "v_zeros", "k_scales", "k_zeros"):
+            getattr(st, n).mul_(f)
+        q /= f
+    elif what == "mixed":
+        st.k_scales[:, :, 7] *= 1e4
+        st.k_zeros[:, :, 7] *= 1e4
+        q[:, :, 7] *= 1e-4
+        st.v_scales.view(U, -1)[:, 5] *= 1e4
+    elif what == "negative":
+        st.v_scales.view(U, -1)[:, 11] *= -1
+        st.k_scales[:, 0, 3] *= -1
+    elif what == "k_inf":
+        st.k_scales[2, -1, 77] = float("inf")
+    elif what == "v_nan":
+        st.v_scales.view(U, -1)[2, 13] = float("nan")
+    elif what == "q_nan":
+        q[1, 0, 100] = float("nan")
+    got, want = (st.attention(q, n_rep=n_rep, path=p) for p in (cabi.ATTN_AUTO, cabi.ATTN_FP32))
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    ok = want.isfinite()
+    assert ok.any() and cabi.device_fault() == 0
+    size = want[ok].abs().max()
+    assert ((got - want)[ok].abs().max() / size).item() < 2 * TOL_F32          # both are within it of the exact result
+
+
+def test_fp32_queries_keep_to_the_scratch_they_are_given(cabi):
+    """Partials of the tensor-core kernel that do not fit the workspace: fewer pieces, then the
+    CUDA-core kernel, whose partials of one piece and one ring part are the least there are."""
+    U, T, n_rep, D = 40, 4096, 4, 128
+    st = cabi.LayerStore(U, D, 32, 1024, T, torch.float32, "cuda")
+    k, v = (torch.randn(U, T + 1000, D, device="cuda") for _ in range(2))
+    cabi.load_state(st, k, v, T)
+    q = torch.randn(U, n_rep, D, device="cuda")
+    want = st.attention(q, n_rep=n_rep, path=cabi.ATTN_FP32)
+    row = U * n_rep * (D + 2) * 4
+    # (pieces asked for, partials of a row the workspace holds); 1000 window tokens are eight ring parts
+    for pieces, ring in ((0, 40), (0, 12), (0, 9), (1, 2), (1, 9), (5, 6)):
+        out = torch.empty_like(q)
+        ws = torch.empty(row * ring, dtype=torch.uint8, device="cuda")
+        rc = cabi.lib.kivi_decode_attention(ctypes.byref(st.c), T, st.res_start, st.res_len, q.data_ptr(), cabi.F32, out.data_ptr(), cabi.F32, n_rep, 0.0,
+                                            ws.data_ptr(), ws.numel(), pieces, cabi.ATTN_AUTO, torch.cuda.current_stream().cuda_stream)
+        assert rc == 0, (pieces, ring, cabi.lib.kivi_last_error())
+        assert rel_err(out, want.cpu()) < 2 * TOL_F32, (pieces, ring)
 
 
 @pytest.mark.parametrize("D,dtype,U,n_rep", [(128, torch.bfloat16, 8, 4), (64, torch.float32, 12, 1), (128, torch.bfloat16, 200, 1), (32, torch.float32, 2, 2)])
