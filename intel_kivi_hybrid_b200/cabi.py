@@ -116,7 +116,7 @@ def _native_ops():
         if not os.environ.get("KIVI_CUDA_LIB"):
             try:
                 from .extension.loader import kivi_native
-                _ops = kivi_native if hasattr(kivi_native, "cache_attention") else False
+                _ops = kivi_native if hasattr(kivi_native, "sample_tokens") else False
             except ImportError:
                 pass
     return _ops or None
@@ -411,6 +411,9 @@ def sample_tokens(logits, temperature=1.0, top_k=0, do_sample=False, seed=0, ste
     """kivi_sample_tokens: [batch, vocab] fp32 / bf16 device logits (last dim
     contiguous) -> int64 [batch] device ids, without a host round trip."""
     assert logits.dim() == 2 and logits.stride(1) == 1
+    ops = _native_ops()
+    if ops is not None:
+        return ops.sample_tokens(logits, float(temperature), int(top_k or 0), bool(do_sample), int(seed) & (2**64 - 1), int(step) & (2**64 - 1), out)
     if not logits.is_cuda:
         raise RuntimeError("tensor must be on a CUDA device")
     if out is None:

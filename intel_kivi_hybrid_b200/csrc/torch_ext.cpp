@@ -280,6 +280,19 @@ int dtype_code(const torch::Tensor& t, const char* name) {
     return t.scalar_type() == torch::kFloat32 ? KIVI_F32 : KIVI_BF16;
 }
 
+// as Python writes it
+std::string dtype_name(torch::ScalarType t) {
+    switch (t) {
+        case torch::kHalf: return "float16";
+        case torch::kDouble: return "float64";
+        case torch::kLong: return "int64";
+        case torch::kInt: return "int32";
+        case torch::kByte: return "uint8";
+        case torch::kBool: return "bool";
+        default: return torch::toString(t);
+    }
+}
+
 // Attention of a layer store of the Python package: `layer` is the address of its
 // struct kivi_layer.  Everything between the Python call and the launches happens
 // here (checks, output allocation, stream lookup): a decode step over a short context
@@ -309,8 +322,7 @@ torch::Tensor cache_attention(int64_t layer, int64_t quant_len, int res_start, i
     auto code = [&](const torch::Tensor& t) {
         if (t.scalar_type() == torch::kFloat32) return KIVI_F32;
         if (t.scalar_type() != torch::kBFloat16)
-            fail(std::string("unsupported dtype torch.") + (t.scalar_type() == torch::kHalf ? "float16" : t.scalar_type() == torch::kDouble ? "float64" : torch::toString(t.scalar_type())) +
-                 ": expected float32 or bfloat16");
+            fail("unsupported dtype torch." + dtype_name(t.scalar_type()) + ": expected float32 or bfloat16");
         return KIVI_BF16;
     };
     const int q_dtype = code(q);
@@ -322,6 +334,30 @@ torch::Tensor cache_attention(int64_t layer, int64_t quant_len, int res_start, i
                                          at::cuda::getCurrentCUDAStream().stream());
     if (rc != KIVI_OK) fail("kivi_cuda error " + std::to_string(rc) + ": " + kivi_last_error());
     return o;
+}
+
+// Next-token choice (cabi.sample_tokens): what lies between the Python call and the launch,
+// 12.3 us of host time call by call from Python (more than the kernel takes), 5.0 here.
+// `logits` is [batch, vocab] with entries side by side.
+torch::Tensor sample_tokens(const torch::Tensor& logits, double temperature, int64_t top_k, bool do_sample, uint64_t seed, uint64_t step,
+                            const c10::optional<torch::Tensor>& out) {
+    auto fail = [](const std::string& what) { throw std::runtime_error(what); };
+    if (!logits.is_cuda()) fail("tensor must be on a CUDA device");
+    if (out.has_value()) {
+        if (!out->is_cuda()) fail("tensor must be on a CUDA device");
+        if (!out->is_contiguous()) fail("tensor must be contiguous");
+        if (out->device() != logits.device())
+            fail("all tensors of one call must be on the same device, got " + logits.device().str() + " and " + out->device().str());
+    }
+    if (logits.scalar_type() != torch::kFloat32 && logits.scalar_type() != torch::kBFloat16)
+        fail("unsupported dtype torch." + dtype_name(logits.scalar_type()) + ": expected float32 or bfloat16");
+    c10::cuda::CUDAGuard guard(logits.device());
+    const torch::Tensor ids = out.has_value() ? *out : at::empty({logits.size(0)}, logits.options().dtype(torch::kLong));
+    const int rc = kivi_sample_tokens(logits.data_ptr(), logits.scalar_type() == torch::kFloat32 ? KIVI_F32 : KIVI_BF16, (int)logits.size(0), (int)logits.size(1),
+                                      logits.stride(0), (float)temperature, (int)top_k, do_sample ? 1 : 0, seed, step, reinterpret_cast<int64_t*>(ids.data_ptr()),
+                                      at::cuda::getCurrentCUDAStream().stream());
+    if (rc != KIVI_OK) fail("kivi_cuda error " + std::to_string(rc) + ": " + kivi_last_error());
+    return ids;
 }
 
 }  // namespace
@@ -448,6 +484,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           "decode_attention over the layer struct at an address (used by cabi.LayerStore); returns the output tensor.",
           py::arg("layer"), py::arg("quant_len"), py::arg("res_start"), py::arg("res_len"), py::arg("q"), py::arg("out"), py::arg("workspace"),
           py::arg("n_rep"), py::arg("sm_scale"), py::arg("num_splits"), py::arg("path"), py::arg("out_dtype"));
+    m.def("sample_tokens", &sample_tokens, py::call_guard<py::gil_scoped_release>(),
+          "Next-token choice over [batch, vocab] device logits (used by cabi.sample_tokens); returns the ids.",
+          py::arg("logits"), py::arg("temperature"), py::arg("top_k"), py::arg("do_sample"), py::arg("seed"), py::arg("step"), py::arg("out"));
     m.def("decode_attention_workspace", [](int num_units, int n_rep, int head_dim, int num_splits) {
               return (int64_t)kivi_decode_attention_workspace(num_units, n_rep, head_dim, num_splits); },
           "Bytes of scratch decode_attention needs.", py::arg("num_units"), py::arg("n_rep"), py::arg("head_dim"), py::arg("num_splits") = 0);

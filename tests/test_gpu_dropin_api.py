@@ -391,6 +391,38 @@ def test_native_attention_call_equals_the_ctypes_call(monkeypatch, dtype, D, n_r
     assert native[1] == general[1]
 
 
+def test_native_sampling_call_equals_the_ctypes_call(monkeypatch):
+    """cabi.sample_tokens goes through the compiled extension; same ids and same refusals
+    as the ctypes binding of the same library call."""
+    from intel_kivi_hybrid_b200 import cabi
+    x = 3 * torch.randn(9, 3, 5003, generator=torch.Generator(device="cuda").manual_seed(2), device="cuda")
+    assert cabi._native_ops() is not None
+
+    def calls():
+        out = torch.full((9,), -1, dtype=torch.int64, device="cuda")
+        got = [cabi.sample_tokens(x[:, 1]), cabi.sample_tokens(x[:, 2], 0.7, None, True), cabi.sample_tokens(x[:, 0].bfloat16(), 1, 40, 1, seed=-5, step=2**63 + 1),
+               cabi.sample_tokens(x[:, 0], 0.0, 2, True, seed=2**64 + 3, out=out)]
+        assert got[3].data_ptr() == out.data_ptr() and all(g.dtype == torch.int64 and g.shape == (9,) for g in got)
+        refused = []
+        for bad in (lambda: cabi.sample_tokens(x[:, 0].cpu()), lambda: cabi.sample_tokens(x[:, 0].half()), lambda: cabi.sample_tokens(x[:, 0].long()),
+                    lambda: cabi.sample_tokens(x[:, 0], top_k=-1, do_sample=True), lambda: cabi.sample_tokens(x[:, 0], out=out.cpu()),
+                    lambda: cabi.sample_tokens(x[:, 0], out=torch.empty(18, dtype=torch.int64, device="cuda")[::2]), lambda: cabi.sample_tokens(x[:0, 0])):
+            with pytest.raises(RuntimeError) as e:
+                bad()
+            refused.append(str(e.value))
+        for bad in (lambda: cabi.sample_tokens(x), lambda: cabi.sample_tokens(x[:, 0, ::2])):
+            with pytest.raises(AssertionError):
+                bad()
+        return got, refused
+
+    native = calls()
+    monkeypatch.setattr(cabi, "_ops", False)
+    general = calls()
+    for a, b in zip(native[0], general[0]):
+        assert torch.equal(a, b)
+    assert native[1] == general[1]
+
+
 def test_attention_refuses_operands_the_kernels_would_overrun(monkeypatch):
     """The kernels take raw pointers: a q or an out too short for the cache, an out in
     pageable host memory or with gaps are refused before the launch, by the extension
