@@ -227,8 +227,10 @@ static int plan_splits_tile(int num_units, int64_t n_groups, int head_dim, int g
 //     a third of a CTA; a CTA's fixed time is c0_waves there.
 // At the two-CTA count the ring CTAs must fit beside the quantized ones, or c1 is that of
 // a crowded SM (256 units x 4k: one piece 51 us, two 44, three 45).
-// Against the best count measured at 308 shapes this is 2 % off on average; where two
-// counts lie close it may take the second (160 units x 8k: two pieces 7 % behind four).
+// Fitted when the kernel's operands were fp16 (2 % off the best count of 308 shapes).  With
+// byte operands it is 4 % off over 130 shapes of four heads; where two counts lie close it may
+// take the second (128 units x 8k: two pieces 7 % behind three, 32 x 32k: thirteen 19 %
+// behind twelve).  A refit in the form below (plan_splits_stages) comes to 3 %.
 static int plan_splits_mma(int num_units, int64_t n_groups, int n_res_splits, int n_sms, int ctas_per_sm) {
     const int per_sm = ctas_per_sm > 0 ? ctas_per_sm : 3;
     const double slots = (double)per_sm * n_sms;
@@ -261,14 +263,19 @@ static int plan_splits_mma(int num_units, int64_t n_groups, int n_res_splits, in
     return best;
 }
 
-// The tensor-core kernel with fp32 queries.  What counts are its stages (two groups a warp,
-// eight a CTA), each of which takes a warp c_one, c_two or c_three us by how many CTAs share
-// the SM, ring CTAs among them.  Fitted to 131 shapes (four heads, 1 to 512 units x 128 to
-// 131072 tokens, 1 to 128 pieces; the times to 11 %): its count is 3.5 % off the best on average.
-static int plan_splits_wide(int num_units, int64_t n_groups, int n_res_splits, int n_sms, int ctas_per_sm) {
+// The tensor-core kernel with fp32 queries and with one head.  What counts are its stages
+// (two groups a warp, eight a CTA), each of which takes a warp c_one, c_two or c_three us by
+// how many CTAs share the SM, ring CTAs among them.  Fitted to 130 shapes each (1 to 800
+// units x 128 to 131072 tokens, 1 to 128 pieces; the times to 11 and 10 %): the counts are
+// 3.5 % off the best on average; the model below, whose costs are those of bf16 queries of
+// four heads, is 9 and 5.8 % off (one head: 256 units x 8k in four pieces 54 us, in its two
+// 64; 12 x 4k in six 8.3, in its eight 10.0).
+struct StageCosts { double c0, c0_waves, c_one, c_two, c_three, c_merge, c_over, ragged, c_start, c_piece; };
+constexpr StageCosts kWideCosts{6.84, 2.2, 1.97, 2.56, 4.32, 1.8, 4.2, 0.48, 0.006, 0.06};
+constexpr StageCosts kOneHeadCosts{5.92, 0.34, 0.82, 0.90, 1.47, 1.07, 2.46, 0.495, 0.006, 0.027};
+static int plan_splits_stages(const StageCosts& c, int num_units, int64_t n_groups, int n_res_splits, int n_sms, int ctas_per_sm) {
     const int per_sm = ctas_per_sm > 0 ? ctas_per_sm : 3;
     const double slots = (double)per_sm * n_sms;
-    const double c0 = 6.84, c0_waves = 2.2, c_one = 1.97, c_two = 2.56, c_three = 4.32, c_merge = 1.8, c_over = 4.2, ragged = 0.48, c_start = 0.006, c_piece = 0.06;
     int best = 1;
     double best_t = 0.0;
     for (int64_t s = 1; s <= kMaxSplitsC && s <= n_groups; ++s) {
@@ -276,14 +283,14 @@ static int plan_splits_wide(int num_units, int64_t n_groups, int n_res_splits, i
         const double stages = (double)(((n_groups + s - 1) / s + 7) / 8);
         double t;
         if (quant <= slots) {
-            t = c0 + stages * (ctas <= n_sms ? c_one : ctas <= 2.0 * n_sms ? c_two : c_three) + (ctas > slots ? c_over * (ctas - slots) / n_sms : 0.0);
+            t = c.c0 + stages * (ctas <= n_sms ? c.c_one : ctas <= 2.0 * n_sms ? c.c_two : c.c_three) + (ctas > slots ? c.c_over * (ctas - slots) / n_sms : 0.0);
         } else {
-            const double one = c0_waves + stages * c_three;
-            t = c0 - c0_waves + quant / slots * one + ragged * one + ring / slots * c_over;
-            if (t < c0 + stages * c_three) t = c0 + stages * c_three;
+            const double one = c.c0_waves + stages * c.c_three;
+            t = c.c0 - c.c0_waves + quant / slots * one + c.ragged * one + ring / slots * c.c_over;
+            if (t < c.c0 + stages * c.c_three) t = c.c0 + stages * c.c_three;
         }
-        if (!folds_in_cluster((int64_t)ctas, (int)s + n_res_splits, n_sms)) t += c_merge + 0.02 * (double)s;
-        t += c_start * ctas + c_piece * (double)(s < 16 ? s : 16);
+        if (!folds_in_cluster((int64_t)ctas, (int)s + n_res_splits, n_sms)) t += c.c_merge + 0.02 * (double)s;
+        t += c.c_start * ctas + c.c_piece * (double)(s < 16 ? s : 16);
         if (s == 1 || t < best_t - 1e-9) { best = (int)s; best_t = t; }
     }
     return best;
@@ -299,7 +306,7 @@ static bool wide_pays(int n_rep, int64_t n_groups) { return n_rep >= 3 && n_grou
 // The piece count of a kernel.  The models above walk up to 128 candidates (1-2 us);
 // a decode loop asks for the same shape again and again, so each thread remembers
 // its last question -- the answer depends on nothing else.
-enum class AttnKernel { kGeneric, kTile, kMma, kMmaWide };
+enum class AttnKernel { kGeneric, kTile, kMma, kMmaOne, kMmaWide };
 static int plan_splits(AttnKernel kernel, int num_units, int64_t n_groups, int requested, int head_dim, int group_size, int n_rep, int n_res,
                        int sms, int ctas_per_sm) {
     if (n_groups <= 0) return 0;
@@ -310,10 +317,11 @@ static int plan_splits(AttnKernel kernel, int num_units, int64_t n_groups, int r
     static thread_local int last = -1;
     if (last >= 0 && memcmp(key, last_key, sizeof(key)) == 0) return last;
     switch (kernel) {
+        case AttnKernel::kMmaOne: last = plan_splits_stages(kOneHeadCosts, num_units, n_groups, n_res, sms, ctas_per_sm); break;
         case AttnKernel::kMma: last = plan_splits_mma(num_units * ((n_rep + 3) / 4), n_groups, n_res, sms, ctas_per_sm); break;
         case AttnKernel::kMmaWide: {
             const int finest = plan_splits_tile(num_units, n_groups, head_dim, group_size, n_rep, n_res > 0 ? 1 : 0, sms);
-            last = plan_splits_wide(num_units * ((n_rep + 3) / 4), n_groups, n_res, sms, ctas_per_sm);
+            last = plan_splits_stages(kWideCosts, num_units * ((n_rep + 3) / 4), n_groups, n_res, sms, ctas_per_sm);
             if (last > finest) last = finest;
             break;
         }
@@ -347,7 +355,7 @@ extern "C" int kivi_decode_attention_plan(int num_units, int64_t quant_len, int 
     *tensor_cores_out = use_mma || wide ? 1 : 0;
     // (arrays on the 16-byte grid, as every allocator places them; fp32 queries: the CUDA-core
     // kernel's count, which the tensor-core kernel does not exceed)
-    const AttnKernel kernel = use_mma ? AttnKernel::kMma : attn_fp32_tile_head_dim(head_dim) ? AttnKernel::kTile : AttnKernel::kGeneric;
+    const AttnKernel kernel = use_mma ? (n_rep == 1 ? AttnKernel::kMmaOne : AttnKernel::kMma) : attn_fp32_tile_head_dim(head_dim) ? AttnKernel::kTile : AttnKernel::kGeneric;
     *quant_splits_out = plan_splits(kernel, num_units, n_groups, num_splits, head_dim, group_size, n_rep, n_res, sms, ctas_per_sm);
     *residual_parts_out = n_parts;
     return KIVI_OK;
@@ -391,7 +399,7 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
     const auto plan = [&]() {
         n_res_splits = res_len > 0 ? 1 : 0; res_chunk = res_len;
         if (use_mma) attn_mma_residual_plan(res_len, &n_res_splits, &res_chunk);
-        kernel = use_mma ? (wide ? AttnKernel::kMmaWide : AttnKernel::kMma) : attn_fp32_tile_ok(L) ? AttnKernel::kTile : AttnKernel::kGeneric;
+        kernel = use_mma ? (wide ? AttnKernel::kMmaWide : n_rep == 1 ? AttnKernel::kMmaOne : AttnKernel::kMma) : attn_fp32_tile_ok(L) ? AttnKernel::kTile : AttnKernel::kGeneric;
         nq_splits = plan_splits(kernel, L->num_units, n_groups, num_splits, D, G, n_rep, n_res_splits, sms, use_mma ? attn_mma_ctas_per_sm() : 0);
     };
     plan();
@@ -406,6 +414,9 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
             plan();
         }
     }
+    // one head: where its plan does not fit the scratch, the general one
+    if (num_splits == 0 && kernel == AttnKernel::kMmaOne && partial_bytes(nq_splits) > workspace_bytes)
+        nq_splits = plan_splits(AttnKernel::kMma, L->num_units, n_groups, 0, D, G, n_rep, n_res_splits, sms, attn_mma_ctas_per_sm());
     // The tile kernel's plan cuts large problems finer than the generic rule (300 units x
     // 8k tokens: 16 pieces against 4): where its partials do not fit the scratch but the
     // coarser cut's do, that one is taken.

@@ -367,3 +367,20 @@ def test_a_plan_too_fine_for_the_scratch_gives_way_to_a_coarser_one(D, n_rep, U,
 def test_attention_split_plan_takes_the_measured_counts(units, tokens, n_rep, pieces):
     from intel_kivi_hybrid_b200 import cabi
     assert cabi.attention_plan(units, tokens, 96, n_rep=n_rep, sms=148, ctas_per_sm=3)[1] == pieces
+
+
+@pytest.mark.parametrize("units,tokens,pieces", [
+    (256, 8192, 4),         # 54 us; in two pieces, as with four heads, 64
+    (12, 4096, 6),          # 8.3 us; in eight 10.0
+    (32, 32768, 8),         # 29.7 us; in thirteen 33.7
+    (64, 128, 1),
+])
+def test_attention_split_plan_of_one_head(units, tokens, pieces):
+    """One query head per KV head has stages of its own cost; whatever the shape, between one
+    piece and as many as there are groups."""
+    from intel_kivi_hybrid_b200 import cabi
+    plan = lambda u, t: cabi.attention_plan(u, t, 96, n_rep=1, sms=148, ctas_per_sm=3)[1]
+    assert plan(units, tokens) == pieces
+    for u in (1, 5, 148, 444, 2000, 65535):
+        for t in (32, 96, 4096, 131072):
+            assert 1 <= plan(u, t) <= min(t // 32, 128), (u, t)
