@@ -403,20 +403,28 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
         nq_splits = plan_splits(kernel, L->num_units, n_groups, num_splits, D, G, n_rep, n_res_splits, sms, use_mma ? attn_mma_ctas_per_sm() : 0);
     };
     plan();
-    // fp32 queries on the tensor cores: where the partials do not fit the scratch, first fewer
-    // pieces (of an automatic count), then the CUDA-core kernel, which has one ring part at most
-    if (wide && partial_bytes(nq_splits) > workspace_bytes) {
-        const int64_t fit = (int64_t)(workspace_bytes / ((size_t)L->num_units * n_rep * (D + 2) * sizeof(float))) - n_res_splits;
-        if (num_splits == 0 && fit >= 1) {
-            nq_splits = (int)fit;
-        } else {
+    // The scratch a call needs is what the plans of the CUDA-core kernel (fp32 queries) and of
+    // four heads (one head) need: smaller is refused, and where only the newer plan's partials
+    // do not fit, the other is followed.  A workspace for any count holds every plan.
+    const bool any_plan_fits = partial_bytes(kMaxSplitsC) <= workspace_bytes && n_res_splits <= 8;
+    if (wide && !any_plan_fits) {
+        const size_t row = (size_t)L->num_units * n_rep * (D + 2) * sizeof(float);
+        const int ring = res_len > 0 ? 1 : 0;
+        const auto core_fits = [&](AttnKernel k) {
+            return row * (plan_splits(k, L->num_units, n_groups, num_splits, D, G, n_rep, ring, sms, 0) + ring) <= workspace_bytes;
+        };
+        const bool served = core_fits(AttnKernel::kTile) || (num_splits == 0 && core_fits(AttnKernel::kGeneric));
+        const int64_t fit = (int64_t)(workspace_bytes / row) - n_res_splits;
+        if (served && num_splits == 0 && nq_splits > fit && fit >= 1) nq_splits = (int)fit;
+        if (!served || nq_splits > fit) {
             use_mma = wide = false;
             plan();
         }
     }
-    // one head: where its plan does not fit the scratch, the general one
-    if (num_splits == 0 && kernel == AttnKernel::kMmaOne && partial_bytes(nq_splits) > workspace_bytes)
-        nq_splits = plan_splits(AttnKernel::kMma, L->num_units, n_groups, 0, D, G, n_rep, n_res_splits, sms, attn_mma_ctas_per_sm());
+    if (num_splits == 0 && kernel == AttnKernel::kMmaOne && !any_plan_fits) {
+        const int general = plan_splits(AttnKernel::kMma, L->num_units, n_groups, 0, D, G, n_rep, n_res_splits, sms, attn_mma_ctas_per_sm());
+        if (partial_bytes(general) > workspace_bytes || partial_bytes(nq_splits) > workspace_bytes) nq_splits = general;
+    }
     // The tile kernel's plan cuts large problems finer than the generic rule (300 units x
     // 8k tokens: 16 pieces against 4): where its partials do not fit the scratch but the
     // coarser cut's do, that one is taken.
