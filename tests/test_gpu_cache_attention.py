@@ -771,8 +771,11 @@ def test_fp32_queries_keep_to_the_scratch_they_are_given(cabi):
     q = torch.randn(U, n_rep, D, device="cuda")
     want = st.attention(q, n_rep=n_rep, path=cabi.ATTN_FP32)
     row = U * n_rep * (D + 2) * 4
+    # the least an automatic count of the CUDA-core kernel needs: its plan or about eight CTAs per SM
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    least = min(cabi.attention_plan(U, T, 1000, n_rep=n_rep, q_dtype=cabi.F32)[1], -(-8 * sms // U), T // 32 // 4) + 1
     # (pieces asked for, partials of a row the workspace holds); 1000 window tokens are eight ring parts
-    for pieces, ring, served in ((0, 40, True), (0, 31, True), (0, 12, False), (1, 2, True), (1, 9, True), (5, 6, True), (5, 5, False)):
+    for pieces, ring, served in ((0, 40, True), (0, least, True), (0, least - 1, False), (1, 2, True), (1, 9, True), (5, 6, True), (5, 5, False)):
         out = torch.empty_like(q)
         ws = torch.empty(row * ring, dtype=torch.uint8, device="cuda")
         rc = cabi.lib.kivi_decode_attention(ctypes.byref(st.c), T, st.res_start, st.res_len, q.data_ptr(), cabi.F32, out.data_ptr(), cabi.F32, n_rep, 0.0,
