@@ -403,11 +403,11 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
         nq_splits = plan_splits(kernel, L->num_units, n_groups, num_splits, D, G, n_rep, n_res_splits, sms, use_mma ? attn_mma_ctas_per_sm() : 0);
     };
     plan();
-    // The scratch a call needs is what the plans of the CUDA-core kernel (fp32 queries) and of
-    // four heads (one head) need: smaller is refused, and where only the newer plan's partials
-    // do not fit, the other is followed.  A workspace for any count holds every plan.
-    const bool any_plan_fits = partial_bytes(kMaxSplitsC) <= workspace_bytes && n_res_splits <= 8;
-    if (wide && !any_plan_fits) {
+    // fp32 queries: the scratch a call needs is what the CUDA-core kernel's plan needs (the one
+    // kivi_decode_attention_plan reports): smaller is refused, and where only the tensor-core
+    // plan's partials do not fit, it takes fewer pieces.  A workspace for any count holds
+    // every plan.
+    if (wide && (partial_bytes(kMaxSplitsC) > workspace_bytes || n_res_splits > 8)) {
         const size_t row = (size_t)L->num_units * n_rep * (D + 2) * sizeof(float);
         const int ring = res_len > 0 ? 1 : 0;
         const auto core_fits = [&](AttnKernel k) {
@@ -421,9 +421,11 @@ static int decode_attention_impl(const kivi_layer* L, int64_t quant_len, int res
             plan();
         }
     }
-    if (num_splits == 0 && kernel == AttnKernel::kMmaOne && !any_plan_fits) {
+    // One head: the plan of four heads may cut coarser; where its partials fit and those of
+    // one head's do not, it is followed.
+    if (num_splits == 0 && kernel == AttnKernel::kMmaOne && partial_bytes(nq_splits) > workspace_bytes) {
         const int general = plan_splits(AttnKernel::kMma, L->num_units, n_groups, 0, D, G, n_rep, n_res_splits, sms, attn_mma_ctas_per_sm());
-        if (partial_bytes(general) > workspace_bytes || partial_bytes(nq_splits) > workspace_bytes) nq_splits = general;
+        if (partial_bytes(general) <= workspace_bytes) nq_splits = general;
     }
     // The tile kernel's plan cuts large problems finer than the generic rule (300 units x
     // 8k tokens: 16 pieces against 4): where its partials do not fit the scratch but the

@@ -384,3 +384,35 @@ def test_attention_split_plan_of_one_head(units, tokens, pieces):
     for u in (1, 5, 148, 444, 2000, 65535):
         for t in (32, 96, 4096, 131072):
             assert 1 <= plan(u, t) <= min(t // 32, 128), (u, t)
+
+
+def _served_with(U, T, res, n_rep, dtype, path, workspace_bytes, num_splits=0):
+    """Whether kivi_decode_attention takes a workspace of this size (at an address it refuses for
+    its alignment, after the size was found to do: nothing is launched)."""
+    from intel_kivi_hybrid_b200 import cabi
+    p = 0x10000
+    layer = cabi.Layer(U, 128, 32, 1024, T, dtype, 0, p, p, p, p, p, p, p, p)
+    rc = cabi.lib.kivi_decode_attention(ctypes.byref(layer), T, 0, res, p, dtype, p, dtype, n_rep, 0.0, 0x10008, workspace_bytes, num_splits, path, None)
+    said = cabi.lib.kivi_last_error().decode()
+    assert rc == 1 and ("aligned" in said or "needed" in said), said
+    return "aligned" in said
+
+
+@pytest.mark.parametrize("n_rep", [1, 2, 3, 4, 5, 8])
+def test_a_workspace_of_the_planned_size_is_served(n_rep):
+    """kivi_decode_attention_plan is there to size a workspace exactly: room for its pieces and
+    ring parts is enough, whatever the kernel.  With one query head per KV head so is room for the
+    plan of four heads, which served one head before it had a plan of its own."""
+    from intel_kivi_hybrid_b200 import cabi
+    refused = []
+    for U in (1, 3, 8, 12, 32, 64, 148, 300, 800):
+        for T in (32, 96, 1024, 2048, 4096, 32768, 131072):
+            for res in (0, 96, 1000):
+                row = U * n_rep * 130 * 4
+                for dtype, path in ((cabi.BF16, cabi.ATTN_AUTO), (cabi.BF16, cabi.ATTN_MMA), (cabi.F32, cabi.ATTN_AUTO), (cabi.F32, cabi.ATTN_FP32)):
+                    pieces = {cabi.attention_plan(U, T, res, n_rep=n_rep, q_dtype=dtype, path=path)[1:]}
+                    if n_rep == 1 and dtype == cabi.BF16:
+                        pieces.add(cabi.attention_plan(U, T, res, n_rep=4, q_dtype=dtype, path=path)[1:])
+                    refused += [(U, T, res, dtype, path, p) for p in pieces if not _served_with(U, T, res, n_rep, dtype, path, sum(p) * row)]
+    assert not refused, (len(refused), refused[:5])
+    assert not _served_with(8, 4096, 96, n_rep, cabi.BF16, cabi.ATTN_AUTO, 2 * 8 * n_rep * 130 * 4)
