@@ -12,12 +12,17 @@
 //   q.k   score[t,h] = sum_d (q[h,d]*s[g,d]) * c[d,t]  +  sum_d q[h,d]*z[g,d]
 //         A = codes of 16 tokens x 32 channels; a byte of four codes is an operand as
 //         it lies, and so is what three masks leave of it (below); B = q*s in 22 bits
-//         and a sign of the largest of the stage, three bytes and a constant (16
+//         and a sign of the largest of the group and head, three bytes and a constant (16
 //         columns = 4 heads x 4 bytes); the zero term is an fp32 dot product.
 //   p.v   out[h,d]   = sum_t (p[h,t]*s[t,gd]) * c[t,d]  +  sum_t p[h,t]*z[t,gd]
 //         A = codes of 16 channels x 32 tokens, same encoding; B = p*s in 16 bits of
-//         the stage's largest (8 columns = 4 heads x 2 bytes); the zero term
-//         accumulates in fp32.
+//         the largest of the stage's tokens, of the same head and channel group (8 columns =
+//         4 heads x 2 bytes); the zero term accumulates in fp32.
+//   What shares a largest value ends in the same sums: scores of one group, outputs of one
+//   channel group.  One for the whole stage cost those beside a louder neighbour their bits
+//   (channel groups 32 times apart: 2.9e-3 of the quiet one's largest output, now 1e-4).
+//   Twice to four times the warp reductions for that: 64 units x 32k 57.1 -> 61.1 us, 128 x 4k
+//   21.8 -> 22.3, one head 512 x 8k 99.4 -> 99.9.
 //   Infinities, NaN and negative value scales take an fp32 form of their own.
 //
 // Bytes instead of fp16 (codes as subnormals, q*s in two parts): 16 codes cost three
@@ -141,8 +146,9 @@ constexpr float kRow1 = 0.25f, kRow2 = 0.0625f, kRow3 = 0.015625f;
 // which is what the top digit's bias adds up to.  22 bits and a sign, against 22 bits of
 // each single element in an fp16 hi/lo pair whose sums the tensor core truncates at 20.
 // p.v: M = 2^23, 0 <= w * F <= 65535: two digits.
-// F follows the largest |w| of a stage and head: the bits of a positive float subtracted from
-// a constant give a float y with x * y between 2 and 2.25 times a power of two.
+// F follows the largest |w| of what goes into the same sums: the bits of a positive float x
+// subtracted from those of (1 + c) * 2^n give a float y with x * y between 1 + c and
+// (1 + c/2)^2 times a power of two (c = 0: 1 and 1.125).
 //
 // Integer accumulators start at the bits of 2^23: read as floats they are 2^23 + sum, since
 // the sums stay below 2^23 (128 * 255 * 255), and differences of them are exact.
@@ -162,9 +168,9 @@ constexpr float kRestV = 255.49f;                         // 0 <= rest < 1 becom
 constexpr float kSmallest = 7.888609052210118e-31f;       // 2^-100: weights below it count as zero beside it
 constexpr uint32_t kExponent = 0x7f800000u, kSmallestBits = 27u << 23;
 constexpr uint32_t kInverseK = 275u << 23;                // largest |w * F| is 2^21 .. 1.125 * 2^21
-constexpr uint32_t kInverseV = 269u << 23;                // 2^15 .. 1.125 * 2^15, and then times kFillV
-constexpr uint32_t kInverseVWide = 276u << 23;            // 2^22 .. 1.125 * 2^22, and then times kFillV
-constexpr float kFillV = 1.7777f;                         // below 65535 / (1.125 * 2^15)
+constexpr uint32_t kInverseV = (269u << 23) + 0x6a0000u;  // 1.828 * 2^15 .. 65523
+constexpr uint32_t kInverseVWide = kInverseV + (7u << 23);         // 2^7 times that
+constexpr uint32_t kLargestScale = 245u << 23;            // 2^118: times a weight (at most 2^8 and a little) still finite
 constexpr float kGrowth = 8.0f;                           // weights up to 2^8 are let stand before the running maximum moves
 
 struct WarpState {
@@ -246,7 +252,7 @@ __device__ __noinline__ float4 weighted_plain(const uint8_t* vc, const float* vs
 template <int NG, bool WIDE>
 __device__ __forceinline__ void qk_phase(const uint8_t* __restrict__ kc, const float* __restrict__ ks, const float* __restrict__ kz,
                                          const LaneView& v, uint8_t* scratch, uint32_t spare, float (&s)[NG][4], float (&fine)[NG][4]) {
-    float w[NG][4][4], sv[NG][4], top[4] = {kSmallest, kSmallest, kSmallest, kSmallest}, qz[NG];
+    float w[NG][4][4], sv[NG][4], top[NG][4], qz[NG];       // top: largest |q * s| of a head, per group of tokens
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
         const float2 sa = *reinterpret_cast<const float2*>(ks + 128 * g + k_channel(v.lane, 0)), sb = *reinterpret_cast<const float2*>(ks + 128 * g + k_channel(v.lane, 2));
@@ -255,11 +261,13 @@ __device__ __forceinline__ void qk_phase(const uint8_t* __restrict__ kc, const f
         for (int h = 0; h < 4; ++h) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) w[g][i][h] = v.qk[i][h] * sv[g][i];
-            top[h] = max3_abs_nan(w[g][2][h], w[g][3][h], max3_abs_nan(w[g][0][h], w[g][1][h], top[h]));
+            top[g][h] = max3_abs_nan(w[g][2][h], w[g][3][h], max3_abs_nan(w[g][0][h], w[g][1][h], kSmallest));
         }
     }
 #pragma unroll
-    for (int h = 0; h < 4; ++h) top[h] = warp_max_abs_nan(top[h]);
+    for (int g = 0; g < NG; ++g)
+#pragma unroll
+        for (int h = 0; h < 4; ++h) top[g][h] = warp_max_abs_nan(top[g][h]);
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
         float z0 = 0.0f, z1 = 0.0f;
@@ -281,7 +289,10 @@ __device__ __forceinline__ void qk_phase(const uint8_t* __restrict__ kc, const f
 #pragma unroll
         for (int g = 0; g < NG; ++g) qz[g] += __shfl_xor_sync(0xffffffffu, qz[g], off);
     __syncwarp();                                           // the scratch is free
-    if (!((top[0] + top[1]) + (top[2] + top[3]) <= 3.0e38f)) {
+    float largest = top[0][0];
+#pragma unroll
+    for (int g = 0; g < NG; ++g) largest = max3_abs_nan(top[g][0], top[g][1], max3_abs_nan(top[g][2], top[g][3], largest));
+    if (!(largest <= 3.0e38f)) {
 #pragma unroll
         for (int h = 0; h < 4; ++h)
 #pragma unroll
@@ -296,21 +307,13 @@ __device__ __forceinline__ void qk_phase(const uint8_t* __restrict__ kc, const f
         }
         return;
     }
-    float F[4], unit;
-    if constexpr (WIDE) {                                   // a power of two, so that unit = 1 / F exactly
-#pragma unroll
-        for (int h = 0; h < 4; ++h) F[h] = __uint_as_float(kInverseK - (1u << 23) - (__float_as_uint(top[h]) & kExponent));
-        unit = __uint_as_float((254u << 23) - __float_as_uint(v.tig == 0 ? F[0] : v.tig == 1 ? F[1] : v.tig == 2 ? F[2] : F[3]));
-        // (the products are made again from here on: 32 of them would not stay in registers)
+    if constexpr (WIDE) {                                   // (the products are made again from here on: 32 of them would not stay in registers)
 #pragma unroll
         for (int g = 0; g < NG; ++g)
 #pragma unroll
             for (int i = 0; i < 4; ++i) asm volatile("" : "+f"(sv[g][i]));
-    } else {
-#pragma unroll
-        for (int h = 0; h < 4; ++h) F[h] = __uint_as_float(kInverseK - __float_as_uint(top[h]));
-        unit = rcp_approx(v.tig == 0 ? F[0] : v.tig == 1 ? F[1] : v.tig == 2 ? F[2] : F[3]);
     }
+    float unit[NG];
     constexpr int kBlocks = WIDE ? 3 : 2;                   // column blocks: digits 0,1 / 2,const / rest 0,1
     constexpr int kDigits = 2 * kBlocks - 1;
     int c[WIDE ? 1 : NG][2][kBlocks][4];                    // [rows of codes 0,1 / 2,3 and up]
@@ -344,11 +347,11 @@ __device__ __forceinline__ void qk_phase(const uint8_t* __restrict__ kc, const f
             for (int i = 0; i < kDigits; ++i) d[i] = y[n][i] - y[n + 1][i];
             if constexpr (WIDE) {
                 const float off = -kMiddle / row;
-                s[g][n] = fmaf(all[2], off, d[2]) * (65536.0f * row) * unit;
+                s[g][n] = fmaf(all[2], off, d[2]) * (65536.0f * row) * unit[g];
                 const float low = fmaf(below, off, fmaf(fmaf(d[4], 256.0f, d[3]), 0x1p-15f, d[0]));
-                fine[g][n] = fmaf(fmaf(fmaf(all[1], off, d[1]), 256.0f, low), unit * row, qz[g]);
+                fine[g][n] = fmaf(fmaf(fmaf(all[1], off, d[1]), 256.0f, low), unit[g] * row, qz[g]);
             } else {
-                s[g][n] = fmaf(fmaf(d[2], 65536.0f, fmaf(d[1], 256.0f, d[0])), unit * row, qz[g]);
+                s[g][n] = fmaf(fmaf(d[2], 65536.0f, fmaf(d[1], 256.0f, d[0])), unit[g] * row, qz[g]);
                 fine[g][n] = 0.0f;
             }
         }
@@ -356,6 +359,12 @@ __device__ __forceinline__ void qk_phase(const uint8_t* __restrict__ kc, const f
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
         if (g > 0) __syncwarp();                            // the operand of the group before has been read
+        float F[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h)                          // (WIDE: a power of two, so that unit = 1 / F exactly)
+            F[h] = __uint_as_float(WIDE ? kInverseK - (1u << 23) - (__float_as_uint(top[g][h]) & kExponent) : kInverseK - __float_as_uint(top[g][h]));
+        const float own = v.tig == 0 ? F[0] : v.tig == 1 ? F[1] : v.tig == 2 ? F[2] : F[3];
+        unit[g] = WIDE ? __uint_as_float((254u << 23) - __float_as_uint(own)) : rcp_approx(own);
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             uint32_t x[2][4], rest[2][4];
@@ -472,21 +481,18 @@ __device__ __forceinline__ void pv_phase(const uint8_t* __restrict__ vc, const f
     }
     __syncwarp();
     float ph[NG][4], sv[NG][4];                             // weights [head], scales [channel group] of the lane's token
-    uint32_t top[4] = {kSmallestBits, kSmallestBits, kSmallestBits, kSmallestBits};
+    uint32_t p_bits = 0u, s_bits = 0u;
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
         const float4 p4 = lds128(v.p_read + 512 * g);
         const float4 s4 = *reinterpret_cast<const float4*>(vs + g * 128 + 4 * v.lane);
         ph[g][0] = p4.x; ph[g][1] = p4.y; ph[g][2] = p4.z; ph[g][3] = p4.w;
         sv[g][0] = s4.x; sv[g][1] = s4.y; sv[g][2] = s4.z; sv[g][3] = s4.w;
-        // as integers, the bits of negative numbers, infinities and NaN all lie above those of a finite one
-        const float smax = __uint_as_float(max(max(__float_as_uint(s4.x), __float_as_uint(s4.y)), max(__float_as_uint(s4.z), __float_as_uint(s4.w))));
 #pragma unroll
-        for (int h = 0; h < 4; ++h) top[h] = max(top[h], __float_as_uint(ph[g][h] * smax));
+        for (int i = 0; i < 4; ++i) { p_bits = max(p_bits, __float_as_uint(ph[g][i])); s_bits = max(s_bits, __float_as_uint(sv[g][i])); }
     }
-#pragma unroll
-    for (int h = 0; h < 4; ++h) top[h] = warp_max_u32(top[h]);
-    if (max(max(top[0], top[1]), max(top[2], top[3])) >= kExponent) {
+    // as integers, the bits of negative numbers, infinities and NaN all lie above those of a finite one
+    if (__any_sync(0xffffffffu, p_bits >= kExponent || s_bits >= kLargestScale)) {
 #pragma unroll
         for (int g = 0; g < NG; ++g)
 #pragma unroll
@@ -510,25 +516,42 @@ __device__ __forceinline__ void pv_phase(const uint8_t* __restrict__ vc, const f
             st.oz[h][2] = fmaf(ph[g][h], z4.z, st.oz[h][2]); st.oz[h][3] = fmaf(ph[g][h], z4.w, st.oz[h][3]);
         }
     }
-    float F[4];
+    // the products of a channel group and the largest of each head, one group ahead of their use
+    float w[2][NG][4], unit[4];
+    uint32_t top[2][4];
+    auto weigh = [&](int gd) {
 #pragma unroll
-    for (int h = 0; h < 4; ++h) F[h] = __uint_as_float((WIDE ? kInverseVWide : kInverseV) - top[h]) * kFillV;
-    const float own = v.tig == 0 ? F[0] : v.tig == 1 ? F[1] : v.tig == 2 ? F[2] : F[3];
-    float unit = rcp_approx(own);
-    if constexpr (WIDE) unit = fmaf(unit, fmaf(-own, unit, 1.0f), unit);
+        for (int h = 0; h < 4; ++h) {
+            uint32_t t = kSmallestBits;
+#pragma unroll
+            for (int g = 0; g < NG; ++g) {
+                w[gd & 1][g][h] = ph[g][h] * sv[g][gd];
+                t = max(t, __float_as_uint(w[gd & 1][g][h]));
+            }
+            top[gd & 1][h] = warp_max_u32(t);
+        }
+    };
+    weigh(0);
     __syncwarp();                                           // every lane has read its weights
     // Rows of 16 bytes per channel group and contraction index k = 4*c + n: the columns
     // [head][digit] of tokens 16*0 + k and 16*1 + k, in the other order for k >= 8 (the writes
     // of a half-warp then touch every bank once; the codes are read in that order too).
 #pragma unroll
-    for (int g = 0; g < NG; ++g)
+    for (int gd = 0; gd < 4; ++gd) {
+        if (gd < 3) weigh(gd + 1);
+        float F[4];
 #pragma unroll
-        for (int gd = 0; gd < 4; ++gd) {
+        for (int h = 0; h < 4; ++h) F[h] = __uint_as_float((WIDE ? kInverseVWide : kInverseV) - top[gd & 1][h]);
+        const float own = v.tig == 0 ? F[0] : v.tig == 1 ? F[1] : v.tig == 2 ? F[2] : F[3];
+        unit[gd] = rcp_approx(own);
+        if constexpr (WIDE) unit[gd] = fmaf(unit[gd], fmaf(-own, unit[gd], 1.0f), unit[gd]);
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
             uint32_t x[4];
             if constexpr (WIDE) {                           // below the 23 bits eight more: the rest of a number rounded down
 #pragma unroll
                 for (int h = 0; h < 4; ++h) {
-                    const float y = ph[g][h] * sv[g][gd], t = __fmaf_rz(y, F[h], kTwo23), r = fmaf(fmaf(y, F[h], kTwo23 - t), kRestV, kTwo23);
+                    const float y = w[gd & 1][g][h], t = __fmaf_rz(y, F[h], kTwo23), r = fmaf(fmaf(y, F[h], kTwo23 - t), kRestV, kTwo23);
                     x[h] = __byte_perm(__float_as_uint(r), __float_as_uint(t), 0x6540);
                 }
                 const uint32_t row = (g == 0 ? v.v_write : v.v_write - v.scratch + spare) + 512 * gd;
@@ -536,10 +559,11 @@ __device__ __forceinline__ void pv_phase(const uint8_t* __restrict__ vc, const f
                 sts64(row + 256, __byte_perm(x[0], x[1], 0x7632), __byte_perm(x[2], x[3], 0x7632));
             } else {
 #pragma unroll
-                for (int h = 0; h < 4; ++h) x[h] = __float_as_uint(fmaf(ph[g][h] * sv[g][gd], F[h], kTwo23));
+                for (int h = 0; h < 4; ++h) x[h] = __float_as_uint(fmaf(w[gd & 1][g][h], F[h], kTwo23));
                 sts64(v.v_write + 1024 * g + 256 * gd, __byte_perm(x[0], x[1], 0x5410), __byte_perm(x[2], x[3], 0x5410));
             }
         }
+    }
     __syncwarp();
     if constexpr (WIDE) {
 #pragma unroll
@@ -578,7 +602,7 @@ __device__ __forceinline__ void pv_phase(const uint8_t* __restrict__ vc, const f
                     d[k] = __int_as_float(acc[mt][k >> 1][r + (k & 1)]) - (i < 3 ? __int_as_float(acc[mt1][k >> 1][r1 + (k & 1)]) : kTwo23);
                 const float low = fmaf(below, off, fmaf(d[2], 256.0f, fmaf(d[0], 1.0f / kRestV, d[1])));
                 float& o = st.o[2 * gd + mt][i & 1];
-                o = fmaf(fmaf(fmaf(all[3], off, d[3]), 65536.0f, low), unit, o);
+                o = fmaf(fmaf(fmaf(all[3], off, d[3]), 65536.0f, low), unit[gd], o);
             }
         }
         return;
@@ -612,7 +636,7 @@ __device__ __forceinline__ void pv_phase(const uint8_t* __restrict__ vc, const f
             const int mt = 2 * gd + (i >> 1), r = 2 * (i & 1), mt1 = 2 * gd + ((i + 1) >> 1), r1 = 2 * ((i + 1) & 1);
             const float n0 = i < 3 ? __int_as_float(acc[i < 3 ? mt1 : 0][r1]) : kTwo23, n1 = i < 3 ? __int_as_float(acc[i < 3 ? mt1 : 0][r1 + 1]) : kTwo23;
             const float d0 = __int_as_float(acc[mt][r]) - n0, d1 = __int_as_float(acc[mt][r + 1]) - n1;
-            st.o[mt][i & 1] = fmaf(fmaf(d1, 256.0f, d0), unit, st.o[mt][i & 1]);
+            st.o[mt][i & 1] = fmaf(fmaf(d1, 256.0f, d0), unit[gd], st.o[mt][i & 1]);
         }
 }
 
@@ -656,18 +680,18 @@ __device__ __forceinline__ int zero_quad_one(int i, int gid, int tig) { return 4
 template <int NG>
 __device__ __forceinline__ void qk_one(const uint8_t* __restrict__ kc, const float* __restrict__ ks, const float* __restrict__ kz,
                                        const OneView& v, uint8_t* scratch, float (&s)[4]) {
-    float w[2][4], top = kSmallest;
+    float w[2][4], top[2];                                  // top: largest |q * s| of a group of tokens
 #pragma unroll
     for (int g = 0; g < 2; ++g) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) w[g][i] = 0.0f;
+        top[g] = kSmallest;
         if (g < NG) {
             const float2 sa = *reinterpret_cast<const float2*>(ks + 128 * g + k_channel(v.lane, 0)), sb = *reinterpret_cast<const float2*>(ks + 128 * g + k_channel(v.lane, 2));
             w[g][0] = v.qk[0] * sa.x; w[g][1] = v.qk[1] * sa.y; w[g][2] = v.qk[2] * sb.x; w[g][3] = v.qk[3] * sb.y;
-            top = max3_abs_nan(w[g][2], w[g][3], max3_abs_nan(w[g][0], w[g][1], top));
+            top[g] = warp_max_abs_nan(max3_abs_nan(w[g][2], w[g][3], max3_abs_nan(w[g][0], w[g][1], kSmallest)));
         }
     }
-    top = warp_max_abs_nan(top);
     const int mine = v.tig < NG ? v.tig : 0;
     float z0 = 0.0f, z1 = 0.0f;
 #pragma unroll
@@ -680,21 +704,22 @@ __device__ __forceinline__ void qk_one(const uint8_t* __restrict__ kc, const flo
 #pragma unroll
     for (int off = 4; off <= 16; off *= 2) qz += __shfl_xor_sync(0xffffffffu, qz, off);
     __syncwarp();                                           // the scratch is free
-    if (!(top <= 3.0e38f)) {
+    if (!(top[0] + top[1] <= 3.0e38f)) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) sts32(v.scratch + 4 * k_channel(v.lane, i), v.qk[i]);
         __syncwarp();
         const float4 r = scores_plain(kc + 1024 * mine, ks + 128 * mine, kz + 128 * mine, reinterpret_cast<const float4*>(scratch), v.gid);
         s[0] = r.x; s[1] = r.y; s[2] = r.z; s[3] = r.w;
     } else {
-        const float F = __uint_as_float(kInverseK - __float_as_uint(top)), unit = rcp_approx(F);
+        const float F[2] = {__uint_as_float(kInverseK - __float_as_uint(top[0])), __uint_as_float(kInverseK - __float_as_uint(top[1]))};
+        const float unit = rcp_approx(mine ? F[1] : F[0]);
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             uint32_t x[2][2];
 #pragma unroll
             for (int k = 0; k < 2; ++k)
 #pragma unroll
-                for (int g = 0; g < 2; ++g) x[k][g] = __float_as_uint(fmaf(w[g][2 * k + e], F, kMagicK));
+                for (int g = 0; g < 2; ++g) x[k][g] = __float_as_uint(fmaf(w[g][2 * k + e], F[g], kMagicK));
             // columns: digits 0 and 1 of the two groups; digit 2 and the constant
             sts128(v.scratch + 512 * e + 16 * v.lane, __byte_perm(x[0][0], x[0][1], 0x5410), 0u, __byte_perm(x[1][0], x[1][1], 0x5410), 0u);
             sts128(v.scratch + 1024 + 512 * e + 16 * v.lane, __byte_perm(x[0][0], x[0][1], 0x7632), 0u, __byte_perm(x[1][0], x[1][1], 0x7632), 0u);
@@ -765,17 +790,18 @@ __device__ __forceinline__ void pv_one(const uint8_t* __restrict__ vc, const flo
     }
     __syncwarp();
     float ph[NG], sv[NG][4];
-    uint32_t top = kSmallestBits;
+    uint32_t top[4] = {kSmallestBits, kSmallestBits, kSmallestBits, kSmallestBits};      // largest p * s of a channel group
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
         ph[g] = lds32(v.scratch + 128 * g + 4 * v.lane);
         const float4 s4 = *reinterpret_cast<const float4*>(vs + g * 128 + 4 * v.lane);
         sv[g][0] = s4.x; sv[g][1] = s4.y; sv[g][2] = s4.z; sv[g][3] = s4.w;
-        const float smax = __uint_as_float(max(max(__float_as_uint(s4.x), __float_as_uint(s4.y)), max(__float_as_uint(s4.z), __float_as_uint(s4.w))));
-        top = max(top, __float_as_uint(ph[g] * smax));
+#pragma unroll
+        for (int gd = 0; gd < 4; ++gd) top[gd] = max(top[gd], __float_as_uint(ph[g] * sv[g][gd]));
     }
-    top = warp_max_u32(top);
-    if (top >= kExponent) {
+#pragma unroll
+    for (int gd = 0; gd < 4; ++gd) top[gd] = warp_max_u32(top[gd]);
+    if (max(max(top[0], top[1]), max(top[2], top[3])) >= kExponent) {
 #pragma unroll
         for (int g = 0; g < NG; ++g) {
             const float4 r = weighted_plain<true>(vc + g * 1024, vs + g * 128, vz + g * 128, reinterpret_cast<const float*>(scratch + 128 * g), v.tig, v.gid, 0);
@@ -783,7 +809,10 @@ __device__ __forceinline__ void pv_one(const uint8_t* __restrict__ vc, const flo
         }
         return;
     }
-    const float F = __uint_as_float(kInverseV - top) * kFillV, unit = rcp_approx(F);
+    float F[4];
+#pragma unroll
+    for (int gd = 0; gd < 4; ++gd) F[gd] = __uint_as_float(kInverseV - top[gd]);
+    const float unit = rcp_approx(v.tig == 0 ? F[0] : v.tig == 1 ? F[1] : v.tig == 2 ? F[2] : F[3]);       // (the lane's columns are of group tig)
     __syncwarp();                                           // every lane has read its weights
 #pragma unroll
     for (int g = 0; g < NG; ++g) {
@@ -792,7 +821,7 @@ __device__ __forceinline__ void pv_one(const uint8_t* __restrict__ vc, const flo
         st.oz[2] = fmaf(ph[g], z4.z, st.oz[2]); st.oz[3] = fmaf(ph[g], z4.w, st.oz[3]);
         uint32_t x[4];
 #pragma unroll
-        for (int gd = 0; gd < 4; ++gd) x[gd] = __float_as_uint(fmaf(ph[g] * sv[g][gd], F, kTwo23));
+        for (int gd = 0; gd < 4; ++gd) x[gd] = __float_as_uint(fmaf(ph[g] * sv[g][gd], F[gd], kTwo23));
         sts64(v.v_write + 256 * g, __byte_perm(x[0], x[1], 0x5410), __byte_perm(x[2], x[3], 0x5410));       // columns [channel group][digit]
     }
     __syncwarp();

@@ -711,6 +711,36 @@ def test_attention_mma_at_the_edges_of_its_fixed_point_operands(cabi, what, toke
     assert ((got - want)[ok].abs().max() / size).item() < 2.9e-3
 
 
+@pytest.mark.parametrize("loud", ["channel group", "token group"])
+@pytest.mark.parametrize("dtype,n_rep", [(torch.bfloat16, 1), (torch.bfloat16, 2), (torch.bfloat16, 4), (torch.bfloat16, 8), (torch.float32, 4)])
+@pytest.mark.parametrize("n_quant,n_res", [(96, 5), (1056, 0)])
+def test_attention_beside_a_louder_neighbour(cabi, n_quant, n_res, dtype, n_rep, loud):
+    """Values of one channel group, or keys of every other token group (far below the others in
+    the softmax), thousands of times larger than their neighbours: every channel group of a row
+    keeps the tolerance against its own largest output.  (A weight is off by 2^-17 of the largest
+    of its own sums at most: 64 of a stage, three at most of a code, as independent roundings
+    3 * 8 * 2^-17 = 1.8e-4 of the largest weight, a tenth of the bf16 tolerance; fp32 2^-15 of that.)"""
+    B, Hkv, D, G, T = 1, 3, 128, 32, n_quant + n_res
+    K, V = ko.make_keys(B, Hkv, T, D, 23), ko.make_values(B, Hkv, T, D, 23)
+    q = ko.make_queries(B, Hkv * n_rep, D, 23)
+    if loud == "channel group":
+        V[..., 32:64] *= 2.0 ** 14
+    else:
+        q[..., 0] = 3.0
+        K[..., 0] = 0.0
+        for t in range(0, n_quant, 2 * G):
+            K[:, :, t:t + G] *= 2.0 ** 14
+            K[:, :, t:t + G, 0] = -100.0 * 2.0 ** 14
+    K, V, q = K.to(dtype), V.to(dtype), q.to(dtype)
+    st = cabi.LayerStore(B * Hkv, D, G, 128, n_quant, dtype, "cuda")
+    cabi.load_state(st, units(K).cuda(), units(V).cuda(), n_quant)
+    out = st.attention(q.cuda(), n_rep=n_rep, out_dtype=torch.float32)
+    ref = ko.kivi_decode_attention(q, K, V, n_quant, G, "half_away", dtype=torch.float64)
+    err = rel_err(out.view(-1, 4, 32), ref.view(-1, 4, 32).float())
+    print(f"[attn beside a louder {loud} {dtype} heads={n_rep} q={n_quant}] rel err {err:.2e}")
+    assert err < (TOL_BF16 if dtype == torch.bfloat16 else TOL_F32) and cabi.device_fault() == 0
+
+
 @pytest.mark.parametrize("n_quant,n_res,n_rep,splits", [(1024, 0, 3, 1), (1056, 77, 4, 0), (1312, 128, 5, 7), (4064, 200, 8, 0), (2080, 1, 4, 65)])
 def test_attention_fp32_queries_on_the_tensor_cores(cabi, n_quant, n_res, n_rep, splits):
     """From three heads and 1024 tokens on fp32 queries are served there: whole and odd
