@@ -245,7 +245,7 @@ __device__ __noinline__ float4 weighted_plain(const uint8_t* vc, const float* vs
 
 // ---- NG token groups (32 tokens each) in three phases -------------------------------
 // q.k: scores of the lane's four tokens (4*gid + n) of each group for head `tig`, log2 domain.
-// A score is s + fine; fine is 0 but for WIDE, where s is a multiple of the top digit's unit,
+// A score is s, or for WIDE s + fine, where s is a multiple of the top digit's unit,
 // so that s less the running maximum, the number exponentiated, keeps all its bits.
 // `spare` (WIDE): the stage's key scales and zeros, kGPS * 1024 bytes, which take operands
 // once they have been read.
@@ -302,8 +302,10 @@ __device__ __forceinline__ void qk_phase(const uint8_t* __restrict__ kc, const f
         for (int g = 0; g < NG; ++g) {
             const float4 r = scores_plain(kc + 1024 * g, ks + 128 * g, kz + 128 * g, reinterpret_cast<const float4*>(scratch) + 32 * v.tig, v.gid);
             s[g][0] = r.x; s[g][1] = r.y; s[g][2] = r.z; s[g][3] = r.w;
+            if constexpr (WIDE) {
 #pragma unroll
-            for (int n = 0; n < 4; ++n) fine[g][n] = 0.0f;
+                for (int n = 0; n < 4; ++n) fine[g][n] = 0.0f;
+            }
         }
         return;
     }
@@ -352,7 +354,6 @@ __device__ __forceinline__ void qk_phase(const uint8_t* __restrict__ kc, const f
                 fine[g][n] = fmaf(fmaf(fmaf(all[1], off, d[1]), 256.0f, low), unit[g] * row, qz[g]);
             } else {
                 s[g][n] = fmaf(fmaf(d[2], 65536.0f, fmaf(d[1], 256.0f, d[0])), unit[g] * row, qz[g]);
-                fine[g][n] = 0.0f;
             }
         }
     };
@@ -432,13 +433,13 @@ __device__ __forceinline__ void qk_phase(const uint8_t* __restrict__ kc, const f
 }
 
 // running max / sum update for NG groups at once; turns scores into weights
-template <int NG>
+template <int NG, bool WIDE>
 __device__ __forceinline__ void softmax_phase(float (&s)[NG][4], const float (&fine)[NG][4], WarpState& st) {
     float gmax = -INFINITY;
 #pragma unroll
     for (int g = 0; g < NG; ++g)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) gmax = fmaxf(gmax, s[g][e] + fine[g][e]);
+        for (int e = 0; e < 4; ++e) gmax = fmaxf(gmax, WIDE ? s[g][e] + fine[g][e] : s[g][e]);
     if (__any_sync(0xffffffffu, gmax > st.m + kGrowth)) {
         gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 4));
         gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, 8));
@@ -459,7 +460,7 @@ __device__ __forceinline__ void softmax_phase(float (&s)[NG][4], const float (&f
 #pragma unroll
     for (int g = 0; g < NG; ++g)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) { s[g][e] = ex2((s[g][e] - st.m) + fine[g][e]); st.l += s[g][e]; }
+        for (int e = 0; e < 4; ++e) { s[g][e] = ex2(WIDE ? (s[g][e] - st.m) + fine[g][e] : s[g][e] - st.m); st.l += s[g][e]; }
 }
 
 // p.v of NG groups; p[g][n] = weight of token 4*gid + n of group g for head tig.
@@ -647,7 +648,7 @@ __device__ __forceinline__ void process_groups(const uint8_t* __restrict__ sb, c
     float s[NG][4], fine[NG][4];
     const uint32_t spare = WIDE ? smem_u32(sb + kGPS * 1024) : 0u;
     qk_phase<NG, WIDE>(sb, reinterpret_cast<const float*>(sb + kGPS * 1024), reinterpret_cast<const float*>(sb + kGPS * 1536), v, scratch, spare, s, fine);
-    softmax_phase<NG>(s, fine, st);
+    softmax_phase<NG, WIDE>(s, fine, st);
     pv_phase<NG, WIDE>(sb + kGPS * 2048, reinterpret_cast<const float*>(sb + kGPS * 3072), reinterpret_cast<const float*>(sb + kGPS * 3584), s, v, scratch, spare, st);
     // what was written over the stage comes before the copy that fills it again
     if constexpr (WIDE) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
