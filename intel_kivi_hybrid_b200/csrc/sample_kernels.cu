@@ -543,8 +543,16 @@ static int sample_threads(int batch, int vocab, int cut) {
     return walk;
 }
 
-// Rows that fit the shared memory of an SM are staged there when every row has an SM of its own.
+// Rows that fit the shared memory of an SM are staged there when every row has an SM of its
+// own and the row is long enough.  Threads take a staged row 16 bytes at a time, so a short one
+// leaves threads without an entry, and with fewer maxima than the cut keeps there is no bound:
+// every entry is a candidate.  us for 32 rows, staged / from memory: k = 20 of 2049 bf16 entries
+// 30.3 / 4.8, k = 300 of 1000 28.1 / 10.8.  Where there is a bound, waiting for the copies
+// costs more than loads in flight until the row outgrows those: k = 50 of 24000 fp32 entries
+// 9.05 / 8.37, of 40000 9.44 / 9.50, of 106000 bf16 a tenth less.  Draws and the radix select,
+// which walk the row more often: 2049 entries 5.06 / 4.73, 4500 7.4 / 7.4, 13000 10.8 / 11.7.
 constexpr size_t kStagedBytes = 208 * 1024;
+constexpr int kStagedFromCut = 40000, kStagedFrom = 4096;
 
 template <typename T, int kThreads, Choice kChoice>
 static cudaError_t allow_staged() {
@@ -567,7 +575,7 @@ static cudaError_t launch_sample(const T* logits, int batch, int vocab, int64_t 
         constexpr Choice c = decltype(choice)::value;
         if constexpr (kThreads > 256) {
             const size_t bytes = ((size_t)vocab * sizeof(T) + 32) / 16 * 16;           // whole 16 bytes at any offset
-            if (batch <= num_sms() && bytes <= kStagedBytes) {
+            if (batch <= num_sms() && bytes <= kStagedBytes && vocab >= (c == Choice::kTopK ? kStagedFromCut : kStagedFrom)) {
                 if (cudaError_t e = allow_staged<T, kThreads, c>(); e != cudaSuccess) return e;
                 return go(sample_kernel<T, kThreads, c, true>, bytes);
             }

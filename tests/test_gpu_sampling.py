@@ -167,3 +167,29 @@ def test_rows_at_any_offset_from_sixteen_bytes(cabi, dtype, vocab, offset):
         wrong += int((got != ko.sample_tokens(x.float(), 0.9, top_k or None, True, seed=5, step=top_k)).sum())
     assert wrong <= 1                                             # (a draw on a boundary: see the oracle test above)
     assert cabi.device_fault() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_a_cut_of_a_short_row_costs_no_more_than_one_of_its_neighbour(cabi, dtype):
+    """With fewer 16-byte pieces in a row than entries to keep, a form that gives threads whole
+    pieces has no bound for the cut and ranks or radix-selects the row instead, at up to six
+    times the time.  A row just above a change of form stays within twice the row below it, a
+    row of 1000 entries below one of 9000."""
+    def us(vocab, top_k):
+        x = (3.0 * torch.randn(32, vocab, generator=torch.Generator().manual_seed(vocab))).to(dtype).cuda()
+        out = torch.empty(32, dtype=torch.int64, device="cuda")
+        best = float("inf")
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda._sleep(2_000_000)                     # the host gets ahead of the GPU
+            a.record()
+            for i in range(50):
+                cabi.sample_tokens(x, 0.9, top_k, True, seed=1, step=i, out=out)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b) * 20)
+        return best
+
+    for top_k in (20, 50, 64):
+        assert us(2049, top_k) < 2 * us(2048, top_k), top_k
+    assert us(1000, 300) < us(9000, 300)
