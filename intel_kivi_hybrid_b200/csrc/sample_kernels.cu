@@ -214,10 +214,16 @@ sample_kernel(const T* logits, int vocab, int64_t row_stride,
             best = better(best, MaxIdx{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)});
         if (lane == 0) { red_f[warp] = best.v; red_i[warp] = best.i; }
         __syncthreads();
-        best = lane < kWarps ? MaxIdx{red_f[lane], red_i[lane]} : MaxIdx{-INFINITY, 0x7fffffff};
+        if constexpr (kWarps <= 8) {                        // (side by side eight reads cost less than five exchanges: 32 x 2048 1.56 us, not 1.66)
+            best = MaxIdx{red_f[0], red_i[0]};
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            best = better(best, MaxIdx{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)});
+            for (int w = 1; w < kWarps; ++w) best = better(best, MaxIdx{red_f[w], red_i[w]});
+        } else {
+            best = lane < kWarps ? MaxIdx{red_f[lane], red_i[lane]} : MaxIdx{-INFINITY, 0x7fffffff};
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                best = better(best, MaxIdx{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)});
+        }
         if (best.i == 0x7fffffff) best.i = 0;
         return best;
     };
