@@ -409,11 +409,13 @@ def merge_token_shards(parts, out_dtype=torch.float32):
 
 def sample_tokens(logits, temperature=1.0, top_k=0, do_sample=False, seed=0, step=0, out=None):
     """kivi_sample_tokens: [batch, vocab] fp32 / bf16 device logits (last dim
-    contiguous) -> int64 [batch] device ids, without a host round trip."""
+    contiguous) -> int64 [batch] device ids, without a host round trip.  out, if
+    given, is an int64 tensor with at least that many elements."""
     assert logits.dim() == 2 and logits.stride(1) == 1
+    top_k = max(-2**31, min(int(top_k or 0), 2**31 - 1))     # (no row has more entries: the same cut, in the library's int)
     ops = _native_ops()
     if ops is not None:
-        return ops.sample_tokens(logits, float(temperature), int(top_k or 0), bool(do_sample), int(seed) & (2**64 - 1), int(step) & (2**64 - 1), out)
+        return ops.sample_tokens(logits, float(temperature), top_k, bool(do_sample), int(seed) & (2**64 - 1), int(step) & (2**64 - 1), out)
     if not logits.is_cuda:
         raise RuntimeError("tensor must be on a CUDA device")
     if out is None:
@@ -421,8 +423,12 @@ def sample_tokens(logits, temperature=1.0, top_k=0, do_sample=False, seed=0, ste
     _dev(out)
     if out.device != logits.device:
         raise RuntimeError(f"all tensors of one call must be on the same device, got {logits.device} and {out.device}")
+    if out.dtype != torch.int64 or out.numel() < logits.shape[0]:
+        raise RuntimeError("out must be int64 and hold an id for every row of logits")
+    if max(logits.shape) > 2**31 - 1:
+        raise RuntimeError("batch and vocab must be below 2**31")
     _check(lib.kivi_sample_tokens(logits.data_ptr(), _dt(logits), logits.shape[0], logits.shape[1], logits.stride(0),
-                                  float(temperature), int(top_k or 0), int(bool(do_sample)), int(seed) & (2**64 - 1),
+                                  float(temperature), top_k, int(bool(do_sample)), int(seed) & (2**64 - 1),
                                   int(step) & (2**64 - 1), out.data_ptr(), _stream()))
     return out
 

@@ -13,6 +13,8 @@
 // Blocking operators return after the kernel has finished, like the reference's
 // wait_and_throw (quantize_kernels.cpp:64-66); *_async operators return a
 // KiviEvent recorded behind the kernel (event.hpp:18-29).
+#include <algorithm>
+
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
@@ -342,19 +344,24 @@ torch::Tensor cache_attention(int64_t layer, int64_t quant_len, int res_start, i
 torch::Tensor sample_tokens(const torch::Tensor& logits, double temperature, int64_t top_k, bool do_sample, uint64_t seed, uint64_t step,
                             const c10::optional<torch::Tensor>& out) {
     auto fail = [](const std::string& what) { throw std::runtime_error(what); };
+    if (logits.dim() != 2 || logits.stride(1) != 1) fail("logits must be [batch, vocab] with entries side by side");
     if (!logits.is_cuda()) fail("tensor must be on a CUDA device");
     if (out.has_value()) {
         if (!out->is_cuda()) fail("tensor must be on a CUDA device");
         if (!out->is_contiguous()) fail("tensor must be contiguous");
         if (out->device() != logits.device())
             fail("all tensors of one call must be on the same device, got " + logits.device().str() + " and " + out->device().str());
+        // (the kernel writes one 64-bit id per row through a raw pointer)
+        if (out->scalar_type() != torch::kLong || out->numel() < logits.size(0)) fail("out must be int64 and hold an id for every row of logits");
     }
+    constexpr int64_t kIntMax = 0x7fffffff;
+    if (logits.size(0) > kIntMax || logits.size(1) > kIntMax) fail("batch and vocab must be below 2**31");
     if (logits.scalar_type() != torch::kFloat32 && logits.scalar_type() != torch::kBFloat16)
         fail("unsupported dtype torch." + dtype_name(logits.scalar_type()) + ": expected float32 or bfloat16");
     c10::cuda::CUDAGuard guard(logits.device());
     const torch::Tensor ids = out.has_value() ? *out : at::empty({logits.size(0)}, logits.options().dtype(torch::kLong));
     const int rc = kivi_sample_tokens(logits.data_ptr(), logits.scalar_type() == torch::kFloat32 ? KIVI_F32 : KIVI_BF16, (int)logits.size(0), (int)logits.size(1),
-                                      logits.stride(0), (float)temperature, (int)top_k, do_sample ? 1 : 0, seed, step, reinterpret_cast<int64_t*>(ids.data_ptr()),
+                                      logits.stride(0), (float)temperature, (int)std::min(std::max(top_k, -kIntMax), kIntMax), do_sample ? 1 : 0, seed, step, reinterpret_cast<int64_t*>(ids.data_ptr()),
                                       at::cuda::getCurrentCUDAStream().stream());
     if (rc != KIVI_OK) fail("kivi_cuda error " + std::to_string(rc) + ": " + kivi_last_error());
     return ids;

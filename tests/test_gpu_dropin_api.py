@@ -423,6 +423,35 @@ def test_native_sampling_call_equals_the_ctypes_call(monkeypatch):
     assert native[1] == general[1]
 
 
+def test_sampling_refuses_ids_it_would_write_out_of_range(monkeypatch):
+    """One 64-bit id per row is written through a raw pointer: an out of another type or with
+    fewer elements is refused before the launch, by both bindings with the same words; a longer
+    one is taken.  A top_k beyond the library's int is no cut, as any above the row's length is."""
+    from intel_kivi_hybrid_b200 import cabi
+    x = 3 * torch.randn(9, 501, generator=torch.Generator(device="cuda").manual_seed(3), device="cuda")
+    ops = cabi._native_ops()
+    said = []
+    for path in (ops, False):
+        monkeypatch.setattr(cabi, "_ops", path)
+        for out in (torch.empty(9, dtype=torch.int32, device="cuda"), torch.empty(18, dtype=torch.int32, device="cuda"),
+                    torch.empty(9, dtype=torch.float64, device="cuda"), torch.empty(8, dtype=torch.int64, device="cuda"), torch.empty(0, dtype=torch.int64, device="cuda")):
+            with pytest.raises(RuntimeError, match="out must be int64") as e:
+                cabi.sample_tokens(x, out=out)
+            said.append(str(e.value))
+        longer = torch.full((11,), -1, dtype=torch.int64, device="cuda")
+        assert torch.equal(cabi.sample_tokens(x, out=longer)[:9], x.argmax(1)) and longer[9:].tolist() == [-1, -1]
+        whole = cabi.sample_tokens(x, 0.9, 0, True, seed=4)
+        for top_k in (501, 2**31 - 1, 2**31, 2**32, 2**32 + 5, 2**63, 10**30):
+            assert torch.equal(cabi.sample_tokens(x, 0.9, top_k, True, seed=4), whole)
+        for top_k in (-1, -2**31, -2**32, -2**64):
+            with pytest.raises(RuntimeError, match="is negative"):
+                cabi.sample_tokens(x, 0.9, top_k, True, seed=4)
+    assert len(set(said)) == 1
+    for bad in (x[0], x[:, None], x[:, ::2]):
+        with pytest.raises(RuntimeError, match="side by side"):
+            ops.sample_tokens(bad, 1.0, 0, False, 0, 0, None)
+
+
 def test_attention_refuses_operands_the_kernels_would_overrun(monkeypatch):
     """The kernels take raw pointers: a q or an out too short for the cache, an out in
     pageable host memory or with gaps are refused before the launch, by the extension
