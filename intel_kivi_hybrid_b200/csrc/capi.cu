@@ -305,17 +305,20 @@ static bool wide_pays(int n_rep, int64_t n_groups) { return n_rep >= 3 && n_grou
 
 // The piece count of a kernel.  The models above walk up to 128 candidates (1-2 us);
 // a decode loop asks for the same shape again and again, so each thread remembers
-// its last question -- the answer depends on nothing else.
+// its last question to each of them (a call whose scratch is too small for one plan asks
+// several) -- the answer depends on nothing else.
 enum class AttnKernel { kGeneric, kTile, kMma, kMmaOne, kMmaWide };
 static int plan_splits(AttnKernel kernel, int num_units, int64_t n_groups, int requested, int head_dim, int group_size, int n_rep, int n_res,
                        int sms, int ctas_per_sm) {
     if (n_groups <= 0) return 0;
     if (requested > 0) return clamp_splits(requested, n_groups);
     if (sms <= 0) sms = 148;
-    const int64_t key[9] = {(int64_t)kernel, num_units, n_groups, head_dim, group_size, n_rep, n_res, sms, ctas_per_sm};
-    static thread_local int64_t last_key[9];
-    static thread_local int last = -1;
-    if (last >= 0 && memcmp(key, last_key, sizeof(key)) == 0) return last;
+    const int64_t key[8] = {num_units, n_groups, head_dim, group_size, n_rep, n_res, sms, ctas_per_sm};
+    struct Question { int64_t key[8]; int pieces; };         // pieces 0: none asked yet
+    static thread_local Question questions[(int)AttnKernel::kMmaWide + 1] = {};
+    Question& asked = questions[(int)kernel];
+    if (asked.pieces > 0 && memcmp(key, asked.key, sizeof(key)) == 0) return asked.pieces;
+    int last = 1;
     switch (kernel) {
         case AttnKernel::kMmaOne: last = plan_splits_stages(kOneHeadCosts, num_units, n_groups, n_res, sms, ctas_per_sm); break;
         case AttnKernel::kMma: last = plan_splits_mma(num_units * ((n_rep + 3) / 4), n_groups, n_res, sms, ctas_per_sm); break;
@@ -328,7 +331,8 @@ static int plan_splits(AttnKernel kernel, int num_units, int64_t n_groups, int r
         case AttnKernel::kTile: last = plan_splits_tile(num_units, n_groups, head_dim, group_size, n_rep, n_res, sms); break;
         case AttnKernel::kGeneric: last = plan_splits_generic(num_units, n_groups, sms); break;
     }
-    memcpy(last_key, key, sizeof(key));
+    memcpy(asked.key, key, sizeof(key));
+    asked.pieces = last;
     return last;
 }
 
