@@ -440,3 +440,13 @@ def test_a_call_with_little_scratch_remembers_its_plans(U, T, n_rep, dtype):
     small = (planned - 1 if n_rep == 1 else planned)         # (one head: the planned count needs no other plan)
     both = [(seconds(small), seconds(200)) for _ in range(40)]
     assert min(a for a, _ in both) < 1.35 * min(b for _, b in both)
+
+
+def test_bench_finds_the_measured_traffic():
+    """bench.py reports DRAM traffic from one line of the kernel's profile summary: it is there,
+    and what it states is the bytes the kernel cannot do without and a little more."""
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("bench", os.path.join(ROOT, "bench.py"))
+    bench = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(bench)
+    assert bench.traffic_factor() is not None and 1.0 <= bench.traffic_factor() < 1.1
