@@ -190,7 +190,9 @@ int kivi_cache_import_keys(const kivi_layer* layer, const uint8_t* packed,
  * 0 = choose from the SM count.  path: KIVI_ATTN_AUTO picks the tensor-core
  * kernel when the shape allows it (fp32 queries: with longer operands, to fp32
  * accuracy, and from the sizes on where it is faster) and the CUDA-core fp32
- * kernel otherwise.
+ * kernel otherwise.  On the tensor cores a weight (softmax weight times value scale)
+ * is exact to 2^-16 of the largest of 64 tokens in the same head and group of 32
+ * channels, fp32 queries to 2^-31; groups of channels do not share it.
  * ---------------------------------------------------------------------- */
 #define KIVI_ATTN_AUTO 0
 #define KIVI_ATTN_FP32 1 /* CUDA-core fp32 kernel, any supported shape */
@@ -206,7 +208,11 @@ int kivi_decode_attention_max_splits(void);
  * holds at a time) and how many CTAs per unit take the residual ring.  For arrays
  * on the 16-byte grid; others take the generic kernel and its coarser cut.  For fp32
  * queries the piece count is the CUDA-core kernel's: where the tensor-core kernel
- * serves them (KIVI_ATTN_AUTO) it is an upper bound.
+ * serves them (KIVI_ATTN_AUTO) it is an upper bound, good for sizing a workspace but
+ * not to be handed back as num_splits, which would cut finer than the call does.  With
+ * num_splits = 0 the cut of such a call, and with it the last bits of its result, also
+ * depends on the workspace: one too small for the tensor-core kernel's own count gets
+ * fewer pieces or the CUDA-core kernel.
  * sms / ctas_per_sm: the SM count and the tensor-core kernel's resident CTAs per
  * SM to plan for; <= 0 asks the current device (148 and 3 without one).
  * No counterpart in the reference. */

@@ -21,16 +21,16 @@
 //   What shares a largest value ends in the same sums: scores of one group, outputs of one
 //   channel group.  One for the whole stage cost those beside a louder neighbour their bits
 //   (channel groups 32 times apart: 2.9e-3 of the quiet one's largest output, now 1e-4).
-//   Twice to four times the warp reductions for that: 64 units x 32k 57.1 -> 61.1 us, 128 x 4k
-//   21.8 -> 22.3, one head 512 x 8k 99.4 -> 99.9.
+//   Two to four times as many warp reductions for that: 64 units x 32k 57.1 -> 60.5 us, 128 x 4k
+//   21.8 -> 22.2, one head 32 x 8k 11.7 -> 11.9.
 //   Infinities, NaN and negative value scales take an fp32 form of their own.
 //
 // Bytes instead of fp16 (codes as subnormals, q*s in two parts): 16 codes cost three
 // ALU operations instead of nine, and every MMA contracts twice as many.  512 units x
-// 32k tokens 416 -> 353 us (6.15 TB/s, 0.94 of a plain copy), 32 x 128k 118 -> 99 us,
-// 128 x 4k 24.0 -> 21.9 us, and the error against the fp32 kernel falls to a seventh.
-// A group of 32 tokens takes about 470 instructions of a warp: 24 MMAs, 48 masks, 96
-// FMAs for the operands and the zero terms, 24 permutes, 44 shared-memory accesses.
+// 32k tokens at boost clocks 416 -> 368 us (5.9 TB/s, 0.90 of a plain copy), under the power
+// cap 484 -> 435 (0.76); 32 x 128k 129 -> 117, 128 x 4k 25.1 -> 23.7, and the error against the
+// fp32 kernel falls to a seventh.  A group of 32 tokens takes about 510 instructions of a
+// warp, 24 of them MMAs.
 //
 // Data movement: every warp streams its own token groups from HBM into a
 // private shared-memory ring with bulk asynchronous copies (cp.async.bulk,
@@ -659,8 +659,8 @@ __device__ __forceinline__ void process_groups(const uint8_t* __restrict__ sb, c
 // groups of the stage (one operand for both, each lane reading the accumulators of its
 // group), in p.v the four channel groups (their contractions go to one accumulator, each
 // with the columns of the others at zero).  A quarter of the operand work, half of the
-// reading of accumulators.  256 units x 4k tokens 40.0 -> 31.3 us with the form for four
-// heads before, 512 x 8k 121 (fp16 form) -> 98, 32 x 8k 14.5 -> 11.5.
+// reading of accumulators.  256 units x 4k tokens 40.0 -> 32.8 us with the form for four
+// heads before, 512 x 8k 121 (fp16 form) -> 97, 32 x 8k 14.5 -> 11.7.
 struct OneView {
     int gid, tig, lane;
     float qk[4];           // pre-scaled query, channel k_channel(lane, i)

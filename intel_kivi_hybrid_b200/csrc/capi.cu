@@ -227,10 +227,11 @@ static int plan_splits_tile(int num_units, int64_t n_groups, int head_dim, int g
 //     a third of a CTA; a CTA's fixed time is c0_waves there.
 // At the two-CTA count the ring CTAs must fit beside the quantized ones, or c1 is that of
 // a crowded SM (256 units x 4k: one piece 51 us, two 44, three 45).
-// Fitted when the kernel's operands were fp16 (2 % off the best count of 308 shapes).  With
-// byte operands it is 4 % off over 130 shapes of four heads; where two counts lie close it may
-// take the second (128 units x 8k: two pieces 7 % behind three, 32 x 32k: thirteen 19 %
-// behind twelve).  A refit in the form below (plan_splits_stages) comes to 3 %.
+// Fitted when the kernel's operands were fp16 (2 % off the best count of 308 shapes; the times
+// above are that kernel's).  With byte operands it was 4 % off over 130 shapes of four heads,
+// and a refit in the form below (plan_splits_stages) 3 % -- or 4 when held to the counts that
+// the tests pin.  Where two counts lie close it may take the second (128 units x 8k: two
+// pieces 36.7 us, three 35.7).
 static int plan_splits_mma(int num_units, int64_t n_groups, int n_res_splits, int n_sms, int ctas_per_sm) {
     const int per_sm = ctas_per_sm > 0 ? ctas_per_sm : 3;
     const double slots = (double)per_sm * n_sms;
@@ -269,7 +270,7 @@ static int plan_splits_mma(int num_units, int64_t n_groups, int n_res_splits, in
 // units x 128 to 131072 tokens, 1 to 128 pieces; the times to 11 and 10 %): the counts are
 // 3.5 % off the best on average; the model below, whose costs are those of bf16 queries of
 // four heads, is 9 and 5.8 % off (one head: 256 units x 8k in four pieces 54 us, in its two
-// 64; 12 x 4k in six 8.3, in its eight 10.0).
+// 64; 12 x 4k in six 7.3, in its eight 9.2).
 struct StageCosts { double c0, c0_waves, c_one, c_two, c_three, c_merge, c_over, ragged, c_start, c_piece; };
 constexpr StageCosts kWideCosts{6.84, 2.2, 1.97, 2.56, 4.32, 1.8, 4.2, 0.48, 0.006, 0.06};
 constexpr StageCosts kOneHeadCosts{5.92, 0.34, 0.82, 0.90, 1.47, 1.07, 2.46, 0.495, 0.006, 0.027};
@@ -298,9 +299,10 @@ static int plan_splits_stages(const StageCosts& c, int num_units, int64_t n_grou
 
 // fp32 queries: the tensor-core kernel costs the same for one to four heads, the CUDA-core
 // kernel about 1500 + 650 n_rep cycles of an SM quarter per group.  us, CUDA cores / tensor
-// cores, each at its best count.  Four heads: 32 units x 8k tokens 37.9 / 21.2, 192 x 4k 102 / 48,
-// 20 x 2k 16.4 / 10.4; 256 x 128 tokens (the ring counts most there) 19.4 / 27.6, 512 x 512
-// 51.5 / 50.1.  One head: 256 x 4k 74 / 65, 32 x 2k 12.3 / 13.7, 192 x 512 14.7 / 19.1.
+// cores, each at its best count.  Four heads: 32 units x 8k tokens 37.0 / 21.1, 192 x 4k 101 / 48,
+// 20 x 2k 14.6 / 9.5; 256 x 128 tokens (the ring counts most there) 19.4 / 27.6, 512 x 512
+// 51.5 / 50.1.  Three heads: 32 x 8k 34.0 / 21.2, 1 x 2k 10.0 / 9.4, the closest 16 x 4k 13.7 / 14.2
+// and 1 x 32k 12.5 / 13.2.  One head: 256 x 4k 74 / 65, 32 x 2k 12.3 / 13.7, 192 x 512 14.7 / 19.1.
 static bool wide_pays(int n_rep, int64_t n_groups) { return n_rep >= 3 && n_groups >= 32; }
 
 // The piece count of a kernel.  The models above walk up to 128 candidates (1-2 us);
@@ -358,7 +360,9 @@ extern "C" int kivi_decode_attention_plan(int num_units, int64_t quant_len, int 
     if (ctas_per_sm <= 0) ctas_per_sm = attn_mma_ctas_per_sm();
     *tensor_cores_out = use_mma || wide ? 1 : 0;
     // (arrays on the 16-byte grid, as every allocator places them; fp32 queries: the CUDA-core
-    // kernel's count, which the tensor-core kernel does not exceed)
+    // kernel's count, which the tensor-core kernel's own does not exceed -- enough scratch for
+    // either, but no num_splits to hand back: 32 units x 8k in its 32 pieces 28.1 us, in the
+    // eight a call would choose 21.1)
     const AttnKernel kernel = use_mma ? (n_rep == 1 ? AttnKernel::kMmaOne : AttnKernel::kMma) : attn_fp32_tile_head_dim(head_dim) ? AttnKernel::kTile : AttnKernel::kGeneric;
     *quant_splits_out = plan_splits(kernel, num_units, n_groups, num_splits, head_dim, group_size, n_rep, n_res, sms, ctas_per_sm);
     *residual_parts_out = n_parts;

@@ -159,8 +159,8 @@ __device__ __forceinline__ void walk(const T* row, uint32_t i0, uint32_t end, ui
 }
 
 // One CTA per row.  What a row costs is latency: how often it is walked, how many bytes are
-// in flight, and the barriers in between.  kStaged (rows that fit shared memory, one row per
-// SM): bulk copies bring the whole row into shared memory, everything in flight at once,
+// in flight, and the barriers in between.  kStaged (long rows that fit shared memory, one row
+// per SM): bulk copies bring the whole row into shared memory, everything in flight at once,
 // and both passes read it there, 16 bytes at a time: the maximum as the pieces arrive, then
 // the candidates or the draw.  Otherwise both passes read memory, strided over the threads.
 //
@@ -535,12 +535,12 @@ sample_kernel(const T* logits, int vocab, int64_t row_stride,
 // eighth: up to one row per SM the row's length decides (as many loads in flight as it can
 // use; past that, barriers and folds cost more than the walk), with more rows than that
 // the rows side by side do.  Measured with 256 / 512 / 1024 threads, us, fp32:
-//   1 row, drawn from the whole row: 1000 entries 4.9 / 5.0 / 6.9, 10000 16 / 13 / 15, 50257 44 / 31 / 22
-//   256 rows x 32000, the same: 46 / 31 / 37; argmax 8.0 / 7.7 / 10.5
-//   1024 rows x 1000: 9.9 / 16 / 39; argmax 4.5 / 7.6 / 19
-// A top-k cut from candidates wants 5k/2 threads (64 rows x 2048, k = 200: 18 / 11 / 12,
-// k = 400: 27 / 30 / 20) and gets them unless that leaves rows waiting for a place; short
-// rows in crowds do as well with the radix select (1024 x 1000, k = 200: 32, and 34 with 512).
+//   1 row, drawn from the whole row: 1000 entries 4.0 / 3.7 / 4.1, 10000 12 / 7.6 / 8.4, 50257 41 / 16 / 15
+//   256 rows x 32000, the same: 41 / 27 / 31; argmax 7.0 / 6.4 / 7.3
+//   1024 rows x 1000: 7.9 / 12 / 26; argmax 3.5 / 5.2 / 11
+// A top-k cut from candidates wants 5k/2 threads (64 rows x 2048, k = 200: 23 / 9.5 / 9.1,
+// k = 400: 25 / 25 / 17) and gets them unless that leaves rows waiting for a place; short
+// rows in crowds do as well with the radix select (1024 x 1000, k = 200: 31, and 30 with 512).
 static int sample_threads(int batch, int vocab, int cut) {
     const int sms = num_sms();
     const int walk = batch <= sms ? (vocab <= 2048 ? 256 : vocab <= 16384 ? 512 : 1024) : batch <= 3 * sms && vocab > 8192 ? 512 : 256;

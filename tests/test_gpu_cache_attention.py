@@ -717,9 +717,9 @@ def test_attention_mma_at_the_edges_of_its_fixed_point_operands(cabi, what, toke
 def test_attention_beside_a_louder_neighbour(cabi, n_quant, n_res, dtype, n_rep, loud):
     """Values of one channel group, or keys of every other token group (far below the others in
     the softmax), thousands of times larger than their neighbours: every channel group of a row
-    keeps the tolerance against its own largest output.  (A weight is off by 2^-17 of the largest
-    of its own sums at most: 64 of a stage, three at most of a code, as independent roundings
-    3 * 8 * 2^-17 = 1.8e-4 of the largest weight, a tenth of the bf16 tolerance; fp32 2^-15 of that.)"""
+    keeps the tolerance against its own largest output.  (A weight is off by less than 2^-16 of the
+    largest of its own sums: 64 of a stage, three at most of a code, as independent roundings
+    3 * 8 * 2^-16 = 3.7e-4 of the largest weight, a fifth of the bf16 tolerance; fp32 2^-15 of that.)"""
     B, Hkv, D, G, T = 1, 3, 128, 32, n_quant + n_res
     K, V = ko.make_keys(B, Hkv, T, D, 23), ko.make_values(B, Hkv, T, D, 23)
     q = ko.make_queries(B, Hkv * n_rep, D, 23)
